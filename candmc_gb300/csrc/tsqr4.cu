@@ -10,8 +10,8 @@
 // dependent FP64 operations and block barriers, so the design minimises the
 // number of sequential steps on the critical path:
 //  * leaves of at most leaf_rows rows, one CTA each: b Householder steps in
-//    the column-owner schedule below, which also yields the leaf's
-//    compact-WY T (T^-1 from the Gram matrix V^T V);
+//    the critical-warp schedule below, then the leaf's compact-WY T (T^-1
+//    from the Gram matrix V^T V);
 //  * a fan-in-4 tree: the node stacks up to four R factors and runs b
 //    Householder steps on the stacked matrix (the zeros below the children's
 //    diagonals stay zero); with V = [I; V_2..V_4] the node's Q blocks are
@@ -38,298 +38,301 @@ namespace candmc {
 
 constexpr int kFan = 4;
 
-// Target rows per TSQR leaf (tuning knob, candmc_set_tuning("leaf_rows", v)).
-int64_t g_leaf_rows = 64;
+// Target rows per TSQR leaf (tuning knob, candmc_set_tuning("leaf_rows", v));
+// 0: kLeafRows, or 256 for panels of kTallPanelRows rows or more.
+int64_t g_leaf_rows = 0;
+// Leaf height of latency-bound panels.  A leaf's step is bound by the FP64
+// pipe from 128 rows on; below, by its chain and reductions, so shorter leaves
+// only add nodes: 8192 x 64 takes 670 us with 128-row leaves, 795 with 64 rows
+// and 809 with 256.
+constexpr int64_t kLeafRows = 128;
 int64_t g_pipe_leaf_rows = 128;
 thread_local int64_t t_leaf_rows = 0;
 // Pipelined tree on/off (tuning knob, candmc_set_tuning("pipe_tree", 0|1)).
 int g_pipe_tree = 1;
-constexpr int kTriScratch = 512 + kDirectB * kDirectB;   // h4_tri_inv workspace (doubles)
 
 __device__ __forceinline__ int64_t t4_leaf_row0(int64_t m, int P, int i) {
   return (m / P) * i + (m % P) * i / P;
 }
 
-// FP64 reciprocal and reciprocal square root by Newton-Raphson refinement of
-// an FP32 seed (Newton's iteration y <- y (2 - x y) and y <- y (3 - x y^2)/2;
-// each step squares the relative error, so two steps take the ~2^-23 seed
-// below FP64 rounding).  On this GPU an FP64 divide or square root costs
-// about ten dependent FP64 operations, which these replace on the reflector's
-// critical path.  Values outside FP32's range fall back to the FP64 operation.
-__device__ __forceinline__ double nr_rcp(double x) {
-  const float xf = (float)x;
-  if (!(fabsf(xf) > 1e-37f && fabsf(xf) < 1e37f)) return 1.0 / x;
-  double y = (double)(1.0f / xf);
-  double e = fma(-x, y, 1.0);
-  y = fma(y, e, y);
-  e = fma(-x, y, 1.0);
-  return fma(y, e, y);
-}
-
-__device__ __forceinline__ double nr_rsqrt(double q) {
-  const float qf = (float)q;
-  if (!(qf > 1e-37f && qf < 1e37f)) return 1.0 / sqrt(q);
-  double y = (double)rsqrtf(qf);
-  const double hq = 0.5 * q;
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const double t = y * y;
-    y = y * fma(-hq, t, 1.5);
-  }
-  return y;
-}
-
-// ---- Householder QR of a shared-memory block, column-owner schedule.
+// ---- Householder QR of a shared-memory block, critical-warp schedule.
 //
-// The block S (column-major, ld rows, b <= 32 columns) is worked by 4 warps;
-// warp w owns the columns c with c % 4 == w for every row, and lane l owns the
-// rows l + 32 t.  Step j applies reflector j (vector v_j: 1 at the head row j,
-// S[j][r] on the tail rows) to every other column and computes reflector j+1:
-//  * the owner of column j+1 updates that column first, then forms reflector
-//    j+1 from it with warp-only reductions (nothing else waits for it but the
-//    next step);
-//  * every warp forms d_c = v_j^T S[c] for its other columns (one transposed
-//    warp reduction for all of them), updates the columns c > j and records
-//    d_c = v_c^T v_j for c < j: these are the strictly upper entries of
-//    T^-1 = striu(V^T V) + diag(V^T V) / 2 (the identity of the reference's
-//    compute_invT_from_Y, alg/QR/qr_2d/qr_2d.cxx:22-60), so T costs no extra
-//    pass over the rows;
-//  * one block barrier per step.
-// On GB300 every warp-wide FP64 instruction holds its SMSP's FP64 pipe for 64
-// cycles, so the schedule keeps one warp per SMSP and the per-step chain of
-// the owner short.  The reflector follows LAPACK dlarfg: beta = -sign(alpha)
-// sqrt(alpha^2 + |x|^2), tau = 1 - alpha / beta, v = x / (alpha - beta); an
-// all-zero tail takes tau = 2, beta = -alpha (a sign flip), the convention of
-// the reconstruction, so that the T^-1 identity holds for every reflector.
-constexpr int kLeafThreads = 128;   // 4 warps, one per SMSP
+// What bounds it: a warp-wide FP64 instruction (fma, add, mul, compare or
+// conversion alike, whatever lanes are active) takes 65 cycles of its SM
+// sub-partition's FP64 pipe and 65 cycles of latency (measured), so the unit
+// of cost is the FP64 instruction: per sub-partition for throughput, per
+// dependent chain for latency.  The schedule therefore
+//  * gives one warp (warp 0, alone with the memory warps on its sub-partition)
+//    the serial chain: apply reflector j-1 to column j, form reflector j;
+//  * spreads the other columns over six warps on the other three
+//    sub-partitions, two warps each, so that one's shuffles and loads hide
+//    behind the other's arithmetic;
+//  * keeps the reflectors unnormalised: H = I - gamma v v^T with
+//    v = (alpha - beta, x), gamma = 1 / (q + |alpha| sigma), q = alpha^2 + |x|^2,
+//    sigma = sqrt(q), beta = -sign(alpha) sigma (LAPACK dlarfg's beta), which
+//    takes the division by alpha - beta and the scaling of x off the chain;
+//    the tails are divided by their heads once, after the last column;
+//  * seeds sigma and gamma with FP32 approximations exchanged by integer
+//    operations (a conversion would cost an FP64 slot) and refines them by one
+//    third-order step;
+//  * forms T from the Gram matrix of the finished reflectors, after the last
+//    column of R has been published.
+// One column step of a 64-row leaf takes about 30 FP64 instructions of chain
+// (2.1 k cycles) instead of two normalised passes with FP64-pipe conversions.
+// An all-zero tail takes v = e_j, gamma = 2, beta = -alpha (a sign flip), the
+// convention of the reconstruction, so that T^-1 = striu(V^T V) +
+// diag(V^T V) / 2 (alg/QR/qr_2d/qr_2d.cxx:22-60) holds for every reflector.
+constexpr int kLeafThreads = 288;   // 9 warps: the critical one, 6 for the columns, 2 for memory
+constexpr int kPollWarp = 4;        // sub-partition 0: waits for the children's columns
+constexpr int kPubWarp = 8;         // sub-partition 0: publishes finished columns
+constexpr int kBulkWarps = 6;       // warps 1-3 and 5-7
+constexpr int kLd = kDirectB + 1;   // leading dimension of the 32 x 32 shared blocks
 constexpr int kMaxR = 8;            // rows per lane: leaves of up to 256 rows, nodes of 4 x 32
 // leaves from which the Y formation takes its path products from a top-down
 // pass over the nodes instead of multiplying each leaf's whole path itself
 constexpr int kNodeMinLeaves = 256;
-// rows from which the lookahead's panels take 256-row leaves
+// rows from which panels take 256-row leaves (65536 x 32: 680 us against 766
+// with 128-row leaves; 262144 x 32: 1866 against 2361)
 constexpr int64_t kTallPanelRows = 32768;
 
-// Sum over the warp of eight values per lane; every lane receives all eight sums.
-__device__ __forceinline__ void warp_sum8(const double (&d)[8], double (&out)[8]) {
-  const int lane = threadIdx.x & 31;
-  const bool u16 = (lane & 16) != 0, u8 = (lane & 8) != 0, u4 = (lane & 4) != 0;
-  double p[4], q[2];
-#pragma unroll
-  for (int k = 0; k < 4; ++k)
-    p[k] = (u16 ? d[k + 4] : d[k]) + __shfl_xor_sync(0xffffffffu, u16 ? d[k] : d[k + 4], 16);
-#pragma unroll
-  for (int k = 0; k < 2; ++k)
-    q[k] = (u8 ? p[k + 2] : p[k]) + __shfl_xor_sync(0xffffffffu, u8 ? p[k] : p[k + 2], 8);
-  double s = (u4 ? q[1] : q[0]) + __shfl_xor_sync(0xffffffffu, u4 ? q[0] : q[1], 4);
-  s += __shfl_xor_sync(0xffffffffu, s, 2);
-  s += __shfl_xor_sync(0xffffffffu, s, 1);
-  // lane l now holds sum number 4 (l & 16 != 0) + 2 (l & 8 != 0) + (l & 4 != 0)
-#pragma unroll
-  for (int k = 0; k < 8; ++k)
-    out[k] = __shfl_sync(0xffffffffu, s, (((k >> 2) & 1) << 4) | (((k >> 1) & 1) << 3) | ((k & 1) << 2));
+// Index 0..5 of a column warp (1-3, 5-7), or -1.
+__device__ __forceinline__ int bulk_index(int warp) {
+  return (warp >= 1 && warp <= 3) ? warp - 1 : (warp >= 5 && warp <= 7) ? warp - 2 : -1;
 }
 
-// The same reduction without the final broadcast: lane l returns sum number
-// 4 (l & 16 != 0) + 2 (l & 8 != 0) + (l & 4 != 0); the four lanes l with equal
-// bits 2..4 hold the same sum.
-__device__ __forceinline__ double warp_sum8_held(const double (&d)[8]) {
+// Sums over the warp of N values per lane (N a power of two): lanes
+// k (32 / N) .. (k + 1) (32 / N) - 1 return sum number k.  Halving the values
+// and the lanes together takes N - 1 + 5 - log2(N) additions instead of 5 N.
+template <int N>
+__device__ __forceinline__ double warp_sum_held(double (&d)[N]) {
   const int lane = threadIdx.x & 31;
-  const bool u16 = (lane & 16) != 0, u8 = (lane & 8) != 0, u4 = (lane & 4) != 0;
-  double p[4], q[2];
+  int o = 16;
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
-    p[k] = (u16 ? d[k + 4] : d[k]) + __shfl_xor_sync(0xffffffffu, u16 ? d[k] : d[k + 4], 16);
+  for (int n = N; n > 1; n >>= 1) {
+    const bool up = (lane & o) != 0;
 #pragma unroll
-  for (int k = 0; k < 2; ++k)
-    q[k] = (u8 ? p[k + 2] : p[k]) + __shfl_xor_sync(0xffffffffu, u8 ? p[k] : p[k + 2], 8);
-  double s = (u4 ? q[1] : q[0]) + __shfl_xor_sync(0xffffffffu, u4 ? q[0] : q[1], 4);
-  s += __shfl_xor_sync(0xffffffffu, s, 2);
-  s += __shfl_xor_sync(0xffffffffu, s, 1);
+    for (int k = 0; k < n / 2; ++k)
+      d[k] = (up ? d[k + n / 2] : d[k]) + __shfl_xor_sync(0xffffffffu, up ? d[k] : d[k + n / 2], o);
+    o >>= 1;
+  }
+  double s = d[0];
+#pragma unroll
+  for (; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   return s;
 }
 
-__device__ __forceinline__ int warp_sum8_index(int lane) {
-  return ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+__device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
+__device__ __forceinline__ bool bits_nonzero(double x) { return (hi_abs(x) | __double2loint(x)) != 0; }
+// x with its sign flipped when `neg` is set
+__device__ __forceinline__ double flip_if(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
+}
+// FP32 value of a positive double with exponent within +-100 (truncated), and back
+__device__ __forceinline__ float f32_of(double x) {
+  return __int_as_float(__funnelshift_l(__double2loint(x), __double2hiint(x) - 0x38000000, 3));
+}
+__device__ __forceinline__ double f64_of(float x) {
+  const int i = __float_as_int(x);
+  return __hiloint2double((i >> 3) + 0x38000000, i << 29);
 }
 
-// Sixteen sums at once, without the broadcast: lane l returns sum number
-// 8 (l & 16 != 0) + 4 (l & 8 != 0) + 2 (l & 4 != 0) + (l & 2 != 0); lanes l and
-// l ^ 1 hold the same sum.
-__device__ __forceinline__ double warp_sum16_held(const double (&d)[16]) {
-  const int lane = threadIdx.x & 31;
-  const bool u16 = (lane & 16) != 0, u8 = (lane & 8) != 0, u4 = (lane & 4) != 0, u2 = (lane & 2) != 0;
-  double p[8], q[4], r[2];
-#pragma unroll
-  for (int k = 0; k < 8; ++k)
-    p[k] = (u16 ? d[k + 8] : d[k]) + __shfl_xor_sync(0xffffffffu, u16 ? d[k] : d[k + 8], 16);
-#pragma unroll
-  for (int k = 0; k < 4; ++k)
-    q[k] = (u8 ? p[k + 4] : p[k]) + __shfl_xor_sync(0xffffffffu, u8 ? p[k] : p[k + 4], 8);
-#pragma unroll
-  for (int k = 0; k < 2; ++k)
-    r[k] = (u4 ? q[k + 2] : q[k]) + __shfl_xor_sync(0xffffffffu, u4 ? q[k] : q[k + 2], 4);
-  double s = (u2 ? r[1] : r[0]) + __shfl_xor_sync(0xffffffffu, u2 ? r[0] : r[1], 2);
-  s += __shfl_xor_sync(0xffffffffu, s, 1);
-  return s;
+// 1 / x: an FP32 seed (relative error below 2^-20) and one third-order step,
+// e = 1 - x y, y (1 + e + e^2), whose error e^3 lies below 2^-60.
+__device__ __forceinline__ double quick_rcp(double x) {
+  const int h = hi_abs(x);
+  if (h < ((1023 - 90) << 20) || h >= ((1023 + 90) << 20)) return 1.0 / x;
+  const double y = flip_if(f64_of(__fdividef(1.0f, f32_of(fabs(x)))), __double2hiint(x) < 0);
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
 }
 
-__device__ __forceinline__ int warp_sum16_index(int lane) {
-  return ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
+// The scalars of one reflector from alpha and q = alpha^2 + |x|^2: sigma =
+// sqrt(q) as q r (1 + e/2 + 3 e^2/8) with e = 1 - q r^2 (the series' next
+// term is below 2^-62), h = alpha + sign(alpha) sigma, gamma = 1 / (q + |alpha|
+// sigma).  Both seeds come from q and alpha in FP32, side by side.
+// q within 2^+-60, alpha^2 <= q.
+__device__ __forceinline__ void h7_scalars(double alpha, double q, double* sigma, double* gam) {
+  const float qf = f32_of(q);
+  const float rf = rsqrtf(qf);
+  const float af = hi_abs(alpha) < ((1023 - 90) << 20) ? 0.0f : f32_of(fabs(alpha));
+  const double g0 = f64_of(__fdividef(1.0f, fmaf(af, qf * rf, qf)));
+  const double r = f64_of(rf);
+  const double t = q * r;
+  const double e = fma(-t, r, 1.0);
+  const double te = t * e;
+  const double p = fma(0.375, e, 0.5);
+  const double sg = fma(te, p, t);
+  const double den = fma(fabs(alpha), sg, q);
+  const double e1 = fma(-den, g0, 1.0);
+  *sigma = sg;
+  *gam = fma(g0, fma(e1, e1, e1), g0);
 }
 
-// Reflector j from column j of S, by one warp: alpha = S[j][j], x = the tail
-// rows (lane l owns rows l + 32 t).  Writes beta to S[j][j],
-// v = x / (alpha - beta) to the tail rows, tau to s_tau[j] and v^T v / 2
-// (with the unit head) to g[j][j] (ld b).
-template <int R, class Tail>
-__device__ void h5_reflector(double* S, int ld, int rows, int j, int b, Tail tail, double* s_tau,
-                             double* g) {
+// One step of the critical warp: column j of S receives reflector j - 1 (in v
+// and gam, kept from the last step) and becomes reflector j.  Lane l owns the
+// rows l + 32 t.  Leaf: head row j, tail rows j + 1 and on.  NODE: head row j
+// of child 0, tail = the rows of the other children (zero below their
+// diagonals).  Writes beta to row j, the unnormalised tail below it, the
+// head to s_h[j] and gamma to s_gam[j].
+template <int R, bool NODE>
+__device__ __forceinline__ void h7_crit(double* S, int ld, int j, double (&v)[R], double& gam, double* s_h,
+                                        double* s_gam) {
   const int lane = threadIdx.x & 31;
   double* col = S + (size_t)j * ld;
   double x[R];
-  double xn2 = 0.0;
 #pragma unroll
-  for (int t = 0; t < R; ++t) {
-    const int r = lane + 32 * t;
-    x[t] = (r < rows && tail(r, j)) ? col[r] : 0.0;
-    xn2 = fma(x[t], x[t], xn2);
+  for (int t = 0; t < R; ++t) x[t] = col[lane + 32 * t];
+  if (j > 0) {
+    double d = v[0] * x[0];
+#pragma unroll
+    for (int t = 1; t < R; ++t) d = fma(v[t], x[t], d);
+    const double f = gam * warp_sum(d);
+#pragma unroll
+    for (int t = 0; t < R; ++t) x[t] = fma(-f, v[t], x[t]);
   }
-  xn2 = warp_sum(xn2);
-  const double alpha = col[j];
-  double tj, sc, beta;
-  if (xn2 == 0.0) {
-    tj = 2.0;
-    sc = 0.0;
-    beta = -alpha;
+  const bool tail0 = !NODE && lane > j;
+  const double y0 = (tail0 || lane == j) ? x[0] : 0.0;
+  int nz = tail0 ? (hi_abs(x[0]) | __double2loint(x[0])) : 0;
+#pragma unroll
+  for (int t = 1; t < R; ++t) nz |= hi_abs(x[t]) | __double2loint(x[t]);
+  double q = y0 * y0;
+#pragma unroll
+  for (int t = 1; t < R; ++t) q = fma(x[t], x[t], q);
+  q = warp_sum(q);
+  const double alpha = __shfl_sync(0xffffffffu, x[0], j);
+  double h, beta;
+  if (!__any_sync(0xffffffffu, nz != 0)) {   // an empty tail: a sign flip
+    h = 1.0;
+    gam = 2.0;
+    beta = flip_if(alpha, true);
   } else {
-    const double q = fma(alpha, alpha, xn2);
-    const double rq = nr_rsqrt(q);
-    const double sg = alpha >= 0.0 ? -1.0 : 1.0;   // -sign(alpha), sign(0) = +
-    beta = sg * q * rq;
-    tj = fma(-alpha, sg * rq, 1.0);
-    sc = nr_rcp(alpha - beta);
-  }
+    const int qh = __double2hiint(q);
+    const bool neg = __double2hiint(alpha) < 0;
+    if (qh >= ((1023 - 60) << 20) && qh < ((1023 + 60) << 20)) {
+      double sigma;
+      h7_scalars(alpha, q, &sigma, &gam);
+      h = alpha + flip_if(sigma, neg);
+      beta = flip_if(sigma, !neg);
+    } else {
+      // squares outside the seeds' range: the reflector of the column scaled
+      // by a power of two is the same reflector (v may carry any factor)
+      int mx = (tail0 || lane == j) ? hi_abs(x[0]) : 0;
 #pragma unroll
-  for (int t = 0; t < R; ++t) {
-    const int r = lane + 32 * t;
-    if (r < rows && tail(r, j)) col[r] = x[t] * sc;
+      for (int t = 1; t < R; ++t) mx = max(mx, hi_abs(x[t]));
+      mx = __reduce_max_sync(0xffffffffu, (unsigned)mx);
+      // Inf and NaN stay unscaled and spread as they would without the scaling
+      const int e = mx >= 0x7ff00000 ? 0 : min(max((mx >> 20) - 1023, -1000), 1000);
+      const double sc = __hiloint2double((1023 - e) << 20, 0), un = __hiloint2double((1023 + e) << 20, 0);
+      if (tail0) x[0] *= sc;
+#pragma unroll
+      for (int t = 1; t < R; ++t) x[t] *= sc;
+      const double as = alpha * sc;
+      const double z0 = lane == j ? as : (tail0 ? x[0] : 0.0);
+      double qs = z0 * z0;
+#pragma unroll
+      for (int t = 1; t < R; ++t) qs = fma(x[t], x[t], qs);
+      qs = warp_sum(qs);
+      const double sigma = sqrt(qs);
+      h = as + flip_if(sigma, neg);
+      gam = 1.0 / fma(fabs(as), sigma, qs);
+      beta = flip_if(sigma, !neg) * un;
+    }
   }
-  __syncwarp();
+  col[lane] = lane == j ? beta : x[0];
+#pragma unroll
+  for (int t = 1; t < R; ++t) col[lane + 32 * t] = x[t];
+  v[0] = lane == j ? h : (tail0 ? x[0] : 0.0);
+#pragma unroll
+  for (int t = 1; t < R; ++t) v[t] = x[t];
   if (lane == 0) {
-    col[j] = beta;
-    s_tau[j] = tj;
-    g[j * b + j] = 0.5 * fma(sc * sc, xn2, 1.0);
+    s_h[j] = h;
+    s_gam[j] = gam;
   }
 }
 
-// Householder QR of S (rows x b, ld >= 32 R, R = ceil(rows / 32) rows per
-// lane); all kLeafThreads threads call it.  Afterwards S holds R (upper
-// triangle) and the reflector tails, s_tau the taus and g (b x b, ld b,
-// zeroed by the caller) T^-1.
-// Step j: warp (j+1) % 4 is the critical warp: it applies reflector j to
-// column j+1 and forms reflector j+1, and does nothing else, because a warp's
-// dependent FP64 chain occupies its SMSP's FP64 pipe.  The other three warps
-// share every other column c: d_c = v_j^T S[c] (a transposed reduction per 8
-// columns), then S[c] -= tau_j v_j d_c for c > j+1, or T^-1[c][j] = d_c for
-// c < j.  After the last reflector all four warps share the work.  The
-// updates load all of a group's rows before the first store, so that
-// independent columns are not serialised through shared memory.
+// Reflector (v, gam) applied to the columns c = q + 6 k, k0 <= k < 6, with
+// c_lo <= c < b, by one warp.
+template <int R, int N>
+__device__ __forceinline__ void h7_apply(double* S, int ld, int b, int q, int k0, int c_lo, const double (&v)[R],
+                                         double gam) {
+  constexpr int NC = N < kBulkWarps ? N : kBulkWarps;
+  constexpr bool keep = R <= 3;   // the columns stay in registers between their dot product and update
+  const int lane = threadIdx.x & 31;
+  double d[N];
+  double xs[NC][keep ? R : 1];
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    d[k] = 0.0;
+    const int c = q + kBulkWarps * (k0 + k);
+    if (k < NC && c >= c_lo && c < b) {
+      const double* sc = S + (size_t)c * ld;
+#pragma unroll
+      for (int t = 0; t < R; ++t) {
+        const double x = sc[lane + 32 * t];
+        if constexpr (keep) xs[k < NC ? k : 0][t] = x;
+        d[k] = fma(v[t], x, d[k]);
+      }
+    }
+  }
+  const double f = gam * warp_sum_held<N>(d);
+#pragma unroll
+  for (int k = 0; k < NC; ++k) {
+    const int c = q + kBulkWarps * (k0 + k);
+    const double fk = __shfl_sync(0xffffffffu, f, k * (32 / N));
+    if (c >= c_lo && c < b) {
+      double* sc = S + (size_t)c * ld;
+      double x[R];
+#pragma unroll
+      for (int t = 0; t < R; ++t) {
+        if constexpr (keep) x[t] = xs[k][t];
+        else x[t] = sc[lane + 32 * t];
+      }
+#pragma unroll
+      for (int t = 0; t < R; ++t) sc[lane + 32 * t] = fma(-fk, v[t], x[t]);
+    }
+  }
+}
+
 struct NoPublish {
   __device__ void operator()(const double*, int, int) const {}
 };
 
-template <int R, class Tail, class Pub = NoPublish>
-__device__ void h5_factor(double* S, int ld, int rows, int b, Tail tail, double* s_tau, double* g,
-                          Pub pub = Pub()) {
+// Householder QR of S (b columns, ld >= 32 R, rows beyond the data zero); all
+// kLeafThreads threads call it after S is filled.  Afterwards S holds R (upper
+// triangle) and the unnormalised tails, s_h the heads, s_gam the gammas.
+// Step j: the critical warp finishes column j (see h7_crit) while the column
+// warps apply reflector j - 1 to the columns after j and the publishing warp
+// hands column j - 1 of R to the parent; one block barrier per step.
+template <int R, bool NODE, class Pub = NoPublish>
+__device__ void h7_factor(double* S, int ld, int b, double* s_h, double* s_gam, Pub pub = Pub()) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (warp == 0) h5_reflector<R>(S, ld, rows, 0, b, tail, s_tau, g);
-  __syncthreads();
+  const int q = bulk_index(warp);
+  double v[R], gam = 0.0;
+#pragma unroll
+  for (int t = 0; t < R; ++t) v[t] = 0.0;
   for (int j = 0; j < b; ++j) {
-    // column j of R is final now (its last update was step j-1): a warp
-    // other than this step's critical one may publish it
-    if (warp == ((j + 2) & 3)) pub(S, ld, j);
-    const double* vj = S + (size_t)j * ld;
-    double vv[R];
-#pragma unroll
-    for (int t = 0; t < R; ++t) {
-      const int r = lane + 32 * t;
-      double v = 0.0;
-      if (r == j) v = 1.0;
-      else if (r < rows && tail(r, j)) v = vj[r];
-      vv[t] = v;
-    }
-    const double tj = s_tau[j];
-    const int nxt = j + 1;
-    const bool has_crit = nxt < b;
-    const int crit = nxt & 3;
-    if (has_crit && warp == crit) {
-      // the next pivot column: apply reflector j, then form reflector j+1
-      double* cn = S + (size_t)nxt * ld;
-      double x[R];
-      double d = 0.0;
-#pragma unroll
-      for (int t = 0; t < R; ++t) {
-        x[t] = cn[lane + 32 * t];
-        d = fma(vv[t], x[t], d);
-      }
-      d = warp_sum(d) * tj;
-#pragma unroll
-      for (int t = 0; t < R; ++t) cn[lane + 32 * t] = fma(-vv[t], d, x[t]);
-      __syncwarp();
-      h5_reflector<R>(S, ld, rows, nxt, b, tail, s_tau, g);
-    } else {
-      // bulk: this warp's share q of the columns other than j and j+1
-      const int nq = has_crit ? 3 : 4;
-      const int q = has_crit ? ((warp - crit + 3) & 3) : warp;   // 0 .. nq-1
-      for (int base = q; base < b; base += 8 * nq) {
-        double dd[8], D[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          dd[k] = 0.0;
-          const int c = base + k * nq;
-          if (c < b && c != j && c != nxt) {
-            const double* sc = S + (size_t)c * ld;
-#pragma unroll
-            for (int t = 0; t < R; ++t) dd[k] = fma(vv[t], sc[lane + 32 * t], dd[k]);
-          }
-        }
-        warp_sum8(dd, D);
-        // T^-1 entries for the columns before j
-        if (lane == 0) {
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const int c = base + k * nq;
-            if (c < j) g[j * b + c] = D[k];   // (V^T V)[c][j]
-          }
-        }
-        // updates of the columns after j+1, four columns per load group
-#pragma unroll
-        for (int h = 0; h < 8; h += 4) {
-          double xs[4][R];
-          bool act[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int c = base + (h + k) * nq;
-            act[k] = c < b && c > nxt;
-            if (act[k]) {
-              const double* sc = S + (size_t)c * ld;
-#pragma unroll
-              for (int t = 0; t < R; ++t) xs[k][t] = sc[lane + 32 * t];
-            }
-          }
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            if (!act[k]) continue;
-            const double dk = D[h + k] * tj;
-            double* sc = S + (size_t)(base + (h + k) * nq) * ld;
-#pragma unroll
-            for (int t = 0; t < R; ++t) sc[lane + 32 * t] = fma(-vv[t], dk, xs[k][t]);
-          }
-        }
-      }
-    }
     __syncthreads();
+    if (warp == 0) {
+      h7_crit<R, NODE>(S, ld, j, v, gam, s_h, s_gam);
+    } else if (j > 0 && q >= 0) {
+      const double* vj = S + (size_t)(j - 1) * ld;
+      const double h = s_h[j - 1];
+#pragma unroll
+      for (int t = 0; t < R; ++t) v[t] = vj[lane + 32 * t];
+      v[0] = lane == j - 1 ? h : (!NODE && lane > j - 1 ? v[0] : 0.0);
+      gam = s_gam[j - 1];
+      // this warp's columns from j + 1 on are its last n
+      const int klo = j + 1 > q ? (j + 1 - q + kBulkWarps - 1) / kBulkWarps : 0;
+      if (klo >= 5) h7_apply<R, 1>(S, ld, b, q, 5, j + 1, v, gam);
+      else if (klo == 4) h7_apply<R, 2>(S, ld, b, q, 4, j + 1, v, gam);
+      else if (klo >= 2) h7_apply<R, 4>(S, ld, b, q, 2, j + 1, v, gam);
+      else h7_apply<R, 8>(S, ld, b, q, 0, j + 1, v, gam);
+    } else if (j > 0 && warp == kPubWarp) {
+      pub(S, ld, j - 1);
+    }
   }
+  __syncthreads();
+  if (warp == kPubWarp) pub(S, ld, b - 1);
 }
 
 // Structure of an operand of h5_mm, on op(X): entries outside it read as 0
@@ -391,29 +394,19 @@ __device__ void h5_mm(const double* A, int lda, bool at, int as, const double* B
   __syncthreads();
 }
 
-// Inverse of the upper triangle of X (b x b, ld b, b <= 32; unit: diagonal
-// taken as 1) into Xi, by recursive 2 x 2 block inversion done bottom-up:
+// Inverse of the upper triangle of X (32 x 32, ld kLd) into Xi (ld kLd), by
+// recursive 2 x 2 block inversion done bottom-up:
 // inv([[A, B], [0, C]]) = [[A^-1, -A^-1 B C^-1], [0, C^-1]].  Every level is
 // two small products computed in parallel, so the dependent FP64 chain is
 // about 2 (1 + 2 + 4 + 8 + 16) operations instead of the b^2 / 2 of a
-// substitution.  The size is padded to a power of two with identity rows.
-// scratch: >= kTriScratch doubles.
-__device__ void h4_tri_inv(const double* X, int b, bool unit, double* Xi, double* scratch) {
-  int bp = 1;
-  while (bp < b) bp <<= 1;
-  auto xat = [&](int i, int k) -> double {
-    if (i >= b || k >= b) return (i == k) ? 1.0 : 0.0;
-    return X[k * b + i];
-  };
-  // Xi is bp x bp here (ld bp); the caller's layout (ld b) is restored at the end
+// substitution.  scratch: 512 doubles.
+__device__ void h4_tri_inv(const double* X, double* Xi, double* scratch) {
+  constexpr int bp = kDirectB;
   for (int idx = threadIdx.x; idx < bp * bp; idx += blockDim.x) {
     const int i = idx % bp, k = idx / bp;
-    double v = 0.0;
-    if (i == k) v = (unit || i >= b) ? 1.0 : 1.0 / X[i * b + i];
-    scratch[512 + idx] = v;
+    Xi[k * kLd + i] = i == k ? quick_rcp(X[i * kLd + i]) : 0.0;
   }
   __syncthreads();
-  double* Z = scratch + 512;
   for (int h = 1; h < bp; h <<= 1) {
     const int npair = bp / (2 * h);
     // M = B C^-1 (h x h per pair)
@@ -421,7 +414,7 @@ __device__ void h4_tri_inv(const double* X, int b, bool unit, double* Xi, double
       const int p = idx / (h * h), e = idx % (h * h), i = e % h, j = e / h;
       const int i0 = p * 2 * h, c0 = i0 + h;
       double acc = 0.0;
-      for (int k = 0; k <= j; ++k) acc = fma(xat(i0 + i, c0 + k), Z[(c0 + j) * bp + c0 + k], acc);
+      for (int k = 0; k <= j; ++k) acc = fma(X[(c0 + k) * kLd + i0 + i], Xi[(c0 + j) * kLd + c0 + k], acc);
       scratch[p * h * h + e] = acc;
     }
     __syncthreads();
@@ -430,37 +423,99 @@ __device__ void h4_tri_inv(const double* X, int b, bool unit, double* Xi, double
       const int p = idx / (h * h), e = idx % (h * h), i = e % h, j = e / h;
       const int i0 = p * 2 * h, c0 = i0 + h;
       double acc = 0.0;
-      for (int k = i; k < h; ++k) acc = fma(Z[(i0 + k) * bp + i0 + i], scratch[p * h * h + j * h + k], acc);
-      Z[(c0 + j) * bp + i0 + i] = -acc;
+      for (int k = i; k < h; ++k) acc = fma(Xi[(i0 + k) * kLd + i0 + i], scratch[p * h * h + j * h + k], acc);
+      Xi[(c0 + j) * kLd + i0 + i] = -acc;
     }
     __syncthreads();
   }
-  for (int idx = threadIdx.x; idx < b * b; idx += blockDim.x) {
-    const int i = idx % b, k = idx / b;
-    Xi[k * b + i] = Z[k * bp + i];
-  }
-  __syncthreads();
 }
 
-__device__ void h4_load(double* dst, const double* src, int b) {
-  for (int idx = threadIdx.x; idx < b * b; idx += blockDim.x) dst[idx] = __ldcg(src + idx);
+// b x b block from global memory (ld b) into shared memory
+__device__ void h4_load(double* dst, const double* src, int b, int ld) {
+  for (int idx = threadIdx.x; idx < b * b; idx += blockDim.x) dst[(idx / b) * ld + idx % b] = __ldcg(src + idx);
   __syncthreads();
 }
 
 // Rows [0, L) of b columns of a column-major block (ld lda) into S (ld ldS),
-// zero below row L: sixteen columns' loads in flight per thread before any
-// store, so the block costs two memory latencies rather than b.
-__device__ void h4_load_block(double* S, int ldS, const double* A, int64_t lda, int L, int b) {
-  for (int r = threadIdx.x; r < ldS; r += blockDim.x) {
-    for (int c0 = 0; c0 < b; c0 += 16) {
-      double t[16];
+// zero up to row `rows` (a multiple of 32) and column 32: eight loads in
+// flight per thread before any store.
+__device__ void h4_load_block(double* S, int ldS, const double* A, int64_t lda, int L, int b, int rows) {
+  const int n = rows * kDirectB;
+  for (int e0 = threadIdx.x; e0 < n; e0 += 8 * kLeafThreads) {
+    double t[8];
 #pragma unroll
-      for (int u = 0; u < 16; ++u) t[u] = (r < L && c0 + u < b) ? A[(int64_t)(c0 + u) * lda + r] : 0.0;
+    for (int u = 0; u < 8; ++u) {
+      const int e = e0 + u * kLeafThreads, c = e / rows, r = e - c * rows;
+      t[u] = (r < L && c < b) ? A[(int64_t)c * lda + r] : 0.0;
+    }
 #pragma unroll
-      for (int u = 0; u < 16; ++u)
-        if (c0 + u < b) S[(c0 + u) * ldS + r] = t[u];
+    for (int u = 0; u < 8; ++u) {
+      const int e = e0 + u * kLeafThreads, c = e / rows, r = e - c * rows;
+      if (e < n) S[c * ldS + r] = t[u];
     }
   }
+}
+
+constexpr int kGramScratch = 4 * 640;   // h7_gram's partial sums (doubles)
+
+// T^-1 = striu(V^T V) + diag(V^T V) / 2 of normalised reflectors into G (32 x
+// 32, ld kLd; columns beyond b get a unit diagonal).  V: rows 0..31 in VT (ld
+// kLd, masked to the reflectors' structure), rows 32..rows-1 in S (ld ldS).
+// Eight warps split the rows; each holds the ten upper 8 x 8 tiles (lane l:
+// row l % 8 of a tile, columns l / 8 and l / 8 + 4), so a row costs 20 FP64
+// instructions and no shuffles; the eight partial sums meet in shared memory.
+__device__ void h7_gram(const double* VT, const double* S, int ldS, int rows, int b, double* G, double* part) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = lane & 7, jj = lane >> 3;
+  double acc[10][2];
+#pragma unroll
+  for (int t = 0; t < 10; ++t) acc[t][0] = acc[t][1] = 0.0;
+  if (warp < 8) {
+    for (int r = warp; r < rows; r += 8) {
+      const double* X = r < kDirectB ? VT : S;
+      const int ld = r < kDirectB ? kLd : ldS;
+      double x[4], y0[4], y1[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        x[t] = X[(8 * t + i) * ld + r];
+        y0[t] = X[(8 * t + jj) * ld + r];
+        y1[t] = X[(8 * t + jj + 4) * ld + r];
+      }
+#pragma unroll
+      for (int tj = 0; tj < 4; ++tj)
+#pragma unroll
+        for (int ti = 0; ti <= tj; ++ti) {
+          const int t = tj * (tj + 1) / 2 + ti;
+          acc[t][0] = fma(x[ti], y0[tj], acc[t][0]);
+          acc[t][1] = fma(x[ti], y1[tj], acc[t][1]);
+        }
+    }
+    if (warp >= 4) {
+#pragma unroll
+      for (int t = 0; t < 10; ++t) {
+        part[(warp - 4) * 640 + t * 64 + lane] = acc[t][0];
+        part[(warp - 4) * 640 + t * 64 + 32 + lane] = acc[t][1];
+      }
+    }
+  }
+  __syncthreads();
+  if (warp < 4) {
+#pragma unroll
+    for (int t = 0; t < 10; ++t) {
+      part[warp * 640 + t * 64 + lane] += acc[t][0];
+      part[warp * 640 + t * 64 + 32 + lane] += acc[t][1];
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 640; e += blockDim.x) {
+    const int t = e >> 6, u = (e >> 5) & 1, l = e & 31;
+    int tj = 0;
+    while ((tj + 1) * (tj + 2) / 2 <= t) ++tj;
+    const int r = 8 * (t - tj * (tj + 1) / 2) + (l & 7), c = 8 * tj + (l >> 3) + 4 * u;
+    const double g = (part[e] + part[640 + e]) + (part[1280 + e] + part[1920 + e]);
+    if (r <= c) G[c * kLd + r] = r == c ? (c < b ? 0.5 * g : 1.0) : g;
+  }
+  __syncthreads();
 }
 
 struct Hr4Args {
@@ -487,7 +542,7 @@ struct Hr4Args {
   double* Mn;       // many leaves: per node, the product of the Q blocks from the root down to it
                     // times U^-1 (nnodes x b x b, by flat id), or nullptr
   int P;
-  int ldS;          // leading dimension of the shared block (>= 32 * ceil(leaf rows / 32), >= 128)
+  int ldS;          // leading dimension of the shared block: 32 row slots + 1
   int depth;
   int nlev[kMaxLevels + 1];
   int base[kMaxLevels + 1];
@@ -500,110 +555,183 @@ __device__ __forceinline__ int h4_children(const Hr4Args& a, int lvl, int node) 
   return n < kFan ? n : kFan;
 }
 
+// barrier `id` of n threads (a multiple of 32)
+__device__ __forceinline__ void named_bar(int id, int n) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+
+constexpr int kBlk = kDirectB * kLd;        // doubles of a 32 x 32 shared block
+constexpr int kRootDoubles = 6 * kBlk;
+constexpr long kSmemSpin = 1L << 22;        // polls of a shared-memory flag
+
+// The root: Q1_top, its sign-choice LU, T, W and U^-1.  The LU runs with a
+// one-column lookahead: warp 0 finishes column i + 1 (the pivot's chain:
+// about 500 cycles) while four warps apply column i to the columns beyond.
+// U^-1 and T are formed column by column behind it, by one warp each on
+// sub-partitions of their own: X U = I gives X[:, c] = (e_c - sum_{k<c} X[:, k]
+// U[k, c]) / U[c, c], and T L^T = -U S gives T[:, c] = -U[:, c] S_c -
+// sum_{k<c} T[:, k] L[c, k]; both need only the columns the LU has finished.
+// 496 FP64 instructions each bound the whole (16 us), where the LU followed
+// by two recursive inversions and a product took 58 us.
 __device__ void h4_root(const Hr4Args& a, double* sm) {
-  const int b = a.b, tid = threadIdx.x;
+  const int b = a.b, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double* sR = sm;
-  double* sM = sR + b * b;
-  double* sQ = sM + b * b;
-  double* sX = sQ + b * b;
-  double* sY = sX + b * b;
-  double* sT = sY + b * b;
+  double* sL = sR + kBlk;    // Q1_top, becomes L\U
+  double* sT = sL + kBlk;
+  double* sX = sT + kBlk;    // U^-1
+  double* sM = sX + kBlk;
+  double* sQ = sM + kBlk;
   __shared__ int s_sign[kDirectB];
-  h4_load(sR, a.Rn + (size_t)a.base[a.depth] * b * b, b);
+  __shared__ double s_rp[kDirectB];
+  __shared__ volatile int s_cols;   // columns of L\U finished
+  h4_load(sR, a.Rn + (size_t)a.base[a.depth] * b * b, b, kLd);
   if (a.Pc) {
     // the pipelined tree multiplied Q1_top up leaf 0's path as its nodes finished
-    h4_load(sX, a.Pc + (size_t)a.depth * b * b, b);
+    h4_load(sL, a.Pc + (size_t)a.depth * b * b, b, kLd);
   } else {
     // chain M = Q1^(1) ... Q1^(depth) of the first-child Q blocks (upper triangular)
-    for (int idx = tid; idx < b * b; idx += blockDim.x) sM[idx] = (idx % b == idx / b) ? 1.0 : 0.0;
+    for (int idx = tid; idx < b * b; idx += blockDim.x) sM[(idx / b) * kLd + idx % b] = (idx % b == idx / b) ? 1.0 : 0.0;
     __syncthreads();
     for (int lvl = a.depth; lvl >= 1; --lvl) {
       if (h4_children(a, lvl, 0) > 1) {
-        h4_load(sX, a.Qn + ((size_t)a.base[lvl] * kFan + 0) * b * b, b);
-        h5_mm(sX, b, false, kSUpper, sM, b, false, kSUpper, sQ, b, b, 1.0, nullptr);
-        for (int idx = tid; idx < b * b; idx += blockDim.x) sM[idx] = sQ[idx];
+        h4_load(sX, a.Qn + ((size_t)a.base[lvl] * kFan + 0) * b * b, b, kLd);
+        h5_mm(sX, kLd, false, kSUpper, sM, kLd, false, kSUpper, sQ, kLd, b, 1.0, nullptr);
+        for (int idx = tid; idx < b * b; idx += blockDim.x) sM[(idx / b) * kLd + idx % b] = sQ[(idx / b) * kLd + idx % b];
         __syncthreads();
       }
     }
     // Q1_top = C0 - V0 (T0 (V0^T C0)), V0 = unit-lower top block of leaf 0, C0 = M
     for (int idx = tid; idx < b * b; idx += blockDim.x) {
       const int r = idx % b, c = idx / b;
-      sY[idx] = (r > c) ? __ldcg(a.Vw + (int64_t)c * a.m + r) : (r == c ? 1.0 : 0.0);
+      sL[c * kLd + r] = (r > c) ? __ldcg(a.Vw + (int64_t)c * a.m + r) : (r == c ? 1.0 : 0.0);
     }
-    h4_load(sT, a.Tl, b);
-    h5_mm(sY, b, true, kSUnitUpper, sM, b, false, kSUpper, sX, b, b, 1.0, nullptr);   // sX = V0^T C0 (upper)
-    h5_mm(sT, b, false, kSUpper, sX, b, false, kSUpper, sQ, b, b, 1.0, nullptr);      // sQ = T0 sX (upper)
-    h5_mm(sY, b, false, kSUnitLower, sQ, b, false, kSUpper, sX, b, b, -1.0, sM);      // sX = C0 - V0 sQ
+    h4_load(sT, a.Tl, b, kLd);
+    h5_mm(sL, kLd, true, kSUnitUpper, sM, kLd, false, kSUpper, sX, kLd, b, 1.0, nullptr);   // V0^T C0 (upper)
+    h5_mm(sT, kLd, false, kSUpper, sX, kLd, false, kSUpper, sQ, kLd, b, 1.0, nullptr);      // T0 of it (upper)
+    h5_mm(sL, kLd, false, kSUnitLower, sQ, kLd, false, kSUpper, sX, kLd, b, -1.0, sM);      // C0 - V0 sQ
+    for (int idx = tid; idx < b * b; idx += blockDim.x) sL[(idx / b) * kLd + idx % b] = sX[(idx / b) * kLd + idx % b];
   }
-  double* sL = sX;   // Q1_top, becomes L\U
-  __shared__ double s_rpiv;
-  // Sign-choice LU without pivoting, with a one-column lookahead: in step i,
-  // warp 0 applies column i to column i + 1 and finishes it (pivot, sign,
-  // multipliers) while the other warps apply column i to the columns beyond;
-  // one barrier per column.
-  const int warp = tid >> 5, lane = tid & 31;
-  auto pivot = [&](int c) {   // warp 0: the diagonal of column c, then its multipliers
-    if (lane == 0) {
-      const double d = sL[c * b + c];
-      const int sg = d > 0.0 ? -1 : 1;
-      s_sign[c] = sg;
-      sL[c * b + c] = d - (double)sg;
-      s_rpiv = nr_rcp(d - (double)sg);   // |d - s| >= 1: the sign choice keeps the pivot away from 0
-    }
-    __syncwarp();
-    const double rp = s_rpiv;
-    for (int r = c + 1 + lane; r < b; r += 32) sL[c * b + r] *= rp;
-  };
-  if (warp == 0) pivot(0);
   __syncthreads();
-  for (int i = 0; i + 1 < b; ++i) {
-    const int c1 = i + 1;
-    if (warp == 0) {
-      for (int r = c1 + lane; r < b; r += 32) sL[c1 * b + r] = fma(-sL[i * b + r], sL[c1 * b + i], sL[c1 * b + r]);
+  for (int idx = tid; idx < kBlk; idx += blockDim.x) sT[idx] = sX[idx] = 0.0;
+  if (tid == 0) s_cols = 0;
+  __syncthreads();
+  const int trail = warp == 3 ? 0 : warp == 7 ? 1 : warp == 4 ? 2 : warp == 8 ? 3 : -1;
+  if (warp == 0) {
+    double x = lane < b ? sL[lane] : 0.0;
+    for (int i = 0; i < b; ++i) {
+      const double d = __shfl_sync(0xffffffffu, x, i);
+      const long long db = __double_as_longlong(d);
+      const bool pos = db > 0 && db <= 0x7ff0000000000000LL;   // d > 0
+      const double piv = d + (pos ? 1.0 : -1.0);   // |piv| >= 1: the sign choice keeps the pivot away from 0
+      const double rp = quick_rcp(piv);
+      const double l = lane > i ? x * rp : (lane == i ? piv : x);
+      if (lane < b) sL[i * kLd + lane] = l;
+      if (lane == 0) {
+        s_sign[i] = pos ? -1 : 1;
+        s_rp[i] = rp;
+      }
+      __threadfence_block();
       __syncwarp();
-      pivot(c1);
-    } else {
-      const int n = b - c1, nc = b - c1 - 1;   // rows i + 1 .., columns i + 2 ..
-      for (int idx = tid - 32; idx < n * nc; idx += blockDim.x - 32) {
-        const int r = c1 + idx % n, c = c1 + 1 + idx / n;
-        sL[c * b + r] = fma(-sL[i * b + r], sL[c * b + i], sL[c * b + r]);
+      if (lane == 0) s_cols = i + 1;
+      named_bar(1, 5 * 32);
+      if (i + 1 < b) {
+        const double xn = lane < b ? sL[(i + 1) * kLd + lane] : 0.0;
+        const double u = __shfl_sync(0xffffffffu, xn, i);
+        x = lane > i ? fma(-l, u, xn) : xn;
       }
     }
-    __syncthreads();
-  }
-  for (int idx = tid; idx < b * b; idx += blockDim.x) {
-    const int r = idx % b, c = idx / b;
-    a.A[c * a.lda + r] = (r > c) ? sL[c * b + r] : (double)s_sign[r] * sR[c * b + r];
-    if (a.W) a.W[c * a.ldW + r] = (r <= c) ? sL[c * b + r] * (double)s_sign[c] : 0.0;
-  }
-  // T = -W L^-T: W (upper) into sQ, L^T (unit upper) into sY, (L^T)^-1 into sM
-  double* scratch = sm + 6 * b * b;
-  for (int idx = tid; idx < b * b; idx += blockDim.x) {
-    const int i = idx % b, k = idx / b;
-    sQ[idx] = (i <= k) ? sL[k * b + i] * (double)s_sign[k] : 0.0;
-    sY[idx] = (i < k) ? sL[i * b + k] : (i == k ? 1.0 : 0.0);
+  } else if (trail >= 0) {
+    for (int i = 0; i < b; ++i) {
+      named_bar(1, 5 * 32);
+      const double l = sL[i * kLd + lane];
+      for (int c = i + 2 + trail; c < b; c += 4) {
+        const double u = sL[c * kLd + i];
+        if (lane > i && lane < b) sL[c * kLd + lane] = fma(-l, u, sL[c * kLd + lane]);
+      }
+    }
+  } else if (warp == 1 || warp == 2) {
+    for (int c = 0; c < b; ++c) {
+      long it = 0;
+      while (s_cols <= c && ++it < kSmemSpin) __nanosleep(20);
+      __syncwarp();
+      if (it >= kSmemSpin) {
+        if (lane == 0) atomicExch(a.status, CANDMC_ERR_TIMEOUT);
+        break;
+      }
+      __threadfence_block();
+      if (warp == 1) {
+        double acc = lane == c ? 1.0 : 0.0;
+#pragma unroll 4
+        for (int k = 0; k < c; ++k) acc = fma(-sX[k * kLd + lane], sL[c * kLd + k], acc);
+        sX[c * kLd + lane] = lane <= c ? acc * s_rp[c] : 0.0;
+      } else {
+        double acc = lane <= c ? flip_if(sL[c * kLd + lane], s_sign[c] > 0) : 0.0;
+#pragma unroll 4
+        for (int k = 0; k < c; ++k) acc = fma(-sT[k * kLd + lane], sL[k * kLd + c], acc);
+        sT[c * kLd + lane] = lane <= c ? acc : 0.0;
+      }
+      __syncwarp();
+    }
   }
   __syncthreads();
-  h4_tri_inv(sY, b, true, sM, scratch);
-  h5_mm(sQ, b, false, kSUpper, sM, b, false, kSUpper, sT, b, b, 1.0, nullptr);
-  for (int idx = tid; idx < b * b; idx += blockDim.x) {
-    const int r = idx % b, c = idx / b;
-    a.T[c * a.ldT + r] = (r <= c) ? -sT[c * b + r] : 0.0;
-  }
-  // U^-1 (the upper triangle of L\U); sM holds it
-  h4_tri_inv(sL, b, false, sM, scratch);
   int bad = 0;
   for (int idx = tid; idx < b * b; idx += blockDim.x) {
-    const double v = sM[idx];
-    if (!isfinite(v)) bad = 1;
+    const int r = idx % b, c = idx / b;
+    const double lu = sL[c * kLd + r];
+    a.A[c * a.lda + r] = (r > c) ? lu : flip_if(sR[c * kLd + r], s_sign[r] < 0);
+    if (a.W) a.W[c * a.ldW + r] = (r <= c) ? flip_if(lu, s_sign[c] < 0) : 0.0;
+    a.T[c * a.ldT + r] = (r <= c) ? sT[c * kLd + r] : 0.0;
+    const double v = sX[c * kLd + r];
+    if (hi_abs(v) >= 0x7ff00000) bad = 1;
     a.Uinv[idx] = v;
   }
   if (bad) atomicExch(a.status, CANDMC_ERR_NUMERIC);
 }
 
-__global__ void __launch_bounds__(kLeafThreads) k_hr4_leaf_tree(Hr4Args a) {
+// The reflectors of a factored leaf: S's tails divided by their heads (s_h
+// becomes the reciprocals), written to Vw (strictly lower part, L rows), and
+// the masked top 32 rows in VT.
+__device__ void h7_leaf_v(double* S, int ldS, int L, int rows, int b, double* s_h, double* VT, double* Vw, int64_t m) {
+  const int tid = threadIdx.x;
+  if (tid < kDirectB) s_h[tid] = tid < b ? quick_rcp(s_h[tid]) : 0.0;
+  __syncthreads();
+  const int n = rows * kDirectB;
+  for (int e = tid; e < n; e += kLeafThreads) {
+    const int c = e / rows, r = e - c * rows;
+    double v = 0.0;
+    if (r > c && c < b) {
+      v = S[c * ldS + r] * s_h[c];
+      S[c * ldS + r] = v;
+    }
+    if (r < kDirectB) VT[c * kLd + r] = (r == c && c < b) ? 1.0 : v;
+    if (r < L && c < b) Vw[(int64_t)c * m + r] = v;
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ int h7_slots(int L) {
+  const int s = (L + 31) >> 5;
+  return s <= 4 ? s : kMaxR;
+}
+
+template <class Pub>
+__device__ void h7_leaf_factor(double* S, int ldS, int slots, int b, double* s_h, double* s_gam, Pub pub) {
+  switch (slots) {
+    case 1: h7_factor<1, false>(S, ldS, b, s_h, s_gam, pub); break;
+    case 2: h7_factor<2, false>(S, ldS, b, s_h, s_gam, pub); break;
+    case 3: h7_factor<3, false>(S, ldS, b, s_h, s_gam, pub); break;
+    case 4: h7_factor<4, false>(S, ldS, b, s_h, s_gam, pub); break;
+    default: h7_factor<kMaxR, false>(S, ldS, b, s_h, s_gam, pub); break;
+  }
+}
+
+// shared memory of a leaf after its block S: VT, G, and the scratch that holds
+// h7_gram's partial sums, then h4_tri_inv's products and T
+constexpr int kLeafScratch = kGramScratch > 512 + kBlk ? kGramScratch : 512 + kBlk;
+
+__global__ void __launch_bounds__(kLeafThreads, 2) k_hr4_leaf_tree(Hr4Args a) {
   extern __shared__ double sm4[];
-  __shared__ double s_tau[kDirectB];
+  __shared__ double s_h[kDirectB], s_gam[kDirectB];
   __shared__ int s_last;
   const int b = a.b, tid = threadIdx.x;
   const int leaf = blockIdx.x;
@@ -611,35 +739,25 @@ __global__ void __launch_bounds__(kLeafThreads) k_hr4_leaf_tree(Hr4Args a) {
   const int L = (int)(t4_leaf_row0(a.m, a.P, leaf + 1) - r0);
   const int ldS = a.ldS;
   double* S = sm4;
-  double* G = S + (size_t)ldS * b;
-  double* Tt = G + b * b;
-  double* scratch = Tt + b * b;
+  double* VT = S + (size_t)ldS * kDirectB;
+  double* G = VT + kBlk;
+  double* scratch = G + kBlk;
+  double* Tt = scratch + 512;
 
-  // ---- leaf: Householder QR of rows [r0, r0 + L); rows L..ldS-1 are zero
-  h4_load_block(S, ldS, a.A + r0, a.lda, L, b);
-  for (int idx = tid; idx < b * b; idx += blockDim.x) G[idx] = 0.0;
-  __syncthreads();
-  {
-    auto tail = [](int r, int j) { return r > j; };
-    switch ((L + 31) >> 5) {
-      case 1: h5_factor<1>(S, ldS, L, b, tail, s_tau, G); break;
-      case 2: h5_factor<2>(S, ldS, L, b, tail, s_tau, G); break;
-      case 3: h5_factor<3>(S, ldS, L, b, tail, s_tau, G); break;
-      case 4: h5_factor<4>(S, ldS, L, b, tail, s_tau, G); break;
-      default: h5_factor<8>(S, ldS, L, b, tail, s_tau, G); break;
-    }
-  }
+  // ---- leaf: Householder QR of rows [r0, r0 + L); the rows beyond L are zero
+  const int slots = h7_slots(L);
+  h4_load_block(S, ldS, a.A + r0, a.lda, L, b, 32 * slots);
+  h7_leaf_factor(S, ldS, slots, b, s_h, s_gam, NoPublish());
   double* Rl = a.Rn + (size_t)(a.base[0] + leaf) * b * b;
   for (int idx = tid; idx < b * b; idx += blockDim.x) {
     const int r = idx % b, c = idx / b;
     Rl[idx] = (r <= c) ? S[c * ldS + r] : 0.0;
   }
-  for (int c = 0; c < b; ++c)
-    for (int r = tid; r < L; r += blockDim.x)
-      a.Vw[(int64_t)c * a.m + r0 + r] = (r > c) ? S[c * ldS + r] : 0.0;
-  h4_tri_inv(G, b, false, Tt, scratch);
+  h7_leaf_v(S, ldS, L, 32 * slots, b, s_h, VT, a.Vw + r0, a.m);
+  h7_gram(VT, S, ldS, 32 * slots, b, G, scratch);
+  h4_tri_inv(G, Tt, scratch);
   double* Tleaf = a.Tl + (size_t)leaf * b * b;
-  for (int idx = tid; idx < b * b; idx += blockDim.x) Tleaf[idx] = Tt[idx];
+  for (int idx = tid; idx < b * b; idx += blockDim.x) Tleaf[idx] = (idx % b <= idx / b) ? Tt[(idx / b) * kLd + idx % b] : 0.0;
 
   // ---- climb the fan-in-4 tree
   int node = leaf;
@@ -662,36 +780,40 @@ __global__ void __launch_bounds__(kLeafThreads) k_hr4_leaf_tree(Hr4Args a) {
     if (!s_last) return;
     __threadfence();
     // stack the children's R factors: child k occupies rows [32 k, 32 k + b)
-    // (rows b..31 of every child stay zero)
-    const int rows = nch * 32;
-    for (int c = 0; c < b; ++c)
-      for (int r = tid; r < rows; r += blockDim.x) {
-        const int k = r >> 5, i = r & 31;
-        const double* Rk = a.Rn + (size_t)(a.base[lvl] + parent * kFan + k) * b * b;
-        S[c * ldS + r] = (i <= c) ? __ldcg(Rk + c * b + i) : 0.0;
-      }
-    for (int idx = tid; idx < b * b; idx += blockDim.x) G[idx] = 0.0;
-    __syncthreads();
+    // (rows b..31 of every child, and the children beyond nch, stay zero)
+    for (int idx = tid; idx < kDirectB * kFan * 32; idx += blockDim.x) {
+      const int c = idx / (kFan * 32), r = idx % (kFan * 32), k = r >> 5, i = r & 31;
+      const double* Rk = a.Rn + (size_t)(a.base[lvl] + parent * kFan + k) * b * b;
+      S[c * ldS + r] = (k < nch && c < b && i <= c) ? __ldcg(Rk + c * b + i) : 0.0;
+    }
     // reflector j: head row j (child 0), tail = rows 0..j of every other child
     // (the children are upper triangular, so nothing below their diagonals is touched)
-    // (rows 32 k .. 32 k + j of children k >= 1 form the tail of reflector j)
-    h5_factor<4>(S, ldS, rows, b, [](int r, int j) { return r >= 32 && (r & 31) <= j; }, s_tau, G);
+    h7_factor<kFan, true>(S, ldS, b, s_h, s_gam);
     for (int idx = tid; idx < b * b; idx += blockDim.x) {
       const int r = idx % b, c = idx / b;
       Rpar[idx] = (r <= c) ? S[c * ldS + r] : 0.0;
     }
-    h4_tri_inv(G, b, false, Tt, scratch);
+    // V = [I; V_1; ..; V_{nch-1}] (V_k upper triangular), normalised
+    if (tid < kDirectB) s_h[tid] = tid < b ? quick_rcp(s_h[tid]) : 0.0;
+    __syncthreads();
+    for (int idx = tid; idx < kDirectB * kFan * 32; idx += blockDim.x) {
+      const int c = idx / (kFan * 32), r = idx % (kFan * 32);
+      if (r >= 32) S[c * ldS + r] *= s_h[c];
+      else VT[c * kLd + r] = (r == c && c < b) ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    h7_gram(VT, S, ldS, kFan * 32, b, G, scratch);
+    h4_tri_inv(G, Tt, scratch);
     double* Qp = a.Qn + (size_t)(a.base[lvl + 1] + parent) * kFan * b * b;
-    // V = [I; V_1; ..; V_{nch-1}] (V_k upper triangular):
     // Q_1 = I - T;  Q_k = -V_k T
     for (int idx = tid; idx < b * b; idx += blockDim.x) {
       const int r = idx % b, c = idx / b;
-      Qp[idx] = ((r == c) ? 1.0 : 0.0) - ((r <= c) ? Tt[c * b + r] : 0.0);
+      Qp[idx] = ((r == c) ? 1.0 : 0.0) - ((r <= c) ? Tt[c * kLd + r] : 0.0);
     }
     for (int k = 1; k < nch; ++k) {
       double* Qk = G;   // G is free once T is formed
-      h5_mm(S + 32 * k, ldS, false, kSUpper, Tt, b, false, kSUpper, Qk, b, b, -1.0, nullptr);
-      for (int idx = tid; idx < b * b; idx += blockDim.x) Qp[(size_t)k * b * b + idx] = Qk[idx];
+      h5_mm(S + 32 * k, ldS, false, kSUpper, Tt, kLd, false, kSUpper, Qk, kLd, b, -1.0, nullptr);
+      for (int idx = tid; idx < b * b; idx += blockDim.x) Qp[(size_t)k * b * b + idx] = Qk[(idx / b) * kLd + idx % b];
       __syncthreads();
     }
     node = parent;
@@ -735,7 +857,7 @@ __device__ bool h6_wait(const Hr4Args& a, const unsigned* p, unsigned v) {
   for (long it = 0; it < kSpinLimit; ++it) {
     if (ld_acquire(p) >= v) return true;
     if (*(volatile int*)a.fail) return false;
-    __nanosleep(100);
+    if (it > 8) __nanosleep(100);
   }
   atomicExch(a.fail, 1);
   atomicExch(a.status, CANDMC_ERR_TIMEOUT);
@@ -750,53 +872,44 @@ __device__ void h6_release_all(const Hr4Args& a, int f) {
   }
 }
 
-struct LeafPublish {
+// Column j of R (rows 0..j of S's column j) handed to the parent by one warp.
+struct Publish {
   double* Rcol;
   int b;
   unsigned* prog;
   __device__ void operator()(const double* S, int ld, int j) const {
     const int lane = threadIdx.x & 31;
     if (lane <= j) Rcol[j * b + lane] = S[j * ld + lane];
-    __threadfence();
-    __syncwarp();
+    __syncwarp();   // orders the lanes' stores before lane 0's release
     if (lane == 0) st_release(prog, (unsigned)(j + 1));
   }
 };
 
-__device__ void h6_leaf(const Hr4Args& a, int leaf, double* sm, double* s_tau) {
+__device__ void h6_leaf(const Hr4Args& a, int leaf, double* sm, double* s_h, double* s_gam) {
   const int b = a.b, tid = threadIdx.x;
   const int64_t r0 = t4_leaf_row0(a.m, a.P, leaf);
   const int L = (int)(t4_leaf_row0(a.m, a.P, leaf + 1) - r0);
   const int ldS = a.ldS;
   double* S = sm;
-  double* G = S + (size_t)ldS * b;
-  double* Tt = G + b * b;
-  double* scratch = Tt + b * b;
-  h4_load_block(S, ldS, a.A + r0, a.lda, L, b);
-  for (int idx = tid; idx < b * b; idx += blockDim.x) G[idx] = 0.0;
-  __syncthreads();
-  const LeafPublish pub{a.Rn + (size_t)leaf * b * b, b, a.prog + leaf};
-  auto tail = [](int r, int j) { return r > j; };
-  switch ((L + 31) >> 5) {
-    case 1: h5_factor<1>(S, ldS, L, b, tail, s_tau, G, pub); break;
-    case 2: h5_factor<2>(S, ldS, L, b, tail, s_tau, G, pub); break;
-    case 3: h5_factor<3>(S, ldS, L, b, tail, s_tau, G, pub); break;
-    case 4: h5_factor<4>(S, ldS, L, b, tail, s_tau, G, pub); break;
-    default: h5_factor<8>(S, ldS, L, b, tail, s_tau, G, pub); break;
-  }
-  for (int c = 0; c < b; ++c)
-    for (int r = tid; r < L; r += blockDim.x)
-      a.Vw[(int64_t)c * a.m + r0 + r] = (r > c) ? S[c * ldS + r] : 0.0;
-  h4_tri_inv(G, b, false, Tt, scratch);
+  double* VT = S + (size_t)ldS * kDirectB;
+  double* G = VT + kBlk;
+  double* scratch = G + kBlk;
+  double* Tt = scratch + 512;
+  const int slots = h7_slots(L);
+  h4_load_block(S, ldS, a.A + r0, a.lda, L, b, 32 * slots);
+  h7_leaf_factor(S, ldS, slots, b, s_h, s_gam, Publish{a.Rn + (size_t)leaf * b * b, b, a.prog + leaf});
+  h7_leaf_v(S, ldS, L, 32 * slots, b, s_h, VT, a.Vw + r0, a.m);
+  h7_gram(VT, S, ldS, 32 * slots, b, G, scratch);
+  h4_tri_inv(G, Tt, scratch);
   double* Tleaf = a.Tl + (size_t)leaf * b * b;
-  for (int idx = tid; idx < b * b; idx += blockDim.x) Tleaf[idx] = Tt[idx];
+  for (int idx = tid; idx < b * b; idx += blockDim.x) Tleaf[idx] = (idx % b <= idx / b) ? Tt[(idx / b) * kLd + idx % b] : 0.0;
   if (leaf == 0 && a.Pc) {
     // P_0 = I - V0 T0 V0^T on the top b rows (V0 unit lower): the first factor
     // of Q1_top, multiplied by the path nodes' Q1 blocks as they finish
-    h5_mm(Tt, b, false, kSUpper, S, ldS, true, kSUnitUpper, G, b, b, 1.0, nullptr);        // G = T0 V0^T
-    h5_mm(S, ldS, false, kSUnitLower, G, b, false, kSUpper, scratch, b, b, 1.0, nullptr);  // V0 G
+    h5_mm(Tt, kLd, false, kSUpper, VT, kLd, true, kSUnitUpper, G, kLd, b, 1.0, nullptr);   // G = T0 V0^T
+    h5_mm(VT, kLd, false, kSUnitLower, G, kLd, false, kSUpper, S, kLd, b, 1.0, nullptr);   // V0 G (S is free)
     for (int idx = tid; idx < b * b; idx += blockDim.x)
-      a.Pc[idx] = ((idx % b == idx / b) ? 1.0 : 0.0) - scratch[idx];
+      a.Pc[idx] = ((idx % b == idx / b) ? 1.0 : 0.0) - S[(idx / b) * kLd + idx % b];
   }
   __threadfence();
   __syncthreads();
@@ -806,208 +919,212 @@ __device__ void h6_leaf(const Hr4Args& a, int leaf, double* sm, double* s_tau) {
   }
 }
 
-__device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_tau, int* s_ok) {
+constexpr int kNodeLd = kFan * 32 + 1;   // child k at rows [32 k, 32 k + b)
+constexpr int kNodeDoubles = kNodeLd * kDirectB + 4 * kBlk + 4 * 96;
+
+// An internal node.  V = [D; V_1; V_2; V_3] with the reflectors unnormalised
+// (D = diag(h)) and T of that form (T_pp = gamma_p).  Step j, between two
+// block barriers:
+//  * warp 0 applies reflector j - 1 to column j and forms reflector j;
+//  * warps 1-3, one per child, apply the reflectors before j to column j + 1:
+//    z = V^T s with one reflector per lane (no reduction over lanes), w = T^T z
+//    with the columns of T the last step knew and w_(j-1) = gamma_(j-1)
+//    (z_(j-1) - (T y)^T z), s -= V w with one row per lane;
+//  * warps 5-7, one per child, form column j - 1 of T: y = V^T v_(j-1),
+//    T[0:j-1, j-1] = -gamma_(j-1) T y;
+//  * the polling warp fetches column j + 2 of the children, and the publishing
+//    warp hands column j - 1 to the parent.
+// Bound: the FP64 pipes of the three sub-partitions with the column warps
+// (about 130 instructions a step at j = 31, 8.5 k cycles; half that on
+// average) against 13 k cycles a step when one warp group did all of it in
+// sequence with seven block barriers.
+__device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_h, double* s_gam) {
   const int b = a.b, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ int s_okv[2];
   int lvl = 1;
   while (lvl < a.depth && f >= a.base[lvl + 1]) ++lvl;
   const int idx = f - a.base[lvl];
   const int nch = h4_children(a, lvl, idx);
   const int child0 = a.base[lvl - 1] + idx * kFan;   // flat id of child 0
   double* Rme = a.Rn + (size_t)f * b * b;
-  constexpr int ld = kFan * 32;   // child k at rows [32 k, 32 k + b)
+  constexpr int ld = kNodeLd;
   double* S = sm;
-  double* Tn = S + ld * b;
-  double* Qk = Tn + b * b;
-  double* zv = Qk + b * b;
-  double* wv = zv + 32;
-  double* yv = wv + 32;
-  double* part = yv + 32;    // 3 x 128 partial sums
-  double* Pb = part + 384;   // prefix product of Q1_top (nodes on leaf 0's path)
-  for (int i = tid; i < ld * b; i += blockDim.x) S[i] = 0.0;
-  for (int i = tid; i < b * b; i += blockDim.x) Tn[i] = 0.0;
-  __syncthreads();
-  auto tail = [](int r, int j) { return r >= 32 && (r & 31) <= j; };
-  // column c of R (head rows 0..c), published to the parent by warp 0
-  auto publish = [&](int c) {
-    if (lane <= c) Rme[c * b + lane] = S[c * ld + lane];
-    __threadfence();
-    __syncwarp();
-    if (lane == 0) st_release(a.prog + f, (unsigned)(c + 1));
-  };
-  for (int j = 0; j < b; ++j) {
-    // (1) column j of every child: lane k of warp 1 waits for child k, while
-    //     warp 0 publishes column j - 1 (finished in the last step)
-    if (warp == 0 && j > 0 && nch > 1) publish(j - 1);
-    if (warp == 1) {
+  double* Tn = S + ld * kDirectB;
+  double* Qk = Tn + kBlk;
+  double* Pb = Qk + kBlk;
+  double* Po = Pb + kBlk;
+  double* zp = Po + kBlk;     // 3 x 32 partial sums each
+  double* yp = zp + 96;
+  double* wp = yp + 96;
+  double* tp = wp + 96;
+  if (nch == 1) {   // a pass-through node: its R is its child's
+    if (warp == 0) {
       bool ok = true;
-      if (lane < nch) ok = h6_wait(a, a.prog + child0 + lane, (unsigned)(j + 1));
-      ok = __all_sync(0xffffffffu, ok);
-      if (lane == 0) *s_ok = ok;
-    }
-    __syncthreads();
-    if (!*s_ok) {
-      h6_release_all(a, f);
-      return;
-    }
-    if (nch == 1) {   // a pass-through node: its R is its child's
-      if (warp == 0) {
+      for (int j = 0; ok && j < b; ++j) {
+        if (lane == 0) ok = h6_wait(a, a.prog + child0, (unsigned)(j + 1));
+        ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+        if (!ok) break;
         if (lane <= j) Rme[j * b + lane] = __ldcg(a.Rn + (size_t)child0 * b * b + j * b + lane);
         __threadfence();
         __syncwarp();
         if (lane == 0) st_release(a.prog + f, (unsigned)(j + 1));
       }
-      continue;
-    }
-    // (2) stack the children's column j
-    if (warp < nch && lane <= j)
-      S[j * ld + 32 * warp + lane] = __ldcg(a.Rn + (size_t)(child0 + warp) * b * b + j * b + lane);
-    __syncthreads();
-    if (j > 0) {
-      // (3) one reduction for two sets of dot products over the children's
-      //     rows: z_p = v_p^T s_j (p < j; the head adds row p of s_j) and
-      //     y_p = v_p^T v_(j-1) (p < j - 1), which give column j - 1 of T
-      double dd[16];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int pp = warp + 4 * q;
-        dd[q] = 0.0;
-        dd[8 + q] = 0.0;
-        if (pp < j)
-          for (int k = 1; k < nch; ++k) {
-            const double vp = S[pp * ld + 32 * k + lane];
-            dd[q] = fma(vp, S[j * ld + 32 * k + lane], dd[q]);
-            if (pp < j - 1) dd[8 + q] = fma(vp, S[(j - 1) * ld + 32 * k + lane], dd[8 + q]);
-          }
-      }
-      {
-        const double sq = warp_sum16_held(dd);
-        const int id = warp_sum16_index(lane);
-        const int pp = warp + 4 * (id & 7);
-        if ((lane & 1) == 0) {
-          if (id < 8) {
-            if (pp < j) zv[pp] = S[j * ld + pp] + sq;
-          } else if (pp < j - 1) {
-            yv[pp] = sq;
-          }
-        }
-      }
-      __syncthreads();
-      // (4) column c = j - 1 of T: T[p][c] = -tau_c sum_{q=p}^{c-1} T[p][q] y_q
-      const int c = j - 1;
-      if (c > 0) {
-        double acc = 0.0;
-        if (lane < c)
-          for (int q = warp; q < c; q += 4)
-            if (q >= lane) acc = fma(Tn[q * b + lane], yv[q], acc);
-        part[warp * 32 + lane] = acc;
-        __syncthreads();
-        if (warp == 0 && lane < c)
-          Tn[c * b + lane] = -s_tau[c] * ((part[lane] + part[32 + lane]) + (part[64 + lane] + part[96 + lane]));
-        __syncthreads();
-      }
-      // (5) w = T^T z
-      {
-        double acc = 0.0;
-        if (lane < j)
-          for (int pp = warp; pp <= lane; pp += 4) acc = fma(Tn[lane * b + pp], zv[pp], acc);
-        part[warp * 32 + lane] = acc;
-      }
-      __syncthreads();
-      if (warp == 0 && lane < j) wv[lane] = (part[lane] + part[32 + lane]) + (part[64 + lane] + part[96 + lane]);
-      __syncthreads();
-      // (6) s_j -= V w: the head rows p < j directly; child k's rows r < j by
-      //     sum_{p<j} V_k[r][p] w_p (V_k[r][p] = 0 for r > p), p split over the warps
-      {
-        double acc[kFan - 1];
-#pragma unroll
-        for (int k = 0; k < kFan - 1; ++k) acc[k] = 0.0;
-        for (int pp = warp; pp < j; pp += 4) {
-          const double wp = wv[pp];
-#pragma unroll
-          for (int k = 1; k < kFan; ++k)
-            if (k < nch) acc[k - 1] = fma(S[pp * ld + 32 * k + lane], wp, acc[k - 1]);
-        }
-#pragma unroll
-        for (int k = 0; k < kFan - 1; ++k) part[k * 128 + warp * 32 + lane] = acc[k];
-      }
-      __syncthreads();
-      if (warp == 0) {
-        if (lane < j) S[j * ld + lane] -= wv[lane];
-      } else if (warp < nch && lane < j) {
-        const double* pk = part + (warp - 1) * 128;
-        S[j * ld + 32 * warp + lane] -= (pk[lane] + pk[32 + lane]) + (pk[64 + lane] + pk[96 + lane]);
-      }
-      __syncthreads();
-    }
-    // (7) reflector j; T[j][j] = tau_j (read from the next step on)
-    if (warp == 0) h5_reflector<kFan>(S, ld, nch * 32, j, b, tail, s_tau, Qk);
-    __syncthreads();
-    if (tid == 0) Tn[j * b + j] = s_tau[j];
-  }
-  if (nch > 1 && b > 1) {
-    // the last column of T: y_p = v_p^T v_(b-1), p < b - 1
-    const int c = b - 1;
-    double dd[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      dd[q] = 0.0;
-      const int pp = warp + 4 * q;
-      if (pp < c)
-        for (int k = 1; k < nch; ++k) dd[q] = fma(S[pp * ld + 32 * k + lane], S[c * ld + 32 * k + lane], dd[q]);
-    }
-    {
-      const double sq = warp_sum8_held(dd);
-      const int pp = warp + 4 * warp_sum8_index(lane);
-      if ((lane & 3) == 0 && pp < c) yv[pp] = sq;
+      if (lane == 0) s_okv[0] = ok;
     }
     __syncthreads();
-    {
-      double acc = 0.0;
-      if (lane < c)
-        for (int q = warp; q < c; q += 4)
-          if (q >= lane) acc = fma(Tn[q * b + lane], yv[q], acc);
-      part[warp * 32 + lane] = acc;
-    }
-    __syncthreads();
-    if (warp == 0 && lane < c)
-      Tn[c * b + lane] = -s_tau[c] * ((part[lane] + part[32 + lane]) + (part[64 + lane] + part[96 + lane]));
-  }
-  __syncthreads();
-  if (nch > 1 && warp == 0) publish(b - 1);
-  if (idx == 0) {
-    // on leaf 0's path: P_lvl = P_(lvl-1) Q1 = P_(lvl-1) (I - T), as soon as the
-    // child on the path has its prefix (it then sets its progress to b + 1).
-    // The root's solver waits for this node's prefix the same way.
-    if (tid == 0) *s_ok = h6_wait(a, a.prog + child0, (unsigned)b + 1u);
-    __syncthreads();
-    if (!*s_ok) {
+    if (!s_okv[0]) {
       h6_release_all(a, f);
       return;
     }
-    h4_load(Qk, a.Pc + (size_t)(lvl - 1) * b * b, b);
+  } else {
+    for (int i = tid; i < ld * kDirectB; i += blockDim.x) S[i] = 0.0;
+    for (int i = tid; i < kBlk; i += blockDim.x) Tn[i] = 0.0;
+    __syncthreads();
+    const Publish pub{Rme, b, a.prog + f};
+    // column c of the children's R into S (polling warp: lane k waits for child k)
+    auto fetch = [&](int c) -> bool {
+      bool ok = true;
+      if (lane < nch) ok = h6_wait(a, a.prog + child0 + lane, (unsigned)(c + 1));
+      if (!__all_sync(0xffffffffu, ok)) return false;
+      double t[kFan];
+#pragma unroll
+      for (int k = 0; k < kFan; ++k)
+        t[k] = (k < nch && lane <= c) ? __ldcg(a.Rn + (size_t)(child0 + k) * b * b + c * b + lane) : 0.0;
+#pragma unroll
+      for (int k = 0; k < kFan; ++k) S[c * ld + 32 * k + lane] = t[k];
+      return true;
+    };
+    if (warp == kPollWarp) {
+      bool ok = fetch(0);
+      if (ok && b > 1) ok = fetch(1);
+      if (lane == 0) s_okv[0] = ok;
+    }
+    const int kc = warp & 3;                 // the child of a column warp: 1..3
+    const bool tgrp = warp >= 5 && warp <= 7;
+    const bool cgrp = warp >= 1 && warp <= 3;
+    // reflectors 0..n-1 are formed: column n - 1 of T, and the reflectors
+    // applied to column c (when c < b)
+    auto bulk = [&](int n, int c) {
+      const double* Vk = S + 32 * kc;
+      const bool live = kc < nch;
+      double acc = 0.0;
+      if (tgrp) {
+        if (live && lane < n - 1) {
+#pragma unroll 4
+          for (int r = 0; r < n - 1; ++r) acc = fma(Vk[lane * ld + r], Vk[(n - 1) * ld + r], acc);
+        }
+        yp[(kc - 1) * 32 + lane] = acc;
+      } else {
+        if (live && c < b && lane < n) {
+#pragma unroll 4
+          for (int r = 0; r < n; ++r) acc = fma(Vk[lane * ld + r], Vk[c * ld + r], acc);
+        }
+        zp[(kc - 1) * 32 + lane] = acc;
+      }
+      named_bar(1, kBulkWarps * 32);
+      double z = 0.0;
+      if (tgrp) {
+        const double y = (yp[lane] + yp[32 + lane]) + yp[64 + lane];
+        acc = 0.0;
+        for (int q = kc - 1; q < n - 1; q += 3) acc = fma(Tn[q * kLd + lane], __shfl_sync(0xffffffffu, y, q), acc);
+        tp[(kc - 1) * 32 + lane] = acc;
+      } else if (c < b) {
+        if (lane < n) z = fma(s_h[lane], S[c * ld + lane], (zp[lane] + zp[32 + lane]) + zp[64 + lane]);
+        acc = 0.0;
+        for (int p = kc - 1; p < n - 1; p += 3) {
+          const double zq = __shfl_sync(0xffffffffu, z, p);
+          acc = fma(lane < n - 1 ? Tn[lane * kLd + p] : 0.0, zq, acc);
+        }
+        wp[(kc - 1) * 32 + lane] = acc;
+      }
+      named_bar(1, kBulkWarps * 32);
+      const double g = s_gam[n - 1];
+      if (tgrp) {
+        if (kc == 1) {
+          const double t = (tp[lane] + tp[32 + lane]) + tp[64 + lane];
+          if (lane < n) Tn[(n - 1) * kLd + lane] = lane < n - 1 ? -g * t : g;
+        }
+      } else if (c < b) {
+        const double t = lane < n - 1 ? ((tp[lane] + tp[32 + lane]) + tp[64 + lane]) * z : 0.0;
+        const double u = warp_sum(t);
+        const double zl = __shfl_sync(0xffffffffu, z, n - 1);
+        double w = (wp[lane] + wp[32 + lane]) + wp[64 + lane];
+        if (lane >= n - 1) w = lane == n - 1 ? g * (zl - u) : 0.0;
+        if (live) {
+          acc = 0.0;
+#pragma unroll 4
+          for (int p = 0; p < n; ++p) acc = fma(Vk[p * ld + lane], __shfl_sync(0xffffffffu, w, p), acc);
+          if (lane < n) S[c * ld + 32 * kc + lane] -= acc;
+        }
+        if (kc == 1 && lane < n) S[c * ld + lane] = fma(-s_h[lane], w, S[c * ld + lane]);
+      }
+    };
+    double v[kFan], gam = 0.0;
+#pragma unroll
+    for (int t = 0; t < kFan; ++t) v[t] = 0.0;
+    for (int j = 0; j < b; ++j) {
+      __syncthreads();
+      if (!s_okv[j & 1]) {   // written before this barrier, rewritten two barriers on
+        h6_release_all(a, f);
+        return;
+      }
+      if (warp == 0) {
+        h7_crit<kFan, true>(S, ld, j, v, gam, s_h, s_gam);
+      } else if (warp == kPollWarp) {
+        bool ok = true;
+        if (j + 2 < b) ok = fetch(j + 2);
+        if (lane == 0) s_okv[(j + 1) & 1] = ok;
+      } else if (warp == kPubWarp) {
+        if (j > 0) pub(S, ld, j - 1);
+      } else if (j > 0 && (tgrp || cgrp)) {
+        bulk(j, j + 1);
+      }
+    }
+    __syncthreads();
+    if (warp == kPubWarp) pub(S, ld, b - 1);
+    if (tgrp || cgrp) bulk(b, b);
+    __syncthreads();
+    // T of normalised heads: Tn = T D (for Q_k = -V_k T D), Qk = D T D (Q_1 = I - D T D)
+    for (int i = tid; i < b * b; i += blockDim.x) {
+      const int r = i % b, c = i / b;
+      const double t = Tn[c * kLd + r] * s_h[c];
+      Tn[c * kLd + r] = t;
+      Qk[c * kLd + r] = s_h[r] * t;
+    }
+    __syncthreads();
+  }
+  if (idx == 0) {
+    // on leaf 0's path: P_lvl = P_(lvl-1) Q1 = P_(lvl-1) (I - D T D), as soon as the
+    // child on the path has its prefix (it then sets its progress to b + 1).
+    // The root's solver waits for this node's prefix the same way.
+    if (tid == 0) s_okv[0] = h6_wait(a, a.prog + child0, (unsigned)b + 1u);
+    __syncthreads();
+    if (!s_okv[0]) {
+      h6_release_all(a, f);
+      return;
+    }
+    const double* Pprev = a.Pc + (size_t)(lvl - 1) * b * b;
     double* Pl = a.Pc + (size_t)lvl * b * b;
     if (nch > 1) {
-      h5_mm(Qk, b, false, kSDense, Tn, b, false, kSUpper, Pb, b, b, -1.0, Qk);
-      for (int i = tid; i < b * b; i += blockDim.x) Pl[i] = Pb[i];
+      h4_load(Pb, Pprev, b, kLd);
+      h5_mm(Pb, kLd, false, kSDense, Qk, kLd, false, kSUpper, Po, kLd, b, -1.0, Pb);
+      for (int i = tid; i < b * b; i += blockDim.x) Pl[i] = Po[(i / b) * kLd + i % b];
     } else {
-      for (int i = tid; i < b * b; i += blockDim.x) Pl[i] = Qk[i];
+      for (int i = tid; i < b * b; i += blockDim.x) Pl[i] = __ldcg(Pprev + i);
     }
     __threadfence();
     __syncthreads();
     if (tid == 0) st_release(a.prog + f, (unsigned)b + 1u);
   }
   if (nch > 1) {
-    // Q blocks of the node (for forming Y): Q_1 = I - T;  Q_k = -V_k T
+    // Q blocks of the node (for forming Y): Q_1 = I - D T D;  Q_k = -V_k T D
     double* Qp = a.Qn + (size_t)f * kFan * b * b;
     for (int i = tid; i < b * b; i += blockDim.x) {
       const int r = i % b, c = i / b;
-      Qp[i] = ((r == c) ? 1.0 : 0.0) - ((r <= c) ? Tn[c * b + r] : 0.0);
+      Qp[i] = ((r == c) ? 1.0 : 0.0) - ((r <= c) ? Qk[c * kLd + r] : 0.0);
     }
-    for (int k = 1; k < nch; ++k) {
-      h5_mm(S + 32 * k, ld, false, kSUpper, Tn, b, false, kSUpper, Qk, b, b, -1.0, nullptr);
-      for (int i = tid; i < b * b; i += blockDim.x) Qp[(size_t)k * b * b + i] = Qk[i];
-      __syncthreads();
-    }
+    for (int k = 1; k < nch; ++k)
+      h5_mm(S + 32 * k, ld, false, kSUpper, Tn, kLd, false, kSUpper, Qp + (size_t)k * b * b, b, b, -1.0, nullptr);
   }
   __threadfence();
   __syncthreads();
@@ -1017,28 +1134,29 @@ __device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_tau, int*
 // The root's solver (one extra CTA): once the top node has published its R
 // and the full prefix Q1_top, the sign-choice LU, T, W and U^-1, while the
 // top node still writes its Q blocks.
-__device__ void h6_root_solver(const Hr4Args& a, double* sm, int* s_ok) {
+__device__ void h6_root_solver(const Hr4Args& a, double* sm) {
+  __shared__ int s_ok;
   const int top = a.base[a.depth];
-  if (threadIdx.x == 0) *s_ok = h6_wait(a, a.prog + top, (unsigned)a.b + 1u);
+  if (threadIdx.x == 0) s_ok = h6_wait(a, a.prog + top, (unsigned)a.b + 1u);
   __syncthreads();
-  if (!*s_ok) return;
+  if (!s_ok) return;
   __threadfence();
   h4_root(a, sm);
 }
 
-__global__ void __launch_bounds__(kLeafThreads) k_hr6_pipe(Hr4Args a) {
+__global__ void __launch_bounds__(kLeafThreads, 2) k_hr6_pipe(Hr4Args a) {
   extern __shared__ double sm6[];
-  __shared__ double s_tau[kDirectB];
-  __shared__ int s_role, s_ok;
+  __shared__ double s_h[kDirectB], s_gam[kDirectB];
+  __shared__ int s_role;
   if (threadIdx.x == 0) s_role = (int)atomicAdd(a.ticket, 1u);
   __syncthreads();
   const int f = s_role;   // flat tree id: leaves 0 .. P-1, the nodes level by level, the root's solver
   if (f < a.P)
-    h6_leaf(a, f, sm6, s_tau);
+    h6_leaf(a, f, sm6, s_h, s_gam);
   else if (f <= a.base[a.depth])
-    h6_node(a, f, sm6, s_tau, &s_ok);
+    h6_node(a, f, sm6, s_h, s_gam);
   else
-    h6_root_solver(a, sm6, &s_ok);
+    h6_root_solver(a, sm6);
 }
 
 // The product of the Q blocks along the root-to-node path times U^-1, for
@@ -1059,8 +1177,8 @@ __global__ void __launch_bounds__(kLeafThreads) k_hr4_node_m(Hr4Args a, int lvl)
   double* sM = sQ + nb2;
   double* sO = sM + nb2;
   if (h4_children(a, lvl + 1, nd) > 1) {
-    h4_load(sQ, a.Qn + ((size_t)(a.base[lvl + 1] + nd) * kFan + (c - nd * kFan)) * nb2, b);
-    h4_load(sM, Mp, b);
+    h4_load(sQ, a.Qn + ((size_t)(a.base[lvl + 1] + nd) * kFan + (c - nd * kFan)) * nb2, b, b);
+    h4_load(sM, Mp, b, b);
     h5_mm(sQ, b, false, kSUpper, sM, b, false, kSUpper, sO, b, b, 1.0, nullptr);
     for (int idx = tid; idx < b * b; idx += blockDim.x) Mo[idx] = sO[idx];
   } else {
@@ -1081,9 +1199,9 @@ __global__ void __launch_bounds__(kThreads) k_hr4_form_y(Hr4Args a) {
   // the levels above 1 come from k_hr4_node_m when it ran (a.Mn)
   const int top = (a.Mn && a.depth >= 2) ? 1 : a.depth;
   if (top < a.depth)
-    h4_load(sM, a.Mn + (size_t)(a.base[1] + leaf / kFan) * b * b, b);
+    h4_load(sM, a.Mn + (size_t)(a.base[1] + leaf / kFan) * b * b, b, b);
   else
-    h4_load(sM, a.Uinv, b);
+    h4_load(sM, a.Uinv, b, b);
   for (int lvl = top; lvl >= 1; --lvl) {
     int nd = leaf;
     for (int l = 0; l < lvl; ++l) nd /= kFan;
@@ -1091,7 +1209,7 @@ __global__ void __launch_bounds__(kThreads) k_hr4_form_y(Hr4Args a) {
     for (int l = 0; l < lvl - 1; ++l) child /= kFan;
     if (h4_children(a, lvl, nd) > 1) {
       const int k = child - nd * kFan;
-      h4_load(sX, a.Qn + ((size_t)(a.base[lvl] + nd) * kFan + k) * b * b, b);
+      h4_load(sX, a.Qn + ((size_t)(a.base[lvl] + nd) * kFan + k) * b * b, b, b);
       h5_mm(sX, b, false, kSUpper, sM, b, false, kSUpper, sY, b, b, 1.0, nullptr);
       for (int idx = tid; idx < b * b; idx += blockDim.x) sM[idx] = sY[idx];
       __syncthreads();
@@ -1102,7 +1220,7 @@ __global__ void __launch_bounds__(kThreads) k_hr4_form_y(Hr4Args a) {
     const int r = idx % b, c = idx / b;
     sY[idx] = (r > c) ? a.Vw[(int64_t)c * a.m + r0 + r] : (r == c ? 1.0 : 0.0);
   }
-  h4_load(sT, a.Tl + (size_t)leaf * b * b, b);
+  h4_load(sT, a.Tl + (size_t)leaf * b * b, b, b);
   h5_mm(sY, b, true, kSUnitUpper, sM, b, false, kSUpper, sX, b, b, 1.0, nullptr);   // sX = V_top^T M
   h5_mm(sT, b, false, kSUpper, sX, b, false, kSUpper, sY, b, b, 1.0, nullptr);      // sY = Z = T sX
   // Z is upper triangular: Y[r][c] = M[r][c] - sum_{k<=c} V[r][k] Z[k][c], eight
@@ -1141,10 +1259,10 @@ __global__ void __launch_bounds__(kThreads) k_hr4_form_y(Hr4Args a) {
 int hr_direct4(double* A, int64_t lda, int64_t m, int b, double* T, int64_t ldT, double* W,
                int64_t ldW, int* d_status, cudaStream_t s) {
   if (b < 1 || b > kDirectB || m < b) return CANDMC_ERR_ARG;
-  int64_t want = t_leaf_rows > 0 ? t_leaf_rows : g_leaf_rows;
-  // the lookahead's tall panels (thousands of leaves: throughput, not the
-  // latency of one leaf, sets the time) take 256-row leaves
-  if (t_leaf_rows > 0 && m >= kTallPanelRows) want = std::max<int64_t>(want, 256);
+  int64_t want = t_leaf_rows > 0 ? t_leaf_rows : g_leaf_rows > 0 ? g_leaf_rows : kLeafRows;
+  // tall panels (throughput, not the latency of one leaf, sets the time) take
+  // 256-row leaves unless the knob asks for a height
+  if ((t_leaf_rows > 0 || g_leaf_rows == 0) && m >= kTallPanelRows) want = std::max<int64_t>(want, 256);
   const int64_t leaf_rows = std::max<int64_t>(32, std::min<int64_t>(want, 256));
   // leaves of at most leaf_rows rows and at least b rows
   int64_t P = std::max<int64_t>(1, std::min<int64_t>((m + leaf_rows - 1) / leaf_rows, m / b));
@@ -1164,22 +1282,20 @@ int hr_direct4(double* A, int64_t lda, int64_t m, int b, double* T, int64_t ldT,
   const int nnodes = total;
   const int64_t Lmax = (m + P - 1) / P;
   const size_t nb2 = (size_t)b * b;
-  // shared block: rows padded to the row slots of the factor instantiation
-  // that runs (1..4 slots of 32 rows, or 8 for leaves of more than 128 rows),
-  // and at least the 4 x 32 rows of a tree node
+  // shared block of the leaves:
+  // rows padded to the row slots of the factor instantiation that runs (1..4
+  // slots of 32 rows, or 8 for leaves of more than 128 rows), and, where the
+  // leaf's CTA also works the nodes, at least the 4 x 32 rows of a node
   const int64_t slots = (Lmax + 31) / 32;
-  const int64_t ldS = std::max<int64_t>(32 * (slots <= 4 ? slots : 8), kFan * 32);
-  if (ldS > 32 * kMaxR) return CANDMC_ERR_ARG;
-  a.ldS = (int)ldS;
-  // block + G + T + tri-inverse workspace; the root reuses the front of the
-  // same area for six b x b buffers plus the workspace
-  const size_t sm = sizeof(double) * std::max<size_t>((size_t)ldS * b + 2 * nb2 + kTriScratch,
-                                                      6 * nb2 + kTriScratch);
-  if (sm > 200 * 1024) return CANDMC_ERR_ARG;
   // the pipelined tree while the whole tree is a modest number of CTAs (a
   // latency-bound panel); the level-by-level tree for many leaves, where the
   // leaves dominate and the pipeline would only add synchronisation
-  const bool pipe = a.depth >= 1 && g_pipe_tree && nnodes <= 4096;
+  const bool pipe = g_pipe_tree && nnodes <= 4096;
+  a.ldS = (int)std::max<int64_t>(32 * (slots <= 4 ? slots : kMaxR), pipe ? 0 : kFan * 32) + 1;
+  if (a.ldS > 32 * kMaxR + 1) return CANDMC_ERR_ARG;
+  const size_t sm = sizeof(double) * std::max<size_t>({(size_t)a.ldS * kDirectB + 2 * kBlk + kLeafScratch,
+                                                       (size_t)kNodeDoubles, (size_t)kRootDoubles});
+  if (sm > 200 * 1024) return CANDMC_ERR_ARG;
   // one workspace, carved in 256-byte aligned pieces; the counters and the
   // node R blocks (read before all their entries are written) lead it, so
   // one memset clears both

@@ -307,7 +307,8 @@ int candmc_batched_ls_f32(int64_t nprob, const int64_t* m, const int64_t* n, flo
  * device-side failures surface here. */
 int candmc_batched_status(void* stream, int* status);
 
-/* tuning knobs: "leaf_rows" (target rows per TSQR leaf, 32..256, default 64);
+/* tuning knobs: "leaf_rows" (target rows per TSQR leaf, 32..256; unset: 128, and 256 for
+ * panels of 32768 rows or more);
  * "pipe_tree" (1, the default: the levels of the TSQR tree overlap column by
  * column; 0: level by level); "oz_reserve_sms" (SMs kept free of the
  * persistent emulated-FP64 update kernel during QR_2D_pipe, for the panel

@@ -1,0 +1,75 @@
+"""The TSQR-HR kernels at the edges of their row slots, widths and ranges.
+
+Inputs are Gaussian panels scaled by a power of two: the reflectors, T and the
+signs do not depend on the scale and R carries it exactly, so one oracle run
+serves every scale.  Beyond 2^+-30 the squares leave the range of the
+reflector's FP32 seeds and the scaled form of the reflector runs.  Tolerance:
+the element-wise bar of the parity tests, 2e-12 max(1, b / 16) relative to the
+largest entry (a few ulps times the panel width).
+"""
+import numpy as np
+import pytest
+
+from oracle import candmc_oracle as co
+from oracle import fixtures as fx
+from oracle import lapack_restated as lp
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def cm():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import candmc_gb300 as cm
+    cm.lib()
+    return cm
+
+
+# leaves of 1, 2, 3, 4 and more than 4 row slots; one leaf, a pass-through
+# node, nodes of 2, 3 and 4 children, two and three levels; widths 1 to 32
+@pytest.mark.parametrize("m,b,leaf", [(32, 32, 32), (33, 1, 32), (63, 2, 64), (96, 31, 96), (97, 32, 96),
+                                      (128, 32, 128), (129, 9, 256), (256, 32, 256), (160, 32, 32), (545, 17, 32),
+                                      (700, 32, 64), (2100, 32, 32), (5000, 25, 256)])
+@pytest.mark.parametrize("exp", [0, 40, -700, 480])
+def test_panel_steps(cm, m, b, leaf, exp):
+    A = fx.gaussian(m, b, 31 * m + b)
+    YRo, Wo = co.hh_recon_qr(A, b)
+    To = co.T_from_W(Wo, lp.unit_lower(YRo, b)[:b])
+    tol = 2e-12 * max(1.0, b / 16)
+    dA = torch.from_numpy(np.ldexp(A, exp)).cuda().t().contiguous().t()
+    for pipe in (1, 0):
+        d = dA.t().clone().t()
+        try:
+            cm.set_tuning("leaf_rows", leaf)
+            cm.set_tuning("pipe_tree", pipe)
+            W, T = cm.hh_recon_qr(d)
+            torch.cuda.synchronize()
+        finally:
+            cm.set_tuning("pipe_tree", 1)
+            cm.set_tuning("leaf_rows", 128)
+        YR = d.cpu().numpy()
+        up = np.triu_indices(b)
+        YR[up] = np.ldexp(YR[up], -exp)
+        assert np.abs(YR - YRo).max() <= tol * max(1.0, np.abs(YRo).max())
+        assert np.abs(W.cpu().numpy() - Wo).max() <= tol
+        assert np.abs(T.cpu().numpy() - To).max() <= tol
+
+
+def test_panel_empty_tails_and_non_finite(cm):
+    """Columns with empty tails keep the sign-flip reflector (tau = 2) exactly,
+    and a NaN stays a NaN instead of hanging or vanishing."""
+    A = np.zeros((300, 16))
+    A[:16] = np.diag(np.arange(1.0, 17.0))
+    d = torch.from_numpy(A).cuda().t().contiguous().t()
+    W, T = cm.hh_recon_qr(d)
+    torch.cuda.synchronize()
+    assert np.array_equal(d.cpu().numpy(), -A)
+    assert np.array_equal(T.diagonal().cpu().numpy(), np.full(16, 2.0))
+    A = fx.gaussian(600, 24, 5)
+    A[410, 7] = np.nan
+    d = torch.from_numpy(A).cuda().t().contiguous().t()
+    cm.hh_recon_qr(d)
+    torch.cuda.synchronize()
+    assert np.isnan(d.cpu().numpy()[:24, 7:]).any()
