@@ -234,8 +234,7 @@ static int check_form(int precision, int64_t b, bool* pair) {
   return CANDMC_OK;
 }
 
-// High-priority, non-blocking side stream per device for the lookahead panels.
-static int device_sms() {
+int device_sms() {
   static std::atomic<int> n{0};
   if (n.load() == 0) {
     int dev = 0, v = 0;
@@ -246,7 +245,7 @@ static int device_sms() {
   return n.load();
 }
 
-// One lookahead stream per host thread and device, so that factorizations
+// One high-priority, non-blocking lookahead stream per host thread and device, so that factorizations
 // issued concurrently from several threads (the request server's workers) do
 // not queue their panels behind one another.
 struct PanelStreams {

@@ -89,6 +89,8 @@ int gram_ozaki(const double* Y, int64_t ldy, int ymask, const double* C, int64_t
 int to_df64(double* X, int64_t ld, int64_t m, int64_t n, cudaStream_t s);
 int from_df64(double* X, int64_t ld, int64_t m, int64_t n, cudaStream_t s);
 
+// capi.cu: SMs of the current device.
+int device_sms();
 // capi.cu: TSQR-HR of one m x b panel (recursive blocking), T (ldT) out.
 int hr_rec(double* A, int64_t lda, int64_t m, int b, double* T, int64_t ldT, int* st, int precision,
            cudaStream_t s);

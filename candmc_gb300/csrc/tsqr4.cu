@@ -24,8 +24,9 @@
 //    b rows, then the sign-choice LU of Q1_top - S, and L\(S R), T, W and
 //    U^-1.  In k_hr6_pipe leaf 0 and the nodes on its path build Q1_top as a
 //    prefix product while they finish, and one extra CTA solves the root;
-//  * kernel 2: each leaf multiplies its root-to-leaf chain of Q blocks into
-//    U^-1 (M) and writes Y = [M; 0] - V (T (V_top^T M)).
+//  * Y = (I - V T V_top^T) (Q^(1) ... Q^(depth)) U^-1 per leaf, the Q blocks
+//    taken along the leaf's path: beside the tree where its CTAs find free
+//    SMs (k_hr6_y), in a launch of its own otherwise (k_hr4_form_y).
 // The Householder factor is canonical, so the result equals the binary-tree
 // reconstruction and LAPACK's dgeqrf up to rounding.
 #include <math.h>
@@ -82,6 +83,11 @@ __device__ __forceinline__ int64_t t4_leaf_row0(int64_t m, int P, int i) {
 // An all-zero tail takes v = e_j, gamma = 2, beta = -alpha (a sign flip), the
 // convention of the reconstruction, so that T^-1 = striu(V^T V) +
 // diag(V^T V) / 2 (alg/QR/qr_2d/qr_2d.cxx:22-60) holds for every reflector.
+// This thread's warp, in a form the compiler knows to be uniform: branches on
+// it (and on columns derived from it) become plain jumps instead of divergent
+// regions, worth 20 % of a column step.
+__device__ __forceinline__ int warp_id() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
+
 constexpr int kLeafThreads = 288;   // 9 warps: the critical one, 6 for the columns, 2 for memory
 constexpr int kPollWarp = 4;        // sub-partition 0: waits for the children's columns
 constexpr int kPubWarp = 8;         // sub-partition 0: publishes finished columns
@@ -305,7 +311,7 @@ struct NoPublish {
 // hands column j - 1 of R to the parent; one block barrier per step.
 template <int R, bool NODE, class Pub = NoPublish>
 __device__ void h7_factor(double* S, int ld, int b, double* s_h, double* s_gam, Pub pub = Pub()) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = warp_id();
   const int q = bulk_index(warp);
   double v[R], gam = 0.0;
 #pragma unroll
@@ -335,64 +341,74 @@ __device__ void h7_factor(double* S, int ld, int b, double* s_h, double* s_gam, 
   if (warp == kPubWarp) pub(S, ld, b - 1);
 }
 
-// Structure of an operand of h5_mm, on op(X): entries outside it read as 0
-// (and the unit diagonals as 1).
-enum : int { kSDense = 0, kSUpper = 1, kSUnitUpper = 2, kSUnitLower = 3 };
+// Structure of an operand of mm32, on op(X).  The zeros (and unit diagonals)
+// are stored; the structure only bounds the k range of a tile.
+enum : int { kSDense = 0, kSUpper = 1, kSLower = 2 };
 
-__device__ __forceinline__ double h5_at(const double* X, int ld, bool tr, int st, int i, int k) {
-  if ((st == kSUpper || st == kSUnitUpper) && k < i) return 0.0;
-  if (st == kSUnitLower && k > i) return 0.0;
-  if ((st == kSUnitUpper || st == kSUnitLower) && k == i) return 1.0;
-  return tr ? X[i * ld + k] : X[k * ld + i];
-}
-
-// C = C0 + alpha op(A) op(B) for b x b shared-memory matrices (b <= 32; C0
-// may be nullptr, or C itself; C must not alias A or B).
-// The 32 x 32 output is cut into 8 x 8 tiles, each owned by one warp (lane l:
-// row l % 8, columns l / 8 and l / 8 + 4), and a tile's k loop only covers
-// the structural nonzeros of its row and column blocks (empty for the zero
-// tiles of a product of two upper-triangular operands), and the tiles are
-// dealt to the warps in order of decreasing work.  A warp-wide FP64 instruction is the unit of cost on this
-// GPU (about 4 per 77 cycles per SM), so this bounds the product by the
-// nonzero tile work instead of by the longest k range of any lane.
-__device__ void h5_mm(const double* A, int lda, bool at, int as, const double* B, int ldb, bool bt,
-                      int bs, double* C, int ldc, int b, double alpha, const double* C0) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  const int nt = (b + 7) >> 3;
-  // tiles in order of decreasing k extent: the diagonal distance d = tj - ti
-  // runs from nt - 1 down to -(nt - 1); tile number p walks that order
+// C = C0 + alpha op(A) op(B) for b x b shared-memory blocks (b <= 32, zero
+// beyond b up to whole 8 x 8 tiles; C0 may be nullptr, or C itself; C must not
+// alias A or B), op(A)[i, k] = A[i ai + k ak], op(B)[k, j] = B[k bk + j bj].
+// bo: rows and columns of C written, b, or up8(b) when C is an operand of a
+// later product.  nb products with the same B at once: A and C advance by
+// anext and cnext doubles.  All threads of the block call it.
+// The 32 x 32 output is cut into 8 x 4 half tiles (lane l: row l % 8, column
+// l / 8), one FP64 instruction per k, and a half tile's k loop covers only the
+// structural nonzeros of its row and column blocks (empty for the zero tiles
+// of a product of two upper-triangular operands).  They are dealt to eight
+// warps (four in a block of four) in order of decreasing work, forward and
+// backward in turn: two upper-triangular operands cost 88 FP64 instructions
+// on the fullest sub-partition (80 on average).  One compact loop serves every
+// product, because a call runs its code once: a version unrolled over the
+// tiles waited for its instructions (7 us a product against 5).  Two sums per
+// lane keep the FP64 pipe at its 65 cycles an instruction (76 in one chain).
+__device__ __noinline__ void mm32(const double* A, int ai, int ak, int as, const double* B, int bk, int bj, int bs,
+                                  double* C, int ldc, int bo, double alpha, const double* C0, int nb = 1,
+                                  int anext = 0, int cnext = 0) {
+  const int lane = threadIdx.x & 31, warp = warp_id();
+  const int nw = blockDim.x >= 256 ? 8 : (int)blockDim.x >> 5;
+  const int nt = (bo + 7) >> 3;
   int p = 0;
-  for (int d = nt - 1; d >= -(nt - 1); --d) {
-    for (int ti = 0; ti < nt; ++ti) {
-      const int tj = ti + d;
-      if (tj < 0 || tj >= nt) continue;
-      const int i0 = ti * 8, j0 = tj * 8;
-      // k range of the tile from the operands' structure
-      int klo = 0, khi = b - 1;
-      if (as == kSUpper || as == kSUnitUpper) klo = i0;
-      if (as == kSUnitLower) khi = khi < i0 + 7 ? khi : i0 + 7;
-      if (bs == kSUpper || bs == kSUnitUpper) khi = khi < j0 + 7 ? khi : j0 + 7;
-      if (bs == kSUnitLower) klo = klo > j0 ? klo : j0;
-      // (an empty range still writes C = C0, or zero)
-      if ((p++ % nwarp) != warp) continue;
-      const int i = i0 + (lane & 7), jA = j0 + (lane >> 3), jB = jA + 4;
-      double acc0 = 0.0, acc1 = 0.0;
-#pragma unroll 4
-      for (int k = klo; k <= khi; ++k) {
-        const double a = (i < b) ? h5_at(A, lda, at, as, i, k) : 0.0;
-        const double b0 = (jA < b) ? h5_at(B, ldb, bt, bs, k, jA) : 0.0;
-        const double b1 = (jB < b) ? h5_at(B, ldb, bt, bs, k, jB) : 0.0;
-        acc0 = fma(a, b0, acc0);
-        acc1 = fma(a, b1, acc1);
-      }
-      if (i < b) {
-        if (jA < b) C[jA * ldc + i] = fma(alpha, acc0, C0 ? C0[jA * ldc + i] : 0.0);
-        if (jB < b) C[jB * ldc + i] = fma(alpha, acc1, C0 ? C0[jB * ldc + i] : 0.0);
+  for (int d = nt - 1; d > -nt; --d) {
+    const int lo = d < 0 ? -d : 0, hi = d < 0 ? nt : nt - d;
+    for (int t = lo * nb; t < hi * nb; ++t) {
+      const int ti = nb == 1 ? t : t / nb, n = nb == 1 ? 0 : t - ti * nb;
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half, ++p) {
+        const int q = p & (2 * nw - 1);
+        if ((q < nw ? q : 2 * nw - 1 - q) != warp) continue;
+        const int i = 8 * ti + (lane & 7), j = 8 * (ti + d) + 4 * half + (lane >> 3);
+        int k0 = 0, k1 = 8 * nt;
+        if (as == kSUpper) k0 = 8 * ti;
+        if (as == kSLower) k1 = min(k1, 8 * ti + 8);
+        if (bs == kSUpper) k1 = min(k1, 8 * (ti + d) + 8);
+        const double* pa = A + n * anext + i * ai + k0 * ak;
+        const double* pb = B + j * bj + k0 * bk;
+        double acc0 = 0.0, acc1 = 0.0;
+#pragma unroll 1
+        for (int k = k0; k < k1; k += 8) {
+          double x[8], y[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            x[u] = pa[u * ak];
+            y[u] = pb[u * bk];
+          }
+          pa += 8 * ak;
+          pb += 8 * bk;
+#pragma unroll
+          for (int u = 0; u < 8; u += 2) {
+            acc0 = fma(x[u], y[u], acc0);
+            acc1 = fma(x[u + 1], y[u + 1], acc1);
+          }
+        }
+        if (i < bo && j < bo)
+          C[n * cnext + j * ldc + i] = fma(alpha, acc0 + acc1, C0 ? C0[j * ldc + i] : 0.0);
       }
     }
   }
   __syncthreads();
 }
+
+__device__ __forceinline__ int up8(int b) { return (b + 7) & ~7; }
 
 // Inverse of the upper triangle of X (32 x 32, ld kLd) into Xi (ld kLd), by
 // recursive 2 x 2 block inversion done bottom-up:
@@ -430,9 +446,12 @@ __device__ void h4_tri_inv(const double* X, double* Xi, double* scratch) {
   }
 }
 
-// b x b block from global memory (ld b) into shared memory
-__device__ void h4_load(double* dst, const double* src, int b, int ld) {
-  for (int idx = threadIdx.x; idx < b * b; idx += blockDim.x) dst[(idx / b) * ld + idx % b] = __ldcg(src + idx);
+// b x b block from global memory (ld b) into a shared block (ld kLd), zero beyond b
+__device__ void h4_load(double* dst, const double* src, int b) {
+  for (int idx = threadIdx.x; idx < kDirectB * kDirectB; idx += blockDim.x) {
+    const int r = idx & 31, c = idx >> 5;
+    dst[c * kLd + r] = (r < b && c < b) ? __ldcg(src + c * b + r) : 0.0;
+  }
   __syncthreads();
 }
 
@@ -465,7 +484,7 @@ constexpr int kGramScratch = 4 * 640;   // h7_gram's partial sums (doubles)
 // row l % 8 of a tile, columns l / 8 and l / 8 + 4), so a row costs 20 FP64
 // instructions and no shuffles; the eight partial sums meet in shared memory.
 __device__ void h7_gram(const double* VT, const double* S, int ldS, int rows, int b, double* G, double* part) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = warp_id();
   const int i = lane & 7, jj = lane >> 3;
   double acc[10][2];
 #pragma unroll
@@ -535,13 +554,15 @@ struct Hr4Args {
   double* Uinv;     // scratch b x b
   int* status;
   unsigned* prog;   // pipelined tree: columns of R published by each node
-  unsigned* done;   // pipelined tree: node finished (T, Q blocks, V written)
+  unsigned* done;   // pipelined tree: node finished (T, Q blocks, V written); the root's U^-1 last
   unsigned* ticket; // pipelined tree: role counter
   int* fail;        // pipelined tree: a wait gave up
-  double* Pc;       // pipelined tree: prefix products of Q1_top along leaf 0's path, (depth + 1) x b x b
+  double* Pc;       // pipelined tree: I - V0 T0 V0^T of leaf 0, then per level the product of the first
+                    // Q blocks up leaf 0's path, (depth + 1) x b x b
   double* Mn;       // many leaves: per node, the product of the Q blocks from the root down to it
                     // times U^-1 (nnodes x b x b, by flat id), or nullptr
   int P;
+  int yparts;       // pipelined tree: CTAs per leaf of k_hr6_y (0: k_hr4_form_y)
   int ldS;          // leading dimension of the shared block: 32 row slots + 1
   int depth;
   int nlev[kMaxLevels + 1];
@@ -555,6 +576,16 @@ __device__ __forceinline__ int h4_children(const Hr4Args& a, int lvl, int node) 
   return n < kFan ? n : kFan;
 }
 
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
 // barrier `id` of n threads (a multiple of 32)
 __device__ __forceinline__ void named_bar(int id, int n) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
@@ -565,16 +596,18 @@ constexpr int kRootDoubles = 6 * kBlk;
 constexpr long kSmemSpin = 1L << 22;        // polls of a shared-memory flag
 
 // The root: Q1_top, its sign-choice LU, T, W and U^-1.  The LU runs with a
-// one-column lookahead: warp 0 finishes column i + 1 (the pivot's chain:
-// about 500 cycles) while four warps apply column i to the columns beyond.
-// U^-1 and T are formed column by column behind it, by one warp each on
-// sub-partitions of their own: X U = I gives X[:, c] = (e_c - sum_{k<c} X[:, k]
-// U[k, c]) / U[c, c], and T L^T = -U S gives T[:, c] = -U[:, c] S_c -
-// sum_{k<c} T[:, k] L[c, k]; both need only the columns the LU has finished.
-// 496 FP64 instructions each bound the whole (16 us), where the LU followed
-// by two recursive inversions and a product took 58 us.
+// one-column lookahead: warp 0 applies column i to column i + 1 and finishes
+// it (pivot, reciprocal, multipliers: a chain of six FP64 instructions) while
+// three warps, with the columns in registers, apply column i to those beyond.
+// U^-1 follows it column by column, X U = I giving X[:, c] = (e_c - sum_{k<c}
+// X[:, k] U[k, c]) / U[c, c], by four warps that split the sum: Y waits for it.
+// The same four then form T from T L^T = -U S, T[:, c] = -U[:, c] S_c -
+// sum_{k<c} T[:, k] L[c, k], beside Y.  All loops are rolled: the role runs
+// once on some SM, and unrolled over the columns it waits for its instructions
+// (LU 32 us with eight columns a warp unrolled, 15 us rolled).  The LU, two
+// inversions and a product one after the other took 58 us.
 __device__ void h4_root(const Hr4Args& a, double* sm) {
-  const int b = a.b, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int b = a.b, tid = threadIdx.x, lane = tid & 31, warp = warp_id();
   double* sR = sm;
   double* sL = sR + kBlk;    // Q1_top, becomes L\U
   double* sT = sL + kBlk;
@@ -582,110 +615,171 @@ __device__ void h4_root(const Hr4Args& a, double* sm) {
   double* sM = sX + kBlk;
   double* sQ = sM + kBlk;
   __shared__ int s_sign[kDirectB];
-  __shared__ double s_rp[kDirectB];
+  __shared__ double s_rp[kDirectB], s_part[3][kDirectB];
   __shared__ volatile int s_cols;   // columns of L\U finished
-  h4_load(sR, a.Rn + (size_t)a.base[a.depth] * b * b, b, kLd);
+  for (int idx = tid; idx < kBlk; idx += blockDim.x) sQ[idx] = sL[idx] = 0.0;
+  __syncthreads();
   if (a.Pc) {
-    // the pipelined tree multiplied Q1_top up leaf 0's path as its nodes finished
-    h4_load(sL, a.Pc + (size_t)a.depth * b * b, b, kLd);
+    // the pipelined tree: sX (loaded by the caller) times the top node's first Q block
+    if (a.depth > 0) {
+      h4_load(sQ, a.Pc + (size_t)a.depth * b * b, b);
+      mm32(sX, 1, kLd, kSDense, sQ, 1, kLd, kSUpper, sL, kLd, up8(b), 1.0, nullptr);
+    } else {
+      h4_load(sL, a.Pc, b);
+    }
   } else {
     // chain M = Q1^(1) ... Q1^(depth) of the first-child Q blocks (upper triangular)
-    for (int idx = tid; idx < b * b; idx += blockDim.x) sM[(idx / b) * kLd + idx % b] = (idx % b == idx / b) ? 1.0 : 0.0;
+    for (int idx = tid; idx < kBlk; idx += blockDim.x) {
+      const int r = idx % kLd, c = idx / kLd;
+      sM[idx] = (r == c && c < b) ? 1.0 : 0.0;
+    }
     __syncthreads();
     for (int lvl = a.depth; lvl >= 1; --lvl) {
       if (h4_children(a, lvl, 0) > 1) {
-        h4_load(sX, a.Qn + ((size_t)a.base[lvl] * kFan + 0) * b * b, b, kLd);
-        h5_mm(sX, kLd, false, kSUpper, sM, kLd, false, kSUpper, sQ, kLd, b, 1.0, nullptr);
+        h4_load(sX, a.Qn + ((size_t)a.base[lvl] * kFan + 0) * b * b, b);
+        mm32(sX, 1, kLd, kSUpper, sM, 1, kLd, kSUpper, sQ, kLd, up8(b), 1.0, nullptr);
         for (int idx = tid; idx < b * b; idx += blockDim.x) sM[(idx / b) * kLd + idx % b] = sQ[(idx / b) * kLd + idx % b];
         __syncthreads();
       }
     }
     // Q1_top = C0 - V0 (T0 (V0^T C0)), V0 = unit-lower top block of leaf 0, C0 = M
-    for (int idx = tid; idx < b * b; idx += blockDim.x) {
-      const int r = idx % b, c = idx / b;
-      sL[c * kLd + r] = (r > c) ? __ldcg(a.Vw + (int64_t)c * a.m + r) : (r == c ? 1.0 : 0.0);
+    for (int idx = tid; idx < kBlk; idx += blockDim.x) {
+      const int r = idx % kLd, c = idx / kLd;
+      sL[idx] = (r < b && c < b) ? (r > c ? __ldcg(a.Vw + (int64_t)c * a.m + r) : (r == c ? 1.0 : 0.0)) : 0.0;
     }
-    h4_load(sT, a.Tl, b, kLd);
-    h5_mm(sL, kLd, true, kSUnitUpper, sM, kLd, false, kSUpper, sX, kLd, b, 1.0, nullptr);   // V0^T C0 (upper)
-    h5_mm(sT, kLd, false, kSUpper, sX, kLd, false, kSUpper, sQ, kLd, b, 1.0, nullptr);      // T0 of it (upper)
-    h5_mm(sL, kLd, false, kSUnitLower, sQ, kLd, false, kSUpper, sX, kLd, b, -1.0, sM);      // C0 - V0 sQ
+    h4_load(sT, a.Tl, b);
+    mm32(sL, kLd, 1, kSUpper, sM, 1, kLd, kSUpper, sX, kLd, up8(b), 1.0, nullptr);    // V0^T C0 (upper)
+    mm32(sT, 1, kLd, kSUpper, sX, 1, kLd, kSUpper, sQ, kLd, up8(b), 1.0, nullptr);   // T0 of it (upper)
+    mm32(sL, 1, kLd, kSLower, sQ, 1, kLd, kSUpper, sX, kLd, up8(b), -1.0, sM);       // C0 - V0 sQ
     for (int idx = tid; idx < b * b; idx += blockDim.x) sL[(idx / b) * kLd + idx % b] = sX[(idx / b) * kLd + idx % b];
+    __syncthreads();
   }
-  __syncthreads();
   for (int idx = tid; idx < kBlk; idx += blockDim.x) sT[idx] = sX[idx] = 0.0;
   if (tid == 0) s_cols = 0;
   __syncthreads();
-  const int trail = warp == 3 ? 0 : warp == 7 ? 1 : warp == 4 ? 2 : warp == 8 ? 3 : -1;
+  // columns before c finished (one warp)
+  auto wait_cols = [&](int c) {
+    long it = 0;
+    while (s_cols < c && ++it < kSmemSpin) __nanosleep(20);
+    __syncwarp();
+    if (it >= kSmemSpin && lane == 0) atomicExch(a.status, CANDMC_ERR_TIMEOUT);
+    __threadfence_block();
+  };
+  // acc minus the sum over k < c, k = h (mod 4), of X[:, k] v[k]: X's columns
+  // from c on are still zero, so the last step may reach beyond c
+  const int h = warp - 1;   // of the four warps 1..4
+  auto minus_sum = [&](double acc, const double* X, const double* v, int ldv, int c) -> double {
+#pragma unroll 1
+    for (int k = h; k < c; k += 16) {
+      double x[4], u[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int kk = k + 4 * q;
+        x[q] = kk < c ? X[kk * kLd + lane] : 0.0;
+        u[q] = kk < c ? v[kk * ldv] : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc = fma(-x[q], u[q], acc);
+    }
+    return acc;
+  };
   if (warp == 0) {
-    double x = lane < b ? sL[lane] : 0.0;
+    double x = sL[lane];
     for (int i = 0; i < b; ++i) {
       const double d = __shfl_sync(0xffffffffu, x, i);
       const long long db = __double_as_longlong(d);
       const bool pos = db > 0 && db <= 0x7ff0000000000000LL;   // d > 0
-      const double piv = d + (pos ? 1.0 : -1.0);   // |piv| >= 1: the sign choice keeps the pivot away from 0
-      const double rp = quick_rcp(piv);
-      const double l = lane > i ? x * rp : (lane == i ? piv : x);
-      if (lane < b) sL[i * kLd + lane] = l;
+      // 1 <= |piv| <= 2: the sign choice keeps the pivot away from 0 (a NaN
+      // passes through the refinement below)
+      const double piv = d + (pos ? 1.0 : -1.0);
+      const double y = flip_if(f64_of(__fdividef(1.0f, f32_of(fabs(piv)))), !pos);
+      const double e = fma(-piv, y, 1.0);
+      const double xy = x * y;
+      const double e2 = fma(e, e, e);
+      const double m = fma(xy, e2, xy);   // the multipliers x / piv
+      sL[i * kLd + lane] = lane > i ? m : (lane == i ? piv : x);
       if (lane == 0) {
         s_sign[i] = pos ? -1 : 1;
-        s_rp[i] = rp;
+        s_rp[i] = fma(y, e2, y);
       }
       __threadfence_block();
       __syncwarp();
       if (lane == 0) s_cols = i + 1;
-      named_bar(1, 5 * 32);
+      named_bar(1, 4 * 32);
       if (i + 1 < b) {
-        const double xn = lane < b ? sL[(i + 1) * kLd + lane] : 0.0;
+        const double xn = sL[(i + 1) * kLd + lane];
         const double u = __shfl_sync(0xffffffffu, xn, i);
-        x = lane > i ? fma(-l, u, xn) : xn;
+        x = lane > i ? fma(-m, u, xn) : xn;
       }
     }
-  } else if (trail >= 0) {
+  } else if (warp >= 5 && warp <= 7) {
+    // columns q, q + 3, .. in registers (one row per lane); column i + 2 goes
+    // back to shared memory for the critical warp when it is next
+    const int q = warp - 5;
+    double x[11];
+#pragma unroll
+    for (int k = 0; k < 11; ++k) {
+      const int c = q + 3 * k;
+      x[k] = c < kDirectB ? sL[c * kLd + lane] : 0.0;
+    }
+#pragma unroll 1
     for (int i = 0; i < b; ++i) {
-      named_bar(1, 5 * 32);
-      const double l = sL[i * kLd + lane];
-      for (int c = i + 2 + trail; c < b; c += 4) {
-        const double u = sL[c * kLd + i];
-        if (lane > i && lane < b) sL[c * kLd + lane] = fma(-l, u, sL[c * kLd + lane]);
+      named_bar(1, 4 * 32);
+      const double l = lane > i ? sL[i * kLd + lane] : 0.0;
+#pragma unroll
+      for (int k = 0; k < 11; ++k) {
+        const int c = q + 3 * k;
+        if (c >= i + 2 && c < b) {
+          x[k] = fma(-l, __shfl_sync(0xffffffffu, x[k], i), x[k]);
+          if (c == i + 2) sL[c * kLd + lane] = x[k];
+        }
       }
     }
-  } else if (warp == 1 || warp == 2) {
+  } else if (warp <= 4) {
+    bool bad = false;
+#pragma unroll 1
     for (int c = 0; c < b; ++c) {
-      long it = 0;
-      while (s_cols <= c && ++it < kSmemSpin) __nanosleep(20);
-      __syncwarp();
-      if (it >= kSmemSpin) {
-        if (lane == 0) atomicExch(a.status, CANDMC_ERR_TIMEOUT);
-        break;
+      wait_cols(c + 1);
+      const double acc = minus_sum((h == 0 && lane == c) ? 1.0 : 0.0, sX, sL + c * kLd, 1, c);
+      if (h) s_part[h - 1][lane] = acc;
+      named_bar(2, 128);
+      if (!h) {
+        const double v =
+            lane <= c ? ((acc + s_part[0][lane]) + (s_part[1][lane] + s_part[2][lane])) * s_rp[c] : 0.0;
+        sX[c * kLd + lane] = v;
+        if (lane < b) a.Uinv[c * b + lane] = v;
+        bad |= hi_abs(v) >= 0x7ff00000;
       }
-      __threadfence_block();
-      if (warp == 1) {
-        double acc = lane == c ? 1.0 : 0.0;
-#pragma unroll 4
-        for (int k = 0; k < c; ++k) acc = fma(-sX[k * kLd + lane], sL[c * kLd + k], acc);
-        sX[c * kLd + lane] = lane <= c ? acc * s_rp[c] : 0.0;
-      } else {
-        double acc = lane <= c ? flip_if(sL[c * kLd + lane], s_sign[c] > 0) : 0.0;
-#pragma unroll 4
-        for (int k = 0; k < c; ++k) acc = fma(-sT[k * kLd + lane], sL[k * kLd + c], acc);
-        sT[c * kLd + lane] = lane <= c ? acc : 0.0;
-      }
-      __syncwarp();
+      named_bar(2, 128);
     }
+    if (!h) {
+      if (bad) atomicExch(a.status, CANDMC_ERR_NUMERIC);
+      __threadfence();
+      __syncwarp();
+      if (lane == 0 && a.Pc) st_release(a.done + a.base[a.depth] + 1, 1u);
+    }
+#pragma unroll 1
+    for (int c = 0; c < b; ++c) {
+      const double acc = minus_sum((h == 0 && lane <= c) ? flip_if(sL[c * kLd + lane], s_sign[c] > 0) : 0.0, sT,
+                                   sL + c, kLd, c);
+      if (h) s_part[h - 1][lane] = acc;
+      named_bar(2, 128);
+      if (!h)
+        sT[c * kLd + lane] = lane <= c ? (acc + s_part[0][lane]) + (s_part[1][lane] + s_part[2][lane]) : 0.0;
+      named_bar(2, 128);
+    }
+  } else if (warp == 8) {   // R while the others work
+    for (int c = 0; c < b; ++c)
+      if (lane < b) sR[c * kLd + lane] = __ldcg(a.Rn + (size_t)a.base[a.depth] * b * b + c * b + lane);
   }
   __syncthreads();
-  int bad = 0;
   for (int idx = tid; idx < b * b; idx += blockDim.x) {
     const int r = idx % b, c = idx / b;
     const double lu = sL[c * kLd + r];
     a.A[c * a.lda + r] = (r > c) ? lu : flip_if(sR[c * kLd + r], s_sign[r] < 0);
     if (a.W) a.W[c * a.ldW + r] = (r <= c) ? flip_if(lu, s_sign[c] < 0) : 0.0;
     a.T[c * a.ldT + r] = (r <= c) ? sT[c * kLd + r] : 0.0;
-    const double v = sX[c * kLd + r];
-    if (hi_abs(v) >= 0x7ff00000) bad = 1;
-    a.Uinv[idx] = v;
   }
-  if (bad) atomicExch(a.status, CANDMC_ERR_NUMERIC);
 }
 
 // The reflectors of a factored leaf: S's tails divided by their heads (s_h
@@ -812,7 +906,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2) k_hr4_leaf_tree(Hr4Args a) {
     }
     for (int k = 1; k < nch; ++k) {
       double* Qk = G;   // G is free once T is formed
-      h5_mm(S + 32 * k, ldS, false, kSUpper, Tt, kLd, false, kSUpper, Qk, kLd, b, -1.0, nullptr);
+      mm32(S + 32 * k, 1, ldS, kSUpper, Tt, 1, kLd, kSUpper, Qk, kLd, b, -1.0, nullptr);
       for (int idx = tid; idx < b * b; idx += blockDim.x) Qp[(size_t)k * b * b + idx] = Qk[(idx / b) * kLd + idx % b];
       __syncthreads();
     }
@@ -840,16 +934,6 @@ __global__ void __launch_bounds__(kLeafThreads, 2) k_hr4_leaf_tree(Hr4Args a) {
 // CANDMC_ERR_TIMEOUT, and the CTA releases its own flags and returns, so no
 // other CTA is left waiting on it.
 constexpr long kSpinLimit = 1L << 22;
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 
 // One thread: wait until *p >= v.  False when the wait gave up or another CTA
 // of this launch did.
@@ -906,8 +990,8 @@ __device__ void h6_leaf(const Hr4Args& a, int leaf, double* sm, double* s_h, dou
   if (leaf == 0 && a.Pc) {
     // P_0 = I - V0 T0 V0^T on the top b rows (V0 unit lower): the first factor
     // of Q1_top, multiplied by the path nodes' Q1 blocks as they finish
-    h5_mm(Tt, kLd, false, kSUpper, VT, kLd, true, kSUnitUpper, G, kLd, b, 1.0, nullptr);   // G = T0 V0^T
-    h5_mm(VT, kLd, false, kSUnitLower, G, kLd, false, kSUpper, S, kLd, b, 1.0, nullptr);   // V0 G (S is free)
+    mm32(Tt, 1, kLd, kSUpper, VT, kLd, 1, kSUpper, G, kLd, up8(b), 1.0, nullptr);   // G = T0 V0^T
+    mm32(VT, 1, kLd, kSLower, G, 1, kLd, kSUpper, S, kLd, b, 1.0, nullptr);        // V0 G (S is free)
     for (int idx = tid; idx < b * b; idx += blockDim.x)
       a.Pc[idx] = ((idx % b == idx / b) ? 1.0 : 0.0) - S[(idx / b) * kLd + idx % b];
   }
@@ -939,7 +1023,7 @@ constexpr int kNodeDoubles = kNodeLd * kDirectB + 4 * kBlk + 4 * 96;
 // average) against 13 k cycles a step when one warp group did all of it in
 // sequence with seven block barriers.
 __device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_h, double* s_gam) {
-  const int b = a.b, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int b = a.b, tid = threadIdx.x, lane = tid & 31, warp = warp_id();
   __shared__ int s_okv[2];
   int lvl = 1;
   while (lvl < a.depth && f >= a.base[lvl + 1]) ++lvl;
@@ -1085,32 +1169,41 @@ __device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_h, double
     if (tgrp || cgrp) bulk(b, b);
     __syncthreads();
     // T of normalised heads: Tn = T D (for Q_k = -V_k T D), Qk = D T D (Q_1 = I - D T D)
-    for (int i = tid; i < b * b; i += blockDim.x) {
-      const int r = i % b, c = i / b;
-      const double t = Tn[c * kLd + r] * s_h[c];
+    for (int i = tid; i < kDirectB * kDirectB; i += blockDim.x) {
+      const int r = i & 31, c = i >> 5;
+      const bool in = r < b && c < b;
+      const double t = in ? Tn[c * kLd + r] * s_h[c] : 0.0;
       Tn[c * kLd + r] = t;
-      Qk[c * kLd + r] = s_h[r] * t;
+      Qk[c * kLd + r] = in ? s_h[r] * t : 0.0;
     }
     __syncthreads();
   }
   if (idx == 0) {
-    // on leaf 0's path: P_lvl = P_(lvl-1) Q1 = P_(lvl-1) (I - D T D), as soon as the
-    // child on the path has its prefix (it then sets its progress to b + 1).
-    // The root's solver waits for this node's prefix the same way.
-    if (tid == 0) s_okv[0] = h6_wait(a, a.prog + child0, (unsigned)b + 1u);
-    __syncthreads();
-    if (!s_okv[0]) {
-      h6_release_all(a, f);
-      return;
+    // on leaf 0's path: U_lvl = U_(lvl-1) Q1 with Q1 = I - D T D and U_0 = I
+    // (upper triangular), as soon as the child on the path has its product (it
+    // then sets its progress to b + 1).  The top node hands its Q1 alone to the
+    // root's solver, which has multiplied what lies below it by then.
+    double* Ul = a.Pc + (size_t)lvl * b * b;
+    const double* Uprev = Ul - (size_t)b * b;
+    const bool mul = lvl > 1 && lvl < a.depth;
+    if (mul) {
+      if (tid == 0) s_okv[0] = h6_wait(a, a.prog + child0, (unsigned)b + 1u);
+      __syncthreads();
+      if (!s_okv[0]) {
+        h6_release_all(a, f);
+        return;
+      }
     }
-    const double* Pprev = a.Pc + (size_t)(lvl - 1) * b * b;
-    double* Pl = a.Pc + (size_t)lvl * b * b;
-    if (nch > 1) {
-      h4_load(Pb, Pprev, b, kLd);
-      h5_mm(Pb, kLd, false, kSDense, Qk, kLd, false, kSUpper, Po, kLd, b, -1.0, Pb);
-      for (int i = tid; i < b * b; i += blockDim.x) Pl[i] = Po[(i / b) * kLd + i % b];
-    } else {
-      for (int i = tid; i < b * b; i += blockDim.x) Pl[i] = __ldcg(Pprev + i);
+    if (mul && nch > 1) {
+      h4_load(Pb, Uprev, b);
+      mm32(Pb, 1, kLd, kSUpper, Qk, 1, kLd, kSUpper, Po, kLd, b, -1.0, Pb);
+    }
+    for (int i = tid; i < b * b; i += blockDim.x) {
+      const int r = i % b, c = i / b;
+      double u = r == c ? 1.0 : 0.0;
+      if (nch > 1) u = mul ? Po[c * kLd + r] : u - Qk[c * kLd + r];
+      else if (mul) u = __ldcg(Uprev + i);
+      Ul[i] = u;
     }
     __threadfence();
     __syncthreads();
@@ -1123,25 +1216,173 @@ __device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_h, double
       const int r = i % b, c = i / b;
       Qp[i] = ((r == c) ? 1.0 : 0.0) - ((r <= c) ? Qk[c * kLd + r] : 0.0);
     }
-    for (int k = 1; k < nch; ++k)
-      h5_mm(S + 32 * k, ld, false, kSUpper, Tn, kLd, false, kSUpper, Qp + (size_t)k * b * b, b, b, -1.0, nullptr);
+    mm32(S + 32, 1, ld, kSUpper, Tn, 1, kLd, kSUpper, Qp + b * b, b, b, -1.0, nullptr, nch - 1, 32, b * b);
   }
   __threadfence();
   __syncthreads();
   if (tid == 0) st_release(a.done + f, 1u);
 }
 
-// The root's solver (one extra CTA): once the top node has published its R
-// and the full prefix Q1_top, the sign-choice LU, T, W and U^-1, while the
-// top node still writes its Q blocks.
+// The root's solver (one extra CTA): leaf 0's block times the product up its
+// path below the top node while that node works; once it has published its R
+// and its own Q block, the sign-choice LU, T, W and U^-1.
 __device__ void h6_root_solver(const Hr4Args& a, double* sm) {
   __shared__ int s_ok;
-  const int top = a.base[a.depth];
-  if (threadIdx.x == 0) s_ok = h6_wait(a, a.prog + top, (unsigned)a.b + 1u);
-  __syncthreads();
-  if (!s_ok) return;
-  __threadfence();
+  const int b = a.b, top = a.base[a.depth];
+  double* sX = sm + 3 * kBlk;
+  double* sM = sX + kBlk;
+  double* sQ = sM + kBlk;
+  auto wait = [&](int f) -> bool {
+    __syncthreads();
+    if (threadIdx.x == 0) s_ok = h6_wait(a, a.prog + f, (unsigned)b + 1u);
+    __syncthreads();
+    return s_ok != 0;
+  };
+  if (!wait(0)) return;
+  if (a.depth > 1) {
+    if (!wait(a.base[a.depth - 1])) return;
+    h4_load(sM, a.Pc, b);
+    h4_load(sQ, a.Pc + (size_t)(a.depth - 1) * b * b, b);
+    mm32(sM, 1, kLd, kSDense, sQ, 1, kLd, kSUpper, sX, kLd, up8(b), 1.0, nullptr);
+  } else {
+    h4_load(sX, a.Pc, b);
+  }
+  if (!wait(top)) return;
   h4_root(a, sm);
+}
+
+constexpr int kYRows = 64;                 // rows of Y one CTA forms
+constexpr int kYLd = kYRows + 1;
+constexpr int kYDoubles = 2 * kDirectB * kYLd + 4 * kBlk;
+
+// Columns 8 CB .. 8 CB + 7 of X U for 32 rows (one per lane), U upper
+// triangular (ld kLd), X column-major (ld kYLd): init + sign * X U.
+template <int CB>
+__device__ __forceinline__ void h6_y_cols(const double* X, const double* U, double sign, double (&acc)[8]) {
+  double p[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) p[u] = 0.0;
+#pragma unroll 4
+  for (int k = 0; k < 8 * CB; ++k) {
+    const double x = X[k * kYLd];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) p[u] = fma(x, U[(8 * CB + u) * kLd + k], p[u]);
+  }
+#pragma unroll
+  for (int kk = 0; kk < 8; ++kk) {
+    const double x = X[(8 * CB + kk) * kYLd];
+#pragma unroll
+    for (int u = kk; u < 8; ++u) p[u] = fma(x, U[(8 * CB + u) * kLd + 8 * CB + kk], p[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < 8; ++u) acc[u] = fma(sign, p[u], acc[u]);
+}
+
+__device__ __forceinline__ void h6_y_mul(int cb, const double* X, const double* U, double sign, double (&acc)[8]) {
+  switch (cb) {
+    case 0: h6_y_cols<0>(X, U, sign, acc); break;
+    case 1: h6_y_cols<1>(X, U, sign, acc); break;
+    case 2: h6_y_cols<2>(X, U, sign, acc); break;
+    default: h6_y_cols<3>(X, U, sign, acc); break;
+  }
+}
+
+// Y of 64 rows of a leaf, while the tree still runs.  Launched as the tree
+// kernel's programmatic dependent: its CTAs start when every CTA of the tree
+// has started, so everything they wait for is running.
+//  * the leaf's rows of its explicit Q, Ql = [I; 0] - V (T V_top^T), while the
+//    tree works;
+//  * B = Q^(1) ... Q^(depth), the Q blocks from the leaf's parent up to the
+//    root, each multiplied in as its node finishes;
+//  * M = B U^-1 when the root's U^-1 is there, and Y = Ql M: 350 FP64
+//    instructions per sub-partition behind the solver for 64 rows, where
+//    k_hr4_form_y multiplies the whole path and forms Y after it (38 us and a
+//    launch at 8192 x 32).
+__device__ void h6_y(const Hr4Args& a, int y, double* sm) {
+  __shared__ int s_ok;
+  const int b = a.b, tid = threadIdx.x, lane = tid & 31, warp = warp_id();
+  const int leaf = y / a.yparts, part = y % a.yparts;
+  const size_t nb2 = (size_t)b * b;
+  const int64_t r0 = t4_leaf_row0(a.m, a.P, leaf);
+  const int L = (int)(t4_leaf_row0(a.m, a.P, leaf + 1) - r0);
+  const int p0 = part * kYRows;
+  const int n = L - p0 < kYRows ? L - p0 : kYRows;   // rows of this part (none in a short leaf's last part)
+  if (n <= 0) return;
+  double* sV = sm;
+  double* sQ1 = sV + kDirectB * kYLd;
+  double* VT = sQ1 + kDirectB * kYLd;
+  double* S1 = VT + kBlk;
+  double* S2 = S1 + kBlk;
+  double* S3 = S2 + kBlk;
+  auto wait = [&](int f) -> bool {
+    __syncthreads();
+    if (tid == 0) s_ok = h6_wait(a, a.done + f, 1u);
+    __syncthreads();
+    return s_ok != 0;
+  };
+  if (!wait(leaf)) return;
+  for (int e = tid; e < kYRows * kDirectB; e += blockDim.x) {
+    const int c = e / kYRows, r = e % kYRows, rl = p0 + r;
+    double v = 0.0;
+    if (r < n && c < b) v = rl == c ? 1.0 : __ldcg(a.Vw + (int64_t)c * a.m + r0 + rl);
+    sV[c * kYLd + r] = v;
+  }
+  for (int e = tid; e < kDirectB * kDirectB; e += blockDim.x) {
+    const int r = e & 31, c = e >> 5;
+    double v = 0.0;
+    if (r < b && c < b) v = r > c ? __ldcg(a.Vw + (int64_t)c * a.m + r0 + r) : (r == c ? 1.0 : 0.0);
+    S1[c * kLd + r] = v;
+  }
+  h4_load(S2, a.Tl + (size_t)leaf * nb2, b);
+  mm32(S2, 1, kLd, kSUpper, S1, kLd, 1, kSUpper, VT, kLd, up8(b), 1.0, nullptr);   // T V_top^T
+  // 32 rows x 8 columns per warp; warps w and w + 4 share a sub-partition and
+  // take column blocks w and 3 - w, so that the triangle's work is even
+  const int g = warp >> 2, cb = g ? 3 - (warp & 3) : warp & 3;
+  const int r = 32 * g + lane, rl = p0 + r;
+  if (warp < 8 && 8 * cb < b) {
+    double acc[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) acc[u] = rl == 8 * cb + u ? 1.0 : 0.0;
+    h6_y_mul(cb, sV + r, VT, -1.0, acc);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) sQ1[(8 * cb + u) * kYLd + r] = acc[u];
+  }
+  // B in S1
+  for (int e = tid; e < kDirectB * kDirectB; e += blockDim.x) {
+    const int r2 = e & 31, c = e >> 5;
+    S1[c * kLd + r2] = (r2 == c && c < b) ? 1.0 : 0.0;
+  }
+  bool any = false;
+  int child = leaf;
+  for (int lvl = 1; lvl <= a.depth; ++lvl) {
+    const int nd = child / kFan;
+    if (h4_children(a, lvl, nd) > 1) {
+      if (!wait(a.base[lvl] + nd)) return;
+      h4_load(any ? S3 : S1, a.Qn + ((size_t)(a.base[lvl] + nd) * kFan + (child - nd * kFan)) * nb2, b);
+      if (any) {
+        mm32(S1, 1, kLd, kSUpper, S3, 1, kLd, kSUpper, S2, kLd, up8(b), 1.0, nullptr);
+        double* t = S1;
+        S1 = S2;
+        S2 = t;
+      }
+      any = true;
+    }
+    child = nd;
+  }
+  if (!wait(a.base[a.depth] + 1)) return;   // U^-1
+  h4_load(S3, a.Uinv, b);
+  mm32(S1, 1, kLd, kSUpper, S3, 1, kLd, kSUpper, S2, kLd, up8(b), 1.0, nullptr);   // M
+  if (warp < 8 && 8 * cb < b) {
+    double acc[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) acc[u] = 0.0;
+    h6_y_mul(cb, sQ1 + r, S2, 1.0, acc);
+    if (r < n && r0 + rl >= b) {   // the panel's top b rows come from the root
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (8 * cb + u < b) a.A[(int64_t)(8 * cb + u) * a.lda + r0 + rl] = acc[u];
+    }
+  }
 }
 
 __global__ void __launch_bounds__(kLeafThreads, 2) k_hr6_pipe(Hr4Args a) {
@@ -1150,13 +1391,23 @@ __global__ void __launch_bounds__(kLeafThreads, 2) k_hr6_pipe(Hr4Args a) {
   __shared__ int s_role;
   if (threadIdx.x == 0) s_role = (int)atomicAdd(a.ticket, 1u);
   __syncthreads();
-  const int f = s_role;   // flat tree id: leaves 0 .. P-1, the nodes level by level, the root's solver
+  // the Y kernel (k_hr6_y) may start once every CTA of this grid is here
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // flat tree id: leaves 0 .. P-1, the nodes level by level, the root's solver
+  const int f = s_role, top = a.base[a.depth];
   if (f < a.P)
     h6_leaf(a, f, sm6, s_h, s_gam);
-  else if (f <= a.base[a.depth])
+  else if (f <= top)
     h6_node(a, f, sm6, s_h, s_gam);
   else
     h6_root_solver(a, sm6);
+}
+
+__global__ void __launch_bounds__(kLeafThreads, 2) k_hr6_y(Hr4Args a) {
+  extern __shared__ double sm6[];
+  h6_y(a, (int)blockIdx.x, sm6);
+  // this grid ends after the tree's: what follows it in the stream follows both
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // The product of the Q blocks along the root-to-node path times U^-1, for
@@ -1174,13 +1425,11 @@ __global__ void __launch_bounds__(kLeafThreads) k_hr4_node_m(Hr4Args a, int lvl)
   const double* Mp = (lvl + 1 == a.depth) ? a.Uinv : a.Mn + (size_t)(a.base[lvl + 1] + nd) * nb2;
   double* Mo = a.Mn + (size_t)(a.base[lvl] + c) * nb2;
   double* sQ = sm4;
-  double* sM = sQ + nb2;
-  double* sO = sM + nb2;
+  double* sM = sQ + kBlk;
   if (h4_children(a, lvl + 1, nd) > 1) {
-    h4_load(sQ, a.Qn + ((size_t)(a.base[lvl + 1] + nd) * kFan + (c - nd * kFan)) * nb2, b, b);
-    h4_load(sM, Mp, b, b);
-    h5_mm(sQ, b, false, kSUpper, sM, b, false, kSUpper, sO, b, b, 1.0, nullptr);
-    for (int idx = tid; idx < b * b; idx += blockDim.x) Mo[idx] = sO[idx];
+    h4_load(sQ, a.Qn + ((size_t)(a.base[lvl + 1] + nd) * kFan + (c - nd * kFan)) * nb2, b);
+    h4_load(sM, Mp, b);
+    mm32(sQ, 1, kLd, kSUpper, sM, 1, kLd, kSUpper, Mo, b, b, 1.0, nullptr);
   } else {
     for (int idx = tid; idx < b * b; idx += blockDim.x) Mo[idx] = __ldcg(Mp + idx);
   }
@@ -1193,15 +1442,15 @@ __global__ void __launch_bounds__(kThreads) k_hr4_form_y(Hr4Args a) {
   const int64_t r0 = t4_leaf_row0(a.m, a.P, leaf);
   const int64_t r1 = t4_leaf_row0(a.m, a.P, leaf + 1);
   double* sM = sm4;
-  double* sX = sM + b * b;
-  double* sY = sX + b * b;
-  double* sT = sY + b * b;
+  double* sX = sM + kBlk;
+  double* sY = sX + kBlk;
+  double* sT = sY + kBlk;
   // the levels above 1 come from k_hr4_node_m when it ran (a.Mn)
   const int top = (a.Mn && a.depth >= 2) ? 1 : a.depth;
   if (top < a.depth)
-    h4_load(sM, a.Mn + (size_t)(a.base[1] + leaf / kFan) * b * b, b, b);
+    h4_load(sM, a.Mn + (size_t)(a.base[1] + leaf / kFan) * b * b, b);
   else
-    h4_load(sM, a.Uinv, b, b);
+    h4_load(sM, a.Uinv, b);
   for (int lvl = top; lvl >= 1; --lvl) {
     int nd = leaf;
     for (int l = 0; l < lvl; ++l) nd /= kFan;
@@ -1209,20 +1458,21 @@ __global__ void __launch_bounds__(kThreads) k_hr4_form_y(Hr4Args a) {
     for (int l = 0; l < lvl - 1; ++l) child /= kFan;
     if (h4_children(a, lvl, nd) > 1) {
       const int k = child - nd * kFan;
-      h4_load(sX, a.Qn + ((size_t)(a.base[lvl] + nd) * kFan + k) * b * b, b, b);
-      h5_mm(sX, b, false, kSUpper, sM, b, false, kSUpper, sY, b, b, 1.0, nullptr);
-      for (int idx = tid; idx < b * b; idx += blockDim.x) sM[idx] = sY[idx];
-      __syncthreads();
+      h4_load(sX, a.Qn + ((size_t)(a.base[lvl] + nd) * kFan + k) * b * b, b);
+      mm32(sX, 1, kLd, kSUpper, sM, 1, kLd, kSUpper, sY, kLd, up8(b), 1.0, nullptr);
+      double* t = sM;
+      sM = sY;
+      sY = t;
     }
   }
   // Z = T (V_top^T M);  Y = [M; 0] - V Z
-  for (int idx = tid; idx < b * b; idx += blockDim.x) {
-    const int r = idx % b, c = idx / b;
-    sY[idx] = (r > c) ? a.Vw[(int64_t)c * a.m + r0 + r] : (r == c ? 1.0 : 0.0);
+  for (int idx = tid; idx < kDirectB * kDirectB; idx += blockDim.x) {
+    const int r = idx & 31, c = idx >> 5;
+    sY[c * kLd + r] = (r < b && c < b) ? (r > c ? a.Vw[(int64_t)c * a.m + r0 + r] : (r == c ? 1.0 : 0.0)) : 0.0;
   }
-  h4_load(sT, a.Tl + (size_t)leaf * b * b, b, b);
-  h5_mm(sY, b, true, kSUnitUpper, sM, b, false, kSUpper, sX, b, b, 1.0, nullptr);   // sX = V_top^T M
-  h5_mm(sT, b, false, kSUpper, sX, b, false, kSUpper, sY, b, b, 1.0, nullptr);      // sY = Z = T sX
+  h4_load(sT, a.Tl + (size_t)leaf * b * b, b);
+  mm32(sY, kLd, 1, kSUpper, sM, 1, kLd, kSUpper, sX, kLd, up8(b), 1.0, nullptr);    // sX = V_top^T M
+  mm32(sT, 1, kLd, kSUpper, sX, 1, kLd, kSUpper, sY, kLd, up8(b), 1.0, nullptr);   // sY = Z = T sX
   // Z is upper triangular: Y[r][c] = M[r][c] - sum_{k<=c} V[r][k] Z[k][c], eight
   // columns at a time with independent accumulators (the loops unroll fully,
   // so the triangle is cut at compile time)
@@ -1238,13 +1488,13 @@ __global__ void __launch_bounds__(kThreads) k_hr4_form_y(Hr4Args a) {
       if (cb < b) {
         double acc[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) acc[u] = (rl < b && cb + u < b) ? sM[(cb + u) * b + rl] : 0.0;
+        for (int u = 0; u < 8; ++u) acc[u] = (rl < b && cb + u < b) ? sM[(cb + u) * kLd + rl] : 0.0;
 #pragma unroll
         for (int k = 0; k < cb + 8; ++k) {
 #pragma unroll
           for (int u = 0; u < 8; ++u)
             if (k <= cb + u) {
-              const double z = (cb + u < b) ? sY[(cb + u) * b + k] : 0.0;
+              const double z = (cb + u < b) ? sY[(cb + u) * kLd + k] : 0.0;
               acc[u] = fma(-v[k], z, acc[u]);
             }
         }
@@ -1293,6 +1543,11 @@ int hr_direct4(double* A, int64_t lda, int64_t m, int b, double* T, int64_t ldT,
   const bool pipe = g_pipe_tree && nnodes <= 4096;
   a.ldS = (int)std::max<int64_t>(32 * (slots <= 4 ? slots : kMaxR), pipe ? 0 : kFan * 32) + 1;
   if (a.ldS > 32 * kMaxR + 1) return CANDMC_ERR_ARG;
+  // Y beside the tree (k_hr6_y) while its CTAs find free SMs; with more of
+  // them than SMs the FP64 pipes bound the panel, and that form spends 1.8
+  // times the instructions of k_hr4_form_y
+  const int64_t yparts = (Lmax + kYRows - 1) / kYRows;
+  a.yparts = (pipe && P * yparts <= device_sms()) ? (int)yparts : 0;
   const size_t sm = sizeof(double) * std::max<size_t>({(size_t)a.ldS * kDirectB + 2 * kBlk + kLeafScratch,
                                                        (size_t)kNodeDoubles, (size_t)kRootDoubles});
   if (sm > 200 * 1024) return CANDMC_ERR_ARG;
@@ -1300,7 +1555,7 @@ int hr_direct4(double* A, int64_t lda, int64_t m, int b, double* T, int64_t ldT,
   // node R blocks (read before all their entries are written) lead it, so
   // one memset clears both
   // counters: cnt (last arriver) or prog + done + ticket + fail (pipelined)
-  const size_t ncnt = pipe ? 2 * (size_t)nnodes + 2 : (size_t)nnodes;
+  const size_t ncnt = pipe ? 2 * (size_t)nnodes + 3 : (size_t)nnodes;
   auto rup256 = [](size_t x) { return (x + 255) & ~(size_t)255; };
   const size_t o_cnt = 0;
   const size_t o_rn = o_cnt + rup256(sizeof(unsigned) * ncnt);
@@ -1326,8 +1581,8 @@ int hr_direct4(double* A, int64_t lda, int64_t m, int b, double* T, int64_t ldT,
   if (pipe) {
     a.prog = a.cnt;
     a.done = a.cnt + nnodes;
-    a.ticket = a.cnt + 2 * nnodes;
-    a.fail = reinterpret_cast<int*>(a.cnt + 2 * nnodes + 1);
+    a.ticket = a.cnt + 2 * nnodes + 1;
+    a.fail = reinterpret_cast<int*>(a.cnt + 2 * nnodes + 2);
     a.Pc = reinterpret_cast<double*>(base + o_pc);
   }
   a.T = T; a.ldT = ldT; a.W = W; a.ldW = ldW;
@@ -1339,6 +1594,7 @@ int hr_direct4(double* A, int64_t lda, int64_t m, int b, double* T, int64_t ldT,
     CANDMC_CK(cudaFuncSetAttribute(k_hr4_leaf_tree, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    200 * 1024));
     CANDMC_CK(cudaFuncSetAttribute(k_hr6_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CANDMC_CK(cudaFuncSetAttribute(k_hr6_y, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     attr = true;
   }
   {
@@ -1352,17 +1608,30 @@ int hr_direct4(double* A, int64_t lda, int64_t m, int b, double* T, int64_t ldT,
   if (node_m) {
     for (int lvl = a.depth - 1; lvl >= 1; --lvl) {
       ProfScope ps(CANDMC_KCLASS_PANEL_Y, 2.0 * a.nlev[lvl] * (double)nb2 * b / 3.0, s);
-      k_hr4_node_m<<<(unsigned)a.nlev[lvl], kLeafThreads, sizeof(double) * 3 * nb2, s>>>(a, lvl);
+      k_hr4_node_m<<<(unsigned)a.nlev[lvl], kLeafThreads, sizeof(double) * 2 * kBlk, s>>>(a, lvl);
       CANDMC_CK(cudaGetLastError());
     }
   }
-  {
+  if (a.yparts) {
+    ProfScope ps(CANDMC_KCLASS_PANEL_Y, 2.0 * m * b * b, s);
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3((unsigned)(P * a.yparts));
+    cfg.blockDim = dim3(kLeafThreads);
+    cfg.dynamicSmemBytes = sizeof(double) * kYDoubles;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CANDMC_CK(cudaLaunchKernelEx(&cfg, k_hr6_y, a));
+  } else {
     // with several waves of leaves, one thread per leaf row: leaves of at most
     // 128 rows take 128-thread CTAs, so two of them (252 registers a thread)
     // share an SM; a single wave keeps 256 threads for the path products
     const unsigned ythreads = (Lmax <= 128 && P >= kNodeMinLeaves) ? 128u : (unsigned)kThreads;
     ProfScope ps(CANDMC_KCLASS_PANEL_Y, 2.0 * m * b * b, s);
-    k_hr4_form_y<<<(unsigned)P, ythreads, sizeof(double) * 4 * nb2, s>>>(a);
+    k_hr4_form_y<<<(unsigned)P, ythreads, sizeof(double) * 4 * kBlk, s>>>(a);
   }
   CANDMC_CK(cudaGetLastError());
   return CANDMC_OK;
