@@ -205,37 +205,90 @@ k_reduce_apply(const double* Zp, int nsplit, int64_t split_stride, int nb, int n
   }
 }
 
-// Triangular inverse of an n x n matrix (ld), one column per thread.
-// lower != 0: lower triangular; unit != 0: unit diagonal implied.
-__global__ void k_tri_inv(const double* X, int64_t ldx, int n, int lower, int unit, double* Xi,
-                          int64_t ldi) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  double* col = Xi + (int64_t)j * ldi;
-  if (lower) {
-    for (int i = 0; i < n; ++i) {
-      double acc;
-      if (i < j) {
-        acc = 0.0;
-      } else {
-        acc = (i == j) ? 1.0 : 0.0;
-        for (int k = j; k < i; ++k) acc -= X[(int64_t)k * ldx + i] * col[k];
-        if (!unit) acc /= X[(int64_t)i * ldx + i];
-      }
-      col[i] = acc;
+// Triangular inverses: batch q inverts the n_q x n_q triangle at X + q xstep,
+// n_q = min(n, ntot - q n), into the n x n block Xi + q istep (zero outside the
+// triangle).  lower != 0: lower triangular, worked as the transpose of an upper
+// one; unit != 0: unit diagonal implied.
+// One warp per column of the inverse (four a CTA), blocked back substitution
+// with one row per lane: the CTA stages 32 x 32 blocks of the triangle (the
+// next one loads while this one is used), a block above the diagonal costs 32
+// FP64 instructions a column and a diagonal block, its columns divided by the
+// diagonal first, a chain of 32 shuffles and fmas.  Bound by those chains: 25 us
+// at n = 128, where a thread per column took 480 us (600 us for the diagonal
+// blocks of a least-squares R).
+constexpr int kTriWarps = 4;
+__global__ void __launch_bounds__(32 * kTriWarps)
+k_tri_inv(const double* X, int64_t ldx, int n, int64_t ntot, int64_t xstep, int lower, int unit, double* Xi,
+          int64_t ldi, int64_t istep) {
+  constexpr int ld = 33, per = 1024 / (32 * kTriWarps);
+  __shared__ double sU[32 * ld];
+  __shared__ double s_rd[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t q = blockIdx.y;
+  X += q * xstep;
+  Xi += q * istep;
+  const int nq = (int)(ntot - q * n < n ? ntot - q * n : n);
+  const int c = blockIdx.x * kTriWarps + warp, J = blockIdx.x * kTriWarps / 32;
+  const int64_t ri = lower ? ldi : 1, ci = lower ? 1 : ldi;     // strides of the upper view of Xi
+  // element (i, k) of the upper view of block (ib, kb); identity beyond nq
+  auto at = [&](int ib, int kb, int e) -> double {
+    const int i = 32 * ib + (lower ? e >> 5 : e & 31), k = 32 * kb + (lower ? e & 31 : e >> 5);
+    if (i < k && k < nq) return lower ? X[i * ldx + k] : X[k * ldx + i];
+    if (i == k) return (i < nq && !unit) ? X[i * ldx + i] : 1.0;
+    return 0.0;
+  };
+  double nxt[per];
+  auto fetch = [&](int ib, int kb) {
+#pragma unroll
+    for (int u = 0; u < per; ++u) nxt[u] = at(ib, kb, tid + 32 * kTriWarps * u);
+  };
+  auto stage = [&]() {
+#pragma unroll
+    for (int u = 0; u < per; ++u) {
+      const int e = tid + 32 * kTriWarps * u;
+      sU[lower ? (e & 31) * ld + (e >> 5) : (e >> 5) * ld + (e & 31)] = nxt[u];
     }
-  } else {
-    for (int i = n - 1; i >= 0; --i) {
-      double acc;
-      if (i > j) {
-        acc = 0.0;
-      } else {
-        acc = (i == j) ? 1.0 : 0.0;
-        for (int k = i + 1; k <= j; ++k) acc -= X[(int64_t)k * ldx + i] * col[k];
-        if (!unit) acc /= X[(int64_t)i * ldx + i];
+  };
+  if (c < n)
+    for (int i = 32 * (J + 1) + lane; i < n; i += 32) Xi[i * ri + c * ci] = 0.0;
+  fetch(J, J);
+  for (int ib = J; ib >= 0; --ib) {
+    const int i = 32 * ib + lane;
+    double r0 = (i == c && c < nq) ? 1.0 : 0.0, r1 = 0.0;
+    for (int kb = J; kb > ib; --kb) {
+      __syncthreads();
+      stage();
+      if (kb - 1 >= ib) fetch(ib, kb - 1);
+      __syncthreads();
+      const int kk = 32 * kb + lane;
+      const double x = (c < n && kk < n) ? Xi[kk * ri + c * ci] : 0.0;
+#pragma unroll 8
+      for (int k = 0; k < 32; k += 2) {
+        r0 = fma(-sU[k * ld + lane], __shfl_sync(0xffffffffu, x, k), r0);
+        r1 = fma(-sU[(k + 1) * ld + lane], __shfl_sync(0xffffffffu, x, k + 1), r1);
       }
-      col[i] = acc;
     }
+    __syncthreads();
+    stage();
+    if (ib > 0) fetch(ib - 1, J);
+    __syncthreads();
+    if (tid < 32) s_rd[tid] = 1.0 / sU[tid * ld + tid];
+    __syncthreads();
+    // columns k divided by U[k][k]: r_i -= (U[i][k] / U[k][k]) r_k, then x = r / diag
+#pragma unroll
+    for (int u = 0; u < per; ++u) {
+      const int e = tid + 32 * kTriWarps * u, k = e >> 5;
+      sU[k * ld + (e & 31)] *= s_rd[k];
+    }
+    __syncthreads();
+    double r = r0 + r1;
+#pragma unroll 8
+    for (int k = 31; k > 0; --k) {
+      const double rk = __shfl_sync(0xffffffffu, r, k);
+      if (lane < k) r = fma(-sU[k * ld + lane], rk, r);
+    }
+    if (c < n && i < n) Xi[i * ri + c * ci] = r * s_rd[lane];
+    __syncwarp();
   }
 }
 
@@ -406,8 +459,21 @@ int tri_inv(const double* X, int64_t ldx, int n, int lower, int unit, double* Xi
             cudaStream_t s) {
   if (n <= 0) return CANDMC_OK;
   ProfScope ps(CANDMC_KCLASS_SMALL, 0.0, s);
-  k_tri_inv<<<(n + 127) / 128, 128, 0, s>>>(X, ldx, n, lower, unit, Xi, ldi);
+  k_tri_inv<<<(n + kTriWarps - 1) / kTriWarps, 32 * kTriWarps, 0, s>>>(X, ldx, n, n, 0, lower, unit, Xi, ldi, 0);
   CANDMC_CK(cudaGetLastError());
+  return CANDMC_OK;
+}
+
+int diag_inv(const double* R, int64_t ldr, int64_t n, int w, double* Dinv, cudaStream_t s) {
+  const int64_t nblk = (n + w - 1) / w;
+  // grid rows are limited to 65535 blocks a launch
+  for (int64_t q = 0; q < nblk; q += 65535) {
+    const int64_t cnt = std::min<int64_t>(65535, nblk - q);
+    ProfScope ps(CANDMC_KCLASS_SMALL, 0.0, s);
+    k_tri_inv<<<dim3((w + kTriWarps - 1) / kTriWarps, (unsigned)cnt), 32 * kTriWarps, 0, s>>>(
+        R + q * w * (ldr + 1), ldr, w, n - q * w, w * (ldr + 1), 0, 0, Dinv + q * (int64_t)w * w, w, (int64_t)w * w);
+    CANDMC_CK(cudaGetLastError());
+  }
   return CANDMC_OK;
 }
 

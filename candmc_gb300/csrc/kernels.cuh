@@ -54,6 +54,9 @@ int gemm_nn_sub(double* C, int64_t ldc, MatRef Y, const double* Z, int64_t ldz, 
                 int64_t n, int nb, cudaStream_t s);
 int tri_inv(const double* X, int64_t ldx, int n, int lower, int unit, double* Xi, int64_t ldi,
             cudaStream_t s);
+// inverses of the w x w diagonal blocks of the upper triangle of R (n x n; the
+// last block may be smaller), w x w each, one after another
+int diag_inv(const double* R, int64_t ldr, int64_t n, int w, double* Dinv, cudaStream_t s);
 int materialize(MatRef X, int64_t n, int64_t k, double* out, int64_t ldo, cudaStream_t s);
 int set_identity(double* out, int64_t ld, int64_t n, int64_t k, cudaStream_t s);
 int invT_from_gram(const double* G, int64_t ldg, int b, double* T, int64_t ldt, cudaStream_t s);

@@ -148,26 +148,6 @@ __global__ void k_ts_reduce(const double* part, int nsplit, int64_t M, int64_t r
   out[c * ldo + i] = v;
 }
 
-// Inverses of the diagonal blocks of the upper triangle of R (w x w each; the
-// last block may be smaller), all blocks at once: block q, one column per thread.
-__global__ void k_diag_inv(const double* R, int64_t ldr, int64_t n, int w, double* Dinv) {
-  const int64_t q = blockIdx.x;
-  const int64_t j0 = q * w;
-  const int bw = (int)((n - j0 < w) ? n - j0 : w);
-  const int j = threadIdx.x;
-  double* col = Dinv + q * (int64_t)w * w + (int64_t)j * w;
-  if (j >= w) return;
-  for (int i = w - 1; i >= 0; --i) {
-    double acc = 0.0;
-    if (j < bw && i < bw && i <= j) {
-      acc = (i == j) ? 1.0 : 0.0;
-      for (int k = i + 1; k <= j; ++k) acc = fma(-R[(j0 + k) * ldr + j0 + i], col[k], acc);
-      acc /= R[(j0 + i) * ldr + j0 + i];
-    }
-    col[i] = acc;
-  }
-}
-
 __global__ void k_add(double* Z, int64_t ldz, const double* C, int64_t ldc, int64_t m, int64_t n) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= m * n) return;
@@ -272,7 +252,7 @@ static int ts_gemm(bool trans, const double* A, int64_t lda, const double* X, in
   return CANDMC_OK;
 }
 
-// X (n x r) <- op(R)^-1 X for the upper triangle of R (ld ldr); Dinv from k_diag_inv.
+// X (n x r) <- op(R)^-1 X for the upper triangle of R (ld ldr); Dinv from diag_inv.
 static int trsm_upper(const double* R, int64_t ldr, int64_t n, const double* Dinv, int w, double* X,
                       int64_t ldx, int64_t r, bool trans, cudaStream_t s) {
   const int64_t nblk = (n + w - 1) / w;
@@ -357,11 +337,7 @@ extern "C" int candmc_ls_solve(const double* A, int64_t lda, int64_t m, int64_t 
   // 3. X0 = R^-1 (Q^T B)[0:n]
   const int64_t nblk = (n + w - 1) / w;
   CANDMC_RET(Dinv.alloc(sizeof(double) * nblk * w * w, s));
-  {
-    ProfScope ps(CANDMC_KCLASS_SMALL, 0.0, s);
-    k_diag_inv<<<(unsigned)nblk, w, 0, s>>>(F.d(), m, n, w, Dinv.d());
-    CANDMC_CK(cudaGetLastError());
-  }
+  CANDMC_RET(diag_inv(F.d(), m, n, w, Dinv.d(), s));
   CANDMC_CK(cudaMemcpy2DAsync(X, sizeof(double) * ldx, Bq.p, sizeof(double) * m, sizeof(double) * n, nrhs,
                               cudaMemcpyDeviceToDevice, s));
   CANDMC_RET(trsm_upper(F.d(), m, n, Dinv.d(), w, X, ldx, nrhs, false, s));

@@ -1,0 +1,82 @@
+"""The triangular inverse at the edges of its 32-row blocks, and the FP64 <->
+float-pair conversions over the exponent range.
+
+Inverse: against numpy's solve in FP64 on triangles with a dominant diagonal
+(off-diagonal row sums at most half the diagonal), whose condition number is
+below 10: a substitution of length n carries at most about n rounding errors, so
+element-wise 4 n 2^-53 relative to the largest entry bounds both sides.
+
+Conversions: A <- A - Y Z with Y = [I; 0] and A's top rows zero leaves the rest
+of A as its float pair, fl(x) + fl(x - fl(x)), which numpy forms the same way:
+equal bits, not close ones.
+"""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def cm():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import candmc_gb300 as cm
+    cm.lib()
+    return cm
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a.T)).cuda().t()
+
+
+def triangle(n, lower, seed):
+    g = np.random.default_rng(seed)
+    X = g.uniform(-1, 1, (n, n)) / (2.0 * n)
+    X[np.diag_indices(n)] = g.uniform(0.5, 2.0, n) * np.where(g.random(n) < 0.5, -1.0, 1.0)
+    return np.tril(X) if lower else np.triu(X)
+
+
+@pytest.mark.parametrize("n", [1, 3, 31, 32, 33, 64, 100, 127, 128, 129, 255, 300])
+def test_triangular_inverse(cm, n):
+    tol = 4 * n * 2.0 ** -53
+    # upper: invT = -W^-T Y1
+    W, Y1 = triangle(n, False, n), triangle(n, True, n + 1)
+    got = cm.compute_invT_from_W(dev(W), dev(Y1)).cpu().numpy()
+    want = -np.linalg.solve(W.T, Y1)
+    assert np.abs(got - want).max() <= tol * np.abs(want).max()
+    if n > 256:
+        return
+    # lower and unit lower: A - Y T^T (Y^T A) with T^T = W^-1, and with T^T = -Y1^-1 W^T
+    g = np.random.default_rng(n + 2)
+    m = n + 40
+    Y = np.tril(g.uniform(-1, 1, (m, n)) / (2.0 * n), -1) + np.eye(m, n)
+    A = g.standard_normal((m, 5))
+    for lower, top in ((True, lambda W: np.linalg.inv(W)), (False, lambda W: -np.linalg.solve(Y[:n], W.T))):
+        W = triangle(n, lower, n + 3)
+        dA = dev(A)
+        cm.upd_A(dev(Y), dA, W=dev(W), W_is_T=lower)
+        want = A - Y @ (top(W) @ (Y.T @ A))
+        assert np.abs(dA.cpu().numpy() - want).max() <= 4 * (n + m) * 2.0 ** -53 * np.abs(want).max() * 4
+
+
+@pytest.mark.parametrize("m,n,ld", [(200, 3, 200), (2500, 70, 2501), (1024 + 128, 1, 1300)])
+@pytest.mark.parametrize("lo,hi", [(-10, 10), (-140, -60), (60, 120)])
+def test_float_pair_round_trip(cm, m, n, ld, lo, hi):
+    g = np.random.default_rng(m + n)
+    b = 64
+    x = np.ldexp(g.uniform(-1, 1, (m, n)), g.integers(lo, hi, (m, n)))
+    x[g.random((m, n)) < 0.05] = 0.0
+    x[b:b + 8] = np.ldexp(1.0, hi - 1) * np.array([1, -1, 1 + 2.0 ** -24, 1 - 2.0 ** -25, 2 - 2.0 ** -52,
+                                                   1 + 2.0 ** -52, 1 + 2.0 ** -23, -(2 - 2.0 ** -25)])[:, None]
+    x[:b] = 0.0
+    buf = torch.zeros(n, ld, dtype=torch.float64, device="cuda")
+    A = buf.t()[:m]
+    A.copy_(torch.from_numpy(x).cuda())
+    cm.upd_A(dev(np.eye(m, b)), A, precision="ozaki")
+    with np.errstate(under="ignore"):
+        h = x.astype(np.float32)
+        l = (x - h.astype(np.float64)).astype(np.float32)
+    want = h.astype(np.float64) + l.astype(np.float64)
+    assert np.array_equal(A.cpu().numpy(), want)
+    assert not buf.t()[m:].any()
