@@ -308,7 +308,8 @@ int qr_2d_pipe_dev(double* A, int64_t lda, int64_t m, int64_t k, int64_t b, int*
       t_oz_cap = saved;
       t_leaf_rows = saved_leaf;
     }
-  } cap_scope(g_oz_reserve_sms > 0 ? std::max(1, device_sms() - g_oz_reserve_sms) : 0, g_pipe_leaf_rows);
+  } cap_scope(g_oz_reserve_sms > 0 ? std::max(1, device_sms() - g_oz_reserve_sms) : 0,
+              g_pipe_leaf_rows > 0 ? g_pipe_leaf_rows : 128);
   cudaStream_t sp = panel_stream();
   if (!sp) return set_error(CANDMC_ERR_CUDA, "could not create the lookahead stream");
   EventRing evs;

@@ -40,14 +40,13 @@ namespace candmc {
 constexpr int kFan = 4;
 
 // Target rows per TSQR leaf (tuning knob, candmc_set_tuning("leaf_rows", v));
-// 0: kLeafRows, or 256 for panels of kTallPanelRows rows or more.
+// 0: chosen by the panel's height (hr_direct4).
 int64_t g_leaf_rows = 0;
 // Leaf height of latency-bound panels.  A leaf's step is bound by the FP64
-// pipe from 128 rows on; below, by its chain and reductions, so shorter leaves
-// only add nodes: 8192 x 64 takes 670 us with 128-row leaves, 795 with 64 rows
-// and 809 with 256.
+// pipe from 128 rows on; below, by its chain.  8192 x 32 takes 194 us with
+// 128-row leaves, 240 with 64 rows (its CTAs share SMs) and 252 with 256.
 constexpr int64_t kLeafRows = 128;
-int64_t g_pipe_leaf_rows = 128;
+int64_t g_pipe_leaf_rows = 0;   // the lookahead's panels (knob "pipe_leaf_rows"); 0: as without it
 thread_local int64_t t_leaf_rows = 0;
 // Pipelined tree on/off (tuning knob, candmc_set_tuning("pipe_tree", 0|1)).
 int g_pipe_tree = 1;
@@ -89,7 +88,7 @@ __device__ __forceinline__ int64_t t4_leaf_row0(int64_t m, int P, int i) {
 __device__ __forceinline__ int warp_id() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
 
 constexpr int kLeafThreads = 288;   // 9 warps: the critical one, 6 for the columns, 2 for memory
-constexpr int kPollWarp = 4;        // sub-partition 0: waits for the children's columns
+constexpr int kPollWarp = 4;        // sub-partition 0: waits for the children's columns; a column warp in leaves
 constexpr int kPubWarp = 8;         // sub-partition 0: publishes finished columns
 constexpr int kBulkWarps = 6;       // warps 1-3 and 5-7
 constexpr int kLd = kDirectB + 1;   // leading dimension of the 32 x 32 shared blocks
@@ -101,10 +100,28 @@ constexpr int kNodeMinLeaves = 256;
 // with 128-row leaves; 262144 x 32: 1866 against 2361)
 constexpr int64_t kTallPanelRows = 32768;
 
-// Index 0..5 of a column warp (1-3, 5-7), or -1.
+// Index 0..5 of a column warp (1-3, 5-7), 6 for the seventh warp of a leaf (4,
+// beside the critical one), or -1.
 __device__ __forceinline__ int bulk_index(int warp) {
-  return (warp >= 1 && warp <= 3) ? warp - 1 : (warp >= 5 && warp <= 7) ? warp - 2 : -1;
+  return (warp >= 1 && warp <= 3) ? warp - 1 : (warp >= 5 && warp <= 7) ? warp - 2 : warp == kPollWarp ? 6 : -1;
 }
+
+// The columns of a block over its warps.  While many columns are left, the six
+// column warps bound a step and the critical warp's sub-partition has time to
+// spare, so warp 6 takes the columns 4, 9, 14 and 19, which are finished before
+// the chain bounds the steps; the other 28, in order, go round the six
+// (slot i = q + 6 k of warp q).
+__device__ __forceinline__ int leaf_col(int q, int k) {
+  const int i = q + kBulkWarps * k, g = i >> 2;
+  return q == kBulkWarps ? (k < 4 ? 5 * k + 4 : kDirectB) : i + (g < 4 ? g : 4);
+}
+// the first k with leaf_col(q, k) >= c
+__device__ __forceinline__ int leaf_first(int q, int c) {
+  if (q == kBulkWarps) return c / 5;
+  const int g = c / 5, i = c - (g < 4 ? g : 4) - q;   // slots of the columns before c
+  return i > 0 ? (i + kBulkWarps - 1) / kBulkWarps : 0;
+}
+constexpr int kLeafCols = 5;   // most columns of a warp
 
 // Sums over the warp of N values per lane (N a power of two): lanes
 // k (32 / N) .. (k + 1) (32 / N) - 1 return sum number k.  Halving the values
@@ -125,6 +142,21 @@ __device__ __forceinline__ double warp_sum_held(double (&d)[N]) {
 #pragma unroll
   for (; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   return s;
+}
+
+// barrier `id` of n threads (a multiple of 32)
+__device__ __forceinline__ void named_bar(int id, int n) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+
+// Polls of a shared-memory flag before a wait gives up.
+constexpr long kSmemSpin = 1L << 22;
+constexpr int kStepThreads = 7 * 32;   // the critical warp and the six column warps of a node
+constexpr int kLeafStepThreads = 8 * 32;   // those of a leaf, with the seventh
+constexpr int kStepBar = 3;            // their barrier, one per column step
+constexpr int kGamBar = 4;             // the critical warp arrives when gamma is written, the others wait
+__device__ __forceinline__ void bar_arrive(int id, int n) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 
 __device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
@@ -156,8 +188,9 @@ __device__ __forceinline__ double quick_rcp(double x) {
 // sqrt(q) as q r (1 + e/2 + 3 e^2/8) with e = 1 - q r^2 (the series' next
 // term is below 2^-62), h = alpha + sign(alpha) sigma, gamma = 1 / (q + |alpha|
 // sigma).  Both seeds come from q and alpha in FP32, side by side.
-// q within 2^+-60, alpha^2 <= q.
-__device__ __forceinline__ void h7_scalars(double alpha, double q, double* sigma, double* gam) {
+// q within 2^+-60, alpha^2 <= q.  gamma is left as its seed and denominator
+// (refine_gamma): nothing needs it before the next dot product is summed.
+__device__ __forceinline__ void h7_scalars(double alpha, double q, double* sigma, double* seed, double* den) {
   const float qf = f32_of(q);
   const float rf = rsqrtf(qf);
   const float af = hi_abs(alpha) < ((1023 - 90) << 20) ? 0.0f : f32_of(fabs(alpha));
@@ -168,31 +201,56 @@ __device__ __forceinline__ void h7_scalars(double alpha, double q, double* sigma
   const double te = t * e;
   const double p = fma(0.375, e, 0.5);
   const double sg = fma(te, p, t);
-  const double den = fma(fabs(alpha), sg, q);
-  const double e1 = fma(-den, g0, 1.0);
   *sigma = sg;
-  *gam = fma(g0, fma(e1, e1, e1), g0);
+  *seed = g0;
+  *den = fma(fabs(alpha), sg, q);
 }
 
-// One step of the critical warp: column j of S receives reflector j - 1 (in v
-// and gam, kept from the last step) and becomes reflector j.  Lane l owns the
-// rows l + 32 t.  Leaf: head row j, tail rows j + 1 and on.  NODE: head row j
-// of child 0, tail = the rows of the other children (zero below their
-// diagonals).  Writes beta to row j, the unnormalised tail below it, the
-// head to s_h[j] and gamma to s_gam[j].
+// 1 / den from its seed (one third-order step; seed exact when den = 1 / seed)
+__device__ __forceinline__ double refine_gamma(double seed, double den) {
+  const double e = fma(-den, seed, 1.0);
+  return fma(seed, fma(e, e, e), seed);
+}
+
+// State of the critical warp between steps: reflector v, and its gamma as seed
+// and denominator.
+template <int R>
+struct Crit {
+  double v[R];
+  double seed, den;
+};
+
+// One step of the critical warp: column j of S receives reflector j - 1 (kept
+// from the last step) and becomes reflector j.  Lane l owns the rows l + 32 t.
+// Leaf: head row j, tail rows j + 1 and on.  NODE: head row j of child 0, tail
+// = the rows of the other children (zero below their diagonals).  Writes beta
+// to row j, the unnormalised tail below it and the head to s_h[j].  gamma_(j-1)
+// is refined here, beside the dot product, written to s_gam[j - 1] and
+// announced on barrier kGamBar, where the column warps wait for it after their
+// own dot products: the step barrier need not wait for it.
 template <int R, bool NODE>
-__device__ __forceinline__ void h7_crit(double* S, int ld, int j, double (&v)[R], double& gam, double* s_h,
-                                        double* s_gam) {
+__device__ __forceinline__ void h7_crit(double* S, int ld, int j, Crit<R>& cr, double* s_h, double* s_gam,
+                                        int nthreads) {
   const int lane = threadIdx.x & 31;
+  double (&v)[R] = cr.v;
   double* col = S + (size_t)j * ld;
   double x[R];
 #pragma unroll
   for (int t = 0; t < R; ++t) x[t] = col[lane + 32 * t];
   if (j > 0) {
-    double d = v[0] * x[0];
+    double d0 = v[0] * x[0], d1 = R > 1 ? v[1 % R] * x[1 % R] : 0.0;
+    const double e = fma(-cr.den, cr.seed, 1.0);
 #pragma unroll
-    for (int t = 1; t < R; ++t) d = fma(v[t], x[t], d);
-    const double f = gam * warp_sum(d);
+    for (int t = 2; t < R; ++t) {
+      if (t & 1) d1 = fma(v[t], x[t], d1);
+      else d0 = fma(v[t], x[t], d0);
+    }
+    const double e2 = fma(e, e, e);
+    if (R > 1) d0 += d1;
+    const double gam = fma(cr.seed, e2, cr.seed);
+    if (lane == 0) s_gam[j - 1] = gam;
+    bar_arrive(kGamBar, nthreads);
+    const double f = gam * warp_sum(d0);
 #pragma unroll
     for (int t = 0; t < R; ++t) x[t] = fma(-f, v[t], x[t]);
   }
@@ -209,14 +267,15 @@ __device__ __forceinline__ void h7_crit(double* S, int ld, int j, double (&v)[R]
   double h, beta;
   if (!__any_sync(0xffffffffu, nz != 0)) {   // an empty tail: a sign flip
     h = 1.0;
-    gam = 2.0;
+    cr.seed = 2.0;
+    cr.den = 0.5;
     beta = flip_if(alpha, true);
   } else {
     const int qh = __double2hiint(q);
     const bool neg = __double2hiint(alpha) < 0;
     if (qh >= ((1023 - 60) << 20) && qh < ((1023 + 60) << 20)) {
       double sigma;
-      h7_scalars(alpha, q, &sigma, &gam);
+      h7_scalars(alpha, q, &sigma, &cr.seed, &cr.den);
       h = alpha + flip_if(sigma, neg);
       beta = flip_if(sigma, !neg);
     } else {
@@ -240,7 +299,8 @@ __device__ __forceinline__ void h7_crit(double* S, int ld, int j, double (&v)[R]
       qs = warp_sum(qs);
       const double sigma = sqrt(qs);
       h = as + flip_if(sigma, neg);
-      gam = 1.0 / fma(fabs(as), sigma, qs);
+      cr.den = fma(fabs(as), sigma, qs);
+      cr.seed = 1.0 / cr.den;
       beta = flip_if(sigma, !neg) * un;
     }
   }
@@ -250,43 +310,45 @@ __device__ __forceinline__ void h7_crit(double* S, int ld, int j, double (&v)[R]
   v[0] = lane == j ? h : (tail0 ? x[0] : 0.0);
 #pragma unroll
   for (int t = 1; t < R; ++t) v[t] = x[t];
-  if (lane == 0) {
-    s_h[j] = h;
-    s_gam[j] = gam;
-  }
+  if (lane == 0) s_h[j] = h;
 }
 
-// Reflector (v, gam) applied to the columns c = q + 6 k, k0 <= k < 6, with
-// c_lo <= c < b, by one warp.
+// Reflector v with *gam applied to this warp's columns k0 <= k < kLeafCols with
+// c_lo <= leaf_col(q, k) < b (*gam is there after barrier kGamBar).
 template <int R, int N>
 __device__ __forceinline__ void h7_apply(double* S, int ld, int b, int q, int k0, int c_lo, const double (&v)[R],
-                                         double gam) {
-  constexpr int NC = N < kBulkWarps ? N : kBulkWarps;
+                                         const double* gam) {
+  constexpr int NC = N < kLeafCols ? N : kLeafCols;
   constexpr bool keep = R <= 3;   // the columns stay in registers between their dot product and update
   const int lane = threadIdx.x & 31;
   double d[N];
   double xs[NC][keep ? R : 1];
+  int cs[NC];
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     d[k] = 0.0;
-    const int c = q + kBulkWarps * (k0 + k);
-    if (k < NC && c >= c_lo && c < b) {
-      const double* sc = S + (size_t)c * ld;
+    if (k < NC) {
+      const int c = leaf_col(q, k0 + k);
+      cs[k < NC ? k : 0] = (c >= c_lo && c < b && k0 + k < kLeafCols) ? c : -1;
+      if (cs[k < NC ? k : 0] >= 0) {
+        const double* sc = S + (size_t)c * ld;
 #pragma unroll
-      for (int t = 0; t < R; ++t) {
-        const double x = sc[lane + 32 * t];
-        if constexpr (keep) xs[k < NC ? k : 0][t] = x;
-        d[k] = fma(v[t], x, d[k]);
+        for (int t = 0; t < R; ++t) {
+          const double x = sc[lane + 32 * t];
+          if constexpr (keep) xs[k < NC ? k : 0][t] = x;
+          d[k] = fma(v[t], x, d[k]);
+        }
       }
     }
   }
-  const double f = gam * warp_sum_held<N>(d);
+  const double sum = warp_sum_held<N>(d);
+  named_bar(kGamBar, kLeafStepThreads);
+  const double f = *gam * sum;
 #pragma unroll
   for (int k = 0; k < NC; ++k) {
-    const int c = q + kBulkWarps * (k0 + k);
     const double fk = __shfl_sync(0xffffffffu, f, k * (32 / N));
-    if (c >= c_lo && c < b) {
-      double* sc = S + (size_t)c * ld;
+    if (cs[k] >= 0) {
+      double* sc = S + (size_t)cs[k] * ld;
       double x[R];
 #pragma unroll
       for (int t = 0; t < R; ++t) {
@@ -300,45 +362,56 @@ __device__ __forceinline__ void h7_apply(double* S, int ld, int b, int q, int k0
 }
 
 struct NoPublish {
-  __device__ void operator()(const double*, int, int) const {}
+  __device__ void all(const double*, int, int, volatile int*, volatile int*) const {}
 };
 
 // Householder QR of S (b columns, ld >= 32 R, rows beyond the data zero); all
 // kLeafThreads threads call it after S is filled.  Afterwards S holds R (upper
 // triangle) and the unnormalised tails, s_h the heads, s_gam the gammas.
 // Step j: the critical warp finishes column j (see h7_crit) while the column
-// warps apply reflector j - 1 to the columns after j and the publishing warp
-// hands column j - 1 of R to the parent; one block barrier per step.
+// warps apply reflector j - 1 to the columns after j; one barrier of those
+// seven warps per step.  The publishing warp follows the count of finished
+// columns on its own, so that its fences (about 1 us) hold nobody up.
 template <int R, bool NODE, class Pub = NoPublish>
-__device__ void h7_factor(double* S, int ld, int b, double* s_h, double* s_gam, Pub pub = Pub()) {
+__device__ void h7_factor(double* S, int ld, int b, double* s_h, double* s_gam, volatile int* s_done,
+                          Pub pub = Pub()) {
   const int lane = threadIdx.x & 31, warp = warp_id();
   const int q = bulk_index(warp);
-  double v[R], gam = 0.0;
+  if (threadIdx.x == 0) *s_done = 0;
+  __syncthreads();
+  if (warp == 0 || q >= 0) {
+    Crit<R> cr;
+    double (&v)[R] = cr.v;
+    cr.seed = cr.den = 0.0;
 #pragma unroll
-  for (int t = 0; t < R; ++t) v[t] = 0.0;
-  for (int j = 0; j < b; ++j) {
-    __syncthreads();
-    if (warp == 0) {
-      h7_crit<R, NODE>(S, ld, j, v, gam, s_h, s_gam);
-    } else if (j > 0 && q >= 0) {
-      const double* vj = S + (size_t)(j - 1) * ld;
-      const double h = s_h[j - 1];
+    for (int t = 0; t < R; ++t) v[t] = 0.0;
+    for (int j = 0; j < b; ++j) {
+      named_bar(kStepBar, kLeafStepThreads);
+      if (warp == 0) {
+        h7_crit<R, NODE>(S, ld, j, cr, s_h, s_gam, kLeafStepThreads);
+        __threadfence_block();
+        __syncwarp();
+        if (lane == 0) *s_done = j + 1;
+      } else if (j > 0) {
+        const double* vj = S + (size_t)(j - 1) * ld;
+        const double h = s_h[j - 1];
 #pragma unroll
-      for (int t = 0; t < R; ++t) v[t] = vj[lane + 32 * t];
-      v[0] = lane == j - 1 ? h : (!NODE && lane > j - 1 ? v[0] : 0.0);
-      gam = s_gam[j - 1];
-      // this warp's columns from j + 1 on are its last n
-      const int klo = j + 1 > q ? (j + 1 - q + kBulkWarps - 1) / kBulkWarps : 0;
-      if (klo >= 5) h7_apply<R, 1>(S, ld, b, q, 5, j + 1, v, gam);
-      else if (klo == 4) h7_apply<R, 2>(S, ld, b, q, 4, j + 1, v, gam);
-      else if (klo >= 2) h7_apply<R, 4>(S, ld, b, q, 2, j + 1, v, gam);
-      else h7_apply<R, 8>(S, ld, b, q, 0, j + 1, v, gam);
-    } else if (j > 0 && warp == kPubWarp) {
-      pub(S, ld, j - 1);
+        for (int t = 0; t < R; ++t) v[t] = vj[lane + 32 * t];
+        v[0] = lane == j - 1 ? h : (!NODE && lane > j - 1 ? v[0] : 0.0);
+        const double* gam = s_gam + j - 1;
+        // this warp's columns from j + 1 on are its last ones
+        const int klo = leaf_first(q, j + 1);
+        if (klo >= 4) h7_apply<R, 1>(S, ld, b, q, 4, j + 1, v, gam);
+        else if (klo == 3) h7_apply<R, 2>(S, ld, b, q, 3, j + 1, v, gam);
+        else if (klo >= 1) h7_apply<R, 4>(S, ld, b, q, 1, j + 1, v, gam);
+        else h7_apply<R, 8>(S, ld, b, q, 0, j + 1, v, gam);
+      }
     }
+    if (warp == 0 && lane == 0) s_gam[b - 1] = refine_gamma(cr.seed, cr.den);
+  } else if (warp == kPubWarp) {
+    pub.all(S, ld, b, s_done, nullptr);
   }
   __syncthreads();
-  if (warp == kPubWarp) pub(S, ld, b - 1);
 }
 
 // Structure of an operand of mm32, on op(X).  The zeros (and unit diagonals)
@@ -416,34 +489,51 @@ __device__ __forceinline__ int up8(int b) { return (b + 7) & ~7; }
 // two small products computed in parallel, so the dependent FP64 chain is
 // about 2 (1 + 2 + 4 + 8 + 16) operations instead of the b^2 / 2 of a
 // substitution.  scratch: 512 doubles.
+template <int H>
+__device__ __forceinline__ void h4_tri_level(const double* X, double* Xi, double* scratch) {
+  constexpr int n = kDirectB / 2 * H;   // elements of the level's off-diagonal blocks
+  constexpr int step = H < 8 ? H : 8;
+  const int idx = threadIdx.x;
+  const int p = idx / (H * H), e = idx % (H * H), i = e % H, j = e / H, i0 = p * 2 * H, c0 = i0 + H;
+  double a0 = 0.0, a1 = 0.0;
+  if (idx < n) {   // M = B C^-1 (C^-1 upper: zero below its diagonal)
+#pragma unroll 1
+    for (int k = 0; k <= j; k += step)
+#pragma unroll
+      for (int u = 0; u < step; ++u) {
+        const double t = X[(c0 + k + u) * kLd + i0 + i], w = Xi[(c0 + j) * kLd + c0 + k + u];
+        if (u & 1) a1 = fma(t, w, a1);
+        else a0 = fma(t, w, a0);
+      }
+    scratch[idx] = a0 + a1;
+  }
+  __syncthreads();
+  if (idx < n) {   // -A^-1 M
+    a0 = a1 = 0.0;
+#pragma unroll 1
+    for (int k = i & ~(step - 1); k < H; k += step)
+#pragma unroll
+      for (int u = 0; u < step; ++u) {
+        const double t = Xi[(i0 + k + u) * kLd + i0 + i], w = scratch[p * H * H + j * H + k + u];
+        if (u & 1) a1 = fma(t, w, a1);
+        else a0 = fma(t, w, a0);
+      }
+    Xi[(c0 + j) * kLd + i0 + i] = -(a0 + a1);
+  }
+  __syncthreads();
+}
+
 __device__ void h4_tri_inv(const double* X, double* Xi, double* scratch) {
-  constexpr int bp = kDirectB;
-  for (int idx = threadIdx.x; idx < bp * bp; idx += blockDim.x) {
-    const int i = idx % bp, k = idx / bp;
+  for (int idx = threadIdx.x; idx < kDirectB * kDirectB; idx += blockDim.x) {
+    const int i = idx & 31, k = idx >> 5;
     Xi[k * kLd + i] = i == k ? quick_rcp(X[i * kLd + i]) : 0.0;
   }
   __syncthreads();
-  for (int h = 1; h < bp; h <<= 1) {
-    const int npair = bp / (2 * h);
-    // M = B C^-1 (h x h per pair)
-    for (int idx = threadIdx.x; idx < npair * h * h; idx += blockDim.x) {
-      const int p = idx / (h * h), e = idx % (h * h), i = e % h, j = e / h;
-      const int i0 = p * 2 * h, c0 = i0 + h;
-      double acc = 0.0;
-      for (int k = 0; k <= j; ++k) acc = fma(X[(c0 + k) * kLd + i0 + i], Xi[(c0 + j) * kLd + c0 + k], acc);
-      scratch[p * h * h + e] = acc;
-    }
-    __syncthreads();
-    // top-right block = -A^-1 M
-    for (int idx = threadIdx.x; idx < npair * h * h; idx += blockDim.x) {
-      const int p = idx / (h * h), e = idx % (h * h), i = e % h, j = e / h;
-      const int i0 = p * 2 * h, c0 = i0 + h;
-      double acc = 0.0;
-      for (int k = i; k < h; ++k) acc = fma(Xi[(i0 + k) * kLd + i0 + i], scratch[p * h * h + j * h + k], acc);
-      Xi[(c0 + j) * kLd + i0 + i] = -acc;
-    }
-    __syncthreads();
-  }
+  h4_tri_level<1>(X, Xi, scratch);
+  h4_tri_level<2>(X, Xi, scratch);
+  h4_tri_level<4>(X, Xi, scratch);
+  h4_tri_level<8>(X, Xi, scratch);
+  h4_tri_level<16>(X, Xi, scratch);
 }
 
 // b x b block from global memory (ld b) into a shared block (ld kLd), zero beyond b
@@ -586,14 +676,8 @@ __device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// barrier `id` of n threads (a multiple of 32)
-__device__ __forceinline__ void named_bar(int id, int n) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
-}
-
 constexpr int kBlk = kDirectB * kLd;        // doubles of a 32 x 32 shared block
 constexpr int kRootDoubles = 6 * kBlk;
-constexpr long kSmemSpin = 1L << 22;        // polls of a shared-memory flag
 
 // The root: Q1_top, its sign-choice LU, T, W and U^-1.  The LU runs with a
 // one-column lookahead: warp 0 applies column i to column i + 1 and finishes
@@ -810,12 +894,13 @@ __device__ __forceinline__ int h7_slots(int L) {
 
 template <class Pub>
 __device__ void h7_leaf_factor(double* S, int ldS, int slots, int b, double* s_h, double* s_gam, Pub pub) {
+  __shared__ volatile int s_done;
   switch (slots) {
-    case 1: h7_factor<1, false>(S, ldS, b, s_h, s_gam, pub); break;
-    case 2: h7_factor<2, false>(S, ldS, b, s_h, s_gam, pub); break;
-    case 3: h7_factor<3, false>(S, ldS, b, s_h, s_gam, pub); break;
-    case 4: h7_factor<4, false>(S, ldS, b, s_h, s_gam, pub); break;
-    default: h7_factor<kMaxR, false>(S, ldS, b, s_h, s_gam, pub); break;
+    case 1: h7_factor<1, false>(S, ldS, b, s_h, s_gam, &s_done, pub); break;
+    case 2: h7_factor<2, false>(S, ldS, b, s_h, s_gam, &s_done, pub); break;
+    case 3: h7_factor<3, false>(S, ldS, b, s_h, s_gam, &s_done, pub); break;
+    case 4: h7_factor<4, false>(S, ldS, b, s_h, s_gam, &s_done, pub); break;
+    default: h7_factor<kMaxR, false>(S, ldS, b, s_h, s_gam, &s_done, pub); break;
   }
 }
 
@@ -827,6 +912,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2) k_hr4_leaf_tree(Hr4Args a) {
   extern __shared__ double sm4[];
   __shared__ double s_h[kDirectB], s_gam[kDirectB];
   __shared__ int s_last;
+  __shared__ volatile int s_done;
   const int b = a.b, tid = threadIdx.x;
   const int leaf = blockIdx.x;
   const int64_t r0 = t4_leaf_row0(a.m, a.P, leaf);
@@ -882,7 +968,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2) k_hr4_leaf_tree(Hr4Args a) {
     }
     // reflector j: head row j (child 0), tail = rows 0..j of every other child
     // (the children are upper triangular, so nothing below their diagonals is touched)
-    h7_factor<kFan, true>(S, ldS, b, s_h, s_gam);
+    h7_factor<kFan, true>(S, ldS, b, s_h, s_gam, &s_done);
     for (int idx = tid; idx < b * b; idx += blockDim.x) {
       const int r = idx % b, c = idx / b;
       Rpar[idx] = (r <= c) ? S[c * ldS + r] : 0.0;
@@ -956,16 +1042,25 @@ __device__ void h6_release_all(const Hr4Args& a, int f) {
   }
 }
 
-// Column j of R (rows 0..j of S's column j) handed to the parent by one warp.
+// R handed to the parent column by column (rows 0..j of S's column j) as the
+// count *s_done of finished columns grows, by one warp.  Stops when *s_fail
+// (may be nullptr) is set.
 struct Publish {
   double* Rcol;
   int b;
   unsigned* prog;
-  __device__ void operator()(const double* S, int ld, int j) const {
+  __device__ void all(const double* S, int ld, int n, volatile int* s_done, volatile int* s_fail) const {
     const int lane = threadIdx.x & 31;
-    if (lane <= j) Rcol[j * b + lane] = S[j * ld + lane];
-    __syncwarp();   // orders the lanes' stores before lane 0's release
-    if (lane == 0) st_release(prog, (unsigned)(j + 1));
+    for (int j = 0; j < n; ++j) {
+      long it = 0;
+      while (*s_done <= j && ++it < kSmemSpin && !(s_fail && *s_fail)) __nanosleep(20);
+      __syncwarp();
+      if (*s_done <= j) return;   // the CTA releases its flags itself
+      __threadfence_block();
+      if (lane <= j) Rcol[j * b + lane] = S[j * ld + lane];
+      __syncwarp();   // orders the lanes' stores before lane 0's release
+      if (lane == 0) st_release(prog, (unsigned)(j + 1));
+    }
   }
 };
 
@@ -1001,30 +1096,71 @@ __device__ void h6_leaf(const Hr4Args& a, int leaf, double* sm, double* s_h, dou
     if (leaf == 0) st_release(a.prog + 0, (unsigned)b + 1u);
     st_release(a.done + leaf, 1u);
   }
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 constexpr int kNodeLd = kFan * 32 + 1;   // child k at rows [32 k, 32 k + b)
-constexpr int kNodeDoubles = kNodeLd * kDirectB + 4 * kBlk + 4 * 96;
+constexpr int kNodeDoubles = kNodeLd * kDirectB + 4 * kBlk + 4 * 96 + 2 * 32;
+
+// One warp's triangular matrix-vector product: lane l < n returns the sum over
+// t <= l of x(l, t) y(l, t).  Row l has l + 1 terms, so rows l and n - 1 - l
+// together have n + 1: the longer one keeps its first h = (n + 2) / 2 terms and
+// the lane of the shorter one takes the rest after its own, which halves the
+// FP64 instructions of a loop over t <= l with idle lanes (17 instead of 31 at
+// n = 31).  Terms outside load as zero: a divergent branch per term cost more
+// than the fma (150 cycles a term instead of 76).
+template <class X, class Y>
+__device__ __forceinline__ double tri_fold(int n, X x, Y y) {
+  const int lane = threadIdx.x & 31;
+  const int mirror = n - 1 - lane, h = (n + 2) >> 1;
+  const bool big = 2 * lane > n - 1;
+  const int sw = (big || lane + 1 >= h) ? 64 : lane + 1;   // from here on the lane helps row `mirror`
+  double acc = 0.0, own = 0.0;
+  for (int t0 = 0; t0 < h; t0 += 4) {
+    double xv[4], yv[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int t = t0 + u;
+      const int l = t >= sw ? mirror : lane, q = t >= sw ? h + t - sw : t;
+      const bool in = t < h && lane < n && q <= l;
+      xv[u] = in ? x(l, q) : 0.0;
+      yv[u] = in ? y(l, q) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (t0 + u == sw) {
+        own = acc;
+        acc = 0.0;
+      }
+      acc = fma(xv[u], yv[u], acc);
+    }
+  }
+  const bool helped = sw < 64;
+  const double rest = __shfl_sync(0xffffffffu, helped ? acc : 0.0, mirror & 31);
+  return big ? acc + rest : (helped ? own : acc);
+}
 
 // An internal node.  V = [D; V_1; V_2; V_3] with the reflectors unnormalised
 // (D = diag(h)) and T of that form (T_pp = gamma_p).  Step j, between two
-// block barriers:
+// barriers of the critical and the column warps:
 //  * warp 0 applies reflector j - 1 to column j and forms reflector j;
 //  * warps 1-3, one per child, apply the reflectors before j to column j + 1:
 //    z = V^T s with one reflector per lane (no reduction over lanes), w = T^T z
-//    with the columns of T the last step knew and w_(j-1) = gamma_(j-1)
-//    (z_(j-1) - (T y)^T z), s -= V w with one row per lane;
+//    with the columns of T the last step knew, s -= V w with one row per lane;
 //  * warps 5-7, one per child, form column j - 1 of T: y = V^T v_(j-1),
-//    T[0:j-1, j-1] = -gamma_(j-1) T y;
-//  * the polling warp fetches column j + 2 of the children, and the publishing
-//    warp hands column j - 1 to the parent.
-// Bound: the FP64 pipes of the three sub-partitions with the column warps
-// (about 130 instructions a step at j = 31, 8.5 k cycles; half that on
-// average) against 13 k cycles a step when one warp group did all of it in
-// sequence with seven block barriers.
+//    T[0:j-1, j-1] = -gamma_(j-1) T y, and the last entry of w, gamma_(j-1)
+//    (z_(j-1) - (T y)^T z), while warps 1-3 apply the others;
+//  * the polling warp fetches the children's columns as they appear, and the
+//    publishing warp hands finished columns to the parent, both at their own
+//    pace (a fence or a trip to L2 takes about as long as a short step).
+// V_k is upper triangular, so z, y and V w run folded (tri_fold).
+// Bound: the FP64 pipes of the three sub-partitions with the column warps,
+// about 92 instructions a step at j = 31 and half that on average (131 with
+// the triangles unfolded: 122 us for 32 columns whose leaves take 79).
 __device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_h, double* s_gam) {
   const int b = a.b, tid = threadIdx.x, lane = tid & 31, warp = warp_id();
   __shared__ int s_okv[2];
+  __shared__ volatile int s_done, s_got, s_fail;   // columns finished, fetched; the poller gave up
   int lvl = 1;
   while (lvl < a.depth && f >= a.base[lvl + 1]) ++lvl;
   const int idx = f - a.base[lvl];
@@ -1041,6 +1177,8 @@ __device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_h, double
   double* yp = zp + 96;
   double* wp = yp + 96;
   double* tp = wp + 96;
+  double* zs = tp + 96;       // z, and w of the last reflector
+  double* wl = zs + 32;
   if (nch == 1) {   // a pass-through node: its R is its child's
     if (warp == 0) {
       bool ok = true;
@@ -1063,6 +1201,7 @@ __device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_h, double
   } else {
     for (int i = tid; i < ld * kDirectB; i += blockDim.x) S[i] = 0.0;
     for (int i = tid; i < kBlk; i += blockDim.x) Tn[i] = 0.0;
+    if (tid == 0) s_done = s_got = s_fail = 0;
     __syncthreads();
     const Publish pub{Rme, b, a.prog + f};
     // column c of the children's R into S (polling warp: lane k waits for child k)
@@ -1078,11 +1217,6 @@ __device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_h, double
       for (int k = 0; k < kFan; ++k) S[c * ld + 32 * k + lane] = t[k];
       return true;
     };
-    if (warp == kPollWarp) {
-      bool ok = fetch(0);
-      if (ok && b > 1) ok = fetch(1);
-      if (lane == 0) s_okv[0] = ok;
-    }
     const int kc = warp & 3;                 // the child of a column warp: 1..3
     const bool tgrp = warp >= 5 && warp <= 7;
     const bool cgrp = warp >= 1 && warp <= 3;
@@ -1093,81 +1227,133 @@ __device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_h, double
       const bool live = kc < nch;
       double acc = 0.0;
       if (tgrp) {
-        if (live && lane < n - 1) {
-#pragma unroll 4
-          for (int r = 0; r < n - 1; ++r) acc = fma(Vk[lane * ld + r], Vk[(n - 1) * ld + r], acc);
-        }
+        if (live)
+          acc = tri_fold(n - 1, [&](int p, int r) { return Vk[p * ld + r]; }, [&](int, int r) { return Vk[(n - 1) * ld + r]; });
         yp[(kc - 1) * 32 + lane] = acc;
       } else {
-        if (live && c < b && lane < n) {
-#pragma unroll 4
-          for (int r = 0; r < n; ++r) acc = fma(Vk[lane * ld + r], Vk[c * ld + r], acc);
-        }
+        if (live && c < b)
+          acc = tri_fold(n, [&](int p, int r) { return Vk[p * ld + r]; }, [&](int, int r) { return Vk[c * ld + r]; });
         zp[(kc - 1) * 32 + lane] = acc;
       }
       named_bar(1, kBulkWarps * 32);
+      // the sums over the children; then this warp's third of T y or T^T z
+      // (columns beyond what is known are zero in Tn)
       double z = 0.0;
+      acc = 0.0;
       if (tgrp) {
         const double y = (yp[lane] + yp[32 + lane]) + yp[64 + lane];
-        acc = 0.0;
-        for (int q = kc - 1; q < n - 1; q += 3) acc = fma(Tn[q * kLd + lane], __shfl_sync(0xffffffffu, y, q), acc);
+        for (int q = kc - 1; q < n - 1; q += 12) {
+          double t[4], w[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int k = q + 3 * u;
+            t[u] = k < n - 1 ? Tn[k * kLd + lane] : 0.0;
+            w[u] = __shfl_sync(0xffffffffu, y, k & 31);
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (q + 3 * u < n - 1) acc = fma(t[u], w[u], acc);
+        }
         tp[(kc - 1) * 32 + lane] = acc;
       } else if (c < b) {
         if (lane < n) z = fma(s_h[lane], S[c * ld + lane], (zp[lane] + zp[32 + lane]) + zp[64 + lane]);
-        acc = 0.0;
-        for (int p = kc - 1; p < n - 1; p += 3) {
-          const double zq = __shfl_sync(0xffffffffu, z, p);
-          acc = fma(lane < n - 1 ? Tn[lane * kLd + p] : 0.0, zq, acc);
+        if (kc == 1) zs[lane] = z;
+        for (int q = kc - 1; q < n - 1; q += 12) {
+          double t[4], w[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int k = q + 3 * u;
+            t[u] = (k < n - 1 && lane < n - 1) ? Tn[lane * kLd + k] : 0.0;
+            w[u] = __shfl_sync(0xffffffffu, z, k & 31);
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (q + 3 * u < n - 1) acc = fma(t[u], w[u], acc);
         }
         wp[(kc - 1) * 32 + lane] = acc;
       }
       named_bar(1, kBulkWarps * 32);
-      const double g = s_gam[n - 1];
+      if (n < b) named_bar(kGamBar, kStepThreads);
       if (tgrp) {
+        const double g = s_gam[n - 1];
+        const double t = (tp[lane] + tp[32 + lane]) + tp[64 + lane];
         if (kc == 1) {
-          const double t = (tp[lane] + tp[32 + lane]) + tp[64 + lane];
           if (lane < n) Tn[(n - 1) * kLd + lane] = lane < n - 1 ? -g * t : g;
+        } else if (kc == 2 && c < b) {
+          // w_(n-1) = gamma (z_(n-1) - (T y)^T z), while warps 1-3 work on the rest
+          const double u = warp_sum(lane < n - 1 ? t * zs[lane] : 0.0);
+          if (lane == 0) *wl = g * (zs[n - 1] - u);
+          named_bar(2, 4 * 32);
         }
       } else if (c < b) {
-        const double t = lane < n - 1 ? ((tp[lane] + tp[32 + lane]) + tp[64 + lane]) * z : 0.0;
-        const double u = warp_sum(t);
-        const double zl = __shfl_sync(0xffffffffu, z, n - 1);
-        double w = (wp[lane] + wp[32 + lane]) + wp[64 + lane];
-        if (lane >= n - 1) w = lane == n - 1 ? g * (zl - u) : 0.0;
-        if (live) {
-          acc = 0.0;
-#pragma unroll 4
-          for (int p = 0; p < n; ++p) acc = fma(Vk[p * ld + lane], __shfl_sync(0xffffffffu, w, p), acc);
-          if (lane < n) S[c * ld + 32 * kc + lane] -= acc;
-        }
-        if (kc == 1 && lane < n) S[c * ld + lane] = fma(-s_h[lane], w, S[c * ld + lane]);
+        // s -= V w: row r = n - 2 - l takes the reflectors p = n - 2 - t >= r,
+        // then reflector n - 1 everywhere
+        const double w = lane < n - 1 ? (wp[lane] + wp[32 + lane]) + wp[64 + lane] : 0.0;
+        double* ws = zp + (kc - 1) * 32;   // the partial z of this warp's child is done
+        ws[lane] = w;
+        __syncwarp();
+        acc = tri_fold(n - 1, [&](int l, int t) { return Vk[(n - 2 - t) * ld + n - 2 - l]; },
+                       [&](int, int t) { return ws[n - 2 - t]; });
+        // to row order: lane l has row n - 2 - l
+        acc = __shfl_sync(0xffffffffu, acc, (n - 2 - lane) & 31);
+        if (lane >= n - 1) acc = 0.0;
+        named_bar(2, 4 * 32);
+        const double wn = *wl;
+        if (live && lane < n) S[c * ld + 32 * kc + lane] -= fma(Vk[(n - 1) * ld + lane], wn, acc);
+        if (kc == 1 && lane < n) S[c * ld + lane] = fma(-s_h[lane], lane == n - 1 ? wn : w, S[c * ld + lane]);
       }
     };
-    double v[kFan], gam = 0.0;
+    if (warp == 0 || tgrp || cgrp) {
+      Crit<kFan> cr;
+      cr.seed = cr.den = 0.0;
 #pragma unroll
-    for (int t = 0; t < kFan; ++t) v[t] = 0.0;
-    for (int j = 0; j < b; ++j) {
-      __syncthreads();
-      if (!s_okv[j & 1]) {   // written before this barrier, rewritten two barriers on
-        h6_release_all(a, f);
-        return;
+      for (int t = 0; t < kFan; ++t) cr.v[t] = 0.0;
+      for (int j = 0; j < b; ++j) {
+        if (warp == 0) {
+          // columns up to j + 1 must have arrived
+          const int need = j + 2 < b ? j + 2 : b;
+          long it = 0;
+          while (s_got < need && !s_fail && ++it < kSmemSpin) {
+          }
+          __syncwarp();
+          if (lane == 0) s_okv[j & 1] = s_got >= need;
+          __threadfence_block();
+        }
+        named_bar(kStepBar, kStepThreads);
+        if (!s_okv[j & 1]) {   // written before this barrier, rewritten two barriers on
+          s_fail = 1;
+          break;
+        }
+        if (warp == 0) {
+          h7_crit<kFan, true>(S, ld, j, cr, s_h, s_gam, kStepThreads);
+          __threadfence_block();
+          __syncwarp();
+          if (lane == 0) s_done = j + 1;
+        } else if (j > 0) {
+          bulk(j, j + 1);
+        }
       }
-      if (warp == 0) {
-        h7_crit<kFan, true>(S, ld, j, v, gam, s_h, s_gam);
-      } else if (warp == kPollWarp) {
-        bool ok = true;
-        if (j + 2 < b) ok = fetch(j + 2);
-        if (lane == 0) s_okv[(j + 1) & 1] = ok;
-      } else if (warp == kPubWarp) {
-        if (j > 0) pub(S, ld, j - 1);
-      } else if (j > 0 && (tgrp || cgrp)) {
-        bulk(j, j + 1);
+      if (warp == 0 && lane == 0) s_gam[b - 1] = refine_gamma(cr.seed, cr.den);
+      named_bar(kStepBar, kStepThreads);
+      if (warp != 0 && !s_fail) bulk(b, b);
+    } else if (warp == kPollWarp) {
+      for (int c = 0; c < b; ++c) {
+        if (!fetch(c)) {
+          s_fail = 1;
+          break;
+        }
+        __threadfence_block();
+        __syncwarp();
+        if (lane == 0) s_got = c + 1;
       }
+    } else {
+      pub.all(S, ld, b, &s_done, &s_fail);
     }
     __syncthreads();
-    if (warp == kPubWarp) pub(S, ld, b - 1);
-    if (tgrp || cgrp) bulk(b, b);
-    __syncthreads();
+    if (s_fail) {
+      h6_release_all(a, f);
+      return;
+    }
     // T of normalised heads: Tn = T D (for Q_k = -V_k T D), Qk = D T D (Q_1 = I - D T D)
     for (int i = tid; i < kDirectB * kDirectB; i += blockDim.x) {
       const int r = i & 31, c = i >> 5;
@@ -1391,8 +1577,10 @@ __global__ void __launch_bounds__(kLeafThreads, 2) k_hr6_pipe(Hr4Args a) {
   __shared__ int s_role;
   if (threadIdx.x == 0) s_role = (int)atomicAdd(a.ticket, 1u);
   __syncthreads();
-  // the Y kernel (k_hr6_y) may start once every CTA of this grid is here
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // The Y kernel (k_hr6_y) may start once every CTA of this grid has started
+  // and the leaves are done: their SMs are then free, one for each of its CTAs
+  // (started with the tree, its CTAs shared SMs and took 20 us for 10).
+  if (s_role >= a.P) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // flat tree id: leaves 0 .. P-1, the nodes level by level, the root's solver
   const int f = s_role, top = a.base[a.depth];
   if (f < a.P)
@@ -1513,6 +1701,10 @@ int hr_direct4(double* A, int64_t lda, int64_t m, int b, double* T, int64_t ldT,
   // tall panels (throughput, not the latency of one leaf, sets the time) take
   // 256-row leaves unless the knob asks for a height
   if ((t_leaf_rows > 0 || g_leaf_rows == 0) && m >= kTallPanelRows) want = std::max<int64_t>(want, 256);
+  // short panels take 64-row leaves while leaves, nodes and the CTAs of Y have
+  // an SM each (2048 x 32: 178 us against 196, 512 x 32: 165 against 187)
+  const int64_t p64 = (m + 63) / 64;
+  if ((t_leaf_rows > 0 ? g_pipe_leaf_rows == 0 : g_leaf_rows == 0) && 2 * p64 + p64 / 3 + 4 <= device_sms()) want = 64;
   const int64_t leaf_rows = std::max<int64_t>(32, std::min<int64_t>(want, 256));
   // leaves of at most leaf_rows rows and at least b rows
   int64_t P = std::max<int64_t>(1, std::min<int64_t>((m + leaf_rows - 1) / leaf_rows, m / b));
