@@ -7,9 +7,10 @@
 // gemm_tn owns a slice of rows and writes a partial Z, and reduce_apply sums
 // the partials in a fixed order and multiplies by T^T in the same pass.
 //
-// GB300 note: FP64 runs at ~1.2 TFLOP/s chip-wide (about 2 DFMA/clk/SM), so
-// these kernels are bound by the FP64 pipe, not by HBM (a 64x64 tile with
-// 4x4 register blocking needs only 8 shared loads per 16 DFMA).
+// GB300 note: FP64 runs at ~1.2 TFLOP/s chip-wide (a warp-wide FP64 instruction
+// takes 65 cycles of its sub-partition), so these kernels are bound by the
+// number of FP64 instructions: tiles that fit the product's odd widths count
+// for more than operand reuse.
 #include <algorithm>
 
 #include "common.cuh"
@@ -17,18 +18,20 @@
 
 namespace candmc {
 
-constexpr int TK = 16;
-
-// out(i, j) = sum_{k in [k0, k1)} opA(i, k) * opB(k, j), a (16 U) x (16 U)
-// tile per CTA (U = 4: 64 x 64; U = 2: 32 x 32 for the narrow products
-// inside a panel, where a 64 x 64 tile would be three quarters padding).
+// ---- products of up to kSmallProduct multiplications: out(i, j) = sum_{k in
+// [k0, k1)} opA(i, k) * opB(k, j), a 16 x 16 tile per CTA, one output a thread.
+// Many small CTAs spread such a product over the SMs and run little code once
+// (1500 x 32 x 32: 9 us against 11 and 20 in the two kernels below; 8192 x 32 x
+// 32: 20 against 27 and 40); from 8192 x 64 x 64 on the others are ahead.
 // mode 0: store into out + split * split_stride (partials), ld ldo.
 // mode 1: out(i, j) -= result (out is the trailing matrix itself).
-template <int U>
+constexpr int TK = 16;
+constexpr int64_t kSmallProduct = 20000000;
+
 __global__ void __launch_bounds__(kThreads)
 k_gemm_f64(MatRef A, MatRef B, int64_t M, int64_t N, int64_t K, int64_t kchunk, double* out,
            int64_t ldo, int64_t split_stride, int mode) {
-  constexpr int TM = 16 * U, TN = 16 * U;
+  constexpr int U = 1, TM = 16, TN = 16;
   __shared__ double sA[TK][TM + 1];
   __shared__ double sB[TK][TN + 1];
   const int tid = threadIdx.x;
@@ -82,6 +85,280 @@ k_gemm_f64(MatRef A, MatRef B, int64_t M, int64_t N, int64_t K, int64_t kchunk, 
       if (gj >= N) continue;
       if (mode == 0) o[gj * ldo + gi] = acc[u][v];
       else o[gj * ldo + gi] -= acc[u][v];
+    }
+  }
+}
+
+// An operand as element (i, j) = p[i si + j sj] with its mask as what to keep by
+// the sign of d = +-(i - j) - off: mat_at with its transposition and mask worked
+// out once, in a dozen instructions an element.  These kernels are short, and
+// code that runs once costs about 30 cycles an instruction to fetch: with
+// mat_at's switch inlined per load, a product of 8192 x 32 x 32 took 45 us.
+struct View {
+  const double* p;
+  int64_t si, sj, off;
+  int sgn;
+  bool pos, zero, neg, unit;   // keep d > 0, d == 0, d < 0; d == 0 reads as one
+};
+
+__device__ __forceinline__ View make_view(const MatRef& X) {
+  View v;
+  v.p = X.p;
+  v.si = X.trans ? X.ld : 1;
+  v.sj = X.trans ? 1 : X.ld;
+  v.off = X.off;
+  v.sgn = X.trans ? -1 : 1;
+  v.pos = X.mask != kUpper;
+  v.neg = X.mask == kUpper || X.mask == kDense;
+  v.unit = X.mask == kUnitLower;
+  v.zero = !v.unit;
+  return v;
+}
+
+__device__ __forceinline__ double view_at(const View& v, int64_t i, int64_t j, bool in) {
+  const int64_t d = v.sgn * (i - j) - v.off;
+  const bool keep = in && (d > 0 ? v.pos : d < 0 ? v.neg : v.zero);
+  const double x = keep ? v.p[i * v.si + j * v.sj] : 0.0;
+  return (in && d == 0 && v.unit) ? 1.0 : x;
+}
+
+// ---- Y^T C, split over rows
+//
+// out + z split_stride, (nb x n, ld nb) = sum over the rows of chunk z of
+// Y(k, i) C(k, j).  A CTA takes up to 64 x (16 CG) outputs in 8 x 4 lane blocks
+// (lane l: row l % 8, column l / 8 of a block), so a product 50 wide pads to 56
+// x 52 and not to 64 x 64.  CG warps share the columns (blocks g, g + CG, ..,
+// at most four each), the 8 / CG groups of them the rows of a stage, 32 at a
+// time through shared memory with the next stage's loads in flight.  The
+// groups' sums meet in shared memory at the end.
+constexpr int kTnK = 32;              // rows per stage
+constexpr int kTnLd = kTnK + 1;
+
+// The sizes are compiled in: a guarded FP64 instruction is predicated, and one
+// whose predicate is off for the whole warp still takes its 65 cycles.
+template <int NU, int NV, int KG>
+__device__ __forceinline__ void tn_stage(const double* sA, const double* sB, int kg, int kn, int bstep,
+                                         double (&acc)[8][4]) {
+#pragma unroll 1
+  for (int k = kg; k < kn; k += KG) {
+    double x[NU], y[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) y[v] = sB[v * bstep + k];
+#pragma unroll
+    for (int u = 0; u < NU; ++u) x[u] = sA[8 * u * kTnLd + k];
+#pragma unroll
+    for (int u = 0; u < NU; ++u)
+#pragma unroll
+      for (int v = 0; v < NV; ++v) acc[u][v] = fma(x[u], y[v], acc[u][v]);
+  }
+}
+
+template <int NV, int KG>
+__device__ __forceinline__ void tn_rows(int nu, const double* sA, const double* sB, int kg, int kn, int bstep,
+                                        double (&acc)[8][4]) {
+  switch (nu) {
+    case 1: tn_stage<1, NV, KG>(sA, sB, kg, kn, bstep, acc); break;
+    case 2: tn_stage<2, NV, KG>(sA, sB, kg, kn, bstep, acc); break;
+    case 3: tn_stage<3, NV, KG>(sA, sB, kg, kn, bstep, acc); break;
+    case 4: tn_stage<4, NV, KG>(sA, sB, kg, kn, bstep, acc); break;
+    case 5: tn_stage<5, NV, KG>(sA, sB, kg, kn, bstep, acc); break;
+    case 6: tn_stage<6, NV, KG>(sA, sB, kg, kn, bstep, acc); break;
+    case 7: tn_stage<7, NV, KG>(sA, sB, kg, kn, bstep, acc); break;
+    default: tn_stage<8, NV, KG>(sA, sB, kg, kn, bstep, acc); break;
+  }
+}
+
+template <int CG>
+__global__ void __launch_bounds__(kThreads, 2)
+k_gemm_tn(MatRef Y, MatRef C, int64_t m, int nb, int64_t n, int rt, int ct, int64_t kchunk, double* out,
+          int64_t split_stride) {
+  constexpr int KG = 8 / CG;
+  __shared__ double sm[2 * 64 * kTnLd];
+  double* sA = sm;                  // [column of Y][row], ld kTnLd
+  double* sB = sm + 64 * kTnLd;     // [column of C][row]
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  // the two groups of CG = 4 pair column groups of different width on a sub-partition
+  const int kg = warp / CG, g = (warp + 2 * kg) % CG;
+  const int i0 = (int)blockIdx.x * rt;
+  const int64_t j0 = (int64_t)blockIdx.y * ct;
+  const int ni = nb - i0 < rt ? nb - i0 : rt;
+  const int nj = (int)(n - j0 < ct ? n - j0 : ct);
+  const int nu = (ni + 7) >> 3;
+  const int nv = ((nj + 3) / 4 - g + CG - 1) / CG;   // column blocks of this warp
+  const int64_t k0 = (int64_t)blockIdx.z * kchunk;
+  const int64_t k1 = (k0 + kchunk < m) ? k0 + kchunk : m;
+  double acc[8][4];
+#pragma unroll
+  for (int u = 0; u < 8; ++u)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) acc[u][v] = 0.0;
+  // element e of a stage: row kb + e % 32 of column e / 32; eight per thread and operand
+  double pa[8], pb[8];
+  const int kr = tid & 31, c0 = tid >> 5;
+  const View vy = make_view(Y), vc = make_view(C);
+  auto fetch = [&](int64_t kb) {
+    const bool row = kb + kr < k1;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) pa[u] = view_at(vy, kb + kr, i0 + c0 + 8 * u, row && c0 + 8 * u < ni);
+#pragma unroll
+    for (int u = 0; u < 2 * CG; ++u) pb[u] = view_at(vc, kb + kr, j0 + c0 + 8 * u, row && c0 + 8 * u < nj);
+  };
+  fetch(k0);
+  const double* wa = sA + (lane & 7) * kTnLd;
+  const double* wb = sB + (4 * g + (lane >> 3)) * kTnLd;
+  constexpr int bstep = 4 * CG * kTnLd;
+  for (int64_t kb = k0; kb < k1; kb += kTnK) {
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 8; ++u) sA[(c0 + 8 * u) * kTnLd + kr] = pa[u];
+#pragma unroll
+    for (int u = 0; u < 2 * CG; ++u) sB[(c0 + 8 * u) * kTnLd + kr] = pb[u];
+    __syncthreads();
+    if (kb + kTnK < k1) fetch(kb + kTnK);
+    const int kn = (int)(k1 - kb < kTnK ? k1 - kb : kTnK);
+    switch (nv) {
+      case 4: tn_rows<4, KG>(nu, wa, wb, kg, kn, bstep, acc); break;
+      case 3: tn_rows<3, KG>(nu, wa, wb, kg, kn, bstep, acc); break;
+      case 2: tn_rows<2, KG>(nu, wa, wb, kg, kn, bstep, acc); break;
+      case 1: tn_rows<1, KG>(nu, wa, wb, kg, kn, bstep, acc); break;
+      default: break;
+    }
+  }
+  // the groups' sums: the upper half of the groups hands its to the lower half
+  constexpr int slot = 64 * 16 * CG;
+#pragma unroll
+  for (int h = KG / 2; h >= 1; h >>= 1) {
+    __syncthreads();
+    if (kg >= h && kg < 2 * h) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          if (u < nu) sm[(kg - h) * slot + ((u * 4 + v) * CG + g) * 32 + lane] = acc[u][v];
+    }
+    __syncthreads();
+    if (kg < h) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (u >= nu) break;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) acc[u][v] += sm[kg * slot + ((u * 4 + v) * CG + g) * 32 + lane];
+      }
+    }
+  }
+  if (kg == 0) {
+    double* o = out + (int64_t)blockIdx.z * split_stride;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const int i = 8 * u + (lane & 7), j = 4 * (v * CG + g) + (lane >> 3);
+        if (i < ni && j < nj) o[(j0 + j) * nb + i0 + i] = acc[u][v];
+      }
+  }
+}
+
+// ---- C -= Y Z
+//
+// C (m x n, ldc) -= opY (m x nb) Z (nb x n, ldz): one row per lane, NC columns
+// in registers, Z broadcast from shared memory (64 rows of it at a time) and Y
+// read straight from memory, coalesced over the lanes, a few columns ahead.
+// Rows and columns pad to 32 and 4.
+constexpr int kNnK = 64;
+constexpr int kNnThreads = 128;   // one warp per sub-partition: small products spread over the SMs
+
+// One row's share of a stage for the first 4 NQ of NC columns; y holds the first
+// PF columns of Y.
+template <int NC, int NQ, int PF>
+__device__ __forceinline__ void nn_stage(const View& vy, int64_t r, bool in, int kb, int kn, const double (*sZ)[NC],
+                                         double (&y)[PF], double (&acc)[NC]) {
+#pragma unroll 1
+  for (int k = 0; k < kn; k += PF) {   // rows of sZ beyond kn are zero
+    double x[PF];
+#pragma unroll
+    for (int u = 0; u < PF; ++u) x[u] = y[u];
+#pragma unroll
+    for (int u = 0; u < PF; ++u) y[u] = view_at(vy, r, kb + k + PF + u, in && k + PF + u < kn);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+#pragma unroll
+      for (int u = 0; u < PF; ++u) {
+        const double2 z0 = *reinterpret_cast<const double2*>(&sZ[k + u][4 * q]);
+        const double2 z1 = *reinterpret_cast<const double2*>(&sZ[k + u][4 * q + 2]);
+        acc[4 * q] = fma(x[u], z0.x, acc[4 * q]);
+        acc[4 * q + 1] = fma(x[u], z0.y, acc[4 * q + 1]);
+        acc[4 * q + 2] = fma(x[u], z1.x, acc[4 * q + 2]);
+        acc[4 * q + 3] = fma(x[u], z1.y, acc[4 * q + 3]);
+      }
+    }
+  }
+}
+
+template <int NC>
+__global__ void __launch_bounds__(kNnThreads)
+k_gemm_nn_sub(double* C, int64_t ldc, MatRef Y, MatRef Z, int64_t m, int64_t n, int nb) {
+  constexpr int PF = NC >= 16 ? 4 : 8;             // columns of Y in flight: about 1000 cycles of FP64 work
+  constexpr int per = kNnK * NC / kNnThreads;      // elements of a stage of Z per thread
+  constexpr bool early = NC <= 16;                 // C's elements load before the products
+  __shared__ __align__(16) double sZ[kNnK][NC];
+  const int64_t r = (int64_t)blockIdx.x * kNnThreads + threadIdx.x;
+  const int64_t j0 = (int64_t)blockIdx.y * NC;
+  const int nj = (int)(n - j0 < NC ? n - j0 : NC);
+  const bool in = r < m;
+  const View vy = make_view(Y);
+  double* c = C + j0 * ldc + r;
+  double acc[NC], old[early ? NC : 1];
+#pragma unroll
+  for (int v = 0; v < NC; ++v) {
+    acc[v] = 0.0;
+    if constexpr (early) old[v] = (in && v < nj) ? c[v * ldc] : 0.0;
+  }
+  for (int kb = 0; kb < nb; kb += kNnK) {
+    const int kn = nb - kb < kNnK ? nb - kb : kNnK;
+    double y[PF], z[per];
+#pragma unroll
+    for (int u = 0; u < per; ++u) {
+      const int e = threadIdx.x + kNnThreads * u, k = e % kNnK, j = e / kNnK;
+      z[u] = (k < kn && j < nj) ? Z.p[(j0 + j) * Z.ld + kb + k] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < PF; ++u) y[u] = view_at(vy, r, kb + u, in && u < kn);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < per; ++u) {
+      const int e = threadIdx.x + kNnThreads * u;
+      sZ[e % kNnK][e / kNnK] = z[u];
+    }
+    __syncthreads();
+    constexpr int Q = NC / 4;
+    switch ((nj + 3) >> 2) {
+      case 1: nn_stage<NC, 1, PF>(vy, r, in, kb, kn, sZ, y, acc); break;
+      case 2: nn_stage<NC, (Q < 2 ? Q : 2), PF>(vy, r, in, kb, kn, sZ, y, acc); break;
+      case 3: nn_stage<NC, (Q < 3 ? Q : 3), PF>(vy, r, in, kb, kn, sZ, y, acc); break;
+      case 4: nn_stage<NC, (Q < 4 ? Q : 4), PF>(vy, r, in, kb, kn, sZ, y, acc); break;
+      case 5: nn_stage<NC, (Q < 5 ? Q : 5), PF>(vy, r, in, kb, kn, sZ, y, acc); break;
+      case 6: nn_stage<NC, (Q < 6 ? Q : 6), PF>(vy, r, in, kb, kn, sZ, y, acc); break;
+      case 7: nn_stage<NC, (Q < 7 ? Q : 7), PF>(vy, r, in, kb, kn, sZ, y, acc); break;
+      default: nn_stage<NC, Q, PF>(vy, r, in, kb, kn, sZ, y, acc); break;
+    }
+  }
+  if (in) {
+    if constexpr (early) {
+#pragma unroll
+      for (int v = 0; v < NC; ++v)
+        if (v < nj) c[v * ldc] = old[v] - acc[v];
+    } else {
+#pragma unroll
+      for (int v0 = 0; v0 < NC; v0 += 8) {
+        if (v0 >= nj) break;
+        double t[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) t[u] = v0 + u < nj ? c[(v0 + u) * ldc] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (v0 + u < nj) c[(v0 + u) * ldc] = t[u] - acc[v0 + u];
+      }
     }
   }
 }
@@ -342,35 +619,36 @@ int small_gemm(int64_t M, int64_t N, int64_t K, double alpha, MatRef A, MatRef B
   return CANDMC_OK;
 }
 
-// Tile width 16 U of the FP64 products (U = 4, 2, 1): the widest tile whose
-// grid still gives every SM work and that is not much wider than the product
-// (a product with a single right-hand side takes 16 x 16 tiles).  Each CTA's FP64 work is serial on its SM
-// (about 2 DFMA/clk), so a narrow product (a panel's own b/2-wide updates,
-// with 64 x 64 outputs or fewer) on a handful of 64 x 64 tiles leaves most of
-// the GPU idle and takes ~60 us; the same product on 16 x 16 tiles spreads
-// over the whole chip.
-static int tile_u(int64_t M, int64_t N, int64_t kparts) {
-  const int64_t want = 2 * (int64_t)num_sms();
-  const int64_t narrow = std::min(M, N);   // no tile much wider than the product itself
-  for (int U : {4, 2}) {
-    if (16 * U > 2 * std::max<int64_t>(narrow, 8)) continue;
-    const int64_t t = ((M + 16 * U - 1) / (16 * U)) * ((N + 16 * U - 1) / (16 * U));
-    if (t * kparts >= want) return U;
+// Z = alpha opT (sum of the nsplit partial products)
+static int reduce_apply(const double* part, int64_t nsplit, int64_t stride, int nb, int64_t n, MatRef Top,
+                        double alpha, double* Z, int64_t ldz, cudaStream_t s) {
+  int nbp = 1;
+  while (nbp < nb) nbp <<= 1;
+  ProfScope ps(CANDMC_KCLASS_REDUCE, 8.0 * stride * nsplit, s);
+  k_reduce_apply<<<(unsigned)n, kThreads, 0, s>>>(part, (int)nsplit, stride, nb, nbp, n, Top, alpha, Z, ldz);
+  CANDMC_CK(cudaGetLastError());
+  return CANDMC_OK;
+}
+
+static int small_tn(MatRef Y, MatRef C, int64_t m, int nb, int64_t n, MatRef Top, double alpha, double* Z,
+                    int64_t ldz, cudaStream_t s) {
+  // about 4 CTAs per SM over slices of TK rows or more
+  const int64_t tiles = (int64_t)((nb + 15) / 16) * ((n + 15) / 16), target = 4 * (int64_t)num_sms();
+  int64_t nsplit = std::max<int64_t>(1, std::min<int64_t>((target + tiles - 1) / tiles, (m + TK - 1) / TK));
+  const int64_t kchunk = ((m + nsplit - 1) / nsplit + TK - 1) / TK * TK;
+  nsplit = std::max<int64_t>(1, (m + kchunk - 1) / kchunk);
+  const int64_t stride = (int64_t)nb * n;
+  DevBuf part;
+  CANDMC_RET(part.alloc(sizeof(double) * (size_t)stride * nsplit, s));
+  MatRef Yt = Y;
+  Yt.trans = !Y.trans;   // element (i, r) of Y^T is Y(r, i)
+  {
+    ProfScope ps(CANDMC_KCLASS_GEMM_TN, 2.0 * nb * n * m, s);
+    const dim3 grid((unsigned)((nb + 15) / 16), (unsigned)((n + 15) / 16), (unsigned)nsplit);
+    k_gemm_f64<<<grid, kThreads, 0, s>>>(Yt, C, nb, n, m, kchunk, part.d(), nb, stride, 0);
   }
-  return 1;
-}
-
-template <int U>
-static void launch_gemm(dim3 grid, MatRef A, MatRef B, int64_t M, int64_t N, int64_t K, int64_t kchunk,
-                        double* out, int64_t ldo, int64_t stride, int mode, cudaStream_t s) {
-  k_gemm_f64<U><<<grid, kThreads, 0, s>>>(A, B, M, N, K, kchunk, out, ldo, stride, mode);
-}
-
-static void launch_gemm_u(int U, dim3 grid, MatRef A, MatRef B, int64_t M, int64_t N, int64_t K,
-                          int64_t kchunk, double* out, int64_t ldo, int64_t stride, int mode, cudaStream_t s) {
-  if (U == 4) launch_gemm<4>(grid, A, B, M, N, K, kchunk, out, ldo, stride, mode, s);
-  else if (U == 2) launch_gemm<2>(grid, A, B, M, N, K, kchunk, out, ldo, stride, mode, s);
-  else launch_gemm<1>(grid, A, B, M, N, K, kchunk, out, ldo, stride, mode, s);
+  CANDMC_CK(cudaGetLastError());
+  return reduce_apply(part.d(), nsplit, stride, nb, n, Top, alpha, Z, ldz, s);
 }
 
 // Z (nb x n, ldz) = alpha * opT * (opY^T * opC), Y and C with m rows.
@@ -400,40 +678,46 @@ int gemm_tn_reduce(MatRef Y, MatRef C, int64_t m, int nb, int64_t n, MatRef Top,
     CANDMC_CK(cudaGetLastError());
     return CANDMC_OK;
   }
-  // the widest tile that, split over 64-row slices, still fills the GPU; for
-  // narrow products 16 x 16 tiles over slices down to TK rows
-  const int U = tile_u(nb, n, std::max<int64_t>(1, m / 64));
-  const int TM = 16 * U, TN = TM;
-  const int64_t tiles = ((nb + TM - 1) / TM) * ((n + TN - 1) / TN);
-  // FP64 work per CTA is what bounds these kernels: aim at ~4 CTAs per SM
-  const int64_t target = 4 * (int64_t)num_sms();
-  const int64_t min_rows = U == 4 ? 64 : (U == 2 ? 32 : TK);
-  int64_t nsplit = std::max<int64_t>(1, std::min<int64_t>((target + tiles - 1) / tiles,
-                                                          (m + min_rows - 1) / min_rows));
+  if (m * nb * n <= kSmallProduct) return small_tn(Y, C, m, nb, n, Top, alpha, Z, ldz, s);
+  // column groups: 4, or 1 (and eight groups of rows) when there are at most
+  // two column blocks; row tiles of at most 64 rows, all alike
+  const int cg = n > 8 ? 4 : 1;
+  int ntr = (nb + 63) / 64, rt = ((nb + ntr - 1) / ntr + 7) / 8 * 8, ct = 16 * cg;
+  auto ntiles = [&]() { return (int64_t)((nb + rt - 1) / rt) * ((n + ct - 1) / ct); };
+  // FP64 work per CTA is what bounds these kernels: full waves of 2 CTAs per
+  // SM, or 1 when their chunks would be shorter than 128 rows.  Chunks shorter
+  // than 64 rows take smaller tiles instead, which leaves fewer partial sums to
+  // add (2000 x 64 x 64: 16 x 32 tiles and 19 chunks, not 125).
+  const int64_t sms = num_sms(), target = sms * (m * ntiles() >= 256 * sms ? 2 : 1);
+  while (m * ntiles() < 64 * sms && (rt > 16 || ct > 16)) {
+    if (rt >= ct && rt > 16) rt = (rt / 2 + 7) / 8 * 8;
+    else if (ct > 16) ct /= 2;
+    else break;
+  }
+  const int64_t tiles = ntiles();
+  int64_t nsplit = std::max<int64_t>(1, std::min<int64_t>(target / tiles, (m + 15) / 16));
   nsplit = std::min<int64_t>(nsplit, 1024);
-  int64_t kchunk = (m + nsplit - 1) / nsplit;
-  kchunk = ((kchunk + TK - 1) / TK) * TK;
+  const int64_t kchunk = (m + nsplit - 1) / nsplit;
   nsplit = std::max<int64_t>(1, (m + kchunk - 1) / kchunk);
   const int64_t stride = (int64_t)nb * n;
   DevBuf part;
   CANDMC_RET(part.alloc(sizeof(double) * (size_t)stride * nsplit, s));
-  MatRef Yt = Y;
-  Yt.trans = !Y.trans;   // element (i, r) of Y^T is Y(r, i)
-  dim3 grid((unsigned)((nb + TM - 1) / TM), (unsigned)((n + TN - 1) / TN), (unsigned)nsplit);
   {
     ProfScope ps(CANDMC_KCLASS_GEMM_TN, 2.0 * nb * n * m, s);
-    launch_gemm_u(U, grid, Yt, C, nb, n, m, kchunk, part.d(), nb, stride, 0, s);
+    // grid rows are limited to 65535 column tiles a launch
+    for (int64_t jt = 0; jt < n; jt += 65535 * (int64_t)ct) {
+      const int64_t nn = std::min<int64_t>(n - jt, 65535 * (int64_t)ct);
+      MatRef Cj = C;
+      Cj.p = C.p + (C.trans ? jt : jt * C.ld);
+      Cj.off = C.trans ? C.off - jt : C.off + jt;
+      const dim3 grid((unsigned)((nb + rt - 1) / rt), (unsigned)((nn + ct - 1) / ct), (unsigned)nsplit);
+      double* o = part.d() + jt * nb;
+      if (cg == 4) k_gemm_tn<4><<<grid, kThreads, 0, s>>>(Y, Cj, m, nb, nn, rt, ct, kchunk, o, stride);
+      else k_gemm_tn<1><<<grid, kThreads, 0, s>>>(Y, Cj, m, nb, nn, rt, ct, kchunk, o, stride);
+    }
   }
   CANDMC_CK(cudaGetLastError());
-  int nbp = 1;
-  while (nbp < nb) nbp <<= 1;
-  {
-    ProfScope ps(CANDMC_KCLASS_REDUCE, 8.0 * stride * nsplit, s);
-    k_reduce_apply<<<(unsigned)n, kThreads, 0, s>>>(part.d(), (int)nsplit, stride, nb, nbp, n, Top, alpha,
-                                                    Z, ldz);
-  }
-  CANDMC_CK(cudaGetLastError());
-  return CANDMC_OK;
+  return reduce_apply(part.d(), nsplit, stride, nb, n, Top, alpha, Z, ldz, s);
 }
 
 // C (m x n, ldc) -= opY (m x nb) * Z (nb x n, ldz)
@@ -446,11 +730,31 @@ int gemm_nn_sub(double* C, int64_t ldc, MatRef Y, const double* Z, int64_t ldz, 
     CANDMC_CK(cudaGetLastError());
     return CANDMC_OK;
   }
-  const int U = tile_u(m, n, 1);
-  const int T = 16 * U;
-  dim3 grid((unsigned)((m + T - 1) / T), (unsigned)((n + T - 1) / T), 1);
+  if (m * n * nb <= kSmallProduct && n <= 16 * (int64_t)65535) {
+    ProfScope ps(CANDMC_KCLASS_GEMM_NN, 2.0 * m * n * nb, s);
+    const dim3 grid((unsigned)((m + 15) / 16), (unsigned)((n + 15) / 16));
+    k_gemm_f64<<<grid, kThreads, 0, s>>>(Y, mref(Z, ldz), m, n, nb, nb, C, ldc, 0, 1);
+    CANDMC_CK(cudaGetLastError());
+    return CANDMC_OK;
+  }
+  // columns per CTA: the fewest column times on the fullest SM (a CTA is one
+  // warp per sub-partition)
+  const int64_t rb = (m + kNnThreads - 1) / kNnThreads, sms = num_sms();
+  auto cost = [&](int64_t nc) { return (rb * ((n + nc - 1) / nc) + sms - 1) / sms * std::min<int64_t>(nc, (n + 3) / 4 * 4); };
+  int nc = 32;
+  for (int t : {16, 8, 4})
+    if (cost(t) < cost(nc)) nc = t;
   ProfScope ps(CANDMC_KCLASS_GEMM_NN, 2.0 * m * n * nb, s);
-  launch_gemm_u(U, grid, Y, mref(Z, ldz), m, n, nb, nb, C, ldc, 0, 1, s);
+  // grid columns are limited to 65535
+  for (int64_t j = 0; j < n; j += 65535 * (int64_t)nc) {
+    const int64_t nn = std::min<int64_t>(n - j, 65535 * (int64_t)nc);
+    const dim3 grid((unsigned)rb, (unsigned)((nn + nc - 1) / nc));
+    const MatRef Zm = mref(Z + j * ldz, ldz);
+    if (nc == 32) k_gemm_nn_sub<32><<<grid, kNnThreads, 0, s>>>(C + j * ldc, ldc, Y, Zm, m, nn, nb);
+    else if (nc == 16) k_gemm_nn_sub<16><<<grid, kNnThreads, 0, s>>>(C + j * ldc, ldc, Y, Zm, m, nn, nb);
+    else if (nc == 8) k_gemm_nn_sub<8><<<grid, kNnThreads, 0, s>>>(C + j * ldc, ldc, Y, Zm, m, nn, nb);
+    else k_gemm_nn_sub<4><<<grid, kNnThreads, 0, s>>>(C + j * ldc, ldc, Y, Zm, m, nn, nb);
+  }
   CANDMC_CK(cudaGetLastError());
   return CANDMC_OK;
 }

@@ -80,3 +80,35 @@ def test_float_pair_round_trip(cm, m, n, ld, lo, hi):
     want = h.astype(np.float64) + l.astype(np.float64)
     assert np.array_equal(A.cpu().numpy(), want)
     assert not buf.t()[m:].any()
+
+
+# products beyond the small-product kernel (2e7 multiplications): tile and
+# column-block remainders of the split-row product (8 x 4 lane blocks, 64 x 64
+# tiles, one or four column groups) and of the row-per-lane product (4-column
+# groups, 64-deep stages), Y dense or read under its unit-lower mask
+@pytest.mark.parametrize("m,nb,n", [(20011, 50, 49), (9001, 33, 70), (70001, 100, 3), (30011, 97, 8), (33333, 64, 9),
+                                    (5003, 129, 65), (2501, 256, 40), (40007, 7, 75), (1700, 64, 300)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_fp64_products(cm, m, nb, n, masked):
+    """Y^T C and C - Y Z against numpy in FP64.  A sum of k products in any
+    order is within k 2^-53 sum |x||y| of the exact one, so two of them are
+    within twice that; Z carries the first product's difference through T = 2 I
+    and |Y|."""
+    g = np.random.default_rng(m + nb + n)
+    Y = g.standard_normal((m, nb)) / np.sqrt(m)
+    C = g.standard_normal((m, n))
+    E = np.tril(Y, -1) + np.eye(m, nb) if masked else Y
+    u = 2.0 ** -53
+    aZ = np.abs(E).T @ np.abs(C)
+    if not masked:
+        got = cm.compute_invT_from_Y2(dev(Y), dev(C)).cpu().numpy()
+        assert (np.abs(got - E.T @ C) <= 2 * m * u * aZ).all()
+    dC = dev(C)
+    W = dev(0.5 * np.eye(nb))          # T^-T = I / 2
+    if masked:
+        cm.update_A(dev(Y), dC, nb, W=W, W_is_T=True)
+    else:
+        cm.upd_A(dev(Y), dC, W=W, W_is_T=True)
+    want = C - E @ (2 * (E.T @ C))
+    bound = 2 * u * (np.abs(C) + (m + nb + 2) * (np.abs(E) @ (2 * aZ)))
+    assert (np.abs(dC.cpu().numpy() - want) <= bound).all()
