@@ -117,11 +117,10 @@ __device__ __forceinline__ int leaf_col(int q, int k) {
 }
 // the first k with leaf_col(q, k) >= c
 __device__ __forceinline__ int leaf_first(int q, int c) {
-  if (q == kBulkWarps) return c / 5;
+  if (q == kBulkWarps) return c / 5 < 4 ? c / 5 : 4;
   const int g = c / 5, i = c - (g < 4 ? g : 4) - q;   // slots of the columns before c
   return i > 0 ? (i + kBulkWarps - 1) / kBulkWarps : 0;
 }
-constexpr int kLeafCols = 5;   // most columns of a warp
 
 // Sums over the warp of N values per lane (N a power of two): lanes
 // k (32 / N) .. (k + 1) (32 / N) - 1 return sum number k.  Halving the values
@@ -313,31 +312,26 @@ __device__ __forceinline__ void h7_crit(double* S, int ld, int j, Crit<R>& cr, d
   if (lane == 0) s_h[j] = h;
 }
 
-// Reflector v with *gam applied to this warp's columns k0 <= k < kLeafCols with
-// c_lo <= leaf_col(q, k) < b (*gam is there after barrier kGamBar).
-template <int R, int N>
-__device__ __forceinline__ void h7_apply(double* S, int ld, int b, int q, int k0, int c_lo, const double (&v)[R],
-                                         const double* gam) {
-  constexpr int NC = N < kLeafCols ? N : kLeafCols;
+// Reflector v with *gam applied to this warp's columns leaf_col(q, k0 + k), k <
+// NC (*gam is there after barrier kGamBar).  The count is compiled in: an FP64
+// instruction whose predicate is off for the whole warp still takes its slot.
+template <int R, int NC>
+__device__ __forceinline__ void h7_apply(double* S, int ld, int q, int k0, const double (&v)[R], const double* gam) {
+  constexpr int N = NC <= 1 ? 1 : NC <= 2 ? 2 : NC <= 4 ? 4 : 8;
   constexpr bool keep = R <= 3;   // the columns stay in registers between their dot product and update
   const int lane = threadIdx.x & 31;
   double d[N];
   double xs[NC][keep ? R : 1];
-  int cs[NC];
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     d[k] = 0.0;
     if (k < NC) {
-      const int c = leaf_col(q, k0 + k);
-      cs[k < NC ? k : 0] = (c >= c_lo && c < b && k0 + k < kLeafCols) ? c : -1;
-      if (cs[k < NC ? k : 0] >= 0) {
-        const double* sc = S + (size_t)c * ld;
+      const double* sc = S + (size_t)leaf_col(q, k0 + k) * ld;
 #pragma unroll
-        for (int t = 0; t < R; ++t) {
-          const double x = sc[lane + 32 * t];
-          if constexpr (keep) xs[k < NC ? k : 0][t] = x;
-          d[k] = fma(v[t], x, d[k]);
-        }
+      for (int t = 0; t < R; ++t) {
+        const double x = sc[lane + 32 * t];
+        if constexpr (keep) xs[k < NC ? k : 0][t] = x;
+        d[k] = fma(v[t], x, d[k]);
       }
     }
   }
@@ -347,17 +341,15 @@ __device__ __forceinline__ void h7_apply(double* S, int ld, int b, int q, int k0
 #pragma unroll
   for (int k = 0; k < NC; ++k) {
     const double fk = __shfl_sync(0xffffffffu, f, k * (32 / N));
-    if (cs[k] >= 0) {
-      double* sc = S + (size_t)cs[k] * ld;
-      double x[R];
+    double* sc = S + (size_t)leaf_col(q, k0 + k) * ld;
+    double x[R];
 #pragma unroll
-      for (int t = 0; t < R; ++t) {
-        if constexpr (keep) x[t] = xs[k][t];
-        else x[t] = sc[lane + 32 * t];
-      }
-#pragma unroll
-      for (int t = 0; t < R; ++t) sc[lane + 32 * t] = fma(-fk, v[t], x[t]);
+    for (int t = 0; t < R; ++t) {
+      if constexpr (keep) x[t] = xs[k][t];
+      else x[t] = sc[lane + 32 * t];
     }
+#pragma unroll
+    for (int t = 0; t < R; ++t) sc[lane + 32 * t] = fma(-fk, v[t], x[t]);
   }
 }
 
@@ -382,6 +374,7 @@ __device__ void h7_factor(double* S, int ld, int b, double* s_h, double* s_gam, 
   if (warp == 0 || q >= 0) {
     Crit<R> cr;
     double (&v)[R] = cr.v;
+    const int kend = q >= 0 ? leaf_first(q, b) : 0;   // columns of this warp
     cr.seed = cr.den = 0.0;
 #pragma unroll
     for (int t = 0; t < R; ++t) v[t] = 0.0;
@@ -401,10 +394,14 @@ __device__ void h7_factor(double* S, int ld, int b, double* s_h, double* s_gam, 
         const double* gam = s_gam + j - 1;
         // this warp's columns from j + 1 on are its last ones
         const int klo = leaf_first(q, j + 1);
-        if (klo >= 4) h7_apply<R, 1>(S, ld, b, q, 4, j + 1, v, gam);
-        else if (klo == 3) h7_apply<R, 2>(S, ld, b, q, 3, j + 1, v, gam);
-        else if (klo >= 1) h7_apply<R, 4>(S, ld, b, q, 1, j + 1, v, gam);
-        else h7_apply<R, 8>(S, ld, b, q, 0, j + 1, v, gam);
+        switch (kend - klo) {
+          case 5: h7_apply<R, 5>(S, ld, q, klo, v, gam); break;
+          case 4: h7_apply<R, 4>(S, ld, q, klo, v, gam); break;
+          case 3: h7_apply<R, 3>(S, ld, q, klo, v, gam); break;
+          case 2: h7_apply<R, 2>(S, ld, q, klo, v, gam); break;
+          case 1: h7_apply<R, 1>(S, ld, q, klo, v, gam); break;
+          default: named_bar(kGamBar, kLeafStepThreads); break;
+        }
       }
     }
     if (warp == 0 && lane == 0) s_gam[b - 1] = refine_gamma(cr.seed, cr.den);
@@ -811,12 +808,11 @@ __device__ void h4_root(const Hr4Args& a, double* sm) {
       named_bar(1, 4 * 32);
       const double l = lane > i ? sL[i * kLd + lane] : 0.0;
 #pragma unroll
-      for (int k = 0; k < 11; ++k) {
+      for (int k = 10; k >= 0; --k) {   // a break, not a predicate: see h7_apply
         const int c = q + 3 * k;
-        if (c >= i + 2 && c < b) {
-          x[k] = fma(-l, __shfl_sync(0xffffffffu, x[k], i), x[k]);
-          if (c == i + 2) sL[c * kLd + lane] = x[k];
-        }
+        if (c < i + 2) break;
+        if (c < kDirectB) x[k] = fma(-l, __shfl_sync(0xffffffffu, x[k], i), x[k]);
+        if (c == i + 2) sL[c * kLd + lane] = x[k];
       }
     }
   } else if (warp <= 4) {
