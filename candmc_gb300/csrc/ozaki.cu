@@ -334,9 +334,9 @@ struct OzArgs {
   int64_t AR;
   const __nv_bfloat16* Bs;   // B-operand slices: S planes of BR x Kpad
   int64_t BR;
-  int64_t Kpad;              // multiple of 16
-  int64_t k_per_cta;         // K extent of one CTA (multiple of kgroup)
-  int64_t kgroup;            // K rows per scale group / accumulator readout
+  int Kpad;                  // multiple of 16
+  int k_per_cta;             // K extent of one CTA (multiple of kgroup)
+  int kgroup;                // K rows per scale group / accumulator readout
   const int* eA;             // [Kpad / kgroup][AR]
   const int* eB;             // [Kpad / kgroup][BR]
   int mode;                  // 0: partial sums (df64) over the CTA's K range; 1: C -= product
@@ -349,7 +349,7 @@ struct OzArgs {
   int c_fp64;                // mode 1: C is stored as FP64 (read and written in FP64)
   int c_assign;              // mode 1 with c_fp64: C = product (C is not read)
   int* status;
-  int64_t n_mt, n_nt, n_ks;  // work items: M tiles x N tiles x K splits
+  int n_mt, n_nt, n_ks;      // work items: M tiles x N tiles x K splits
 };
 
 __device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
@@ -379,75 +379,119 @@ constexpr int OZ_EPI_WARPS = 12;                     // epilogue warps: 4 TMEM l
 constexpr int OZ_EPI_COLS = OZ_N * 4 / OZ_EPI_WARPS;  // accumulator columns per epilogue warp
 constexpr int OZ_WARPS = 2 + OZ_EPI_WARPS;             // producer, MMA issuer, epilogue
 constexpr int OZ_THREADS = OZ_WARPS * 32;
-static_assert(OZ_EPI_WARPS % 4 == 0 && OZ_EPI_COLS % 16 == 0, "epilogue split");
+static_assert(OZ_EPI_WARPS % 4 == 0 && OZ_EPI_COLS == 32, "epilogue split: one column per lane for the exponents");
 
-// The five accumulators of one output element as one df64 value.  Groups 0..3
-// hold the diagonals i + j = g of the slice products, exact multiples of
-// 2^-8g with |g0| <= 2^23, |g1| <= 2^15, |g2| <= 2^8, |g3| < 1 (digits of at
-// most 8 bits over a 128-row group); group 4 holds the rest, down to about
-// 2^-40.  Rounding g1 and g2 to integers and g3 to a multiple of 2^-16 (the
-// 1.5 * 2^23 and 1.5 * 2^7 shifts) splits them exactly: H = g0 + [g1] + [g2]
-// is an integer below 2^24, M = frac(g1) + frac(g2) + [g3] a multiple of 2^-16
-// below 2 in magnitude, both exact, and only L = (g3 - [g3]) + g4 rounds.  The
-// two fast TwoSums are exact here (H is zero or at least 1 in magnitude), so
-// the result carries about 2^-47 relative error, as a df64 sum of the five.
-// The operations are round-to-nearest intrinsics, which the compiler neither
-// contracts into FMAs nor reorders.
-__device__ __forceinline__ f2 combine_groups(float g0, float g1, float g2, float g3, float g4) {
-  const float kShift = 12582912.0f;   // 1.5 * 2^23: rounds to an integer
-  const float kShift3 = 192.0f;       // 1.5 * 2^7: rounds to a multiple of 2^-16
-  const float r1 = __fsub_rn(__fadd_rn(g1, kShift), kShift);
-  const float r2 = __fsub_rn(__fadd_rn(g2, kShift), kShift);
-  const float r3 = __fsub_rn(__fadd_rn(g3, kShift3), kShift3);
-  const float H = __fadd_rn(__fadd_rn(g0, r1), r2);
-  const float M = __fadd_rn(__fadd_rn(__fsub_rn(g1, r1), __fsub_rn(g2, r2)), r3);
-  const float L = __fadd_rn(__fsub_rn(g3, r3), g4);
-  const float s = __fadd_rn(H, M);
-  const float e = __fsub_rn(M, __fsub_rn(s, H));
-  const float l = __fadd_rn(e, L);
-  const float h = __fadd_rn(s, l);
-  return {h, __fsub_rn(l, __fsub_rn(h, s))};
+// Two floats in one 64-bit register: the f32x2 instructions round each half
+// as the scalar ones do and take one issue slot for both.
+struct f2x2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ f2x2 pack2(float a, float b) {
+  f2x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f2x2 x) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x.v));
+  return r;
+}
+__device__ __forceinline__ f2x2 add2(f2x2 a, f2x2 b) {
+  f2x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f2x2 mul2(f2x2 a, f2x2 b) {
+  f2x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f2x2 sub2(f2x2 a, f2x2 b) {   // a - b, rounded once
+  f2x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(b.v), "l"(0xbf800000bf800000ull), "l"(a.v));
+  return r;
 }
 
-// The accumulators of one output element as one value: the exact five-group
-// combine of the emulated-FP64 form, or, for the FP32 form (one group per
-// level, FP32 accuracy wanted), their FP32 sum.
+// two df64 values: high words, low words
+struct df2 {
+  f2x2 h, l;
+};
+
+// The accumulators of two output elements (columns j, j + 1 of gr) as df64
+// values.  Groups 0..3 hold the diagonals i + j = g of the slice products,
+// exact multiples of 2^-8g with |g0| <= 2^23, |g1| <= 2^15, |g2| <= 2^8,
+// |g3| < 1 (digits of at most 8 bits over a 128-row group); group 4 holds the
+// rest, down to about 2^-40.  Rounding g1 and g2 to integers and g3 to a
+// multiple of 2^-16 (the 1.5 * 2^23 and 1.5 * 2^7 shifts) splits them exactly:
+// H = g0 + [g1] + [g2] is an integer below 2^24, M = frac(g1) + frac(g2) + [g3]
+// a multiple of 2^-16 below 2 in magnitude, both exact, and only
+// L = (g3 - [g3]) + g4 rounds.  The two fast TwoSums are exact here (H is zero
+// or at least 1 in magnitude), so the result carries about 2^-47 relative
+// error, as a df64 sum of the five.  The FP32 form (G < 5, one group per level,
+// FP32 accuracy wanted) takes their FP32 sum.
 template <int G>
-__device__ __forceinline__ f2 combine_g(const float (&gv)[G][8], int j) {
-  if constexpr (G == 5) {
-    return combine_groups(gv[0][j], gv[1][j], gv[2][j], gv[3][j], gv[4][j]);
-  } else {
-    float h = gv[G - 1][j];
+__device__ __forceinline__ df2 combine2(const uint32_t (&gr)[G][8], int j) {
+  f2x2 g[G];
 #pragma unroll
-    for (int g = G - 2; g >= 0; --g) h = __fadd_rn(gv[g][j], h);
-    return {h, 0.0f};
+  for (int q = 0; q < G; ++q) g[q] = pack2(__uint_as_float(gr[q][j]), __uint_as_float(gr[q][j + 1]));
+  if constexpr (G == 5) {
+    const f2x2 shift = pack2(12582912.0f, 12582912.0f);   // 1.5 * 2^23: rounds to an integer
+    const f2x2 shift3 = pack2(192.0f, 192.0f);            // 1.5 * 2^7: rounds to a multiple of 2^-16
+    const f2x2 r1 = sub2(add2(g[1], shift), shift);
+    const f2x2 r2 = sub2(add2(g[2], shift), shift);
+    const f2x2 r3 = sub2(add2(g[3], shift3), shift3);
+    const f2x2 H = add2(add2(g[0], r1), r2);
+    const f2x2 M = add2(add2(sub2(g[1], r1), sub2(g[2], r2)), r3);
+    const f2x2 L = add2(sub2(g[3], r3), g[4]);
+    const f2x2 s = add2(H, M);
+    const f2x2 l = add2(sub2(M, sub2(s, H)), L);
+    const f2x2 h = add2(s, l);
+    return {h, sub2(l, sub2(h, s))};
+  } else {
+    f2x2 h = g[G - 1];
+#pragma unroll
+    for (int q = G - 2; q >= 0; --q) h = add2(g[q], h);
+    return {h, {0ull}};
   }
 }
 
-// x + y without the lo-part TwoSum: relative error of order 2^-46 of |x| + |y|
-__device__ __forceinline__ f2 df_add_sloppy(f2 x, f2 y) {
-  const float s = __fadd_rn(x.h, y.h);
-  const float bb = __fsub_rn(s, x.h);
-  const float e = __fadd_rn(__fsub_rn(x.h, __fsub_rn(s, bb)), __fsub_rn(y.h, bb));
-  const float l = __fadd_rn(e, __fadd_rn(x.l, y.l));
-  const float h = __fadd_rn(s, l);
-  return {h, __fsub_rn(l, __fsub_rn(h, s))};
+// Accumulation of the epilogue, x + y without the lo-part TwoSum: relative
+// error of order 2^-46 of |x| + |y|.  For the FP32 form (G < 5, products
+// accurate to FP32) plain FP32, which keeps C in the df64 slots with a zero
+// low word.
+template <int G>
+__device__ __forceinline__ df2 oz_accumulate(df2 x, df2 y) {
+  const f2x2 s = add2(x.h, y.h);
+  if constexpr (G != 5) return {s, {0ull}};
+  const f2x2 bb = sub2(s, x.h);
+  const f2x2 e = add2(sub2(x.h, sub2(s, bb)), sub2(y.h, bb));
+  const f2x2 l = add2(e, add2(x.l, y.l));
+  const f2x2 h = add2(s, l);
+  return {h, sub2(l, sub2(h, s))};
 }
 
-// Accumulation of the epilogue: df64 for the emulated-FP64 form (G = 5); for
-// the FP32 form (G < 5, products accurate to FP32) plain FP32, which keeps C
-// in the df64 slots with a zero low word.
+// C - p for the read-modify-write of MODE 1, as df_add of C and -p does it
+// (same split by form)
 template <int G>
-__device__ __forceinline__ f2 oz_accumulate(f2 x, f2 y) {
-  if constexpr (G == 5) return df_add_sloppy(x, y);
-  else return {__fadd_rn(x.h, y.h), 0.0f};
+__device__ __forceinline__ df2 oz_subtract(df2 c, df2 p) {
+  if constexpr (G != 5) return {sub2(add2(c.h, c.l), p.h), {0ull}};
+  const f2x2 s = sub2(c.h, p.h), sb = sub2(s, c.h);
+  const f2x2 e = sub2(sub2(c.h, sub2(s, sb)), add2(p.h, sb));
+  const f2x2 t = sub2(c.l, p.l), tb = sub2(t, c.l);
+  const f2x2 te = sub2(sub2(c.l, sub2(t, tb)), add2(p.l, tb));
+  const f2x2 e1 = add2(e, t);
+  const f2x2 s1 = add2(s, e1);
+  const f2x2 e2 = add2(sub2(e1, sub2(s1, s)), te);
+  const f2x2 h = add2(s1, e2);
+  return {h, sub2(e2, sub2(h, s1))};
 }
 
-// C - p for the read-modify-write of MODE 1 (same split by form)
-template <int G>
-__device__ __forceinline__ f2 oz_subtract(f2 c, f2 p) {
-  if constexpr (G == 5) return df_add(c, {-p.h, -p.l});
-  else return {__fsub_rn(__fadd_rn(c.h, c.l), p.h), 0.0f};
+// v * 2^e for e beyond the normal floats' range (e >= -312 for float inputs):
+// three normal factors, so the partial products stay exact unless the result
+// leaves the range
+__device__ __forceinline__ float scale_wide(float v, int e) {
+  const int e1 = min(max(e, -126), 127), e2 = min(max(e - e1, -126), 127);
+  return __fmul_rn(__fmul_rn(__fmul_rn(v, pow2f(e1)), pow2f(e2)), pow2f(e - e1 - e2));
 }
 
 __device__ __forceinline__ void mbar_init(uint64_t* b, unsigned count) {
@@ -490,52 +534,81 @@ __device__ __forceinline__ bool oz_wait(uint64_t* b, uint32_t parity, volatile i
   return false;
 }
 
+// Where a product of slice A_i stands among the products of A_i in one step:
+// the first one fills the tensor core's A collector, the others reuse it.
+enum OzCollect { kOzSingle, kOzFill, kOzUse, kOzLast };
+
 // One 128 x 96 x 16 BF16 MMA into the accumulator at TMEM column address dt;
-// accum = 0 overwrites it.
+// accum = 0 overwrites it.  The whole warp calls it, one elected lane issues:
+// in a branch on the lane index the operands go through the vector registers
+// and an MMA takes 50 cycles to issue at any width, here 24 (N = 32).
+template <OzCollect U>
 __device__ __forceinline__ void umma_bf16(uint32_t dt, uint64_t ad, uint64_t bd, uint32_t idesc,
                                           uint32_t accum) {
+#define OZ_UMMA(COLLECT)                                                                            \
+  asm volatile(                                                                                     \
+      "{\n\t.reg .pred p, one;\n\telect.sync _|one, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"       \
+      "@one tcgen05.mma.cta_group::1.kind::f16" COLLECT " [%0], %1, %2, %3, p;\n\t}" ::"r"(dt),    \
+      "l"(ad), "l"(bd), "r"(idesc), "r"(accum)                                                      \
+      : "memory")
+  if constexpr (U == kOzFill) OZ_UMMA(".collector::a::fill");
+  else if constexpr (U == kOzUse) OZ_UMMA(".collector::a::use");
+  else if constexpr (U == kOzLast) OZ_UMMA(".collector::a::lastuse");
+  else OZ_UMMA("");
+#undef OZ_UMMA
+}
+
+// arrives on b once every MMA issued so far has completed (one elected lane)
+__device__ __forceinline__ void umma_commit(uint64_t* b) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dt),
-      "l"(ad), "l"(bd), "r"(idesc), "r"(accum));
+      "{\n\t.reg .pred one;\n\telect.sync _|one, 0xffffffff;\n\t"
+      "@one tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
+          smem_u32(b))
+      : "memory");
 }
 
 // The slice-pair MMAs of one K16 step.  da / db: descriptors of the stage's
 // first A and B slice (the slices follow at fixed byte strides, and a
 // descriptor's address field is the shared-memory address / 16, so slice
 // descriptors are the base plus a constant).  In loop order the first product
-// of accumulator group g is (0, g): in a group's first step (FIRST) those
-// overwrite their accumulator, every other product adds to it.
-template <int S, int G, bool FIRST>
-__device__ __forceinline__ void oz_issue_step(uint32_t tmem, uint64_t da, uint64_t db, uint32_t idesc) {
-#pragma unroll
-  for (int i = 0; i < S; ++i) {
-#pragma unroll
-    for (int j = 0; j < S; ++j) {
-      if (i + j >= S) continue;
-      const int g = (i + j < G - 1) ? i + j : G - 1;
-      const bool first = FIRST && i == 0 && j < G;
-      umma_bf16(tmem + (uint32_t)(g * OZ_N), da + (uint64_t)(i * (OZ_ABYTES >> 4)),
-                db + (uint64_t)(j * (OZ_BBYTES >> 4)), idesc, first ? 0u : 1u);
-    }
-  }
+// of accumulator group g is (0, g): with accum = 0 (a group's first step)
+// those overwrite their accumulator, every other product adds to it.  The
+// products of one A slice follow one another and take it from the collector:
+// without that a 128 x 96 x 16 MMA is bound by its 7 KB of operand reads (58
+// cycles instead of 50; its multiplications take 48).
+template <int S, int G, int I = 0, int J = 0>
+__device__ __forceinline__ void oz_issue_step(uint32_t tmem, uint64_t da, uint64_t db, uint32_t idesc,
+                                              uint32_t accum) {
+  constexpr int g = (I + J < G - 1) ? I + J : G - 1;
+  constexpr OzCollect u = (I == S - 1) ? kOzSingle : (J == 0) ? kOzFill : (J == S - 1 - I) ? kOzLast : kOzUse;
+  umma_bf16<u>(tmem + (uint32_t)(g * OZ_N), da + (uint64_t)(I * (OZ_ABYTES >> 4)),
+               db + (uint64_t)(J * (OZ_BBYTES >> 4)), idesc, (I == 0 && J < G) ? accum : 1u);
+  if constexpr (I + J + 1 < S) oz_issue_step<S, G, I, J + 1>(tmem, da, db, idesc, accum);
+  else if constexpr (I + 1 < S) oz_issue_step<S, G, I + 1, 0>(tmem, da, db, idesc, accum);
+}
+
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e != 0;
 }
 
 // Work item w of a launch: (M tile, N tile, K range).  M tiles run fastest so
 // that consecutive items of a CTA share the B operand's slices in L2.
 struct OzItem {
-  int64_t m0, n0, kbeg, kend;
+  int64_t m0, n0;
+  int kbeg, kend;
   int split;
 };
 
-__device__ __forceinline__ OzItem oz_item(const OzArgs& a, int64_t w) {
+__device__ __forceinline__ OzItem oz_item(const OzArgs& a, int w) {
   OzItem it;
-  const int64_t mt = w % a.n_mt, rest = w / a.n_mt;
-  const int64_t nt = rest % a.n_nt, ks = rest / a.n_nt;
-  it.m0 = mt * OZ_M;
-  it.n0 = nt * OZ_N;
-  it.kbeg = ks * a.k_per_cta;
-  it.kend = (it.kbeg + a.k_per_cta < a.Kpad) ? it.kbeg + a.k_per_cta : a.Kpad;
+  const unsigned rest = (unsigned)w / (unsigned)a.n_mt, mt = (unsigned)w % (unsigned)a.n_mt;
+  const unsigned ks = rest / (unsigned)a.n_nt, nt = rest % (unsigned)a.n_nt;
+  it.m0 = (int64_t)mt * OZ_M;
+  it.n0 = (int64_t)nt * OZ_N;
+  it.kbeg = (int)ks * a.k_per_cta;
+  it.kend = min(it.kbeg + a.k_per_cta, a.Kpad);
   it.split = (int)ks;
   return it;
 }
@@ -557,10 +630,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
   __shared__ uint32_t tmem_base_s;
   __shared__ volatile int s_fail;
   __shared__ int s_eb[OZ_EPI_WARPS][OZ_EPI_COLS];   // per epilogue warp: its columns' exponents
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   unsigned char* ring = (unsigned char*)(((uintptr_t)oz_smem + 1023) & ~(uintptr_t)1023);
-  const int64_t nitems = a.n_mt * a.n_nt * a.n_ks;
-  const int steps_per_group = (int)(a.kgroup / 16);
+  const int nitems = a.n_mt * a.n_nt * a.n_ks;
+  const int steps_per_group = a.kgroup / 16;
 
   if (tid == 0) {
     for (int st = 0; st < OZ_STAGES; ++st) {
@@ -599,113 +672,112 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
   const uint32_t tmem = tmem_base_s;
 
   if (warp == 0) {
-    // ---------------- producer
-    if (lane == 0) {
-      int64_t gs = 0;   // stage fills issued by this CTA
-      for (int64_t w = blockIdx.x; w < nitems && !s_fail; w += gridDim.x) {
-        const OzItem it = oz_item(a, w);
-        for (int64_t kb = it.kbeg >> 4; kb < (it.kend >> 4); ++kb, ++gs) {
-          const int st = (int)(gs % OZ_STAGES);
-          if (!oz_wait(&empty_b[st], (uint32_t)(((gs / OZ_STAGES) & 1) ^ 1), &s_fail)) break;
-          const int abytes = (MODE == 0 && a.AR < OZ_M) ? (int)a.AR * 32 : OZ_ABYTES;
+    // ---------------- producer: the whole warp walks the stages, one elected lane copies
+    const int abytes = (MODE == 0 && a.AR < OZ_M) ? (int)a.AR * 32 : OZ_ABYTES;
+    const int64_t aplane = a.AR * a.Kpad, bplane = a.BR * a.Kpad;
+    int st = 0;
+    uint32_t parity = 1;
+    bool ok = true;
+    for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
+      const OzItem it = oz_item(a, w);
+      const __nv_bfloat16* as = a.As + (int64_t)it.kbeg * a.AR + it.m0 * 16;
+      const __nv_bfloat16* bs = a.Bs + (int64_t)it.kbeg * a.BR + it.n0 * 16;
+      for (int k = it.kbeg; k < it.kend; k += 16) {
+        ok = oz_wait(&empty_b[st], parity, &s_fail);
+        if (!ok) break;
+        if (elect_one()) {
           mbar_expect_tx(&full_b[st], (unsigned)(S * (abytes + OZ_BBYTES)));
-          unsigned char* sb = ring + (size_t)st * STAGE_BYTES;
-#pragma unroll 1
+          const uint32_t sa = smem_u32(ring + (size_t)st * STAGE_BYTES), sb = sa + S * OZ_ABYTES;
+#pragma unroll
           for (int sl = 0; sl < S; ++sl) {
-            bulk_g2s(smem_u32(sb + sl * OZ_ABYTES),
-                     a.As + (int64_t)sl * a.AR * a.Kpad + kb * a.AR * 16 + (it.m0 >> 3) * 128,
-                     (unsigned)abytes, &full_b[st]);
-            bulk_g2s(smem_u32(sb + S * OZ_ABYTES + sl * OZ_BBYTES),
-                     a.Bs + (int64_t)sl * a.BR * a.Kpad + kb * a.BR * 16 + (it.n0 >> 3) * 128,
-                     (unsigned)OZ_BBYTES, &full_b[st]);
+            bulk_g2s(sa + sl * OZ_ABYTES, as + sl * aplane, (unsigned)abytes, &full_b[st]);
+            bulk_g2s(sb + sl * OZ_BBYTES, bs + sl * bplane, (unsigned)OZ_BBYTES, &full_b[st]);
           }
+        }
+        __syncwarp();
+        as += a.AR * 16;
+        bs += a.BR * 16;
+        if (++st == OZ_STAGES) {
+          st = 0;
+          parity ^= 1;
         }
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_N >> 3) << 17) |
-                             ((uint32_t)(OZ_M >> 4) << 24);
-      // ring stages are 1024-byte aligned and the ring ends below 256 KB, so
-      // base + offset / 16 stays inside the descriptor's 14-bit address field
-      const uint64_t ring_desc = make_desc(smem_u32(ring));
-      static_assert((OZ_STAGES * STAGE_BYTES + 2048) < (1 << 18), "ring within the descriptor's range");
-      static_assert(STAGE_BYTES % 16 == 0 && OZ_ABYTES % 16 == 0 && OZ_BBYTES % 16 == 0, "16-byte strides");
-      int64_t gs = 0, ngroups = 0;
-      for (int64_t w = blockIdx.x; w < nitems && !s_fail; w += gridDim.x) {
-        const OzItem it = oz_item(a, w);
-        const int nsteps = (int)((it.kend - it.kbeg) >> 4);
-        for (int t = 0; t < nsteps && !s_fail; ++t, ++gs) {
-          const int sig = t % steps_per_group;
-          if (sig == 0) {
-            // the epilogue has read the previous group's accumulators
-            if (!oz_wait(&acc_empty, (uint32_t)((ngroups & 1) ^ 1), &s_fail)) break;
-          }
-          const int st = (int)(gs % OZ_STAGES);
-          if (!oz_wait(&full_b[st], (uint32_t)((gs / OZ_STAGES) & 1), &s_fail)) break;
+    // ---------------- MMA issuer: the whole warp walks the stages, one elected lane issues
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_N >> 3) << 17) |
+                           ((uint32_t)(OZ_M >> 4) << 24);
+    // ring stages are 1024-byte aligned and the ring ends below 256 KB, so
+    // base + offset / 16 stays inside the descriptor's 14-bit address field
+    const uint64_t ring_desc = make_desc(smem_u32(ring));
+    static_assert((OZ_STAGES * STAGE_BYTES + 2048) < (1 << 18), "ring within the descriptor's range");
+    static_assert(STAGE_BYTES % 16 == 0 && OZ_ABYTES % 16 == 0 && OZ_BBYTES % 16 == 0, "16-byte strides");
+    int st = 0;
+    uint32_t parity = 0, acc_parity = 1;
+    bool ok = true;
+    for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
+      const OzItem it = oz_item(a, w);
+      for (int left = (it.kend - it.kbeg) >> 4; left > 0 && ok; left -= steps_per_group) {
+        const int steps = min(left, steps_per_group);
+        // the epilogue has read the previous group's accumulators
+        ok = oz_wait(&acc_empty, acc_parity, &s_fail);
+        acc_parity ^= 1;
+        for (int t = 0; t < steps && ok; ++t) {
+          ok = oz_wait(&full_b[st], parity, &s_fail);
+          if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint64_t da = ring_desc + (uint64_t)(st * (STAGE_BYTES >> 4));
-          const uint64_t db = da + (uint64_t)((S * OZ_ABYTES) >> 4);
-          if (sig == 0)
-            oz_issue_step<S, G, true>(tmem, da, db, idesc);
-          else
-            oz_issue_step<S, G, false>(tmem, da, db, idesc);
-          // the stage is free once these MMAs have read it
-          asm volatile(
-              "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                  smem_u32(&empty_b[st]))
-              : "memory");
-          if (sig == steps_per_group - 1 || t == nsteps - 1) {
-            asm volatile(
-                "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                    smem_u32(&acc_full))
-                : "memory");
-            ++ngroups;
+          oz_issue_step<S, G>(tmem, da, da + (uint64_t)((S * OZ_ABYTES) >> 4), idesc, t > 0 ? 1u : 0u);
+          umma_commit(&empty_b[st]);   // the stage is free once these MMAs have read it
+          if (++st == OZ_STAGES) {
+            st = 0;
+            parity ^= 1;
           }
         }
+        if (ok) umma_commit(&acc_full);
       }
-      // every MMA this thread issued has completed before TMEM is released
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                       smem_u32(&fin))
-                   : "memory");
-      volatile int dummy = 0;
-      oz_wait(&fin, 0u, &dummy);
     }
+    // every MMA this warp issued has completed before TMEM is released
+    umma_commit(&fin);
+    volatile int dummy = 0;
+    oz_wait(&fin, 0u, &dummy);
   } else {
     // ---------------- epilogue: warps 2 .. 2 + OZ_EPI_WARPS - 1
     const int q = warp & 3;                // TMEM lane quarter this warp may access
     const int part = (warp - 2) >> 2;      // column part
     const int row = q * 32 + lane;
     int64_t ngroups = 0;
-    f2 acc[OZ_EPI_COLS];   // MODE 0: sums over the item's K range; MODE 1: this group's product
-    for (int64_t w = blockIdx.x; w < nitems && !s_fail; w += gridDim.x) {
+    df2 acc[OZ_EPI_COLS / 2];   // MODE 0: sums over the item's K range; MODE 1: this group's product
+    for (int w = blockIdx.x; w < nitems && !s_fail; w += gridDim.x) {
       const OzItem it = oz_item(a, w);
-      const int nsteps = (int)((it.kend - it.kbeg) >> 4);
-      const int64_t gm = it.m0 + row;
-      if (MODE == 1 && w + gridDim.x < nitems) {
-        // the next item's C tile streams into L2 while this one is computed
+      const int nsteps = (it.kend - it.kbeg) >> 4;
+      const int64_t gm = it.m0 + row, gn0 = it.n0 + part * OZ_EPI_COLS;
+      const int nc = (int)min((int64_t)OZ_EPI_COLS, a.Nvalid - gn0);   // this warp's columns (<= 0: none)
+      if (MODE == 1 && w + gridDim.x < nitems && !a.c_fp64) {
+        // the next item's C tile streams into L2 while this one is computed:
+        // a lane takes one column, 32 rows of 8 bytes
         const OzItem nx = oz_item(a, w + gridDim.x);
-        const int64_t pm = nx.m0 + row;
-        if (pm < a.Mvalid) {
-          for (int j = 0; j < OZ_EPI_COLS; ++j) {
-            const int64_t gn = nx.n0 + part * OZ_EPI_COLS + j;
-            if (gn < a.Nvalid && (lane & 15) == 0)
-              asm volatile("prefetch.global.L2 [%0];" ::"l"(a.C + gn * a.ldc + pm));
-          }
+        const int64_t pm = nx.m0 + q * 32, pn = nx.n0 + part * OZ_EPI_COLS + lane;
+        if (pn < a.Nvalid && pm < a.Mvalid) {
+          const float2* pc = a.C + pn * a.ldc + pm;
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(pc));
+          if (pm + 16 < a.Mvalid) asm volatile("prefetch.global.L2 [%0];" ::"l"(pc + 16));
         }
       }
 #pragma unroll
-      for (int j = 0; j < OZ_EPI_COLS; ++j) acc[j] = {0.0f, 0.0f};
+      for (int j = 0; j < OZ_EPI_COLS / 2; ++j) acc[j] = {{0ull}, {0ull}};
       for (int t0 = 0; t0 < nsteps; t0 += steps_per_group) {
-        // the group's exponents are loaded while its MMAs run
-        const int64_t grp = (it.kbeg + (int64_t)t0 * 16) / a.kgroup;
+        // The group's exponents are loaded while its MMAs run, shifted to
+        // where a float has its exponent: 2^(eA + eB - 16) takes one addition.
+        const int64_t grp = (it.kbeg + t0 * 16) / a.kgroup;
         const int eA = (gm < a.AR) ? a.eA[grp * a.AR + gm] : 0;
-        int* eb = s_eb[warp - 2];
-        for (int c = lane; c < OZ_EPI_COLS; c += 32) {
-          const int64_t gn = it.n0 + part * OZ_EPI_COLS + c;
-          eb[c] = (gn < a.BR) ? __ldg(a.eB + grp * a.BR + gn) : 0;
-        }
+        const int eb = (gn0 + lane < a.BR) ? __ldg(a.eB + grp * a.BR + gn0 + lane) : 0;
+        int* ebs = s_eb[warp - 2];
+        ebs[lane] = eb << 23;
+        // one warp-uniform test: every scale a normal float
+        const int eb_min = __reduce_min_sync(0xffffffffu, eb), eb_max = __reduce_max_sync(0xffffffffu, eb);
+        const bool normal = __all_sync(0xffffffffu, eA + eb_min - 16 >= -126 && eA + eb_max - 16 <= 127);
+        const int fA = (eA - 16 + 127) << 23;
         __syncwarp();
         if (!oz_wait(&acc_full, (uint32_t)(ngroups & 1), &s_fail)) break;
         ++ngroups;
@@ -713,103 +785,99 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
         // drain the five accumulators, 8 columns at a time
 #pragma unroll
         for (int c8 = 0; c8 < OZ_EPI_COLS / 8; ++c8) {
-          const int cbase = part * OZ_EPI_COLS + c8 * 8;
-          int eB[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) eB[j] = eb[c8 * 8 + j];
           uint32_t gr[G][8];
 #pragma unroll
           for (int g = 0; g < G; ++g)
-            tmem_ld8(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(g * OZ_N + cbase), gr[g]);
+            tmem_ld8(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(g * OZ_N + part * OZ_EPI_COLS + c8 * 8), gr[g]);
+          int f[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) f[j] = ebs[c8 * 8 + j];
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          float gv[G][8];
 #pragma unroll
-          for (int g = 0; g < G; ++g) {
-            tmem_regs_ready(gr[g]);
+          for (int g = 0; g < G; ++g) tmem_regs_ready(gr[g]);
+          if (normal) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) gv[g][j] = __uint_as_float(gr[g][j]);
-          }
-          // one warp-uniform test: every scale 2^(eA + eB - 16) a normal float
-          bool normal = true;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int e = eA + eB[j] - 16;
-            normal = normal && e >= -126 && e <= 127;
-          }
-          if (__all_sync(0xffffffffu, normal)) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const f2 v = combine_g<G>(gv, j);
-              const float f = pow2f(eA + eB[j] - 16);
-              const f2 sv = {__fmul_rn(v.h, f), __fmul_rn(v.l, f)};
-              if (MODE == 0) acc[c8 * 8 + j] = oz_accumulate<G>(acc[c8 * 8 + j], sv);
-              else acc[c8 * 8 + j] = sv;
+            for (int j = 0; j < 8; j += 2) {
+              df2 v = combine2<G>(gr, j);
+              const f2x2 sc = pack2(__int_as_float(fA + f[j]), __int_as_float(fA + f[j + 1]));
+              v = {mul2(v.h, sc), mul2(v.l, sc)};
+              df2& x = acc[c8 * 4 + j / 2];
+              x = (MODE == 0) ? oz_accumulate<G>(x, v) : v;
             }
           } else {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const f2 v = combine_g<G>(gv, j);
-              // 2^e as three normal factors (e >= -312 for float inputs): the
-              // partial products stay exact unless the result leaves the range
-              const int e = eA + eB[j] - 16;
-              const int e1 = min(max(e, -126), 127), e2 = min(max(e - e1, -126), 127);
-              const float f1 = pow2f(e1), f2v = pow2f(e2), f3 = pow2f(e - e1 - e2);
-              const f2 sv = {__fmul_rn(__fmul_rn(__fmul_rn(v.h, f1), f2v), f3),
-                             __fmul_rn(__fmul_rn(__fmul_rn(v.l, f1), f2v), f3)};
-              if (MODE == 0) acc[c8 * 8 + j] = oz_accumulate<G>(acc[c8 * 8 + j], sv);
-              else acc[c8 * 8 + j] = sv;
+            for (int j = 0; j < 8; j += 2) {
+              df2 v = combine2<G>(gr, j);
+              const int e0 = eA + (f[j] >> 23) - 16, e1 = eA + (f[j + 1] >> 23) - 16;
+              const float2 h = unpack2(v.h), l = unpack2(v.l);
+              v = {pack2(scale_wide(h.x, e0), scale_wide(h.y, e1)), pack2(scale_wide(l.x, e0), scale_wide(l.y, e1))};
+              df2& x = acc[c8 * 4 + j / 2];
+              x = (MODE == 0) ? oz_accumulate<G>(x, v) : v;
             }
           }
         }
-        // the accumulators are free for the next group (and eb may be rewritten)
+        // the accumulators are free for the next group (and ebs may be rewritten)
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(&acc_empty);
         if (MODE == 1 && gm < a.Mvalid) {
-          // C -= product, 16 columns per batch of loads
+          if (a.c_fp64) {
+            // FP64 storage (a panel's own columns): one FP64 subtraction per element
+            double* cp = a.C64 + gn0 * a.ldc + gm;
 #pragma unroll
-          for (int c16 = 0; c16 < OZ_EPI_COLS / 16; ++c16) {
-            if (a.c_fp64) {
-              // FP64 storage (a panel's own columns): one FP64 subtraction per element
+            for (int c16 = 0; c16 < OZ_EPI_COLS; c16 += 16) {
               double cd[16];
 #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const int64_t gn = it.n0 + part * OZ_EPI_COLS + c16 * 16 + j;
-                cd[j] = (gn < a.Nvalid && !a.c_assign) ? a.C64[gn * a.ldc + gm] : 0.0;
-              }
+              for (int j = 0; j < 16; ++j) cd[j] = (c16 + j < nc && !a.c_assign) ? cp[(c16 + j) * a.ldc] : 0.0;
 #pragma unroll
               for (int j = 0; j < 16; ++j) {
-                const int64_t gn = it.n0 + part * OZ_EPI_COLS + c16 * 16 + j;
-                if (gn >= a.Nvalid) continue;
-                const double pv = df_to_double(acc[c16 * 16 + j]);
-                a.C64[gn * a.ldc + gm] = a.c_assign ? pv : cd[j] - pv;
+                if (c16 + j >= nc) continue;
+                const float2 h = unpack2(acc[(c16 + j) / 2].h), l = unpack2(acc[(c16 + j) / 2].l);
+                const double pv = df_to_double((j & 1) ? f2{h.y, l.y} : f2{h.x, l.x});
+                cp[(c16 + j) * a.ldc] = a.c_assign ? pv : cd[j] - pv;
               }
-              continue;
             }
-            float2 cv[16];
+          } else {
+            // C -= product, 16 columns per batch of loads
+            float2* cp = a.C + gn0 * a.ldc + gm;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int64_t gn = it.n0 + part * OZ_EPI_COLS + c16 * 16 + j;
-              cv[j] = (gn < a.Nvalid) ? a.C[gn * a.ldc + gm] : make_float2(0.0f, 0.0f);
-            }
+            for (int c16 = 0; c16 < OZ_EPI_COLS; c16 += 16) {
+              float2 cv[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int64_t gn = it.n0 + part * OZ_EPI_COLS + c16 * 16 + j;
-              if (gn >= a.Nvalid) continue;
-              const int64_t ci = gn * a.ldc + gm;
-              const f2 r = oz_subtract<G>({cv[j].x, cv[j].y}, acc[c16 * 16 + j]);
-              if (gm < a.fp64_rows) a.C64[ci] = df_to_double(r);
-              else a.C[ci] = make_float2(r.h, r.l);
+              for (int j = 0; j < 16; ++j) cv[j] = (c16 + j < nc) ? cp[(c16 + j) * a.ldc] : make_float2(0.0f, 0.0f);
+#pragma unroll
+              for (int j = 0; j < 16; j += 2) {
+                const df2 r = oz_subtract<G>({pack2(cv[j].x, cv[j + 1].x), pack2(cv[j].y, cv[j + 1].y)},
+                                             acc[(c16 + j) / 2]);
+                const float2 h = unpack2(r.h), l = unpack2(r.l);
+                cv[j] = make_float2(h.x, l.x);
+                cv[j + 1] = make_float2(h.y, l.y);
+              }
+              if (it.m0 >= a.fp64_rows) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                  if (c16 + j < nc) cp[(c16 + j) * a.ldc] = cv[j];
+              } else {
+                // the tile holds finished rows: tested here for the tile, since the
+                // FP64 addition of a row's test takes its slot also where it is off
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                  if (c16 + j >= nc) continue;
+                  double* cd = reinterpret_cast<double*>(cp + (c16 + j) * a.ldc);
+                  if (gm < a.fp64_rows) *cd = df_to_double({cv[j].x, cv[j].y});
+                  else *reinterpret_cast<float2*>(cd) = cv[j];
+                }
+              }
             }
           }
         }
       }
       if (MODE == 0 && !s_fail && gm < a.AR) {
-        float2* out = a.part + (int64_t)it.split * a.Nvalid * a.AR;
+        float2* out = a.part + ((int64_t)it.split * a.Nvalid + gn0) * a.AR + gm;
 #pragma unroll
         for (int j = 0; j < OZ_EPI_COLS; ++j) {
-          const int64_t gn = it.n0 + part * OZ_EPI_COLS + j;
-          if (gn < a.Nvalid) out[gn * a.AR + gm] = make_float2(acc[j].h, acc[j].l);
+          const float2 h = unpack2(acc[j / 2].h), l = unpack2(acc[j / 2].l);
+          if (j < nc) out[j * a.AR] = (j & 1) ? make_float2(h.y, l.y) : make_float2(h.x, l.x);
         }
       }
     }
@@ -939,6 +1007,33 @@ thread_local int t_oz_cap = 0;
 
 // one persistent CTA per SM at most (fewer under a cap), each taking every
 // gridDim-th work item
+static int64_t oz_ctas() {
+  const int64_t sms = num_sms_oz();
+  return (t_oz_cap > 0 && t_oz_cap < sms) ? t_oz_cap : sms;
+}
+
+// K groups of 128 rows per work item of Y^T C, for `groups` of them and ntiles
+// column tiles.  The CTAs take the items in turn, so the time is that of the
+// CTA with the most: rounds x (groups per item + what an item costs besides).
+// An item's partial tile, written once and read once by the reduction, takes
+// about 0.8 of a group's time.  Two rounds of equal items, whatever their
+// number came to, left 16384 x 8192 (86 tiles) at 96 groups per CTA, where
+// the mean is 72.4; this rule gives 76.
+static int64_t oz_groups_per_item(int64_t groups, int64_t ntiles) {
+  const int64_t ctas = oz_ctas();
+  int64_t best = groups;
+  double best_cost = 1e300;
+  for (int64_t ks = 1; ks <= groups && (ks == 1 || ntiles * (ks - 1) < 8 * ctas); ++ks) {
+    const int64_t per = (groups + ks - 1) / ks;
+    const int64_t items = ntiles * ((groups + per - 1) / per);
+    const double cost = (double)((items + ctas - 1) / ctas) * ((double)per + 0.8);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = per;
+    }
+  }
+  return best;
+}
 template <int S>
 static int launch_oz(OzArgs a, unsigned gm, unsigned gn, unsigned gk, int cls, double flops,
                      cudaStream_t s) {
@@ -949,13 +1044,10 @@ static int launch_oz(OzArgs a, unsigned gm, unsigned gn, unsigned gk, int cls, d
     CANDMC_CK(cudaFuncSetAttribute(k_oz_mma<1, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     attr = true;
   }
-  a.n_mt = gm;
-  a.n_nt = gn;
-  a.n_ks = gk;
-  const int64_t items = (int64_t)gm * gn * gk;
-  int64_t ctas = num_sms_oz();
-  if (t_oz_cap > 0 && t_oz_cap < ctas) ctas = t_oz_cap;
-  const unsigned grid = (unsigned)std::min<int64_t>(items, ctas);
+  a.n_mt = (int)gm;
+  a.n_nt = (int)gn;
+  a.n_ks = (int)gk;
+  const unsigned grid = (unsigned)std::min<int64_t>((int64_t)gm * gn * gk, oz_ctas());
   ProfScope ps(cls, flops, s);
   if (a.mode == 0)
     k_oz_mma<0, S><<<grid, OZ_THREADS, SMEM, s>>>(a);
@@ -985,15 +1077,13 @@ static int oz_tn(const SliceSrc& ysrc, const SliceSrc& csrc, int64_t m, int nb, 
   auto* cbs = static_cast<__nv_bfloat16*>(cb.p);
   CANDMC_RET(launch_slice_kcol<S>(ysrc, 0, m, nb, AR1, Kp1, (int)KG, yas, static_cast<int*>(ea.p), s));
   CANDMC_RET(launch_slice_kcol<S>(csrc, 0, m, n, BR1, Kp1, (int)KG, cbs, static_cast<int*>(eb.p), s));
-  // K split: about two waves of CTAs
   const int64_t ntiles = BR1 / OZ_N;
-  int64_t ksplit = std::max<int64_t>(1, std::min<int64_t>(Kp1 / KG, (2 * num_sms_oz() + ntiles - 1) / ntiles));
-  int64_t kper = rup((Kp1 + ksplit - 1) / ksplit, KG);
-  ksplit = (Kp1 + kper - 1) / kper;
+  const int64_t kper = KG * oz_groups_per_item(Kp1 / KG, ntiles);
+  const int64_t ksplit = (Kp1 + kper - 1) / kper;
   CANDMC_RET(part.alloc(sizeof(float2) * ksplit * n * AR1, s));
   OzArgs g1{};
-  g1.As = yas; g1.AR = AR1; g1.Bs = cbs; g1.BR = BR1; g1.Kpad = Kp1; g1.k_per_cta = kper;
-  g1.kgroup = KG; g1.eA = static_cast<int*>(ea.p); g1.eB = static_cast<int*>(eb.p);
+  g1.As = yas; g1.AR = AR1; g1.Bs = cbs; g1.BR = BR1; g1.Kpad = (int)Kp1; g1.k_per_cta = (int)kper;
+  g1.kgroup = (int)KG; g1.eA = static_cast<int*>(ea.p); g1.eB = static_cast<int*>(eb.p);
   g1.mode = 0; g1.part = static_cast<float2*>(part.p); g1.Mvalid = nb; g1.Nvalid = n;
   g1.status = status;
   CANDMC_RET(launch_oz<S>(g1, 1, (unsigned)ntiles, (unsigned)ksplit, cls, 2.0 * nb * n * m, s));
@@ -1030,7 +1120,7 @@ static int oz_top_times(MatRef Top, int nb, const double* Z, int64_t n, double* 
                                   static_cast<int*>(ez.p), s));
   OzArgs g{};
   g.As = tas; g.AR = OZ_M; g.Bs = zbs; g.BR = BR;
-  g.Kpad = Kp; g.k_per_cta = Kp; g.kgroup = Kp;
+  g.Kpad = g.k_per_cta = g.kgroup = (int)Kp;
   g.eA = static_cast<int*>(et.p); g.eB = static_cast<int*>(ez.p);
   g.mode = 1; g.C = reinterpret_cast<float2*>(Zt); g.C64 = Zt; g.ldc = nb;
   g.Mvalid = nb; g.Nvalid = n; g.fp64_rows = 0; g.status = status;
@@ -1084,7 +1174,7 @@ static int apply_qt_slices(const double* Y, int64_t ldy, int ymask, int64_t m, i
   OzArgs g2{};
   g2.As = static_cast<__nv_bfloat16*>(y2.p); g2.AR = AR2;
   g2.Bs = static_cast<__nv_bfloat16*>(z2.p); g2.BR = BR2;
-  g2.Kpad = Kp2; g2.k_per_cta = Kp2; g2.kgroup = Kp2;
+  g2.Kpad = g2.k_per_cta = g2.kgroup = (int)Kp2;
   g2.eA = static_cast<int*>(ey2.p); g2.eB = static_cast<int*>(ez2.p);
   g2.mode = 1; g2.C = reinterpret_cast<float2*>(C); g2.C64 = C; g2.ldc = ldc;
   g2.Mvalid = m; g2.Nvalid = n; g2.fp64_rows = fp64_rows; g2.status = status;

@@ -1,0 +1,66 @@
+"""The emulated-FP64 contractions at the edges of their tiles, K groups, K
+splits and scale exponents.
+
+C - Y (Y^T C) / 2 (the operator is the inverse of W = 2 I) against numpy in
+FP64.  The bound is worked out from the
+format, per element.  An operand entry is its digits to half a unit of the
+last one, 2^-57 of its scale, which is at most twice its row's largest entry;
+the slice products left out come to less than 2^-55 of both scales: together
+less than 2^-52 max|x| max|y| per product.  Float pairs, the exact combine of
+the accumulators and the pair additions round at 2^-46, which over a sum is
+taken as 2^-44 of sum |x||y|.  A float pair resolves 2^-149.  The reference's
+own k-term sums are within k 2^-53 sum |x||y|.
+"""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def cm():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import candmc_gb300 as cm
+    cm.lib()
+    return cm
+
+
+def dev(a):
+    return torch.from_numpy(np.asfortranarray(a)).cuda().t().contiguous().t()
+
+
+def product_bound(X, Y, dX, dY):
+    """|error| of the emulated X Y for operands with errors dX, dY."""
+    k = X.shape[1]
+    a = np.abs(X) @ np.abs(Y)
+    scales = np.abs(X).max(axis=1, keepdims=True) * np.abs(Y).max(axis=0, keepdims=True)
+    return k * 2.0 ** -52 * scales + (2.0 ** -44 + k * 2.0 ** -53) * a + dX @ np.abs(Y) + np.abs(X) @ dY
+
+
+# rows: one group of 128, one more or less, 16-row blocks, many K splits (157
+# groups); columns: 96-column tiles, below and from 1024 columns (the operator
+# product on the tensor cores); panel widths: 8-row core matrices, 16-deep K steps
+@pytest.mark.parametrize("m,nb,n", [(1, 1, 1), (128, 16, 96), (129, 17, 97), (127, 8, 95), (255, 128, 193),
+                                    (656, 9, 1100), (1000, 100, 1024), (20000, 128, 30), (20090, 33, 289)])
+@pytest.mark.parametrize("scales", [(0,), (0, -60, 60, -112)])
+def test_update_edges(cm, m, nb, n, scales):
+    g = np.random.default_rng(m + nb + n)
+    Y = g.standard_normal((m, nb)) / np.sqrt(m)
+    C = np.ldexp(g.standard_normal((m, n)), np.resize(scales, n)[None, :])
+    if n > 2:
+        C[:, 2] = 0.0
+    out = dev(C)
+    cm.upd_A(dev(Y), out, W=dev(2.0 * np.eye(nb)), W_is_T=True, precision="ozaki")
+    tiny = 2.0 ** -148
+    zero = lambda a: np.zeros_like(a)
+    Z = Y.T @ C
+    dZ = product_bound(Y.T, C, zero(Y.T), np.full_like(C, tiny)) + tiny
+    T = 0.5 * np.eye(nb)
+    Z2 = T @ Z
+    dZ2 = product_bound(T, Z, zero(T), dZ) + tiny
+    want = C - Y @ Z2
+    bound = product_bound(Y, Z2, zero(Y), dZ2) + 2.0 ** -46 * (np.abs(C) + np.abs(Y @ Z2)) + 4 * tiny
+    got = out.cpu().numpy()
+    assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
