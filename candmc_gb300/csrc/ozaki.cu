@@ -136,15 +136,41 @@ __device__ __forceinline__ double widen(float f) {
 
 __device__ __forceinline__ double df_to_double(f2 x) { return widen(x.h) + widen(x.l); }
 
+// Two floats in one 64-bit register: the f32x2 instructions round each half
+// as the scalar ones do and take one issue slot for both.
+struct f2x2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ f2x2 pack2(float a, float b) {
+  f2x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f2x2 x) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x.v));
+  return r;
+}
+__device__ __forceinline__ f2x2 add2(f2x2 a, f2x2 b) {
+  f2x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f2x2 mul2(f2x2 a, f2x2 b) {
+  f2x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f2x2 sub2(f2x2 a, f2x2 b) {   // a - b, rounded once
+  f2x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(b.v), "l"(0xbf800000bf800000ull), "l"(a.v));
+  return r;
+}
+
 // ------------------------------------------------------------------ slicing
 // 2^e for -126 <= e <= 127 (a normal float): x * pow2f(e) rounds once, as
 // ldexpf(x, e) does
 __device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }
-
-// x * 2^k rounded once: one multiplication when 2^k is a normal float
-__device__ __forceinline__ float scale_pow2(float x, int k) {
-  return (k >= -126 && k <= 127) ? __fmul_rn(x, pow2f(k)) : ldexpf(x, k);
-}
 
 // Scale exponent of a group maximum: smallest e with max < 2^e (0 for 0).
 __device__ __forceinline__ int scale_exp(float mx) {
@@ -154,20 +180,28 @@ __device__ __forceinline__ int scale_exp(float mx) {
   return e;
 }
 
-// Write the S natural-weight digits of v = (h + l) * 2^(8 - e) to slices.
-template <int S>
-__device__ __forceinline__ void slice_value(f2 v, int e, __nv_bfloat16* out, int64_t plane,
-                                            int64_t off) {
-  float p = scale_pow2(v.h, 8 - e), q = scale_pow2(v.l, 8 - e);
-  float w = 1.0f;
+// The S digits of two values (p + q scaled below 2^8, |q| at most half an ulp
+// of p), each at its natural weight 2^(-8i): digit i is the rest rounded to a
+// multiple of that weight by adding and taking away 1.5 * 2^(23 - 8i), and the
+// rest stays exact.  The low word comes in before every second digit: a rest
+// below 2^(-8i-1) and a q below half an ulp of it are still balanced digits.
+// put(i, d) takes the digits of both values.
+template <int S, class Put>
+__device__ __forceinline__ void slice_digits(f2x2 p, f2x2 q, Put put) {
 #pragma unroll
   for (int i = 0; i < S; ++i) {
-    f2 s = two_sum(p, q);
-    float d = rintf(s.h);
-    out[i * plane + off] = __float2bfloat16_rn(d * w);
-    p = (s.h - d) * 256.0f;
-    q = s.l * 256.0f;
-    w *= 0.00390625f;
+    if (i > 0 && i == S - 1) {
+      p = add2(p, q);
+    } else if (i > 0 && i % 2 == 0) {
+      const f2x2 t = add2(p, q);
+      q = sub2(q, sub2(t, p));
+      p = t;
+    }
+    const float m = 12582912.0f * __int_as_float((127 - 8 * i) << 23);
+    const f2x2 shift = pack2(m, m);
+    const f2x2 d = sub2(add2(p, shift), shift);
+    put(i, d);
+    if (i + 1 < S) p = sub2(p, d);
   }
 }
 
@@ -194,138 +228,92 @@ __device__ __forceinline__ f2 src_at(const SliceSrc& s, int64_t r, int64_t c) {
   return df_from_double(x);
 }
 
-// Operand element (n, k) = src(k, n): K runs down the columns of a column-major
-// source (rows k0 .. k0 + K).  One warp per (n, K group of G); n in [0, Nvalid)
-// are data, rows beyond are zero padding up to Rpad; k beyond Kvalid are zero.
-// Slices: S planes of Rpad x Kpad (cm order); exponents e[(k/G) * Rpad + n].
-template <int S>
-__global__ void k_slice_kcol(SliceSrc src, int64_t k0, int64_t Kvalid, int64_t Nvalid, int64_t Rpad,
-                             int64_t Kpad, int G, __nv_bfloat16* out, int* eout) {
-  const int lane = threadIdx.x & 31;
-  const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t ngroups = Kpad / G;
-  if (wid >= Rpad * ngroups) return;
-  const int64_t n = wid % Rpad, g = wid / Rpad;
-  const int64_t plane = Rpad * Kpad;
-  float mx = 0.0f;
-  if (n < Nvalid) {
-    for (int64_t k = g * G + lane; k < (g + 1) * G && k < Kvalid; k += 32) {
-      f2 v = src_at(src, k0 + k, n);
-      mx = fmaxf(mx, fabsf(v.h));
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  // the lo part can push |x| just above |hi|'s bound; leave one ulp of room
-  const int e = scale_exp(mx * (1.0f + 1.0e-6f));
-  if (lane == 0) eout[g * Rpad + n] = e;
-  for (int64_t k = g * G + lane; k < (g + 1) * G; k += 32) {
-    f2 v = {0.0f, 0.0f};
-    if (n < Nvalid && k < Kvalid) v = src_at(src, k0 + k, n);
-    slice_value<S>(v, e, out, plane, cm_off(n, k, Rpad));
-  }
-}
+// Slices of an R x K operand (rows n, the contraction index k), with one scale
+// exponent per row and K group of G (a multiple of 16, at most 128).  Element
+// (n, k) is src(k, n) (KROW = false: K runs down the source's columns) or
+// src(n, k) (KROW = true: K runs along its rows); rows from Nvalid to Rpad
+// and k from Kvalid on are zero.  Slices: S planes of Rpad x Kpad in the
+// core-matrix order; exponents e[(k / G) * Rpad + n].
+// A CTA takes kSliceRows rows and one group: it stages the group in shared
+// memory, warp w finds the exponents of rows 2w and 2w + 1, and then the
+// 16 x 16 elements of K16 block w are, in every plane, one contiguous 512-byte
+// run, of which a lane writes the 16 bytes of 8 consecutive k.  The rows' pitch
+// shifts a row by 16 bytes, so the lanes' 16-byte reads (8 rows at one k)
+// fall on different banks.  Bound by memory (8 bytes read and 2 S written per
+// element) once the digits take some 15 issue slots: at about 100, one TwoSum
+// for each, 16384 x 8192 elements took 599 us, with 8-way bank conflicts.
+constexpr int kSliceRows = 16;
 
-// The same slicing with coalesced stores: one CTA per 8 rows n of the operand
-// (one core-matrix row block) and one K group of G <= 128 (a multiple of 16).
-// Warp w reads column n0 + w of the source into shared memory and finds its
-// scale exponent; then, for every K16 block, the 8 x 16 elements of a slice
-// plane are one contiguous 256-byte run of the core-matrix order, which a
-// warp writes with 8-byte stores (4 elements per lane).
-template <int S>
-__global__ void __launch_bounds__(256) k_slice_kcol8(SliceSrc src, int64_t k0, int64_t Kvalid,
-                                                     int64_t Nvalid, int64_t Rpad, int64_t Kpad, int G,
-                                                     __nv_bfloat16* out, int* eout) {
-  __shared__ float2 tile[8][128];
-  __shared__ int s_e[8];
+template <int S, bool KROW>
+__global__ void __launch_bounds__(256) k_slice(SliceSrc src, int64_t Kvalid, int64_t Nvalid,
+                                               int64_t Rpad, int64_t Kpad, int G, __nv_bfloat16* out, int* eout) {
+  __shared__ __align__(16) float2 tile[kSliceRows][128 + 2];
+  __shared__ int s_e[kSliceRows];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t n0 = (int64_t)blockIdx.x * 8;
-  const int64_t g = blockIdx.y;
-  const int64_t kb0 = g * G;
-  {
-    const int64_t n = n0 + warp;
-    float mx = 0.0f;
-    for (int k = lane; k < G; k += 32) {
-      f2 v = {0.0f, 0.0f};
-      if (n < Nvalid && kb0 + k < Kvalid) v = src_at(src, k0 + kb0 + k, n);
-      tile[warp][k] = make_float2(v.h, v.l);
-      mx = fmaxf(mx, fabsf(v.h));
+  const unsigned nblocks = (unsigned)((Rpad + kSliceRows - 1) / kSliceRows);
+  const int64_t n0 = (int64_t)(blockIdx.x % nblocks) * kSliceRows;
+  const int64_t g = blockIdx.x / nblocks, kb0 = g * G;
+  if (KROW) {
+    const int r = threadIdx.x & 15;
+    f2 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int k = (threadIdx.x >> 4) + 16 * u;
+      v[u] = {0.0f, 0.0f};
+      if (k < G && n0 + r < Nvalid && kb0 + k < Kvalid) v[u] = src_at(src, n0 + r, kb0 + k);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    for (int u = 0; u < 8; ++u) tile[r][(threadIdx.x >> 4) + 16 * u] = make_float2(v[u].h, v[u].l);
+  } else {
+    f2 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int64_t n = n0 + 2 * warp + (u >> 2);
+      const int k = lane + 32 * (u & 3);
+      v[u] = {0.0f, 0.0f};
+      if (k < G && n < Nvalid && kb0 + k < Kvalid) v[u] = src_at(src, kb0 + k, n);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) tile[2 * warp + (u >> 2)][lane + 32 * (u & 3)] = make_float2(v[u].h, v[u].l);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int r = 2 * warp + u;
+    float mx = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 128; k += 32) mx = fmaxf(mx, fabsf(tile[r][k + lane].x));
+    mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
     // the lo part can push |x| just above |hi|'s bound; leave one ulp of room
     const int e = scale_exp(mx * (1.0f + 1.0e-6f));
     if (lane == 0) {
-      s_e[warp] = e;
-      if (n < Rpad) eout[g * Rpad + n] = e;
+      s_e[r] = e;
+      if (n0 + r < Rpad) eout[g * Rpad + n0 + r] = e;
     }
   }
   __syncthreads();
+  const int r = (lane >> 4) * 8 + (lane & 7), khalf = (lane >> 3) & 1;
+  if (n0 + r >= Rpad || warp >= G / 16) return;
+  // 2^(8 - e) as two normal factors, the second one 1 unless e < -119
+  const int k1 = min(8 - s_e[r], 127);
+  const float f1 = pow2f(k1), f2v = pow2f(8 - s_e[r] - k1);
+  const f2x2 sc1 = pack2(f1, f1), sc2 = pack2(f2v, f2v);
+  const float4* t4 = reinterpret_cast<const float4*>(&tile[r][warp * 16 + khalf * 8]);
+  uint32_t d[S][4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const float4 x = t4[c];
+    slice_digits<S>(mul2(mul2(pack2(x.x, x.z), sc1), sc2), mul2(mul2(pack2(x.y, x.w), sc1), sc2),
+                    [&](int i, f2x2 v) {
+                      const float2 w = unpack2(v);
+                      asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d[i][c]) : "f"(w.y), "f"(w.x));
+                    });
+  }
   const int64_t plane = Rpad * Kpad;
-  // lane u of a warp: elements 4u .. 4u+3 of a 128-element core-matrix run:
-  // k-half (u / 16), row (u % 16) / 2, k & 7 = 4 (u % 2) .. +3
-  const int u = lane;
-  const int khalf = u >> 4, r = (u & 15) >> 1, k7 = (u & 1) * 4;
-  const int e = s_e[r];
-  for (int blk = warp; blk < G / 16; blk += 8) {
-    float p[4], q[4];
+  __nv_bfloat16* o = out + ((kb0 >> 4) + warp) * (Rpad * 16) + ((n0 >> 3) + (lane >> 4)) * 128 + khalf * 64 + (lane & 7) * 8;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 t = tile[r][blk * 16 + khalf * 8 + k7 + i];
-      p[i] = scale_pow2(t.x, 8 - e);
-      q[i] = scale_pow2(t.y, 8 - e);
-    }
-    const int64_t base = ((kb0 >> 4) + blk) * (Rpad * 16) + (n0 >> 3) * 128 + 4 * u;
-    float w = 1.0f;
-#pragma unroll
-    for (int sl = 0; sl < S; ++sl) {
-      __align__(8) __nv_bfloat16 d4[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const f2 sv = two_sum(p[i], q[i]);
-        const float d = rintf(sv.h);
-        d4[i] = __float2bfloat16_rn(d * w);
-        p[i] = (sv.h - d) * 256.0f;
-        q[i] = sv.l * 256.0f;
-      }
-      *reinterpret_cast<uint2*>(out + sl * plane + base) = *reinterpret_cast<const uint2*>(d4);
-      w *= 0.00390625f;
-    }
-  }
-}
-
-// Operand element (n, k) = src(n, k): K runs along the rows of a column-major
-// source (rows n0 + n, columns 0 .. K).  Scale group = the whole row (G = Kpad).
-// A CTA stages 32 rows x Kpad columns through shared memory.
-template <int S>
-__global__ void k_slice_krow(SliceSrc src, int64_t n0, int64_t Nvalid, int64_t Kvalid, int64_t Rpad,
-                             int64_t Kpad, __nv_bfloat16* out, int* eout) {
-  extern __shared__ float2 tile[];   // [32][Kpad]
-  const int64_t nb = (int64_t)blockIdx.x * 32;
-  for (int64_t idx = threadIdx.x; idx < 32 * Kpad; idx += blockDim.x) {
-    int64_t rr = idx % 32, k = idx / 32;
-    int64_t n = nb + rr;
-    f2 v = {0.0f, 0.0f};
-    if (n < Nvalid && k < Kvalid) v = src_at(src, n0 + n, k);
-    tile[rr * Kpad + k] = make_float2(v.h, v.l);
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int64_t plane = Rpad * Kpad;
-  for (int rr = warp; rr < 32; rr += nw) {
-    const int64_t n = nb + rr;
-    if (n >= Rpad) continue;
-    float mx = 0.0f;
-    for (int64_t k = lane; k < Kpad; k += 32) mx = fmaxf(mx, fabsf(tile[rr * Kpad + k].x));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    const int e = scale_exp(mx * (1.0f + 1.0e-6f));
-    if (lane == 0) eout[n] = e;
-    for (int64_t k = lane; k < Kpad; k += 32) {
-      float2 t = tile[rr * Kpad + k];
-      slice_value<S>({t.x, t.y}, e, out, plane, cm_off(n, k, Rpad));
-    }
-  }
+  for (int i = 0; i < S; ++i)
+    *reinterpret_cast<uint4*>(o + i * plane) = make_uint4(d[i][0], d[i][1], d[i][2], d[i][3]);
 }
 
 // ------------------------------------------------------------------ tcgen05 kernel
@@ -380,37 +368,6 @@ constexpr int OZ_EPI_COLS = OZ_N * 4 / OZ_EPI_WARPS;  // accumulator columns per
 constexpr int OZ_WARPS = 2 + OZ_EPI_WARPS;             // producer, MMA issuer, epilogue
 constexpr int OZ_THREADS = OZ_WARPS * 32;
 static_assert(OZ_EPI_WARPS % 4 == 0 && OZ_EPI_COLS == 32, "epilogue split: one column per lane for the exponents");
-
-// Two floats in one 64-bit register: the f32x2 instructions round each half
-// as the scalar ones do and take one issue slot for both.
-struct f2x2 {
-  unsigned long long v;
-};
-__device__ __forceinline__ f2x2 pack2(float a, float b) {
-  f2x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(f2x2 x) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x.v));
-  return r;
-}
-__device__ __forceinline__ f2x2 add2(f2x2 a, f2x2 b) {
-  f2x2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ f2x2 mul2(f2x2 a, f2x2 b) {
-  f2x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
-  return r;
-}
-__device__ __forceinline__ f2x2 sub2(f2x2 a, f2x2 b) {   // a - b, rounded once
-  f2x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(b.v), "l"(0xbf800000bf800000ull), "l"(a.v));
-  return r;
-}
 
 // two df64 values: high words, low words
 struct df2 {
@@ -973,33 +930,27 @@ int from_df64(double* X, int64_t ld, int64_t m, int64_t n, cudaStream_t s) {
   return CANDMC_OK;
 }
 
-template <int S>
-static int launch_slice_kcol(SliceSrc src, int64_t k0, int64_t Kvalid, int64_t Nvalid, int64_t Rpad,
-                             int64_t Kpad, int G, __nv_bfloat16* out, int* e, cudaStream_t s) {
+// KROW and the other arguments as in k_slice; Kpad is a multiple of G
+template <int S, bool KROW>
+static int launch_slice(SliceSrc src, int64_t Kvalid, int64_t Nvalid, int64_t Rpad, int64_t Kpad, int G,
+                        __nv_bfloat16* out, int* e, cudaStream_t s) {
   ProfScope ps(CANDMC_KCLASS_OZ_SLICE, 8.0 * Nvalid * Kvalid + 2.0 * S * Rpad * Kpad, s);
-  if (G <= 128 && G % 16 == 0 && Rpad % 8 == 0) {
-    k_slice_kcol8<S><<<dim3((unsigned)(Rpad / 8), (unsigned)(Kpad / G)), 256, 0, s>>>(src, k0, Kvalid, Nvalid,
-                                                                                  Rpad, Kpad, G, out, e);
-    CANDMC_CK(cudaGetLastError());
-    return CANDMC_OK;
-  }
-  int64_t warps = Rpad * (Kpad / G);
-  k_slice_kcol<S><<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s>>>(src, k0, Kvalid, Nvalid, Rpad,
-                                                                      Kpad, G, out, e);
+  const int64_t ctas = (Rpad + kSliceRows - 1) / kSliceRows * (Kpad / G);
+  k_slice<S, KROW><<<(unsigned)ctas, 256, 0, s>>>(src, Kvalid, Nvalid, Rpad, Kpad, G, out, e);
   CANDMC_CK(cudaGetLastError());
   return CANDMC_OK;
 }
 
 template <int S>
-static int launch_slice_krow(SliceSrc src, int64_t n0, int64_t Nvalid, int64_t Kvalid, int64_t Rpad,
-                             int64_t Kpad, __nv_bfloat16* out, int* e, cudaStream_t s) {
-  size_t sm = sizeof(float2) * 32 * (size_t)Kpad;
-  if (sm > 48 * 1024)
-    CANDMC_CK(cudaFuncSetAttribute(k_slice_krow<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  ProfScope ps(CANDMC_KCLASS_OZ_SLICE, 8.0 * Nvalid * Kvalid + 2.0 * S * Rpad * Kpad, s);
-  k_slice_krow<S><<<(unsigned)((Rpad + 31) / 32), 256, sm, s>>>(src, n0, Nvalid, Kvalid, Rpad, Kpad, out, e);
-  CANDMC_CK(cudaGetLastError());
-  return CANDMC_OK;
+static int launch_slice_cols(SliceSrc src, int64_t Kvalid, int64_t Nvalid, int64_t Rpad, int64_t Kpad, int G,
+                             __nv_bfloat16* out, int* e, cudaStream_t s) {
+  return launch_slice<S, false>(src, Kvalid, Nvalid, Rpad, Kpad, G, out, e, s);
+}
+
+template <int S>
+static int launch_slice_rows(SliceSrc src, int64_t Kvalid, int64_t Nvalid, int64_t Rpad, int64_t Kpad, int G,
+                             __nv_bfloat16* out, int* e, cudaStream_t s) {
+  return launch_slice<S, true>(src, Kvalid, Nvalid, Rpad, Kpad, G, out, e, s);
 }
 
 int g_oz_reserve_sms = 32;
@@ -1075,8 +1026,8 @@ static int oz_tn(const SliceSrc& ysrc, const SliceSrc& csrc, int64_t m, int nb, 
   CANDMC_RET(eb.alloc(sizeof(int) * (Kp1 / KG) * BR1, s));
   auto* yas = static_cast<__nv_bfloat16*>(ya.p);
   auto* cbs = static_cast<__nv_bfloat16*>(cb.p);
-  CANDMC_RET(launch_slice_kcol<S>(ysrc, 0, m, nb, AR1, Kp1, (int)KG, yas, static_cast<int*>(ea.p), s));
-  CANDMC_RET(launch_slice_kcol<S>(csrc, 0, m, n, BR1, Kp1, (int)KG, cbs, static_cast<int*>(eb.p), s));
+  CANDMC_RET(launch_slice_cols<S>(ysrc, m, nb, AR1, Kp1, (int)KG, yas, static_cast<int*>(ea.p), s));
+  CANDMC_RET(launch_slice_cols<S>(csrc, m, n, BR1, Kp1, (int)KG, cbs, static_cast<int*>(eb.p), s));
   const int64_t ntiles = BR1 / OZ_N;
   const int64_t kper = KG * oz_groups_per_item(Kp1 / KG, ntiles);
   const int64_t ksplit = (Kp1 + kper - 1) / kper;
@@ -1113,10 +1064,10 @@ static int oz_top_times(MatRef Top, int nb, const double* Z, int64_t n, double* 
   // A operand element (i, k) = Top(i, k): X[k, i] of a transposed reference
   // (a column of X per operand row), X[i, k] otherwise (a row of X)
   if (Top.trans)
-    CANDMC_RET(launch_slice_kcol<S>(tsrc, 0, nb, nb, OZ_M, Kp, (int)Kp, tas, static_cast<int*>(et.p), s));
+    CANDMC_RET(launch_slice_cols<S>(tsrc, nb, nb, OZ_M, Kp, (int)Kp, tas, static_cast<int*>(et.p), s));
   else
-    CANDMC_RET(launch_slice_krow<S>(tsrc, 0, nb, nb, OZ_M, Kp, tas, static_cast<int*>(et.p), s));
-  CANDMC_RET(launch_slice_kcol<S>(SliceSrc{Z, nullptr, nb, kDense, 0}, 0, nb, n, BR, Kp, (int)Kp, zbs,
+    CANDMC_RET(launch_slice_rows<S>(tsrc, nb, nb, OZ_M, Kp, (int)Kp, tas, static_cast<int*>(et.p), s));
+  CANDMC_RET(launch_slice_cols<S>(SliceSrc{Z, nullptr, nb, kDense, 0}, nb, n, BR, Kp, (int)Kp, zbs,
                                   static_cast<int*>(ez.p), s));
   OzArgs g{};
   g.As = tas; g.AR = OZ_M; g.Bs = zbs; g.BR = BR;
@@ -1166,10 +1117,10 @@ static int apply_qt_slices(const double* Y, int64_t ldy, int ymask, int64_t m, i
   CANDMC_RET(ey2.alloc(sizeof(int) * AR2, s));
   CANDMC_RET(z2.alloc(sizeof(__nv_bfloat16) * S * BR2 * Kp2, s));
   CANDMC_RET(ez2.alloc(sizeof(int) * BR2, s));
-  CANDMC_RET(launch_slice_krow<S>(ysrc, 0, m, nb, AR2, Kp2, static_cast<__nv_bfloat16*>(y2.p),
+  CANDMC_RET(launch_slice_rows<S>(ysrc, nb, m, AR2, Kp2, (int)Kp2, static_cast<__nv_bfloat16*>(y2.p),
                                static_cast<int*>(ey2.p), s));
   SliceSrc zsrc{zt.d(), nullptr, nb, kDense, 0};
-  CANDMC_RET(launch_slice_kcol<S>(zsrc, 0, nb, n, BR2, Kp2, (int)Kp2, static_cast<__nv_bfloat16*>(z2.p),
+  CANDMC_RET(launch_slice_cols<S>(zsrc, nb, n, BR2, Kp2, (int)Kp2, static_cast<__nv_bfloat16*>(z2.p),
                                static_cast<int*>(ez2.p), s));
   OzArgs g2{};
   g2.As = static_cast<__nv_bfloat16*>(y2.p); g2.AR = AR2;
