@@ -18,19 +18,22 @@
 // split, fast TwoSum), scaled by a power of two and accumulated or subtracted
 // in df64.  Finished rows (the panel's R block) are written back as FP64.
 //
-// Kernel layout (k_oz_mma): persistent CTAs (at most one per SM) over work
-// items of one 128 x 96 output tile and K range each; 14 warps.  Operand
-// slices are pre-sliced in global memory in the UMMA "K-major, no swizzle"
-// core-matrix order, so each K16 step of a tile is a contiguous 4 KB (A, 128
-// rows) and 3 KB (B, 96 rows) block per slice: a producer warp streams them
-// with bulk asynchronous copies into a 4-stage shared-memory ring, an MMA
-// warp issues the 28 tcgen05.mma of a step and commits them to the stage's
-// "empty" mbarrier (and, at the end of an exact-accumulation group, to the
-// epilogue's "full" mbarrier), and twelve epilogue warps drain and combine
-// the accumulators and release them; the df64 read-modify-write of C (MODE
-// 1) then overlaps the next group's MMAs.  Every wait is bounded; a wait that
-// runs out sets the status word, the roles stop, the MMA warp waits for its
-// last MMAs, and the CTA frees its TMEM and returns.
+// Kernel layout: persistent CTAs (at most one per SM) over work items of one
+// 128 x 96 output tile and K range each; 14 warps.  k_oz_mma takes operand
+// slices from global memory in the UMMA "K-major, no swizzle" core-matrix
+// order, so each K16 step of a tile is a contiguous 4 KB (A, 128 rows) and 3 KB
+// (B, 96 rows) block per slice: a producer warp streams them with bulk
+// asynchronous copies into a 4-stage shared-memory ring, an MMA warp issues the
+// 28 tcgen05.mma of a step and commits them to the stage's "empty" mbarrier
+// (and, at the end of an exact-accumulation group, to the epilogue's "full"
+// mbarrier), and twelve epilogue warps drain and combine the accumulators and
+// release them; the read-modify-write of C then overlaps the next group's MMAs.
+// k_oz_tn (Y^T C for float pairs) has only A sliced beforehand: its twelve warps
+// slice C on the way.  Every wait is bounded; a wait that runs out sets the
+// status word, the roles stop, the MMA warp waits for its last MMAs, and the CTA
+// frees its TMEM and returns.  Both kernels are kept short: what runs once per
+// group costs some 30 cycles an instruction where the loop does not fit the
+// instruction cache.
 #include <cuda_bf16.h>
 #include <math.h>
 
@@ -56,7 +59,7 @@ struct OzCfg {
   static constexpr int STAGE_BYTES = S * (OZ_ABYTES + OZ_BBYTES);
   static constexpr int SMEM = OZ_STAGES * STAGE_BYTES + 1024;
 };
-constexpr long OZ_WAIT_LIMIT = 1L << 22;                // bounded mbarrier polls
+constexpr int OZ_WAIT_LIMIT = 1 << 22;                // bounded mbarrier polls
 
 // element (r, k) of an R x K operand slice plane in core-matrix K-major order
 __host__ __device__ __forceinline__ int64_t cm_off(int64_t r, int64_t k, int64_t R) {
@@ -124,14 +127,15 @@ __device__ __forceinline__ f2 df_from_double(double x) {
   return {h, l};
 }
 
-// A float as a double by its bits (no FP64 conversion) where it is normal or zero.
+// A float as a double by its bits (no FP64 conversion): a subnormal is scaled to
+// a normal float first, and the exponent of an infinity or NaN becomes the double's.
 __device__ __forceinline__ double widen(float f) {
-  const unsigned i = __float_as_uint(f), m = i & 0x7fffffffu;
-  if (m - 0x00800000u < 0x7f000000u) {
-    return __hiloint2double((int)((m >> 3) + 0x38000000u | (i & 0x80000000u)), (int)(i << 29));
-  }
-  if (m == 0) return __hiloint2double((int)i, 0);
-  return (double)f;
+  const bool sub = (__float_as_uint(f) & 0x7f800000u) == 0;
+  const unsigned i = __float_as_uint(sub ? __fmul_rn(f, 18446744073709551616.0f) : f), m = i & 0x7fffffffu;   // 2^64
+  unsigned h = (m >> 3) + (sub ? 0x38000000u - (64u << 20) : 0x38000000u);
+  if (m >= 0x7f800000u) h += 0x38000000u;
+  if (m == 0) h = 0;
+  return __hiloint2double((int)(h | (i & 0x80000000u)), (int)(i << 29));
 }
 
 __device__ __forceinline__ double df_to_double(f2 x) { return widen(x.h) + widen(x.l); }
@@ -172,12 +176,13 @@ __device__ __forceinline__ f2x2 sub2(f2x2 a, f2x2 b) {   // a - b, rounded once
 // ldexpf(x, e) does
 __device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }
 
-// Scale exponent of a group maximum: smallest e with max < 2^e (0 for 0).
+// Scale exponent of a group maximum: smallest e with max < 2^e (0 for 0 and for
+// an infinity), from the bits (frexpf took 700 cycles where it stands between
+// two groups of a contraction).
 __device__ __forceinline__ int scale_exp(float mx) {
-  if (!(mx > 0.0f)) return 0;
-  int e;
-  frexpf(mx, &e);   // mx = f * 2^e, f in [0.5, 1)
-  return e;
+  const unsigned b = __float_as_uint(mx);
+  if (!(mx > 0.0f) || b >= 0x7f800000u) return 0;
+  return b >= 0x00800000u ? (int)(b >> 23) - 126 : 32 - __clz((int)b) - 149;
 }
 
 // The S digits of two values (p + q scaled below 2^8, |q| at most half an ulp
@@ -203,6 +208,14 @@ __device__ __forceinline__ void slice_digits(f2x2 p, f2x2 q, Put put) {
     put(i, d);
     if (i + 1 < S) p = sub2(p, d);
   }
+}
+
+// Two digits as BF16: they have at most 8 significant bits, so the upper halves
+// of the floats are exact (a conversion takes a quarter-rate slot, this a byte
+// permutation; a NaN keeps its quiet bit there).
+__device__ __forceinline__ uint32_t to_bf16x2(f2x2 v) {
+  const float2 w = unpack2(v);
+  return __byte_perm(__float_as_uint(w.x), __float_as_uint(w.y), 0x7632);
 }
 
 struct SliceSrc {
@@ -304,10 +317,7 @@ __global__ void __launch_bounds__(256) k_slice(SliceSrc src, int64_t Kvalid, int
   for (int c = 0; c < 4; ++c) {
     const float4 x = t4[c];
     slice_digits<S>(mul2(mul2(pack2(x.x, x.z), sc1), sc2), mul2(mul2(pack2(x.y, x.w), sc1), sc2),
-                    [&](int i, f2x2 v) {
-                      const float2 w = unpack2(v);
-                      asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d[i][c]) : "f"(w.y), "f"(w.x));
-                    });
+                    [&](int i, f2x2 v) { d[i][c] = to_bf16x2(v); });
   }
   const int64_t plane = Rpad * Kpad;
   __nv_bfloat16* o = out + ((kb0 >> 4) + warp) * (Rpad * 16) + ((n0 >> 3) + (lane >> 4)) * 128 + khalf * 64 + (lane & 7) * 8;
@@ -320,22 +330,21 @@ __global__ void __launch_bounds__(256) k_slice(SliceSrc src, int64_t Kvalid, int
 struct OzArgs {
   const __nv_bfloat16* As;   // A-operand slices: S planes of AR x Kpad
   int64_t AR;
-  const __nv_bfloat16* Bs;   // B-operand slices: S planes of BR x Kpad
+  const __nv_bfloat16* Bs;   // k_oz_mma: B-operand slices, S planes of BR x Kpad
   int64_t BR;
-  int Kpad;                  // multiple of 16
-  int k_per_cta;             // K extent of one CTA (multiple of kgroup)
-  int kgroup;                // K rows per scale group / accumulator readout
+  int Kpad;                  // multiple of 16 (k_oz_tn: of 128)
+  int k_per_cta;             // K extent of one work item (multiple of kgroup)
+  int kgroup;                // K rows per scale group / accumulator readout (k_oz_tn: 128)
   const int* eA;             // [Kpad / kgroup][AR]
-  const int* eB;             // [Kpad / kgroup][BR]
-  int mode;                  // 0: partial sums (df64) over the CTA's K range; 1: C -= product
-  float2* part;              // mode 0: [split][Nvalid][AR] (ld AR per column)
-  float2* C;                 // mode 1: df64 matrix (ld ldc)
-  double* C64;               // mode 1: same storage viewed as FP64
+  const int* eB;             // k_oz_mma: [Kpad / kgroup][BR]
+  float2* part;              // sums: [split][Nvalid][AR] (ld AR per column), df64 sums over an item's K range
+  float2* C;                 // float pairs (ld ldc): k_oz_tn's B operand, kOzPairs' C
+  double* C64;               // kOzDoubles: C
   int64_t ldc;
   int64_t Mvalid, Nvalid;
-  int64_t fp64_rows;         // mode 1: rows < fp64_rows are written as FP64 (final)
-  int c_fp64;                // mode 1: C is stored as FP64 (read and written in FP64)
-  int c_assign;              // mode 1 with c_fp64: C = product (C is not read)
+  int64_t Kvalid;            // k_oz_tn: rows of C
+  int64_t fp64_rows;         // kOzPairs: rows < fp64_rows are written as FP64 (final)
+  int c_assign;              // kOzDoubles: C = product (C is not read)
   int* status;
   int n_mt, n_nt, n_ks;      // work items: M tiles x N tiles x K splits
 };
@@ -427,7 +436,7 @@ __device__ __forceinline__ df2 oz_accumulate(df2 x, df2 y) {
   return {h, sub2(l, sub2(h, s))};
 }
 
-// C - p for the read-modify-write of MODE 1, as df_add of C and -p does it
+// C - p for the read-modify-write of float pairs, as df_add of C and -p does it
 // (same split by form)
 template <int G>
 __device__ __forceinline__ df2 oz_subtract(df2 c, df2 p) {
@@ -476,7 +485,8 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, unsigned
 // bounded wait; gives up early when another role of the CTA failed
 __device__ __forceinline__ bool oz_wait(uint64_t* b, uint32_t parity, volatile int* fail) {
   const uint32_t addr = smem_u32(b);
-  for (long it = 0; it < OZ_WAIT_LIMIT; ++it) {
+#pragma unroll 1
+  for (int it = 0; it < OZ_WAIT_LIMIT; ++it) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\t"
@@ -570,15 +580,101 @@ __device__ __forceinline__ OzItem oz_item(const OzArgs& a, int w) {
   return it;
 }
 
-// Persistent, warp-specialised emulated-FP64 contraction.  Warp 0 streams the
-// operands' pre-sliced K16 blocks into a ring of OZ_STAGES stages with bulk
-// copies; warp 1 issues the 28 slice-pair MMAs of a stage into the five TMEM
-// accumulator groups and commits them (freeing the stage, and at the end of
-// an exact-accumulation group, handing the accumulators to the epilogue);
-// the epilogue warps 2.. read the accumulators (warp w owns TMEM lanes
-// 32 (w % 4) .. +31 and column part (w - 2) / 4), release them, and combine
-// them in df64.
-template <int MODE, int S>
+// Read one group's accumulators (columns of this warp from TMEM address taddr,
+// 8 at a time), scale them by 2^(eA + eB - 16) and set acc to them (ADD =
+// false) or add them to it.  ebs: the columns' exponents shifted to where a
+// float has its exponent, so that a scale takes one addition; eb: this lane's
+// column's exponent, for one warp-uniform test that every scale is a normal
+// float.
+template <int G, bool ADD>
+__device__ __forceinline__ void oz_drain(uint32_t taddr, const int* ebs, int eb, int eA, df2 (&acc)[OZ_EPI_COLS / 2]) {
+  const int eb_min = __reduce_min_sync(0xffffffffu, eb), eb_max = __reduce_max_sync(0xffffffffu, eb);
+  const bool normal = __all_sync(0xffffffffu, eA + eb_min - 16 >= -126 && eA + eb_max - 16 <= 127);
+  const int fA = (eA - 16 + 127) << 23;
+  if (!normal) {
+    // one column at a time, the sums in local memory: short code for a rare case (the
+    // unrolled form of both cases did not fit the instruction cache)
+    float2 x[OZ_EPI_COLS];
+#pragma unroll
+    for (int j = 0; j < OZ_EPI_COLS; j += 2) {
+      const float2 h = unpack2(acc[j / 2].h), l = unpack2(acc[j / 2].l);
+      x[j] = make_float2(h.x, l.x);
+      x[j + 1] = make_float2(h.y, l.y);
+    }
+#pragma unroll 1
+    for (int j = 0; j < OZ_EPI_COLS; ++j) {
+      uint32_t gr[G][8];
+#pragma unroll
+      for (int g = 0; g < G; ++g) tmem_ld8(taddr + (uint32_t)(g * OZ_N + (j & ~7)), gr[g]);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        tmem_regs_ready(gr[g]);
+#pragma unroll
+        for (int c = 1; c < 8; ++c)
+          if (c == (j & 7)) gr[g][0] = gr[g][c];
+      }
+      const df2 v = combine2<G>(gr, 0);
+      const int e = eA + (ebs[j] >> 23) - 16;
+      const df2 sv = {pack2(scale_wide(unpack2(v.h).x, e), 0.0f), pack2(scale_wide(unpack2(v.l).x, e), 0.0f)};
+      const df2 r = ADD ? oz_accumulate<G>({pack2(x[j].x, 0.0f), pack2(x[j].y, 0.0f)}, sv) : sv;
+      x[j] = make_float2(unpack2(r.h).x, unpack2(r.l).x);
+    }
+#pragma unroll
+    for (int j = 0; j < OZ_EPI_COLS; j += 2)
+      acc[j / 2] = {pack2(x[j].x, x[j + 1].x), pack2(x[j].y, x[j + 1].y)};
+    return;
+  }
+#pragma unroll
+  for (int c8 = 0; c8 < OZ_EPI_COLS / 8; ++c8) {
+    uint32_t gr[G][8];
+#pragma unroll
+    for (int g = 0; g < G; ++g) tmem_ld8(taddr + (uint32_t)(g * OZ_N + c8 * 8), gr[g]);
+    int f[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = ebs[c8 * 8 + j];
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int g = 0; g < G; ++g) tmem_regs_ready(gr[g]);
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      df2 v = combine2<G>(gr, j);
+      const f2x2 sc = pack2(__int_as_float(fA + f[j]), __int_as_float(fA + f[j + 1]));
+      v = {mul2(v.h, sc), mul2(v.l, sc)};
+      df2& x = acc[c8 * 4 + j / 2];
+      x = ADD ? oz_accumulate<G>(x, v) : v;
+    }
+  }
+}
+
+// an item's sums: this lane's row, this warp's columns
+__device__ __forceinline__ void oz_store_sums(const OzArgs& a, const OzItem& it, int row, int part,
+                                              const df2 (&acc)[OZ_EPI_COLS / 2]) {
+  const int64_t gn0 = it.n0 + part * OZ_EPI_COLS;
+  float2* out = a.part + ((int64_t)it.split * a.Nvalid + gn0) * a.AR + row;
+#pragma unroll
+  for (int j = 0; j < OZ_EPI_COLS; ++j) {
+    const float2 h = unpack2(acc[j / 2].h), l = unpack2(acc[j / 2].l);
+    if (row < a.AR && gn0 + j < a.Nvalid) out[j * a.AR] = (j & 1) ? make_float2(h.y, l.y) : make_float2(h.x, l.x);
+  }
+}
+
+// What k_oz_mma does with the products: sums over an item's K range (the Y^T C
+// of a panel's own FP64 columns), C -= product for float pairs, and C -= product
+// or C = product for FP64 storage.
+enum OzEpilogue { kOzSums, kOzPairs, kOzDoubles };
+
+// Contraction of two pre-sliced operands: persistent, warp-specialised.  Warp 0
+// streams their K16 blocks into a ring of OZ_STAGES stages with bulk copies; warp
+// 1 issues the 28 slice-pair MMAs of a stage into the five TMEM accumulator groups
+// and commits them (freeing the stage, and at the end of an exact-accumulation
+// group, handing the accumulators to the epilogue); the epilogue warps 2.. read
+// the accumulators (warp w owns TMEM lanes 32 (w % 4) .. +31 and column part
+// (w - 2) / 4), release them, and combine them in df64.  Bound by the MMAs (1390
+// cycles a K16 step) and the readout between groups (3100, FP32 additions).  One
+// kernel per epilogue: with all of them in one it was 165 KB of instructions
+// beside a 32 KB cache, and C -= Y Z' at 16384 x 8192 x 128 took 707 us, now 620.
+template <int S, OzEpilogue E>
 __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
   constexpr int G = OzCfg<S>::G;
   constexpr int STAGE_BYTES = OzCfg<S>::STAGE_BYTES;
@@ -612,7 +708,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
   // fills only the first AR x 32 bytes of each slice block; the rest of every
   // stage's A blocks is zeroed once here and never written again, so the
   // 128-row MMA reads zeros there.
-  if (MODE == 0 && a.AR < OZ_M) {
+  if (E == kOzSums && a.AR < OZ_M) {
     const int abytes = (int)a.AR * 32;
     const int tail = (OZ_ABYTES - abytes) / 16;
     for (int idx = tid; idx < OZ_STAGES * S * tail; idx += blockDim.x) {
@@ -630,7 +726,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
 
   if (warp == 0) {
     // ---------------- producer: the whole warp walks the stages, one elected lane copies
-    const int abytes = (MODE == 0 && a.AR < OZ_M) ? (int)a.AR * 32 : OZ_ABYTES;
+    const int abytes = (E == kOzSums && a.AR < OZ_M) ? (int)a.AR * 32 : OZ_ABYTES;
     const int64_t aplane = a.AR * a.Kpad, bplane = a.BR * a.Kpad;
     int st = 0;
     uint32_t parity = 1;
@@ -704,13 +800,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
     const int part = (warp - 2) >> 2;      // column part
     const int row = q * 32 + lane;
     int64_t ngroups = 0;
-    df2 acc[OZ_EPI_COLS / 2];   // MODE 0: sums over the item's K range; MODE 1: this group's product
+    df2 acc[OZ_EPI_COLS / 2];   // this group's product, or the sums over the item's groups
     for (int w = blockIdx.x; w < nitems && !s_fail; w += gridDim.x) {
       const OzItem it = oz_item(a, w);
       const int nsteps = (it.kend - it.kbeg) >> 4;
       const int64_t gm = it.m0 + row, gn0 = it.n0 + part * OZ_EPI_COLS;
       const int nc = (int)min((int64_t)OZ_EPI_COLS, a.Nvalid - gn0);   // this warp's columns (<= 0: none)
-      if (MODE == 1 && w + gridDim.x < nitems && !a.c_fp64) {
+      if (E == kOzPairs && w + gridDim.x < nitems) {
         // the next item's C tile streams into L2 while this one is computed:
         // a lane takes one column, 32 rows of 8 bytes
         const OzItem nx = oz_item(a, w + gridDim.x);
@@ -721,64 +817,28 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
           if (pm + 16 < a.Mvalid) asm volatile("prefetch.global.L2 [%0];" ::"l"(pc + 16));
         }
       }
+      if constexpr (E == kOzSums) {
 #pragma unroll
-      for (int j = 0; j < OZ_EPI_COLS / 2; ++j) acc[j] = {{0ull}, {0ull}};
+        for (int j = 0; j < OZ_EPI_COLS / 2; ++j) acc[j] = {{0ull}, {0ull}};
+      }
       for (int t0 = 0; t0 < nsteps; t0 += steps_per_group) {
-        // The group's exponents are loaded while its MMAs run, shifted to
-        // where a float has its exponent: 2^(eA + eB - 16) takes one addition.
+        // the group's exponents are loaded while its MMAs run
         const int64_t grp = (it.kbeg + t0 * 16) / a.kgroup;
         const int eA = (gm < a.AR) ? a.eA[grp * a.AR + gm] : 0;
         const int eb = (gn0 + lane < a.BR) ? __ldg(a.eB + grp * a.BR + gn0 + lane) : 0;
         int* ebs = s_eb[warp - 2];
         ebs[lane] = eb << 23;
-        // one warp-uniform test: every scale a normal float
-        const int eb_min = __reduce_min_sync(0xffffffffu, eb), eb_max = __reduce_max_sync(0xffffffffu, eb);
-        const bool normal = __all_sync(0xffffffffu, eA + eb_min - 16 >= -126 && eA + eb_max - 16 <= 127);
-        const int fA = (eA - 16 + 127) << 23;
         __syncwarp();
         if (!oz_wait(&acc_full, (uint32_t)(ngroups & 1), &s_fail)) break;
         ++ngroups;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // drain the five accumulators, 8 columns at a time
-#pragma unroll
-        for (int c8 = 0; c8 < OZ_EPI_COLS / 8; ++c8) {
-          uint32_t gr[G][8];
-#pragma unroll
-          for (int g = 0; g < G; ++g)
-            tmem_ld8(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(g * OZ_N + part * OZ_EPI_COLS + c8 * 8), gr[g]);
-          int f[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) f[j] = ebs[c8 * 8 + j];
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int g = 0; g < G; ++g) tmem_regs_ready(gr[g]);
-          if (normal) {
-#pragma unroll
-            for (int j = 0; j < 8; j += 2) {
-              df2 v = combine2<G>(gr, j);
-              const f2x2 sc = pack2(__int_as_float(fA + f[j]), __int_as_float(fA + f[j + 1]));
-              v = {mul2(v.h, sc), mul2(v.l, sc)};
-              df2& x = acc[c8 * 4 + j / 2];
-              x = (MODE == 0) ? oz_accumulate<G>(x, v) : v;
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; j += 2) {
-              df2 v = combine2<G>(gr, j);
-              const int e0 = eA + (f[j] >> 23) - 16, e1 = eA + (f[j + 1] >> 23) - 16;
-              const float2 h = unpack2(v.h), l = unpack2(v.l);
-              v = {pack2(scale_wide(h.x, e0), scale_wide(h.y, e1)), pack2(scale_wide(l.x, e0), scale_wide(l.y, e1))};
-              df2& x = acc[c8 * 4 + j / 2];
-              x = (MODE == 0) ? oz_accumulate<G>(x, v) : v;
-            }
-          }
-        }
+        oz_drain<G, E == kOzSums>(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(part * OZ_EPI_COLS), ebs, eb, eA, acc);
         // the accumulators are free for the next group (and ebs may be rewritten)
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(&acc_empty);
-        if (MODE == 1 && gm < a.Mvalid) {
-          if (a.c_fp64) {
+        if (E != kOzSums && gm < a.Mvalid) {
+          if constexpr (E == kOzDoubles) {
             // FP64 storage (a panel's own columns): one FP64 subtraction per element
             double* cp = a.C64 + gn0 * a.ldc + gm;
 #pragma unroll
@@ -810,34 +870,389 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
                 cv[j] = make_float2(h.x, l.x);
                 cv[j + 1] = make_float2(h.y, l.y);
               }
-              if (it.m0 >= a.fp64_rows) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                  if (c16 + j < nc) cp[(c16 + j) * a.ldc] = cv[j];
-              } else {
-                // the tile holds finished rows: tested here for the tile, since the
-                // FP64 addition of a row's test takes its slot also where it is off
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                  if (c16 + j >= nc) continue;
-                  double* cd = reinterpret_cast<double*>(cp + (c16 + j) * a.ldc);
-                  if (gm < a.fp64_rows) *cd = df_to_double({cv[j].x, cv[j].y});
-                  else *reinterpret_cast<float2*>(cd) = cv[j];
-                }
+              for (int j = 0; j < 16; ++j)
+                if (c16 + j < nc) cp[(c16 + j) * a.ldc] = cv[j];
+            }
+            // Finished rows become FP64 in a short loop of their own, over what this
+            // lane has just stored: the FP64 addition takes its slot of the pipe in
+            // every tile where it stands in the loop above, also where it is off.
+            if (gm < a.fp64_rows) {
+#pragma unroll 1
+              for (int j = 0; j < nc; ++j) {
+                const float2 v = cp[j * a.ldc];
+                *reinterpret_cast<double*>(cp + j * a.ldc) = df_to_double({v.x, v.y});
               }
             }
           }
         }
       }
-      if (MODE == 0 && !s_fail && gm < a.AR) {
-        float2* out = a.part + ((int64_t)it.split * a.Nvalid + gn0) * a.AR + gm;
+      if (E == kOzSums && !s_fail) oz_store_sums(a, it, row, part, acc);
+    }
+  }
+  __syncthreads();
+  if (s_fail && tid == 0) atomicExch(a.status, CANDMC_ERR_TIMEOUT);
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+}
+
+// Z = Y^T C over K splits, C read as it is stored: a column of C meets the
+// tensor cores once (one M tile, b <= 128), so slicing it in its own kernel
+// wrote 14 bytes per element that were read back once (450 us at 16384 x 8192
+// beside the 605 us of the contraction).  Here twelve warps slice it on the
+// way, in two teams of six: team v takes the K16 steps t = v (mod 2) of a group
+// and so one stage of the two-stage B ring, a warp 16 columns of them.  (With
+// every warp in every step, a step took the 1900 cycles of one warp's chain of
+// loads, digits, fence and copies, for 1390 of MMAs.)  The 128 rows of a group
+// come into shared memory by asynchronous copies one group ahead, 98 KB, each
+// warp its own part, so that only the warp waits for it.  Per group the warps
+// find their columns' maxima over their steps' rows and exchange them, then slice
+// step after step and ask for the same rows of the next group.  The first step of
+// the next group is sliced before the accumulators of the last one are read, so
+// the tensor cores go on as soon as they are free.  For the sums, warp w reads TMEM
+// lanes 32 (w % 4) .., column part (w - 2) / 4.
+constexpr int TN_ASTAGES = 3, TN_BSTAGES = 2;
+template <int S>
+struct TnCfg {
+  static constexpr int A = S * OZ_ABYTES, B = S * OZ_BBYTES;
+  static constexpr int RAW = OZ_N * 128 * 8;
+  static constexpr int SMEM = TN_ASTAGES * A + TN_BSTAGES * B + RAW + 1024;
+};
+constexpr int TN_TEAM = OZ_EPI_WARPS / TN_BSTAGES;   // warps of a slicing team
+static_assert(OZ_N == 16 * TN_TEAM && 8 % TN_BSTAGES == 0, "two core-matrix row blocks of B per slicing warp");
+
+// asynchronous copies of `bytes` bytes (0 up to 8 or 16), the rest zero
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// Where the 16 bytes of rows 2c, 2c + 1 of a warp's column r stand in its 8 x 16
+// block (a column takes 128 bytes): moved among the 8 places of the column so that the
+// slicing lanes' reads (rows of 4 columns, 2 places apart) fall on different banks.
+__device__ __forceinline__ uint32_t raw_place(int r, int c) {
+  return (uint32_t)(r * 128 + ((c ^ ((r & 1) | ((r & 2) << 1))) << 4));
+}
+
+// the scale exponent of a column whose halves have these maxima (the lo part can
+// push |x| just above |hi|'s bound; leave one ulp of room)
+__device__ __forceinline__ int tn_exp(float m0, float m1) { return scale_exp(fmaxf(m0, m1) * (1.0f + 1.0e-6f)); }
+
+template <int S>
+__global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_tn(OzArgs a) {
+  constexpr int G = OzCfg<S>::G;
+  using Cfg = TnCfg<S>;
+  extern __shared__ __align__(1024) unsigned char oz_smem[];
+  __shared__ __align__(8) uint64_t a_full[TN_ASTAGES], a_empty[TN_ASTAGES], b_full[TN_BSTAGES], b_empty[TN_BSTAGES];
+  __shared__ __align__(8) uint64_t acc_full, acc_empty, exp_full, fin;
+  __shared__ uint32_t tmem_base_s;
+  __shared__ volatile int s_fail;
+  __shared__ float s_mx[2][TN_BSTAGES][OZ_N];      // column maxima by group parity and team
+  __shared__ int s_eb[OZ_EPI_WARPS][OZ_EPI_COLS];   // per warp: the exponents of its sums' columns
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  unsigned char* ring = (unsigned char*)(((uintptr_t)oz_smem + 1023) & ~(uintptr_t)1023);
+  const int nitems = a.n_nt * a.n_ks;
+
+  if (tid == 0) {
+    for (int st = 0; st < TN_ASTAGES; ++st) {
+      mbar_init(&a_full[st], 1);
+      mbar_init(&a_empty[st], 1);
+    }
+    for (int st = 0; st < TN_BSTAGES; ++st) {
+      mbar_init(&b_full[st], TN_TEAM);
+      mbar_init(&b_empty[st], 1);
+    }
+    mbar_init(&acc_full, 1);
+    mbar_init(&acc_empty, OZ_EPI_WARPS);
+    mbar_init(&exp_full, OZ_EPI_WARPS);
+    mbar_init(&fin, 1);
+    s_fail = 0;
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&tmem_base_s)),
+                 "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  // An A operand of fewer than 128 rows (a narrow Y^T, stored with AR rows)
+  // fills only the first AR x 32 bytes of each slice block; the rest of every
+  // stage's A blocks is zeroed once here and never written again, so the
+  // 128-row MMA reads zeros there.
+  if (a.AR < OZ_M) {
+    const int abytes = (int)a.AR * 32;
+    const int tail = (OZ_ABYTES - abytes) / 16;
+    for (int idx = tid; idx < TN_ASTAGES * S * tail; idx += blockDim.x) {
+      const int blk = idx / tail, q = idx % tail;
+      *reinterpret_cast<uint4*>(ring + (size_t)blk * OZ_ABYTES + abytes +
+                                16 * q) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_base_s;
+  unsigned char* bring = ring + TN_ASTAGES * Cfg::A;
+
+  if (warp == 0) {
+    // ---------------- producer of A: the whole warp walks the stages, one elected lane copies
+    const int abytes = (a.AR < OZ_M) ? (int)a.AR * 32 : OZ_ABYTES;
+    const int64_t aplane = a.AR * a.Kpad;
+    int st = 0;
+    uint32_t parity = 1;
+    bool ok = true;
+    for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
+      const OzItem it = oz_item(a, w);
+      const __nv_bfloat16* as = a.As + (int64_t)it.kbeg * a.AR;
+      for (int k = it.kbeg; k < it.kend; k += 16, as += a.AR * 16) {
+        ok = oz_wait(&a_empty[st], parity, &s_fail);
+        if (!ok) break;
+        if (elect_one()) {
+          mbar_expect_tx(&a_full[st], (unsigned)(S * abytes));
+          const uint32_t sa = smem_u32(ring + st * Cfg::A);
 #pragma unroll
-        for (int j = 0; j < OZ_EPI_COLS; ++j) {
-          const float2 h = unpack2(acc[j / 2].h), l = unpack2(acc[j / 2].l);
-          if (j < nc) out[j * a.AR] = (j & 1) ? make_float2(h.y, l.y) : make_float2(h.x, l.x);
+          for (int sl = 0; sl < S; ++sl) bulk_g2s(sa + sl * OZ_ABYTES, as + sl * aplane, (unsigned)abytes, &a_full[st]);
+        }
+        __syncwarp();
+        if (++st == TN_ASTAGES) {
+          st = 0;
+          parity ^= 1;
         }
       }
     }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer: the whole warp walks the stages, one elected lane issues
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_N >> 3) << 17) |
+                           ((uint32_t)(OZ_M >> 4) << 24);
+    // the rings end below 256 KB: base + offset / 16 stays inside the
+    // descriptor's 14-bit address field
+    const uint64_t a_desc = make_desc(smem_u32(ring)), b_desc = make_desc(smem_u32(bring));
+    static_assert(Cfg::A % 1024 == 0 && Cfg::B % 1024 == 0 && Cfg::SMEM + 2048 < (1 << 18), "stage alignment, range");
+    int sa = 0, sb = 0;
+    uint32_t a_parity = 0, b_parity = 0, acc_parity = 1;
+    bool ok = true;
+    for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
+      const OzItem it = oz_item(a, w);
+      for (int k = it.kbeg; k < it.kend && ok; k += 128) {
+        // the previous group's accumulators have been read
+        ok = oz_wait(&acc_empty, acc_parity, &s_fail);
+        acc_parity ^= 1;
+        for (int t = 0; t < 8 && ok; ++t) {
+          ok = oz_wait(&a_full[sa], a_parity, &s_fail) && oz_wait(&b_full[sb], b_parity, &s_fail);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          oz_issue_step<S, G>(tmem, a_desc + (uint64_t)(sa * (Cfg::A >> 4)), b_desc + (uint64_t)(sb * (Cfg::B >> 4)),
+                              idesc, t > 0 ? 1u : 0u);
+          umma_commit(&b_empty[sb]);   // the stages are free once these MMAs have read them
+          umma_commit(&a_empty[sa]);
+          if (++sa == TN_ASTAGES) {
+            sa = 0;
+            a_parity ^= 1;
+          }
+          if (++sb == TN_BSTAGES) {
+            sb = 0;
+            b_parity ^= 1;
+          }
+        }
+        if (ok) umma_commit(&acc_full);
+      }
+    }
+    // every MMA this warp issued has completed before TMEM is released
+    umma_commit(&fin);
+    volatile int dummy = 0;
+    oz_wait(&fin, 0u, &dummy);
+  } else {
+    // ---------------- slicing of C and sums: warps 2 .. 2 + OZ_EPI_WARPS - 1
+    const int cw = warp - 2;
+    const int team = cw / TN_TEAM, c0 = (cw % TN_TEAM) * 16;   // steps team, team + 2, ..; columns c0 .. c0 + 15
+    const int q = warp & 3;                // TMEM lane quarter this warp may access
+    const int part = cw >> 2;              // column part of the sums
+    const int row = q * 32 + lane;
+    const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(part * OZ_EPI_COLS);
+    unsigned char* raw = bring + TN_BSTAGES * Cfg::B + cw * 8192;   // 4 K16 blocks of 16 columns x 16 rows
+    const double* C = reinterpret_cast<const double*>(a.C);   // a float pair takes 8 bytes
+    // Asynchronous copies of this warp's part of a group, block after block: a lane
+    // takes 16 bytes (2 rows) of every fourth column where C's columns are aligned to
+    // that, else 8 bytes (1 row) of every second.  load_from sets the lane's first element.
+    const bool wide = ((a.ldc | (int64_t)(reinterpret_cast<uintptr_t>(C) >> 3)) & 1) == 0;
+    const int lrow = wide ? 2 * (lane & 7) : (lane & 15), lcol = wide ? lane >> 3 : lane >> 4;
+    const uint32_t ldst = smem_u32(raw);
+    const double* lp = C;
+    int lleft = 0, lcols = 0;   // rows and columns from the lane's first element to the matrix' end
+    auto load_from = [&](int64_t n0, int k) {
+      const int64_t n = n0 + c0 + lcol;
+      lp = C + n * a.ldc + k + team * 16 + lrow;
+      lleft = (int)a.Kvalid - k - team * 16 - lrow;
+      lcols = (int)min(a.Nvalid - n, (int64_t)16);
+    };
+    auto load_block = [&](int u) {   // the warp's u-th step of the group
+      const double* p = lp + u * 32;
+      const int left = lleft - u * 32;
+      if (wide) {
+        const int bytes = min(max(left, 0), 2) * 8;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int b = 4 * i < lcols ? bytes : 0;
+          cp_async16(ldst + u * 2048 + raw_place(lcol + 4 * i, lrow >> 1), b ? p + i * 4 * a.ldc : C, b);
+        }
+      } else {
+        const int bytes = left > 0 ? 8 : 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int b = 2 * i < lcols ? bytes : 0;
+          cp_async8(ldst + u * 2048 + raw_place(lcol + 2 * i, lrow >> 1) + (lane & 1) * 8, b ? p + i * 2 * a.ldc : C, b);
+        }
+      }
+    };
+    // lane's part of a block: columns r and r + 8, rows kr .. kr + 3
+    const int r = (lane & 15) >> 1, kr = (lane >> 4) * 8 + (lane & 1) * 4;
+    const uint32_t place0 = raw_place(r, kr >> 1), place1 = raw_place(r, (kr >> 1) + 1);
+    // maxima of the lane's columns over a block's rows, once they have arrived
+    float mx[2] = {0.0f, 0.0f};
+    auto scan_block = [&](int u) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float4 x = *reinterpret_cast<const float4*>(raw + u * 2048 + (c >> 1) * 1024 + ((c & 1) ? place1 : place0));
+        mx[c >> 1] = fmaxf(mx[c >> 1], fmaxf(fabsf(x.x), fabsf(x.z)));
+      }
+    };
+    df2 acc[OZ_EPI_COLS / 2];   // sums over the item's K range
+#pragma unroll
+    for (int j = 0; j < OZ_EPI_COLS / 2; ++j) acc[j] = {{0ull}, {0ull}};
+
+    // The accumulators of the group at row k of item it are read and added up;
+    // after its last group the item's sums are written.
+    uint32_t drained = 0;
+    auto drain = [&](const OzItem& it, int k, int eA) -> bool {
+      const uint32_t par = drained & 1;
+      const int c = part * OZ_EPI_COLS + lane;
+      const int eb = tn_exp(s_mx[par][0][c], s_mx[par][1][c]);
+      s_eb[cw][lane] = eb << 23;
+      if (!oz_wait(&acc_full, par, &s_fail)) return false;
+      ++drained;
+      __syncwarp();
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      oz_drain<G, true>(taddr, s_eb[cw], eb, eA, acc);
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty);
+      if (k + 128 < it.kend) return true;
+      oz_store_sums(a, it, row, part, acc);
+#pragma unroll
+      for (int j = 0; j < OZ_EPI_COLS / 2; ++j) acc[j] = {{0ull}, {0ull}};
+      return true;
+    };
+
+    OzItem it = oz_item(a, blockIdx.x), last_it = it;
+    int w = blockIdx.x, k = it.kbeg, last_k = -1, last_eA = 0;
+    uint32_t b_parity = 1, group = 0;
+    bool ok = true;
+    load_from(it.n0, k);
+#pragma unroll 1
+    for (int u = 0; u < 4; ++u) load_block(u);
+    bool have = true;   // a group to slice; the last pass only reads the last group's sums
+    while (true) {
+      const int eA = (have && row < a.AR) ? a.eA[(int64_t)(k >> 7) * a.AR + row] : 0;
+      OzItem nit = it;
+      int nw = w, nk = k + 128;
+      bool more = have;
+      int e[2] = {0, 0};
+      if (have) {
+      // the last of this warp's rows of the group have arrived (the first group: all)
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();
+#pragma unroll 1
+      for (int u = group ? 3 : 0; u < 4; ++u) scan_block(u);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
+        mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 16));
+        if ((lane & 17) == 0) s_mx[group & 1][team][c0 + r + 8 * h] = mx[h];
+        mx[h] = 0.0f;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&exp_full);
+      // the group after this one
+      if (nk >= it.kend) {
+        nw = w + gridDim.x;
+        more = nw < nitems;
+        if (more) {
+          nit = oz_item(a, nw);
+          nk = nit.kbeg;
+        }
+      }
+      load_from(nit.n0, nk);
+      ok = oz_wait(&exp_full, group & 1, &s_fail);
+      if (!ok) break;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        e[h] = tn_exp(s_mx[group & 1][0][c0 + r + 8 * h], s_mx[group & 1][1][c0 + r + 8 * h]);
+      }
+      const bool tiny = __any_sync(0xffffffffu, min(e[0], e[1]) < -119);
+      // Team 0 prepares the first step before it reads the last group's sums; the second
+      // step's stage is free only with the last group's last MMA, so team 1 reads them first.
+#pragma unroll 1
+      for (int u = 0; u < 4; ++u) {
+        if (u == 1 - team && last_k >= 0) {
+          ok = drain(last_it, last_k, last_eA);
+          if (!ok) break;
+        }
+        if (!have) continue;
+        unsigned char* sd = bring + team * Cfg::B + c0 * 32 + lane * 8;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float4 x0 = *reinterpret_cast<const float4*>(raw + u * 2048 + h * 1024 + place0);
+          const float4 x1 = *reinterpret_cast<const float4*>(raw + u * 2048 + h * 1024 + place1);
+          // times 2^(8 - e): two normal factors, the second one 1 unless e < -119
+          const int k1 = min(8 - e[h], 127);
+          const float f1 = pow2f(k1);
+          f2x2 v[4] = {pack2(x0.x, x0.z), pack2(x0.y, x0.w), pack2(x1.x, x1.z), pack2(x1.y, x1.w)};
+          if (tiny) {
+            const float f2v = pow2f(8 - e[h] - k1);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) v[c] = mul2(v[c], pack2(f2v, f2v));
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c) v[c] = mul2(v[c], pack2(f1, f1));
+          uint32_t d[S][2];
+          slice_digits<S>(v[0], v[1], [&](int i, f2x2 y) { d[i][0] = to_bf16x2(y); });
+          slice_digits<S>(v[2], v[3], [&](int i, f2x2 y) { d[i][1] = to_bf16x2(y); });
+          if (h == 0) {
+            // while the stage is in use: the block asked for one step ago
+            if (u > 0 && more) {
+              asm volatile("cp.async.wait_all;" ::: "memory");
+              __syncwarp();
+              scan_block(u - 1);
+            }
+            ok = oz_wait(&b_empty[team], b_parity, &s_fail);
+            if (!ok) break;
+          }
+#pragma unroll
+          for (int i = 0; i < S; ++i)
+            *reinterpret_cast<uint2*>(sd + h * 256 + i * OZ_BBYTES) = make_uint2(d[i][0], d[i][1]);
+        }
+        if (!ok) break;
+        b_parity ^= 1;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&b_full[team]);
+        if (more) load_block(u);
+      }
+      last_it = it;
+      last_k = k;
+      last_eA = eA;
+      ++group;
+      if (!ok || !have) break;
+      have = more;
+      it = nit;
+      w = nw;
+      k = nk;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   }
   __syncthreads();
   if (s_fail && tid == 0) atomicExch(a.status, CANDMC_ERR_TIMEOUT);
@@ -985,25 +1400,37 @@ static int64_t oz_groups_per_item(int64_t groups, int64_t ntiles) {
   }
   return best;
 }
-template <int S>
-static int launch_oz(OzArgs a, unsigned gm, unsigned gn, unsigned gk, int cls, double flops,
-                     cudaStream_t s) {
-  constexpr int SMEM = OzCfg<S>::SMEM;
+// Dynamic shared memory above the default limit, allowed once per kernel.
+template <class K>
+static int allow_smem(K kernel, int bytes, std::atomic<bool>& done) {
+  if (done) return CANDMC_OK;
+  CANDMC_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  done = true;
+  return CANDMC_OK;
+}
+
+template <int S, OzEpilogue E>
+static int launch_oz_mma(OzArgs a, int64_t gm, int64_t gn, int64_t gk, int cls, double flops, cudaStream_t s) {
   static std::atomic<bool> attr{false};
-  if (!attr) {
-    CANDMC_CK(cudaFuncSetAttribute(k_oz_mma<0, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-    CANDMC_CK(cudaFuncSetAttribute(k_oz_mma<1, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-    attr = true;
-  }
+  CANDMC_RET(allow_smem(k_oz_mma<S, E>, OzCfg<S>::SMEM, attr));
   a.n_mt = (int)gm;
   a.n_nt = (int)gn;
   a.n_ks = (int)gk;
-  const unsigned grid = (unsigned)std::min<int64_t>((int64_t)gm * gn * gk, oz_ctas());
   ProfScope ps(cls, flops, s);
-  if (a.mode == 0)
-    k_oz_mma<0, S><<<grid, OZ_THREADS, SMEM, s>>>(a);
-  else
-    k_oz_mma<1, S><<<grid, OZ_THREADS, SMEM, s>>>(a);
+  k_oz_mma<S, E><<<(unsigned)std::min<int64_t>(gm * gn * gk, oz_ctas()), OZ_THREADS, OzCfg<S>::SMEM, s>>>(a);
+  CANDMC_CK(cudaGetLastError());
+  return CANDMC_OK;
+}
+
+template <int S>
+static int launch_oz_tn(OzArgs a, int64_t gn, int64_t gk, int cls, double flops, cudaStream_t s) {
+  static std::atomic<bool> attr{false};
+  CANDMC_RET(allow_smem(k_oz_tn<S>, TnCfg<S>::SMEM, attr));
+  a.n_mt = 1;
+  a.n_nt = (int)gn;
+  a.n_ks = (int)gk;
+  ProfScope ps(cls, flops, s);
+  k_oz_tn<S><<<(unsigned)std::min<int64_t>(gn * gk, oz_ctas()), OZ_THREADS, TnCfg<S>::SMEM, s>>>(a);
   CANDMC_CK(cudaGetLastError());
   return CANDMC_OK;
 }
@@ -1018,26 +1445,37 @@ static int oz_tn(const SliceSrc& ysrc, const SliceSrc& csrc, int64_t m, int nb, 
   const int64_t Kp1 = rup(m, KG);
   // the A operand keeps only its nb rows (rounded to a core matrix of 8):
   // the kernel zero-fills the rest of the 128-row tile in shared memory
-  const int64_t AR1 = rup(nb, 8), BR1 = rup(n, OZ_N);
+  const int64_t AR1 = rup(nb, 8), ntiles = (n + OZ_N - 1) / OZ_N;
   DevBuf ya, ea, cb, eb, part;
   CANDMC_RET(ya.alloc(sizeof(__nv_bfloat16) * S * AR1 * Kp1, s));
   CANDMC_RET(ea.alloc(sizeof(int) * (Kp1 / KG) * AR1, s));
-  CANDMC_RET(cb.alloc(sizeof(__nv_bfloat16) * S * BR1 * Kp1, s));
-  CANDMC_RET(eb.alloc(sizeof(int) * (Kp1 / KG) * BR1, s));
   auto* yas = static_cast<__nv_bfloat16*>(ya.p);
-  auto* cbs = static_cast<__nv_bfloat16*>(cb.p);
   CANDMC_RET(launch_slice_cols<S>(ysrc, m, nb, AR1, Kp1, (int)KG, yas, static_cast<int*>(ea.p), s));
-  CANDMC_RET(launch_slice_cols<S>(csrc, m, n, BR1, Kp1, (int)KG, cbs, static_cast<int*>(eb.p), s));
-  const int64_t ntiles = BR1 / OZ_N;
   const int64_t kper = KG * oz_groups_per_item(Kp1 / KG, ntiles);
   const int64_t ksplit = (Kp1 + kper - 1) / kper;
   CANDMC_RET(part.alloc(sizeof(float2) * ksplit * n * AR1, s));
   OzArgs g1{};
-  g1.As = yas; g1.AR = AR1; g1.Bs = cbs; g1.BR = BR1; g1.Kpad = (int)Kp1; g1.k_per_cta = (int)kper;
-  g1.kgroup = (int)KG; g1.eA = static_cast<int*>(ea.p); g1.eB = static_cast<int*>(eb.p);
-  g1.mode = 0; g1.part = static_cast<float2*>(part.p); g1.Mvalid = nb; g1.Nvalid = n;
-  g1.status = status;
-  CANDMC_RET(launch_oz<S>(g1, 1, (unsigned)ntiles, (unsigned)ksplit, cls, 2.0 * nb * n * m, s));
+  g1.As = yas; g1.AR = AR1; g1.Kpad = (int)Kp1; g1.k_per_cta = (int)kper;
+  g1.kgroup = (int)KG; g1.eA = static_cast<int*>(ea.p); g1.part = static_cast<float2*>(part.p);
+  g1.Mvalid = nb; g1.Nvalid = n; g1.Kvalid = m; g1.status = status;
+  const double flops = 2.0 * nb * n * m;
+  // Float pairs are sliced on their way through the contraction.  FP64 columns (a
+  // panel's own, few column tiles) are sliced by k_slice first: splitting a double
+  // by its bits takes more issue slots than the twelve warps have beside the MMAs
+  // (the half-panel update of 16384 x 32: 44 us fused, 33 in two kernels).
+  if (csrc.df) {
+    g1.C = const_cast<float2*>(csrc.df);
+    g1.ldc = csrc.ld;
+    CANDMC_RET(launch_oz_tn<S>(g1, ntiles, ksplit, cls, flops, s));
+  } else {
+    const int64_t BR1 = ntiles * OZ_N;
+    CANDMC_RET(cb.alloc(sizeof(__nv_bfloat16) * S * BR1 * Kp1, s));
+    CANDMC_RET(eb.alloc(sizeof(int) * (Kp1 / KG) * BR1, s));
+    g1.Bs = static_cast<__nv_bfloat16*>(cb.p); g1.BR = BR1; g1.eB = static_cast<int*>(eb.p);
+    CANDMC_RET(launch_slice_cols<S>(csrc, m, n, BR1, Kp1, (int)KG, static_cast<__nv_bfloat16*>(cb.p),
+                                    static_cast<int*>(eb.p), s));
+    CANDMC_RET((launch_oz_mma<S, kOzSums>(g1, 1, ntiles, ksplit, cls, flops, s)));
+  }
   ProfScope ps(CANDMC_KCLASS_REDUCE, 8.0 * ksplit * n * AR1, s);
   k_oz_sum_partials<<<(unsigned)((nb * n + 255) / 256), 256, 0, s>>>(static_cast<float2*>(part.p),
                                                                       (int)ksplit, AR1, nb, n, Z);
@@ -1047,7 +1485,7 @@ static int oz_tn(const SliceSrc& ysrc, const SliceSrc& csrc, int64_t m, int nb, 
 
 // Zt (nb x n, FP64, ld nb) = Top (nb x nb) * Z (nb x n, FP64, ld nb) with the
 // S-slice contraction: Top is the A operand (sliced from its stored matrix,
-// transposed or not), Z the B operand, and the MODE 1 epilogue stores the
+// transposed or not), Z the B operand, and the epilogue stores the
 // product into Zt instead of subtracting it.
 template <int S>
 static int oz_top_times(MatRef Top, int nb, const double* Z, int64_t n, double* Zt, int* status,
@@ -1073,10 +1511,10 @@ static int oz_top_times(MatRef Top, int nb, const double* Z, int64_t n, double* 
   g.As = tas; g.AR = OZ_M; g.Bs = zbs; g.BR = BR;
   g.Kpad = g.k_per_cta = g.kgroup = (int)Kp;
   g.eA = static_cast<int*>(et.p); g.eB = static_cast<int*>(ez.p);
-  g.mode = 1; g.C = reinterpret_cast<float2*>(Zt); g.C64 = Zt; g.ldc = nb;
+  g.C = reinterpret_cast<float2*>(Zt); g.C64 = Zt; g.ldc = nb;
   g.Mvalid = nb; g.Nvalid = n; g.fp64_rows = 0; g.status = status;
-  g.c_fp64 = 1; g.c_assign = 1;
-  return launch_oz<S>(g, 1, (unsigned)(BR / OZ_N), 1, cls, 2.0 * nb * nb * n, s);
+  g.c_assign = 1;
+  return launch_oz_mma<S, kOzDoubles>(g, 1, BR / OZ_N, 1, cls, 2.0 * nb * nb * n, s);
 }
 
 // Width from which the operator product T^T Z of an update runs on the
@@ -1127,12 +1565,11 @@ static int apply_qt_slices(const double* Y, int64_t ldy, int ymask, int64_t m, i
   g2.Bs = static_cast<__nv_bfloat16*>(z2.p); g2.BR = BR2;
   g2.Kpad = g2.k_per_cta = g2.kgroup = (int)Kp2;
   g2.eA = static_cast<int*>(ey2.p); g2.eB = static_cast<int*>(ez2.p);
-  g2.mode = 1; g2.C = reinterpret_cast<float2*>(C); g2.C64 = C; g2.ldc = ldc;
+  g2.C = reinterpret_cast<float2*>(C); g2.C64 = C; g2.ldc = ldc;
   g2.Mvalid = m; g2.Nvalid = n; g2.fp64_rows = fp64_rows; g2.status = status;
-  g2.c_fp64 = c_fp64 ? 1 : 0;
-  CANDMC_RET(launch_oz<S>(g2, (unsigned)(AR2 / OZ_M), (unsigned)(BR2 / OZ_N), 1, cls_nn,
-                       2.0 * m * n * nb, s));
-  return CANDMC_OK;
+  const double flops = 2.0 * m * n * nb;
+  if (c_fp64) return launch_oz_mma<S, kOzDoubles>(g2, AR2 / OZ_M, BR2 / OZ_N, 1, cls_nn, flops, s);
+  return launch_oz_mma<S, kOzPairs>(g2, AR2 / OZ_M, BR2 / OZ_N, 1, cls_nn, flops, s);
 }
 
 // The emulated-FP64 form: 7 slices, 28 slice products per K16 step.

@@ -39,19 +39,13 @@ def product_bound(X, Y, dX, dY):
     return k * 2.0 ** -52 * scales + (2.0 ** -44 + k * 2.0 ** -53) * a + dX @ np.abs(Y) + np.abs(X) @ dY
 
 
-# rows: one group of 128, one more or less, 16-row blocks, many K splits (157
-# groups); columns: 96-column tiles, below and from 1024 columns (the operator
-# product on the tensor cores); panel widths: 8-row core matrices, 16-deep K steps
-@pytest.mark.parametrize("m,nb,n", [(1, 1, 1), (128, 16, 96), (129, 17, 97), (127, 8, 95), (255, 128, 193),
-                                    (656, 9, 1100), (1000, 100, 1024), (20000, 128, 30), (20090, 33, 289)])
-@pytest.mark.parametrize("scales", [(0,), (0, -60, 60, -112)])
-def test_update_edges(cm, m, nb, n, scales):
+def check_update(cm, m, nb, n, scales, store):
     g = np.random.default_rng(m + nb + n)
     Y = g.standard_normal((m, nb)) / np.sqrt(m)
     C = np.ldexp(g.standard_normal((m, n)), np.resize(scales, n)[None, :])
     if n > 2:
         C[:, 2] = 0.0
-    out = dev(C)
+    out = store(C)
     cm.upd_A(dev(Y), out, W=dev(2.0 * np.eye(nb)), W_is_T=True, precision="ozaki")
     tiny = 2.0 ** -148
     zero = lambda a: np.zeros_like(a)
@@ -64,3 +58,29 @@ def test_update_edges(cm, m, nb, n, scales):
     bound = product_bound(Y, Z2, zero(Y), dZ2) + 2.0 ** -46 * (np.abs(C) + np.abs(Y @ Z2)) + 4 * tiny
     got = out.cpu().numpy()
     assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
+
+
+# rows: one group of 128, one more or less, 16-row blocks, many K splits (157
+# groups); columns: 96-column tiles, below and from 1024 columns (the operator
+# product on the tensor cores); panel widths: 8-row core matrices, 16-deep K steps
+@pytest.mark.parametrize("m,nb,n", [(1, 1, 1), (128, 16, 96), (129, 17, 97), (127, 8, 95), (255, 128, 193),
+                                    (656, 9, 1100), (1000, 100, 1024), (20000, 128, 30), (20090, 33, 289)])
+@pytest.mark.parametrize("scales", [(0,), (0, -60, 60, -112)])
+def test_update_edges(cm, m, nb, n, scales):
+    check_update(cm, m, nb, n, scales, dev)
+
+
+# C as rows of a larger matrix: columns aligned to 16 bytes with an odd number of
+# rows, and columns at every 8-byte boundary; what lies around C stays
+@pytest.mark.parametrize("m,nb,n", [(129, 17, 97), (1003, 64, 200), (20001, 32, 40)])
+@pytest.mark.parametrize("off,extra", [(0, 1), (2, 5), (1, 3), (1, 2)])
+def test_update_within_matrix(cm, m, nb, n, off, extra):
+    buf = torch.full((n, m + extra), 3.0, dtype=torch.float64, device="cuda")
+
+    def store(C):
+        A = buf.t()[off:off + m]
+        A.copy_(torch.from_numpy(C).cuda())
+        return A
+
+    check_update(cm, m, nb, n, (0,), store)
+    assert (buf[:, :off] == 3.0).all() and (buf[:, off + m:] == 3.0).all()
