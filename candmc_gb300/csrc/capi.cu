@@ -110,19 +110,15 @@ int hr_rec(double* A, int64_t lda, int64_t m, int b, double* T, int64_t ldT, int
   CANDMC_RET(hr_rec(A + (int64_t)b1 * lda + b1, lda, m - b1, b2, T22, ldT, st, precision, s));
   // G = Y1[b1:m, :]^T * Y2   (Y2 unit-lower in A[b1:, b1:]); with the half
   // update on the tensor cores, this (m - b1) x b1 x b2 product goes there too
-  DevBuf g, x;
+  DevBuf g;
   CANDMC_RET(g.alloc(sizeof(double) * b1 * b2, s));
-  CANDMC_RET(x.alloc(sizeof(double) * b1 * b2, s));
   if (oz)
     CANDMC_RET(gram_ozaki(A + b1, lda, kDense, A + (int64_t)b1 * lda + b1, lda, kUnitLower, m - b1, b1, b2,
                           g.d(), st, s));
   else
     CANDMC_RET(gemm_tn_reduce(mref(A + b1, lda), mref(A + (int64_t)b1 * lda + b1, lda, 0, kUnitLower),
                               m - b1, b1, b2, mref(nullptr, 0), 1.0, g.d(), b1, s));
-  // X = T11 * G;  T12 = -X * T22
-  CANDMC_RET(small_gemm(b1, b2, b1, 1.0, mref(T, ldT, 0, kUpper), mref(g.d(), b1), 0.0, x.d(), b1, s));
-  CANDMC_RET(small_gemm(b1, b2, b2, -1.0, mref(x.d(), b1), mref(T22, ldT, 0, kUpper), 0.0,
-                        T + (int64_t)b1 * ldT, ldT, s));
+  CANDMC_RET(merge_t(g.d(), T, ldT, b1, b2, s));   // T12 = -T11 G T22
   CANDMC_CK(cudaMemset2DAsync(T + b1, sizeof(double) * ldT, 0, sizeof(double) * b2, b1, s));
   return CANDMC_OK;
 }

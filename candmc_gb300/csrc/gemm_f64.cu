@@ -426,8 +426,11 @@ k_small_gemm(MatRef A, MatRef B, int64_t M, int64_t N, int64_t K, double alpha, 
       sB[k2][jj] = (gj < N && gk2 < K) ? mat_at(B, gk2, gj) : 0.0;
     }
     __syncthreads();
-#pragma unroll 16
-    for (int kk = 0; kk < 64; ++kk) acc = fma(sA[ti][kk], sB[kk][tj], acc);
+    const int kn = (int)(K - kb < 64 ? K - kb : 64);
+    for (int k0 = 0; k0 < kn; k0 += 8) {   // zeros beyond K
+#pragma unroll
+      for (int kk = k0; kk < k0 + 8; ++kk) acc = fma(sA[ti][kk], sB[kk][tj], acc);
+    }
     __syncthreads();
   }
   int64_t gi = i0 + ti, gj = j0 + tj;
@@ -435,6 +438,42 @@ k_small_gemm(MatRef A, MatRef B, int64_t M, int64_t N, int64_t K, double alpha, 
     double v = alpha * acc;
     if (beta != 0.0) v += beta * C[gj * ldc + gi];
     C[gj * ldc + gi] = v;
+  }
+}
+
+// T12 = -T11 G T22 of two upper-triangular factors (T11: b1 x b1, T22: b2 x b2, T12
+// beside them with the same ld) and G (b1 x b2, ld b1).  One CTA per column j, as
+// in k_reduce_apply: thread (i, g) takes every 256 / nbp-th term of row i, first of
+// t = G T22(:, j), then of T11 t.  One launch of 6 us where two small products took
+// 9 each (bound by the latencies of loads and of the FP64 pipe).
+__global__ void __launch_bounds__(kThreads)
+k_merge_t(const double* G, double* T, int64_t ldT, int b1, int b2, int nbp) {
+  __shared__ double part[kThreads];
+  __shared__ double col[kThreads];
+  const int NG = kThreads / nbp;
+  const int i = threadIdx.x % nbp, g = threadIdx.x / nbp, j = blockIdx.x;
+  const double* t22 = T + (int64_t)(b1 + j) * ldT + b1;
+  for (int k = threadIdx.x; k <= j; k += kThreads) col[k] = t22[k];
+  __syncthreads();
+  double v = 0.0;
+  if (i < b1)
+    for (int k = g; k <= j; k += NG) v = fma(G[(int64_t)k * b1 + i], col[k], v);
+  part[g * nbp + i] = v;
+  __syncthreads();
+  if (g == 0) {
+    double t = 0.0;
+    for (int h = 0; h < NG; ++h) t += part[h * nbp + i];
+    col[i] = t;
+  }
+  __syncthreads();
+  v = 0.0;
+  for (int k = i + g; k < b1; k += NG) v = fma(T[(int64_t)k * ldT + i], col[k], v);
+  part[g * nbp + i] = v;
+  __syncthreads();
+  if (g == 0 && i < b1) {
+    double t = 0.0;
+    for (int h = 0; h < NG; ++h) t += part[h * nbp + i];
+    T[(int64_t)(b1 + j) * ldT + i] = -t;
   }
 }
 
@@ -615,6 +654,16 @@ int small_gemm(int64_t M, int64_t N, int64_t K, double alpha, MatRef A, MatRef B
   dim3 grid((unsigned)((M + 15) / 16), (unsigned)((N + 15) / 16));
   ProfScope ps(CANDMC_KCLASS_SMALL, 2.0 * M * N * K, s);
   k_small_gemm<<<grid, kThreads, 0, s>>>(A, B, M, N, K, alpha, beta, C, ldc);
+  CANDMC_CK(cudaGetLastError());
+  return CANDMC_OK;
+}
+
+int merge_t(const double* G, double* T, int64_t ldT, int b1, int b2, cudaStream_t s) {
+  if (b1 > kThreads || b2 > kThreads) return set_error(CANDMC_ERR_ARG, "merge_t needs widths of at most 256");
+  int nbp = 1;
+  while (nbp < b1) nbp <<= 1;
+  ProfScope ps(CANDMC_KCLASS_SMALL, 2.0 * b1 * b2 * (b1 + b2), s);
+  k_merge_t<<<(unsigned)b2, kThreads, 0, s>>>(G, T, ldT, b1, b2, nbp);
   CANDMC_CK(cudaGetLastError());
   return CANDMC_OK;
 }

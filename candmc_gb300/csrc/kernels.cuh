@@ -46,6 +46,8 @@ int hr_direct4(double* A, int64_t lda, int64_t m, int b, double* T, int64_t ldT,
                int64_t ldW, int* d_status, cudaStream_t s);
 
 // gemm_f64.cu
+// T12 = -T11 G T22 of two upper-triangular factors stored one after the other (T: ld ldT)
+int merge_t(const double* G, double* T, int64_t ldT, int b1, int b2, cudaStream_t s);
 int small_gemm(int64_t M, int64_t N, int64_t K, double alpha, MatRef A, MatRef B, double beta,
                double* C, int64_t ldc, cudaStream_t s);
 int gemm_tn_reduce(MatRef Y, MatRef C, int64_t m, int nb, int64_t n, MatRef Top, double alpha,

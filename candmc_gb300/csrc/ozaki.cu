@@ -38,6 +38,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <initializer_list>
 
 #include "kernels.cuh"
 
@@ -243,10 +244,12 @@ __device__ __forceinline__ f2 src_at(const SliceSrc& s, int64_t r, int64_t c) {
 
 // Slices of an R x K operand (rows n, the contraction index k), with one scale
 // exponent per row and K group of G (a multiple of 16, at most 128).  Element
-// (n, k) is src(k, n) (KROW = false: K runs down the source's columns) or
-// src(n, k) (KROW = true: K runs along its rows); rows from Nvalid to Rpad
+// (n, k) is src(k, n) (krow = 0: K runs down the source's columns) or
+// src(n, k) (krow = 1: K runs along its rows); rows from Nvalid to Rpad
 // and k from Kvalid on are zero.  Slices: S planes of Rpad x Kpad in the
-// core-matrix order; exponents e[(k / G) * Rpad + n].
+// core-matrix order; exponents e[(k / G) * Rpad + n].  A launch takes up to three
+// operands, one block range each: those of a panel's own products are small,
+// and the second and third launch cost 9 us each beside a first of 10.
 // A CTA takes kSliceRows rows and one group: it stages the group in shared
 // memory, warp w finds the exponents of rows 2w and 2w + 1, and then the
 // 16 x 16 elements of K16 block w are, in every plane, one contiguous 512-byte
@@ -257,16 +260,35 @@ __device__ __forceinline__ f2 src_at(const SliceSrc& s, int64_t r, int64_t c) {
 // for each, 16384 x 8192 elements took 599 us, with 8-way bank conflicts.
 constexpr int kSliceRows = 16;
 
-template <int S, bool KROW>
-__global__ void __launch_bounds__(256) k_slice(SliceSrc src, int64_t Kvalid, int64_t Nvalid,
-                                               int64_t Rpad, int64_t Kpad, int G, __nv_bfloat16* out, int* eout) {
+struct SliceJob {
+  SliceSrc src;
+  int krow;
+  int64_t Kvalid, Nvalid, Rpad, Kpad;
+  int G;
+  __nv_bfloat16* out;
+  int* e;
+  unsigned blocks() const { return (unsigned)((Rpad + kSliceRows - 1) / kSliceRows * (Kpad / G)); }
+};
+struct SliceJobs {
+  SliceJob job[3];
+  unsigned end[3];   // first block after each job's
+};
+
+template <int S>
+__global__ void __launch_bounds__(256) k_slice(const __grid_constant__ SliceJobs jobs) {
   __shared__ __align__(16) float2 tile[kSliceRows][128 + 2];
   __shared__ int s_e[kSliceRows];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int jb = blockIdx.x < jobs.end[0] ? 0 : blockIdx.x < jobs.end[1] ? 1 : 2;
+  const SliceJob& J = jobs.job[jb];
+  const unsigned block = blockIdx.x - (jb ? jobs.end[jb - 1] : 0);
+  const SliceSrc& src = J.src;
+  const int64_t Kvalid = J.Kvalid, Nvalid = J.Nvalid, Rpad = J.Rpad, Kpad = J.Kpad;
+  const int G = J.G;
   const unsigned nblocks = (unsigned)((Rpad + kSliceRows - 1) / kSliceRows);
-  const int64_t n0 = (int64_t)(blockIdx.x % nblocks) * kSliceRows;
-  const int64_t g = blockIdx.x / nblocks, kb0 = g * G;
-  if (KROW) {
+  const int64_t n0 = (int64_t)(block % nblocks) * kSliceRows;
+  const int64_t g = block / nblocks, kb0 = g * G;
+  if (J.krow) {
     const int r = threadIdx.x & 15;
     f2 v[8];
 #pragma unroll
@@ -301,7 +323,7 @@ __global__ void __launch_bounds__(256) k_slice(SliceSrc src, int64_t Kvalid, int
     const int e = scale_exp(mx * (1.0f + 1.0e-6f));
     if (lane == 0) {
       s_e[r] = e;
-      if (n0 + r < Rpad) eout[g * Rpad + n0 + r] = e;
+      if (n0 + r < Rpad) J.e[g * Rpad + n0 + r] = e;
     }
   }
   __syncthreads();
@@ -320,7 +342,7 @@ __global__ void __launch_bounds__(256) k_slice(SliceSrc src, int64_t Kvalid, int
                     [&](int i, f2x2 v) { d[i][c] = to_bf16x2(v); });
   }
   const int64_t plane = Rpad * Kpad;
-  __nv_bfloat16* o = out + ((kb0 >> 4) + warp) * (Rpad * 16) + ((n0 >> 3) + (lane >> 4)) * 128 + khalf * 64 + (lane & 7) * 8;
+  __nv_bfloat16* o = J.out + ((kb0 >> 4) + warp) * (Rpad * 16) + ((n0 >> 3) + (lane >> 4)) * 128 + khalf * 64 + (lane & 7) * 8;
 #pragma unroll
   for (int i = 0; i < S; ++i)
     *reinterpret_cast<uint4*>(o + i * plane) = make_uint4(d[i][0], d[i][1], d[i][2], d[i][3]);
@@ -1289,30 +1311,37 @@ __global__ void __launch_bounds__(256) k_cvt_df64(double* X, int64_t ld, int64_t
 }
 
 // Z (nb x n, FP64, ld nb) = sum over splits of the df64 partials [split][n][AR],
-// added in split order.  Eight partials are loaded before they are added, so a
-// narrow update's many splits (up to one per 128 rows) cost a few memory
-// latencies per output instead of one per split.
-__global__ void k_oz_sum_partials(const float2* part, int nsplit, int64_t AR, int nb, int64_t n,
-                                  double* Z) {
-  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (int64_t)nb * n) return;
-  int64_t i = idx % nb, j = idx / nb;
+// added in a fixed order.  Eight partials are loaded before they are added, so
+// that a narrow update's many splits (up to one per 128 rows) cost a few memory
+// latencies per output; and with W > 1 each of W warps takes 1 / W of the splits
+// of a CTA's 256 / W outputs, added up in shared memory (W = 8 from 16 splits:
+// 64 splits of 32 x 32 outputs took 12 us with one thread per output).
+template <int W>
+__global__ void __launch_bounds__(256) k_oz_sum_partials(const float2* part, int nsplit, int64_t AR, int nb,
+                                                         int64_t n, double* Z) {
+  constexpr int OUT = 256 / W;
+  __shared__ float2 sums[W][OUT];
+  const int o = threadIdx.x % OUT, w = threadIdx.x / OUT;
+  const int64_t idx = (int64_t)blockIdx.x * OUT + o;
+  const bool valid = idx < (int64_t)nb * n;
+  const int64_t i = idx % nb, j = idx / nb, stride = n * AR;
   const float2* p = part + j * AR + i;
-  const int64_t stride = n * AR;
+  const int per = (nsplit + W - 1) / W, end = min(nsplit, (w + 1) * per);
   f2 s = {0.0f, 0.0f};
-  int sp = 0;
-  for (; sp + 8 <= nsplit; sp += 8) {
+  for (int sp = w * per; valid && sp < end; sp += 8) {
     float2 v[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = p[(int64_t)(sp + u) * stride];
+    for (int u = 0; u < 8; ++u) v[u] = sp + u < end ? p[(int64_t)(sp + u) * stride] : make_float2(0.0f, 0.0f);
 #pragma unroll
     for (int u = 0; u < 8; ++u) s = df_add(s, {v[u].x, v[u].y});
   }
-  for (; sp < nsplit; ++sp) {
-    const float2 v = p[(int64_t)sp * stride];
-    s = df_add(s, {v.x, v.y});
+  if (W > 1) {
+    sums[w][o] = make_float2(s.h, s.l);
+    __syncthreads();
+    if (w) return;
+    for (int u = 1; u < W; ++u) s = df_add(s, {sums[u][o].x, sums[u][o].y});
   }
-  Z[j * nb + i] = df_to_double(s);
+  if (valid) Z[j * nb + i] = df_to_double(s);
 }
 
 // ------------------------------------------------------------------ host side
@@ -1345,27 +1374,24 @@ int from_df64(double* X, int64_t ld, int64_t m, int64_t n, cudaStream_t s) {
   return CANDMC_OK;
 }
 
-// KROW and the other arguments as in k_slice; Kpad is a multiple of G
-template <int S, bool KROW>
-static int launch_slice(SliceSrc src, int64_t Kvalid, int64_t Nvalid, int64_t Rpad, int64_t Kpad, int G,
-                        __nv_bfloat16* out, int* e, cudaStream_t s) {
-  ProfScope ps(CANDMC_KCLASS_OZ_SLICE, 8.0 * Nvalid * Kvalid + 2.0 * S * Rpad * Kpad, s);
-  const int64_t ctas = (Rpad + kSliceRows - 1) / kSliceRows * (Kpad / G);
-  k_slice<S, KROW><<<(unsigned)ctas, 256, 0, s>>>(src, Kvalid, Nvalid, Rpad, Kpad, G, out, e);
+// One launch over the operands of `jobs`.
+template <int S>
+static int launch_slices(std::initializer_list<SliceJob> jobs, cudaStream_t s) {
+  SliceJobs a{};
+  unsigned blocks = 0;
+  double bytes = 0.0;
+  int i = 0;
+  for (const SliceJob& j : jobs) {
+    a.job[i] = j;
+    blocks += j.out ? j.blocks() : 0;   // a job without an output is none
+    a.end[i++] = blocks;
+    if (j.out) bytes += 8.0 * j.Nvalid * j.Kvalid + 2.0 * S * j.Rpad * j.Kpad;
+  }
+  for (; i < 3; ++i) a.end[i] = blocks;
+  ProfScope ps(CANDMC_KCLASS_OZ_SLICE, bytes, s);
+  k_slice<S><<<blocks, 256, 0, s>>>(a);
   CANDMC_CK(cudaGetLastError());
   return CANDMC_OK;
-}
-
-template <int S>
-static int launch_slice_cols(SliceSrc src, int64_t Kvalid, int64_t Nvalid, int64_t Rpad, int64_t Kpad, int G,
-                             __nv_bfloat16* out, int* e, cudaStream_t s) {
-  return launch_slice<S, false>(src, Kvalid, Nvalid, Rpad, Kpad, G, out, e, s);
-}
-
-template <int S>
-static int launch_slice_rows(SliceSrc src, int64_t Kvalid, int64_t Nvalid, int64_t Rpad, int64_t Kpad, int G,
-                             __nv_bfloat16* out, int* e, cudaStream_t s) {
-  return launch_slice<S, true>(src, Kvalid, Nvalid, Rpad, Kpad, G, out, e, s);
 }
 
 int g_oz_reserve_sms = 32;
@@ -1439,7 +1465,7 @@ static int launch_oz_tn(OzArgs a, int64_t gn, int64_t gk, int cls, double flops,
 // (m x n) read through their slice sources; split-K partials summed in df64.
 template <int S>
 static int oz_tn(const SliceSrc& ysrc, const SliceSrc& csrc, int64_t m, int nb, int64_t n, double* Z,
-                 int* status, cudaStream_t s, int cls) {
+                 int* status, cudaStream_t s, int cls, const SliceJob& also = SliceJob{}) {
   const int64_t KG = 128;                       // K rows per exact accumulation
   // A-op = Y^T (rows = Householder index, K = m), B-op = C (rows = columns)
   const int64_t Kp1 = rup(m, KG);
@@ -1450,7 +1476,7 @@ static int oz_tn(const SliceSrc& ysrc, const SliceSrc& csrc, int64_t m, int nb, 
   CANDMC_RET(ya.alloc(sizeof(__nv_bfloat16) * S * AR1 * Kp1, s));
   CANDMC_RET(ea.alloc(sizeof(int) * (Kp1 / KG) * AR1, s));
   auto* yas = static_cast<__nv_bfloat16*>(ya.p);
-  CANDMC_RET(launch_slice_cols<S>(ysrc, m, nb, AR1, Kp1, (int)KG, yas, static_cast<int*>(ea.p), s));
+  const SliceJob yjob{ysrc, 0, m, nb, AR1, Kp1, (int)KG, yas, static_cast<int*>(ea.p)};
   const int64_t kper = KG * oz_groups_per_item(Kp1 / KG, ntiles);
   const int64_t ksplit = (Kp1 + kper - 1) / kper;
   CANDMC_RET(part.alloc(sizeof(float2) * ksplit * n * AR1, s));
@@ -1466,19 +1492,24 @@ static int oz_tn(const SliceSrc& ysrc, const SliceSrc& csrc, int64_t m, int nb, 
   if (csrc.df) {
     g1.C = const_cast<float2*>(csrc.df);
     g1.ldc = csrc.ld;
+    CANDMC_RET(launch_slices<S>({yjob, also}, s));
     CANDMC_RET(launch_oz_tn<S>(g1, ntiles, ksplit, cls, flops, s));
   } else {
     const int64_t BR1 = ntiles * OZ_N;
     CANDMC_RET(cb.alloc(sizeof(__nv_bfloat16) * S * BR1 * Kp1, s));
     CANDMC_RET(eb.alloc(sizeof(int) * (Kp1 / KG) * BR1, s));
     g1.Bs = static_cast<__nv_bfloat16*>(cb.p); g1.BR = BR1; g1.eB = static_cast<int*>(eb.p);
-    CANDMC_RET(launch_slice_cols<S>(csrc, m, n, BR1, Kp1, (int)KG, static_cast<__nv_bfloat16*>(cb.p),
-                                    static_cast<int*>(eb.p), s));
+    const SliceJob cjob{csrc, 0, m, n, BR1, Kp1, (int)KG, static_cast<__nv_bfloat16*>(cb.p), static_cast<int*>(eb.p)};
+    CANDMC_RET(launch_slices<S>({yjob, cjob, also}, s));
     CANDMC_RET((launch_oz_mma<S, kOzSums>(g1, 1, ntiles, ksplit, cls, flops, s)));
   }
   ProfScope ps(CANDMC_KCLASS_REDUCE, 8.0 * ksplit * n * AR1, s);
-  k_oz_sum_partials<<<(unsigned)((nb * n + 255) / 256), 256, 0, s>>>(static_cast<float2*>(part.p),
-                                                                      (int)ksplit, AR1, nb, n, Z);
+  const int64_t outs = (int64_t)nb * n;
+  const auto* pp = static_cast<const float2*>(part.p);
+  if (ksplit >= 16)
+    k_oz_sum_partials<8><<<(unsigned)((outs + 31) / 32), 256, 0, s>>>(pp, (int)ksplit, AR1, nb, n, Z);
+  else
+    k_oz_sum_partials<1><<<(unsigned)((outs + 255) / 256), 256, 0, s>>>(pp, (int)ksplit, AR1, nb, n, Z);
   CANDMC_CK(cudaGetLastError());
   return CANDMC_OK;
 }
@@ -1501,12 +1532,9 @@ static int oz_top_times(MatRef Top, int nb, const double* Z, int64_t n, double* 
   const SliceSrc tsrc{Top.p, nullptr, Top.ld, Top.mask, Top.off};
   // A operand element (i, k) = Top(i, k): X[k, i] of a transposed reference
   // (a column of X per operand row), X[i, k] otherwise (a row of X)
-  if (Top.trans)
-    CANDMC_RET(launch_slice_cols<S>(tsrc, nb, nb, OZ_M, Kp, (int)Kp, tas, static_cast<int*>(et.p), s));
-  else
-    CANDMC_RET(launch_slice_rows<S>(tsrc, nb, nb, OZ_M, Kp, (int)Kp, tas, static_cast<int*>(et.p), s));
-  CANDMC_RET(launch_slice_cols<S>(SliceSrc{Z, nullptr, nb, kDense, 0}, nb, n, BR, Kp, (int)Kp, zbs,
-                                  static_cast<int*>(ez.p), s));
+  const SliceJob tjob{tsrc, Top.trans ? 0 : 1, nb, nb, OZ_M, Kp, (int)Kp, tas, static_cast<int*>(et.p)};
+  const SliceJob zjob{SliceSrc{Z, nullptr, nb, kDense, 0}, 0, nb, n, BR, Kp, (int)Kp, zbs, static_cast<int*>(ez.p)};
+  CANDMC_RET(launch_slices<S>({tjob, zjob}, s));
   OzArgs g{};
   g.As = tas; g.AR = OZ_M; g.Bs = zbs; g.BR = BR;
   g.Kpad = g.k_per_cta = g.kgroup = (int)Kp;
@@ -1539,7 +1567,14 @@ static int apply_qt_slices(const double* Y, int64_t ldy, int ymask, int64_t m, i
                          : SliceSrc{nullptr, reinterpret_cast<const float2*>(C), ldc, kDense, 0};
   DevBuf z, zt;
   CANDMC_RET(z.alloc(sizeof(double) * nb * n, s));
-  CANDMC_RET(oz_tn<S>(ysrc, csrc, m, nb, n, z.d(), status, s, cls_tn));
+  // Y as the A operand of GEMM2 (rows = m, K = nb) is sliced in the same launch
+  const int64_t Kp2 = rup(nb, 16);
+  const int64_t AR2 = rup(m, OZ_M), BR2 = rup(n, OZ_N);
+  DevBuf y2, ey2, z2, ez2;
+  CANDMC_RET(y2.alloc(sizeof(__nv_bfloat16) * S * AR2 * Kp2, s));
+  CANDMC_RET(ey2.alloc(sizeof(int) * AR2, s));
+  const SliceJob y2job{ysrc, 1, nb, m, AR2, Kp2, (int)Kp2, static_cast<__nv_bfloat16*>(y2.p), static_cast<int*>(ey2.p)};
+  CANDMC_RET(oz_tn<S>(ysrc, csrc, m, nb, n, z.d(), status, s, cls_tn, y2job));
   // ---- Z' = T^T * Z   (FP64 storage, nb x n); counted, as on the FP64 pipe,
   // under the small-product class, apart from the two contractions with Y
   CANDMC_RET(zt.alloc(sizeof(double) * nb * n, s));
@@ -1548,18 +1583,10 @@ static int apply_qt_slices(const double* Y, int64_t ldy, int ymask, int64_t m, i
   else
     CANDMC_RET(small_gemm(nb, n, nb, 1.0, Top, mref(z.d(), nb), 0.0, zt.d(), nb, s));
   // ---- GEMM2: C -= Y * Z'.  A-op = Y (rows = m, K = nb), B-op = Z'^T (rows = columns, K = nb)
-  const int64_t Kp2 = rup(nb, 16);
-  const int64_t AR2 = rup(m, OZ_M), BR2 = rup(n, OZ_N);
-  DevBuf y2, ey2, z2, ez2;
-  CANDMC_RET(y2.alloc(sizeof(__nv_bfloat16) * S * AR2 * Kp2, s));
-  CANDMC_RET(ey2.alloc(sizeof(int) * AR2, s));
   CANDMC_RET(z2.alloc(sizeof(__nv_bfloat16) * S * BR2 * Kp2, s));
   CANDMC_RET(ez2.alloc(sizeof(int) * BR2, s));
-  CANDMC_RET(launch_slice_rows<S>(ysrc, nb, m, AR2, Kp2, (int)Kp2, static_cast<__nv_bfloat16*>(y2.p),
-                               static_cast<int*>(ey2.p), s));
-  SliceSrc zsrc{zt.d(), nullptr, nb, kDense, 0};
-  CANDMC_RET(launch_slice_cols<S>(zsrc, nb, n, BR2, Kp2, (int)Kp2, static_cast<__nv_bfloat16*>(z2.p),
-                               static_cast<int*>(ez2.p), s));
+  CANDMC_RET(launch_slices<S>({SliceJob{SliceSrc{zt.d(), nullptr, nb, kDense, 0}, 0, nb, n, BR2, Kp2, (int)Kp2,
+                                        static_cast<__nv_bfloat16*>(z2.p), static_cast<int*>(ez2.p)}}, s));
   OzArgs g2{};
   g2.As = static_cast<__nv_bfloat16*>(y2.p); g2.AR = AR2;
   g2.Bs = static_cast<__nv_bfloat16*>(z2.p); g2.BR = BR2;

@@ -73,3 +73,28 @@ def test_panel_empty_tails_and_non_finite(cm):
     cm.hh_recon_qr(d)
     torch.cuda.synchronize()
     assert np.isnan(d.cpu().numpy()[:24, 7:]).any()
+
+
+# T from two halves' factors (T12 = -T11 G T22): halves of 16 to 128 columns, even
+# and odd, FP64 products and, from 16 row splits on, the emulated ones
+@pytest.mark.parametrize("m,b,oz", [(300, 33, 0), (300, 47, 0), (700, 64, 0), (333, 65, 0), (600, 100, 0), (520, 128, 0),
+                                    (600, 255, 0), (2500, 96, 1), (2049, 50, 1), (1900, 128, 1)])
+def test_merged_factors(cm, m, b, oz):
+    A = fx.gaussian(m, b, 7 * m + b)
+    YRo, Wo = co.hh_recon_qr(A, b)
+    To = co.T_from_W(Wo, lp.unit_lower(YRo, b)[:b])
+    tol = 2e-12 * max(1.0, b / 16)
+    d = torch.from_numpy(np.asfortranarray(A)).cuda().t().contiguous().t()
+    if oz:   # one panel; T enters through the next half's update only
+        try:
+            cm.set_tuning("panel_oz_min_rows", 1024)
+            cm.QR_2D(d, b, precision="ozaki")
+            torch.cuda.synchronize()
+        finally:
+            cm.set_tuning("panel_oz_min_rows", 8192)
+    else:
+        W, T = cm.hh_recon_qr(d)
+        torch.cuda.synchronize()
+        assert np.abs(T.cpu().numpy() - To).max() <= tol
+        assert np.array_equal(np.tril(T.cpu().numpy(), -1), np.zeros((b, b)))
+    assert np.abs(d.cpu().numpy() - YRo).max() <= tol * max(1.0, np.abs(YRo).max())
