@@ -483,13 +483,17 @@ k_merge_t(const double* G, double* T, int64_t ldT, int b1, int b2, int nbp) {
 // groups are combined in shared memory, and the product with opT splits its k
 // range over the groups the same way, so every dependent FP64 chain is about
 // nsplit / G + nb / G long instead of nsplit + nb.  The summation order is
-// fixed, so the result is deterministic.
-__global__ void __launch_bounds__(kThreads)
+// fixed, so the result is deterministic.  With few columns of 128 rows or more a CTA
+// has 1024 threads: its loads and FP64 chains bound the launch then (a 128 x 16
+// step of a triangular solve with 32 partials: 17 + 6 us as a product and a
+// reduction, 8 here).
+template <int TH>
+__global__ void __launch_bounds__(TH)
 k_reduce_apply(const double* Zp, int nsplit, int64_t split_stride, int nb, int nbp, int64_t n,
                MatRef Top, double alpha, double* Z, int64_t ldz) {
-  __shared__ double part[kThreads];
+  __shared__ double part[TH];
   __shared__ double col[256];
-  const int G = kThreads / nbp;
+  const int G = TH / nbp;
   const int i = threadIdx.x % nbp, g = threadIdx.x / nbp;
   const int64_t jc = blockIdx.x;
   double sacc = 0.0;
@@ -669,12 +673,15 @@ int merge_t(const double* G, double* T, int64_t ldT, int b1, int b2, cudaStream_
 }
 
 // Z = alpha opT (sum of the nsplit partial products)
-static int reduce_apply(const double* part, int64_t nsplit, int64_t stride, int nb, int64_t n, MatRef Top,
+int reduce_apply(const double* part, int64_t nsplit, int64_t stride, int nb, int64_t n, MatRef Top,
                         double alpha, double* Z, int64_t ldz, cudaStream_t s) {
   int nbp = 1;
   while (nbp < nb) nbp <<= 1;
   ProfScope ps(CANDMC_KCLASS_REDUCE, 8.0 * stride * nsplit, s);
-  k_reduce_apply<<<(unsigned)n, kThreads, 0, s>>>(part, (int)nsplit, stride, nb, nbp, n, Top, alpha, Z, ldz);
+  if (nbp >= 128 && n <= 2 * num_sms())
+    k_reduce_apply<1024><<<(unsigned)n, 1024, 0, s>>>(part, (int)nsplit, stride, nb, nbp, n, Top, alpha, Z, ldz);
+  else
+    k_reduce_apply<kThreads><<<(unsigned)n, kThreads, 0, s>>>(part, (int)nsplit, stride, nb, nbp, n, Top, alpha, Z, ldz);
   CANDMC_CK(cudaGetLastError());
   return CANDMC_OK;
 }
@@ -720,12 +727,7 @@ int gemm_tn_reduce(MatRef Y, MatRef C, int64_t m, int nb, int64_t n, MatRef Top,
       k_gemv_tn<<<dim3((unsigned)cblk, (unsigned)nsplit), kThreads, 0, s>>>(Y, C, m, nb, kchunk, part.d());
     }
     CANDMC_CK(cudaGetLastError());
-    int nbp = 1;
-    while (nbp < nb) nbp <<= 1;
-    ProfScope ps(CANDMC_KCLASS_REDUCE, 8.0 * nb * nsplit, s);
-    k_reduce_apply<<<1u, kThreads, 0, s>>>(part.d(), (int)nsplit, nb, nb, nbp, 1, Top, alpha, Z, ldz);
-    CANDMC_CK(cudaGetLastError());
-    return CANDMC_OK;
+    return reduce_apply(part.d(), nsplit, nb, nb, 1, Top, alpha, Z, ldz, s);
   }
   if (m * nb * n <= kSmallProduct) return small_tn(Y, C, m, nb, n, Top, alpha, Z, ldz, s);
   // column groups: 4, or 1 (and eight groups of rows) when there are at most

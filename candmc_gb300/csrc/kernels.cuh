@@ -50,6 +50,9 @@ int hr_direct4(double* A, int64_t lda, int64_t m, int b, double* T, int64_t ldT,
 int merge_t(const double* G, double* T, int64_t ldT, int b1, int b2, cudaStream_t s);
 int small_gemm(int64_t M, int64_t N, int64_t K, double alpha, MatRef A, MatRef B, double beta,
                double* C, int64_t ldc, cudaStream_t s);
+// Z (nb x n, ldz) = alpha opT (sum of nsplit partials of nb x n, ld nb); nb <= 256
+int reduce_apply(const double* part, int64_t nsplit, int64_t stride, int nb, int64_t n, MatRef Top, double alpha,
+                 double* Z, int64_t ldz, cudaStream_t s);
 int gemm_tn_reduce(MatRef Y, MatRef C, int64_t m, int nb, int64_t n, MatRef Top, double alpha,
                    double* Z, int64_t ldz, cudaStream_t s);
 int gemm_nn_sub(double* C, int64_t ldc, MatRef Y, const double* Z, int64_t ldz, int64_t m,

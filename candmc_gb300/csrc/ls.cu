@@ -33,30 +33,37 @@
 
 namespace candmc {
 
-constexpr int TS_M = 128;   // output rows per CTA
 constexpr int TS_R = 16;    // right-hand sides per CTA
 constexpr int TS_K = 32;
 
-// part[z] (r x M, ld M) = op(A)[rows of the tile, K chunk z] * X[K chunk, cols]
-// op(A) = A (M x K, ld lda) or A^T (A is K x M).
-template <int TRANS>
+// part[z] (r x M, ld M) = op(A)[rows of the tile, K chunk z] * X[K chunk, cols],
+// less Cin in chunk 0 (Cin: may be null).  op(A) = A (M x K, ld lda) or A^T (A is
+// K x M).  A CTA takes RM rows and 16 right-hand sides, a thread 16 RM / 256 of
+// one row's.  Bound by the FP64 pipe: 128 rows x 128 of K take 68 us of one SM, so
+// products of few rows (a block row of a triangular solve) take RM = 32 and short
+// chunks (4.3 us for 32 of K).
+template <int TRANS, int RM>
 __global__ void __launch_bounds__(256) k_ts_gemm(const double* A, int64_t lda, const double* X,
                                                  int64_t ldx, int64_t M, int64_t K, int64_t r,
-                                                 int64_t kchunk, double* part) {
-  __shared__ double sA[TS_K][TS_M + 1];
+                                                 int64_t kchunk, const double* Cin, int64_t ldc, double* part) {
+  constexpr int NC = TS_R * RM / 256;   // columns per thread
+  __shared__ double sA[TS_K][RM + 1];
   __shared__ double sX[TS_K][TS_R];
   const int tid = threadIdx.x;
-  const int row = tid % TS_M, half = tid / TS_M;      // 2 x 8 columns
-  const int64_t i0 = (int64_t)blockIdx.x * TS_M, c0 = (int64_t)blockIdx.y * TS_R;
+  const int row = tid % RM, grp = tid / RM;
+  const int64_t i0 = (int64_t)blockIdx.x * RM, c0 = (int64_t)blockIdx.y * TS_R;
   const int64_t k0 = (int64_t)blockIdx.z * kchunk;
   const int64_t k1 = (k0 + kchunk < K) ? k0 + kchunk : K;
-  double acc[8];
+  double acc[NC];
 #pragma unroll
-  for (int v = 0; v < 8; ++v) acc[v] = 0.0;
+  for (int v = 0; v < NC; ++v) {
+    const int64_t gc = c0 + grp * NC + v;
+    acc[v] = (Cin && blockIdx.z == 0 && i0 + row < M && gc < r) ? -Cin[gc * ldc + i0 + row] : 0.0;
+  }
   for (int64_t kb = k0; kb < k1; kb += TS_K) {
-    for (int idx = tid; idx < TS_K * TS_M; idx += 256) {
+    for (int idx = tid; idx < TS_K * RM; idx += 256) {
       int kk, ii;
-      if (TRANS) { kk = idx % TS_K; ii = idx / TS_K; } else { ii = idx % TS_M; kk = idx / TS_M; }
+      if (TRANS) { kk = idx % TS_K; ii = idx / TS_K; } else { ii = idx % RM; kk = idx / RM; }
       const int64_t gi = i0 + ii, gk = kb + kk;
       double v = 0.0;
       if (gi < M && gk < k1) v = TRANS ? A[gi * lda + gk] : A[gk * lda + gi];
@@ -72,7 +79,7 @@ __global__ void __launch_bounds__(256) k_ts_gemm(const double* A, int64_t lda, c
     for (int kk = 0; kk < TS_K; ++kk) {
       const double a = sA[kk][row];
 #pragma unroll
-      for (int v = 0; v < 8; ++v) acc[v] = fma(a, sX[kk][half * 8 + v], acc[v]);
+      for (int v = 0; v < NC; ++v) acc[v] = fma(a, sX[kk][grp * NC + v], acc[v]);
     }
     __syncthreads();
   }
@@ -80,8 +87,8 @@ __global__ void __launch_bounds__(256) k_ts_gemm(const double* A, int64_t lda, c
   if (gi >= M) return;
   double* out = part + (int64_t)blockIdx.z * r * M;
 #pragma unroll
-  for (int v = 0; v < 8; ++v) {
-    const int64_t gc = c0 + half * 8 + v;
+  for (int v = 0; v < NC; ++v) {
+    const int64_t gc = c0 + grp * NC + v;
     if (gc < r) out[gc * M + gi] = acc[v];
   }
 }
@@ -198,6 +205,43 @@ static int ls_sms() {
   return n;
 }
 
+// Row tile and K split of k_ts_gemm: tiles of 128 rows and chunks of at least 128
+// of K (about 4 CTAs per SM) where those fill the chip, else tiles of 32 rows and
+// chunks from 32 (about one CTA per SM; more splits would cost the reduction).
+struct TsSplit {
+  bool small;
+  int64_t kchunk, nsplit;
+};
+static TsSplit ts_split(int64_t M, int64_t K, int64_t r) {
+  const int64_t cols = (r + TS_R - 1) / TS_R, t128 = (M + 127) / 128 * cols, t32 = (M + 31) / 32 * cols;
+  TsSplit p;
+  p.small = t128 * ((K + 127) / 128) < ls_sms();
+  int64_t n = p.small ? std::min<int64_t>((ls_sms() + t32 - 1) / t32, (K + TS_K - 1) / TS_K)
+                      : std::min<int64_t>((4 * ls_sms() + t128 - 1) / t128, (K + 127) / 128);
+  n = std::max<int64_t>(1, n);
+  p.kchunk = std::max<int64_t>(TS_K, ((K + n - 1) / n + TS_K - 1) / TS_K * TS_K);
+  p.nsplit = std::max<int64_t>(1, (K + p.kchunk - 1) / p.kchunk);
+  return p;
+}
+
+// the partial products of p, K > 0
+static int ts_parts(const TsSplit& p, bool trans, const double* A, int64_t lda, const double* X, int64_t ldx,
+                    int64_t M, int64_t K, int64_t r, const double* Cin, int64_t ldc, double* part, cudaStream_t s) {
+  ProfScope ps(CANDMC_KCLASS_GEMM_TN, 2.0 * M * K * r, s);
+  const int64_t rm = p.small ? 32 : 128;
+  const dim3 g((unsigned)((M + rm - 1) / rm), (unsigned)((r + TS_R - 1) / TS_R), (unsigned)p.nsplit);
+  auto run = [&](auto kernel) { kernel<<<g, 256, 0, s>>>(A, lda, X, ldx, M, K, r, p.kchunk, Cin, ldc, part); };
+  if (p.small) {
+    if (trans) run(k_ts_gemm<1, 32>);
+    else run(k_ts_gemm<0, 32>);
+  } else {
+    if (trans) run(k_ts_gemm<1, 128>);
+    else run(k_ts_gemm<0, 128>);
+  }
+  CANDMC_CK(cudaGetLastError());
+  return CANDMC_OK;
+}
+
 // out (M x r) = beta * Cin + alpha * op(A) X, FP64, op(A) M x K
 static int ts_gemm(bool trans, const double* A, int64_t lda, const double* X, int64_t ldx, int64_t M,
                    int64_t K, int64_t r, double alpha, double beta, const double* Cin, int64_t ldc,
@@ -227,24 +271,14 @@ static int ts_gemm(bool trans, const double* A, int64_t lda, const double* X, in
     CANDMC_CK(cudaGetLastError());
     return CANDMC_OK;
   }
-  const int64_t tiles = ((M + TS_M - 1) / TS_M) * ((r + TS_R - 1) / TS_R);
-  int64_t nsplit = std::max<int64_t>(1, std::min<int64_t>((4 * ls_sms() + tiles - 1) / tiles, (K + 127) / 128));
-  int64_t kchunk = ((K + nsplit - 1) / nsplit + TS_K - 1) / TS_K * TS_K;
-  if (kchunk <= 0) kchunk = TS_K;
-  nsplit = std::max<int64_t>(1, (K + kchunk - 1) / kchunk);
+  const TsSplit p = ts_split(M, K, r);
+  const int64_t nsplit = p.nsplit;
   DevBuf part;
   CANDMC_RET(part.alloc(sizeof(double) * nsplit * M * r, s));
-  if (K > 0) {
-    ProfScope ps(CANDMC_KCLASS_GEMM_TN, 2.0 * M * K * r, s);
-    dim3 g((unsigned)((M + TS_M - 1) / TS_M), (unsigned)((r + TS_R - 1) / TS_R), (unsigned)nsplit);
-    if (trans)
-      k_ts_gemm<1><<<g, 256, 0, s>>>(A, lda, X, ldx, M, K, r, kchunk, part.d());
-    else
-      k_ts_gemm<0><<<g, 256, 0, s>>>(A, lda, X, ldx, M, K, r, kchunk, part.d());
-    CANDMC_CK(cudaGetLastError());
-  } else {
+  if (K > 0)
+    CANDMC_RET(ts_parts(p, trans, A, lda, X, ldx, M, K, r, nullptr, 0, part.d(), s));
+  else
     CANDMC_CK(cudaMemsetAsync(part.p, 0, sizeof(double) * M * r, s));
-  }
   ProfScope ps(CANDMC_KCLASS_REDUCE, 8.0 * nsplit * M * r, s);
   k_ts_reduce<<<(unsigned)((M * r + 255) / 256), 256, 0, s>>>(part.d(), (int)nsplit, M, r, alpha, beta,
                                                               Cin, ldc, out, ldo);
@@ -262,7 +296,18 @@ static int trsm_upper(const double* R, int64_t ldr, int64_t n, const double* Din
     const int64_t q = trans ? qq : nblk - 1 - qq;
     const int64_t j0 = q * w, bw = std::min<int64_t>(w, n - j0);
     double* Xj = X + j0;
-    if (!trans) {
+    const int64_t K = trans ? j0 : n - j0 - bw;
+    if (r > 1 && K > 0) {
+      // X_j = D_q^-1 (X_j - R_jk X_k): partial products with -X_j in the first, then
+      // their sum times -D_q^-1
+      const TsSplit p = ts_split(bw, K, r);
+      DevBuf part;
+      CANDMC_RET(part.alloc(sizeof(double) * p.nsplit * bw * r, s));
+      CANDMC_RET(ts_parts(p, trans, trans ? R + j0 * ldr : R + (j0 + bw) * ldr + j0, ldr, trans ? X : X + j0 + bw, ldx,
+                          bw, K, r, Xj, ldx, part.d(), s));
+      CANDMC_RET(reduce_apply(part.d(), p.nsplit, bw * r, (int)bw, r, mref(Dinv + q * w * w, w, trans ? 1 : 0), -1.0,
+                              Xj, ldx, s));
+    } else if (!trans) {
       // tmp = X_j - R[j0:j0+bw, j0+bw:n] X[j0+bw:n]
       CANDMC_RET(ts_gemm(false, R + (j0 + bw) * ldr + j0, ldr, X + j0 + bw, ldx, bw, n - j0 - bw, r, -1.0,
                          1.0, Xj, ldx, tmp.d(), w, s));

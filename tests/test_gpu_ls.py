@@ -149,3 +149,24 @@ def test_ls_fp32_form_refined_at_moderate_kappa(cm, smin, refine):
     X = host(X)
     err = np.linalg.norm(X - Xo, axis=0) / np.linalg.norm(Xo, axis=0)
     assert err.max() <= max(LS_TOL, 100 * (1 / smin) * 2.2e-16), (err, st)
+
+
+# block rows of the triangular solves: remainders of the 32-row tiles and of the 128-row
+# blocks, one and several column tiles, chunks of 32 and more of K; and products of
+# the refinement on both sides of the row-tile rule
+@pytest.mark.parametrize("m,n,nrhs", [(200, 129, 2), (300, 255, 16), (700, 513, 17), (1500, 1100, 33), (3000, 2305, 5)])
+@pytest.mark.parametrize("refine", [0, 1])
+def test_ls_solve_block_rows(cm, m, n, nrhs, refine):
+    A = fx.gaussian(m, n, m + n)
+    B = fx.gaussian(m, nrhs, 11)
+    Xo = co.ls_solve(A, B, 128)
+    try:
+        cm.set_tuning("ls_refine", refine)
+        X, st = cm.ls_solve(dev(A), dev(B), b=64, precision="fp64", max_refine=30, tol=1e-15)
+        torch.cuda.synchronize()
+    finally:
+        cm.set_tuning("ls_refine", 0)
+    X = host(X)
+    err = np.linalg.norm(X - Xo, axis=0) / np.linalg.norm(Xo, axis=0)
+    assert err.max() <= LS_TOL, (err.max(), st)
+    assert st["status"] == 0
