@@ -748,6 +748,21 @@ int gemm_tn_reduce(MatRef Y, MatRef C, int64_t m, int nb, int64_t n, MatRef Top,
   const int64_t tiles = ntiles();
   int64_t nsplit = std::max<int64_t>(1, std::min<int64_t>(target / tiles, (m + 15) / 16));
   nsplit = std::min<int64_t>(nsplit, 1024);
+  if (nsplit <= 4) {
+    // Many tiles: CTAs on one SM share its FP64 pipe, so the fullest SM's rows
+    // count, and a split that leaves it few more than the mean is worth its
+    // partials (a CTA's start and end cost about 24 rows, adding a partial 4).
+    // 2048 x 128 x 16384, 512 tiles: one chunk 8.45 ms (4 rounds where 3.37 would
+    // do), 2 chunks 7.35; 16384 x 128 x 8192, 256 tiles: 34.3, and 28.7 with 7.
+    int64_t best = INT64_MAX;
+    for (int64_t ns = 1; ns <= 8 && (ns == 1 || m / ns >= 128); ++ns) {
+      const int64_t cost = (tiles * ns + sms - 1) / sms * ((m + ns - 1) / ns + 24) + 4 * ns;
+      if (cost < best) {
+        best = cost;
+        nsplit = ns;
+      }
+    }
+  }
   const int64_t kchunk = (m + nsplit - 1) / nsplit;
   nsplit = std::max<int64_t>(1, (m + kchunk - 1) / kchunk);
   const int64_t stride = (int64_t)nb * n;

@@ -112,3 +112,10 @@ def test_fp64_products(cm, m, nb, n, masked):
     want = C - E @ (2 * (E.T @ C))
     bound = 2 * u * (np.abs(C) + (m + nb + 2) * (np.abs(E) @ (2 * aZ)))
     assert (np.abs(dC.cpu().numpy() - want) <= bound).all()
+
+
+# many column tiles, where the row split balances the rounds: one tile more than a
+# round of SMs, odd chunks, chunks of the smallest length
+@pytest.mark.parametrize("m,nb,n", [(1111, 65, 4900), (900, 128, 2500), (256, 70, 9800), (2050, 33, 3300)])
+def test_fp64_products_wide(cm, m, nb, n):
+    test_fp64_products(cm, m, nb, n, False)
