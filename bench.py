@@ -592,7 +592,7 @@ def wl_caqr(args, ctx):
                 "frac": achieved / pk if achieved else None,
                 "bf16_issued_tflops": achieved * 28.0 if achieved else None,
                 "traffic": traffic_from_profile("ozaki_gemm_caqr_n16384.md"),
-                "kernel": "k_oz_mma (Ozaki BF16 slice contractions on tcgen05, Y^T A and A -= Y Z; "
+                "kernel": "k_oz_tn, k_oz_mma (Ozaki BF16 slice contractions on tcgen05, Y^T A and A -= Y Z; "
                           "the b x b operator product T^T Z is counted under 'small')",
                 "launches": dom_l, "share_of_step": dom_ms / t_max if t_max else None,
                 "peak_source": "MEASURED_PEAKS.json bf16_tflops_sustained / 28 slice products "
@@ -602,7 +602,7 @@ def wl_caqr(args, ctx):
         pk = measured_peaks().get("bf16_tflops_sustained", 1700.0) / 6.0
         roof = {"bound": "tensor", "achieved": achieved, "peak": pk, "unit": "TFLOP/s",
                 "frac": achieved / pk if achieved else None, "traffic": None,
-                "kernel": "k_oz_mma<., 3> (FP32 form: 3 BF16 slices on tcgen05)", "launches": dom_l,
+                "kernel": "k_oz_tn<3>, k_oz_mma<3, .> (FP32 form: 3 BF16 slices on tcgen05)", "launches": dom_l,
                 "share_of_step": dom_ms / t_max if t_max else None,
                 "peak_source": "MEASURED_PEAKS.json bf16_tflops_sustained / 6 slice products (of measured)"}
     else:
@@ -831,7 +831,7 @@ def wl_forms(args, ctx):
         ach = sum(prof[c][1] for c in dom) / (dom_ms / 1e3) / 1e12 if dom_ms else None
         roof = {"bound": "tensor", "achieved": ach, "peak": pk, "unit": "TFLOP/s",
                 "frac": ach / pk if ach else None, "traffic": None,
-                "kernel": "k_oz_mma", "peak_source": "bf16_tflops_sustained / 28 (of measured)"}
+                "kernel": "k_oz_tn, k_oz_mma", "peak_source": "bf16_tflops_sustained / 28 (of measured)"}
     line = base_line(args, ctx, "CAQR TFLOP/s by precision form (FP64-equivalent, 2mn^2 - 2/3 n^3)",
                      tf * ctx.world, "TFLOP/s", ms, f"{form} trailing update, f64 panels",
                      {"workload": f"CAQR {m}x{n} b={b}, A=U diag(logspace(0,-10|-3,n)) V^T, U,V Haar "

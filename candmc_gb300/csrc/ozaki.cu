@@ -106,7 +106,7 @@ __device__ __forceinline__ f2 df_add(f2 x, f2 y) {
 
 // x as FP32 hi + lo, each rounded to nearest even.  A conversion or an addition
 // of doubles costs a slot of the FP64 pipe (65 cycles a warp on each
-// sub-partition: four of them per element held k_to_df64 at 2.2 TB/s), so in
+// sub-partition: four of them per element held the conversion at 2.2 TB/s), so in
 // the range where both parts are normal the split works on the bits: hi is the
 // significand rounded to 24 bits, lo the exact difference of the two bit
 // patterns (an integer below 2^28 in units of 2^(e - 52)).
