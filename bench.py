@@ -606,7 +606,7 @@ def wl_caqr(args, ctx):
                 "share_of_step": dom_ms / t_max if t_max else None,
                 "peak_source": "MEASURED_PEAKS.json bf16_tflops_sustained / 6 slice products (of measured)"}
     else:
-        roof = fp64_roof(prof, dom, "k_gemm_f64 (Y^T A split-K partials and A -= Y Z)", t_max)
+        roof = fp64_roof(prof, dom, "k_gemm_tn, k_gemm_nn_sub (Y^T A split-row partials and A -= Y Z)", t_max)
         roof["traffic"] = traffic_from_profile("gemm_f64_caqr_n16384.md")
 
     log(f"caqr {prec}: {t_max / args.steps:.1f} ms/step")
@@ -678,7 +678,7 @@ def wl_caqr(args, ctx):
 def caqr_fp64_leg(args, ctx, A0, A, steps=2, warmup=1):
     """The plain FP64 form on the same matrix: TFLOP/s and accuracy."""
     _, dom, t_max, launches, prof, clk = caqr_form_run(ctx, A0, A, args.b, "fp64", args.entry, steps, warmup)
-    roof = fp64_roof(prof, dom, "k_gemm_f64", t_max)
+    roof = fp64_roof(prof, dom, "k_gemm_tn, k_gemm_nn_sub", t_max)
     bwd, orth = full_accuracy(ctx.cm, A0, A, args.b, precision="fp64")
     return {"value": flops(args.n) * steps / (t_max / 1e3) / 1e12, "unit": "TFLOP/s", "steps": steps,
             "warmup": warmup, "ms_per_step": t_max / steps, "gpu_launches": launches,
@@ -714,7 +714,7 @@ def wl_tsqr_hr(args, ctx):
     f = qr_flops(m, b)
     value = ctx.world * f * args.steps / (t_max / 1e3) / 1e9
     roof = fp64_roof(prof, ["panel_leaf", "panel_y"],
-                     "k_hr6_pipe (pipelined TSQR tree) or k_hr4_leaf_tree, + k_hr4_form_y (reconstruction, Y)",
+                     "k_hr6_pipe (pipelined TSQR tree) or k_hr4_leaf_tree, + k_hr6_y or k_hr4_form_y (reconstruction, Y)",
                      t_max)
     roof["traffic"] = traffic_from_profile("tsqr_hr_panel_8192x64.md")
     shares = kernel_time_shares(ctx, step)
@@ -972,7 +972,7 @@ def wl_batched(args, ctx):
         step()                                   # the chosen form's result for the accuracy check
     f = sum(qr_flops(m, n) for m, n in sizes)
     by = sum(16.0 * m * n for m, n in sizes)
-    roof = fp64_roof(prof, ["panel_leaf", "panel_y"], "k_hr6_pipe / k_hr4_leaf_tree + k_hr4_form_y", t_max)
+    roof = fp64_roof(prof, ["panel_leaf", "panel_y"], "k_hr6_pipe / k_hr4_leaf_tree + k_hr6_y or k_hr4_form_y", t_max)
     hbm = measured_peaks().get("hbm_gbs", 6778.0)
     roof["step_fp64_tflops"] = f * args.steps / (t_max / 1e3) / 1e12
     if roof["achieved"] is None:
