@@ -200,6 +200,11 @@ extern "C" int candmc_set_tuning(const char* key, int64_t value) {
     g_pipe_tree = (int)value;
     return CANDMC_OK;
   }
+  if (std::string(key) == "panel_polls" || std::string(key) == "panel_smem_polls") {
+    if (value < 1 || value > (1 << 30)) return set_error(CANDMC_ERR_ARG, "panel_polls, panel_smem_polls in [1, 2^30]");
+    (std::string(key) == "panel_polls" ? g_panel_polls : g_panel_smem_polls) = (int)value;
+    return CANDMC_OK;
+  }
   return set_error(CANDMC_ERR_ARG, "unknown tuning key");
 }
 
@@ -221,11 +226,13 @@ extern "C" int candmc_batched_ls(int64_t nprob, const int64_t* m, const int64_t*
   }
   if (!use_graph) return batched_issue(nprob, m, n, A, lda, B, nstreams, s);
   std::vector<int64_t> key;
-  key.reserve(6 * nprob + 4);
+  key.reserve(5 * nprob + 8);
   key.push_back(nprob);
   key.push_back(nstreams);
   key.push_back(g_leaf_rows);
   key.push_back(g_pipe_tree);
+  key.push_back(g_panel_polls);
+  key.push_back(g_panel_smem_polls);
   key.push_back(g_batched_form);
   key.push_back(g_panel_oz_min_rows);
   for (int64_t i = 0; i < nprob; ++i) {

@@ -32,6 +32,8 @@ int hr_direct(double* A, int64_t lda, int64_t m, int b, double* T, int64_t ldT, 
 // tsqr4.cu: direct TSQR-HR with a fan-in-4 tree and compact-WY Q blocks.
 extern int64_t g_leaf_rows;
 extern int g_pipe_tree;
+// limits of the panel kernels' bounded waits (knobs "panel_polls", "panel_smem_polls")
+extern int g_panel_polls, g_panel_smem_polls;
 // leaf height of the panels factored by the lookahead (tuning knob
 // "pipe_leaf_rows"), and the per-host-thread override it sets (0: none)
 extern int64_t g_pipe_leaf_rows;

@@ -148,8 +148,10 @@ __device__ __forceinline__ void named_bar(int id, int n) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 
-// Polls of a shared-memory flag before a wait gives up.
-constexpr long kSmemSpin = 1L << 22;
+// Polls before a bounded wait gives up (tuning knobs "panel_polls": on another CTA
+// of the panel; "panel_smem_polls": on another warp of the CTA).  About 100 ns each.
+int g_panel_polls = 1 << 22;
+int g_panel_smem_polls = 1 << 22;
 constexpr int kStepThreads = 7 * 32;   // the critical warp and the six column warps of a node
 constexpr int kLeafStepThreads = 8 * 32;   // those of a leaf, with the seventh
 constexpr int kStepBar = 3;            // their barrier, one per column step
@@ -354,7 +356,7 @@ __device__ __forceinline__ void h7_apply(double* S, int ld, int q, int k0, const
 }
 
 struct NoPublish {
-  __device__ void all(const double*, int, int, volatile int*, volatile int*) const {}
+  __device__ void all(const double*, int, int, volatile int*, volatile int*) {}
 };
 
 // Householder QR of S (b columns, ld >= 32 R, rows beyond the data zero); all
@@ -644,6 +646,7 @@ struct Hr4Args {
   unsigned* done;   // pipelined tree: node finished (T, Q blocks, V written); the root's U^-1 last
   unsigned* ticket; // pipelined tree: role counter
   int* fail;        // pipelined tree: a wait gave up
+  int polls, smem_polls;   // limits of the bounded waits
   double* Pc;       // pipelined tree: I - V0 T0 V0^T of leaf 0, then per level the product of the first
                     // Q blocks up leaf 0's path, (depth + 1) x b x b
   double* Mn;       // many leaves: per node, the product of the Q blocks from the root down to it
@@ -673,6 +676,13 @@ __device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// A wait ran out: the call's status, and in the pipelined tree the flag that ends the
+// other CTAs' waits.
+__device__ __forceinline__ void h6_give_up(int* fail, int* status) {
+  if (fail) atomicExch(fail, 1);
+  atomicExch(status, CANDMC_ERR_TIMEOUT);
+}
+
 constexpr int kBlk = kDirectB * kLd;        // doubles of a 32 x 32 shared block
 constexpr int kRootDoubles = 6 * kBlk;
 
@@ -697,7 +707,7 @@ __device__ void h4_root(const Hr4Args& a, double* sm) {
   double* sQ = sM + kBlk;
   __shared__ int s_sign[kDirectB];
   __shared__ double s_rp[kDirectB], s_part[3][kDirectB];
-  __shared__ volatile int s_cols;   // columns of L\U finished
+  __shared__ volatile int s_cols, s_late;   // columns of L\U finished; a wait for one gave up
   for (int idx = tid; idx < kBlk; idx += blockDim.x) sQ[idx] = sL[idx] = 0.0;
   __syncthreads();
   if (a.Pc) {
@@ -736,14 +746,17 @@ __device__ void h4_root(const Hr4Args& a, double* sm) {
     __syncthreads();
   }
   for (int idx = tid; idx < kBlk; idx += blockDim.x) sT[idx] = sX[idx] = 0.0;
-  if (tid == 0) s_cols = 0;
+  if (tid == 0) s_cols = s_late = 0;
   __syncthreads();
   // columns before c finished (one warp)
   auto wait_cols = [&](int c) {
-    long it = 0;
-    while (s_cols < c && ++it < kSmemSpin) __nanosleep(20);
+    int it = 0;
+    while (s_cols < c && ++it < a.smem_polls) __nanosleep(it < 1024 ? 20 : 100);
     __syncwarp();
-    if (it >= kSmemSpin && lane == 0) atomicExch(a.status, CANDMC_ERR_TIMEOUT);
+    if (lane == 0 && it >= a.smem_polls) {
+      h6_give_up(a.fail, a.status);
+      s_late = 1;
+    }
     __threadfence_block();
   };
   // acc minus the sum over k < c, k = h (mod 4), of X[:, k] v[k]: X's columns
@@ -836,7 +849,7 @@ __device__ void h4_root(const Hr4Args& a, double* sm) {
       if (bad) atomicExch(a.status, CANDMC_ERR_NUMERIC);
       __threadfence();
       __syncwarp();
-      if (lane == 0 && a.Pc) st_release(a.done + a.base[a.depth] + 1, 1u);
+      if (lane == 0 && a.Pc && !s_late) st_release(a.done + a.base[a.depth] + 1, 1u);
     }
 #pragma unroll 1
     for (int c = 0; c < b; ++c) {
@@ -1012,46 +1025,48 @@ __global__ void __launch_bounds__(kLeafThreads, 2) k_hr4_leaf_tree(Hr4Args a) {
 // panel costs about b + depth steps.  Roles come from an atomic ticket
 // (leaves first, then the nodes level by level), so a node only waits for
 // CTAs that took a lower ticket and are already running, whatever the
-// scheduling order.  Every wait is bounded: a wait that runs out records
-// CANDMC_ERR_TIMEOUT, and the CTA releases its own flags and returns, so no
-// other CTA is left waiting on it.
-constexpr long kSpinLimit = 1L << 22;
+// scheduling order.  Every wait is bounded: a wait that runs out, on another CTA
+// or on a warp of its own, records CANDMC_ERR_TIMEOUT and sets the flag that every
+// wait on another CTA polls, and the CTA returns without publishing anything more,
+// so no other CTA is left waiting on it or takes what it did not finish.
 
 // One thread: wait until *p >= v.  False when the wait gave up or another CTA
 // of this launch did.
 __device__ bool h6_wait(const Hr4Args& a, const unsigned* p, unsigned v) {
-  for (long it = 0; it < kSpinLimit; ++it) {
+  for (int it = 0; it < a.polls; ++it) {
     if (ld_acquire(p) >= v) return true;
     if (*(volatile int*)a.fail) return false;
     if (it > 8) __nanosleep(100);
   }
-  atomicExch(a.fail, 1);
-  atomicExch(a.status, CANDMC_ERR_TIMEOUT);
+  h6_give_up(a.fail, a.status);
   return false;
-}
-
-__device__ void h6_release_all(const Hr4Args& a, int f) {
-  if (threadIdx.x == 0) {
-    __threadfence();
-    st_release(a.prog + f, (unsigned)a.b);
-    st_release(a.done + f, 1u);
-  }
 }
 
 // R handed to the parent column by column (rows 0..j of S's column j) as the
 // count *s_done of finished columns grows, by one warp.  Stops when *s_fail
-// (may be nullptr) is set.
+// (may be nullptr) is set; where its own wait runs out it sets *s_short (apart
+// from s_fail, which the column warps read between their barriers).
 struct Publish {
   double* Rcol;
   int b;
   unsigned* prog;
-  __device__ void all(const double* S, int ld, int n, volatile int* s_done, volatile int* s_fail) const {
+  volatile int* s_short;
+  int polls;
+  int *fail, *status;
+  __device__ void all(const double* S, int ld, int n, volatile int* s_done, volatile int* s_fail) {
     const int lane = threadIdx.x & 31;
     for (int j = 0; j < n; ++j) {
-      long it = 0;
-      while (*s_done <= j && ++it < kSmemSpin && !(s_fail && *s_fail)) __nanosleep(20);
-      __syncwarp();
-      if (*s_done <= j) return;   // the CTA releases its flags itself
+      for (int it = 0; *s_done <= j && !(s_fail && *s_fail);) {
+        if (++it >= polls) break;
+        __nanosleep(it < 1024 ? 20 : 100);
+      }
+      if (__any_sync(0xffffffffu, *s_done <= j)) {
+        if (lane == 0 && !(s_fail && *s_fail)) {
+          h6_give_up(fail, status);
+          *s_short = 1;
+        }
+        return;
+      }
       __threadfence_block();
       if (lane <= j) Rcol[j * b + lane] = S[j * ld + lane];
       __syncwarp();   // orders the lanes' stores before lane 0's release
@@ -1061,6 +1076,7 @@ struct Publish {
 };
 
 __device__ void h6_leaf(const Hr4Args& a, int leaf, double* sm, double* s_h, double* s_gam) {
+  __shared__ volatile int s_short;
   const int b = a.b, tid = threadIdx.x;
   const int64_t r0 = t4_leaf_row0(a.m, a.P, leaf);
   const int L = (int)(t4_leaf_row0(a.m, a.P, leaf + 1) - r0);
@@ -1071,8 +1087,11 @@ __device__ void h6_leaf(const Hr4Args& a, int leaf, double* sm, double* s_h, dou
   double* scratch = G + kBlk;
   double* Tt = scratch + 512;
   const int slots = h7_slots(L);
+  if (tid == 0) s_short = 0;   // read after the barriers of the factorization
   h4_load_block(S, ldS, a.A + r0, a.lda, L, b, 32 * slots);
-  h7_leaf_factor(S, ldS, slots, b, s_h, s_gam, Publish{a.Rn + (size_t)leaf * b * b, b, a.prog + leaf});
+  h7_leaf_factor(S, ldS, slots, b, s_h, s_gam,
+                 Publish{a.Rn + (size_t)leaf * b * b, b, a.prog + leaf, &s_short, a.smem_polls, a.fail, a.status});
+  if (s_short) return;
   h7_leaf_v(S, ldS, L, 32 * slots, b, s_h, VT, a.Vw + r0, a.m);
   h7_gram(VT, S, ldS, 32 * slots, b, G, scratch);
   h4_tri_inv(G, Tt, scratch);
@@ -1156,7 +1175,8 @@ __device__ __forceinline__ double tri_fold(int n, X x, Y y) {
 __device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_h, double* s_gam) {
   const int b = a.b, tid = threadIdx.x, lane = tid & 31, warp = warp_id();
   __shared__ int s_okv[2];
-  __shared__ volatile int s_done, s_got, s_fail;   // columns finished, fetched; the poller gave up
+  __shared__ volatile int s_done, s_got, s_fail;   // columns finished, fetched; a wait for a column gave up
+  __shared__ volatile int s_short;                 // the publishing warp's gave up
   int lvl = 1;
   while (lvl < a.depth && f >= a.base[lvl + 1]) ++lvl;
   const int idx = f - a.base[lvl];
@@ -1190,16 +1210,13 @@ __device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_h, double
       if (lane == 0) s_okv[0] = ok;
     }
     __syncthreads();
-    if (!s_okv[0]) {
-      h6_release_all(a, f);
-      return;
-    }
+    if (!s_okv[0]) return;
   } else {
     for (int i = tid; i < ld * kDirectB; i += blockDim.x) S[i] = 0.0;
     for (int i = tid; i < kBlk; i += blockDim.x) Tn[i] = 0.0;
-    if (tid == 0) s_done = s_got = s_fail = 0;
+    if (tid == 0) s_done = s_got = s_fail = s_short = 0;
     __syncthreads();
-    const Publish pub{Rme, b, a.prog + f};
+    Publish pub{Rme, b, a.prog + f, &s_short, a.smem_polls, a.fail, a.status};
     // column c of the children's R into S (polling warp: lane k waits for child k)
     auto fetch = [&](int c) -> bool {
       bool ok = true;
@@ -1306,12 +1323,14 @@ __device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_h, double
       for (int t = 0; t < kFan; ++t) cr.v[t] = 0.0;
       for (int j = 0; j < b; ++j) {
         if (warp == 0) {
-          // columns up to j + 1 must have arrived
+          // columns up to j + 1 must have arrived (the polling warp's own wait is as
+          // long, and sets s_fail)
           const int need = j + 2 < b ? j + 2 : b;
-          long it = 0;
-          while (s_got < need && !s_fail && ++it < kSmemSpin) {
-          }
+          int it = 0, polls = a.smem_polls;
+          while (s_got < need && !s_fail && ++it < polls)
+            if (it >= 4096) __nanosleep(100);
           __syncwarp();
+          if (lane == 0 && it >= polls) h6_give_up(a.fail, a.status);
           if (lane == 0) s_okv[j & 1] = s_got >= need;
           __threadfence_block();
         }
@@ -1346,10 +1365,7 @@ __device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_h, double
       pub.all(S, ld, b, &s_done, &s_fail);
     }
     __syncthreads();
-    if (s_fail) {
-      h6_release_all(a, f);
-      return;
-    }
+    if (s_fail || s_short) return;
     // T of normalised heads: Tn = T D (for Q_k = -V_k T D), Qk = D T D (Q_1 = I - D T D)
     for (int i = tid; i < kDirectB * kDirectB; i += blockDim.x) {
       const int r = i & 31, c = i >> 5;
@@ -1371,10 +1387,7 @@ __device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_h, double
     if (mul) {
       if (tid == 0) s_okv[0] = h6_wait(a, a.prog + child0, (unsigned)b + 1u);
       __syncthreads();
-      if (!s_okv[0]) {
-        h6_release_all(a, f);
-        return;
-      }
+      if (!s_okv[0]) return;
     }
     if (mul && nch > 1) {
       h4_load(Pb, Uprev, b);
@@ -1777,6 +1790,8 @@ int hr_direct4(double* A, int64_t lda, int64_t m, int b, double* T, int64_t ldT,
   a.Uinv = reinterpret_cast<double*>(base + o_uinv);
   a.Mn = node_m ? reinterpret_cast<double*>(base + o_mn) : nullptr;
   a.status = d_status;
+  a.polls = g_panel_polls;
+  a.smem_polls = g_panel_smem_polls;
   static std::atomic<bool> attr{false};
   if (!attr) {
     CANDMC_CK(cudaFuncSetAttribute(k_hr4_leaf_tree, cudaFuncAttributeMaxDynamicSharedMemorySize,

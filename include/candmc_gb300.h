@@ -322,7 +322,10 @@ int candmc_batched_status(void* stream, int* status);
  * [I A; A^T 0] refining x and r); "batched_form" (CANDMC_PREC_OZAKI, the
  * default: candmc_batched_ls's panels apply each half-panel's Q^T to the
  * other half on the tensor cores from "panel_oz_min_rows" rows on, in
- * emulated FP64 on FP64 storage; CANDMC_PREC_FP64: on the FP64 pipe) */
+ * emulated FP64 on FP64 storage; CANDMC_PREC_FP64: on the FP64 pipe); "panel_polls", "panel_smem_polls" (polls
+ * after which a wait of the panel kernels on another thread block, or on another
+ * warp of its own, gives up with CANDMC_ERR_TIMEOUT; 1..2^30, default 2^22, about
+ * half a second) */
 int candmc_set_tuning(const char* key, int64_t value);
 
 /* ---- least-squares request server (no counterpart in the reference) ---------

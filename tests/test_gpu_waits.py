@@ -1,0 +1,57 @@
+"""The bounded waits of the kernels: one that runs out makes the call return
+CANDMC_ERR_TIMEOUT (the limits are lowered from the host; nothing is left
+waiting), and the next call with the usual limits is right again.
+"""
+import numpy as np
+import pytest
+
+from oracle import candmc_oracle as co
+from oracle import fixtures as fx
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+POLLS = 1 << 22
+TIMEOUT = 4
+
+
+@pytest.fixture(scope="module")
+def cm():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import candmc_gb300 as cm
+    cm.lib()
+    return cm
+
+
+def status_of(cm, f):
+    try:
+        f()
+    except cm.CandmcError as e:
+        return e.status
+    return 0
+
+
+# one leaf (only its publishing warp and the root's solver wait), a node of three
+# leaves, two levels of nodes with a pass-through one
+@pytest.mark.parametrize("knob", ["panel_smem_polls", "panel_polls"])
+@pytest.mark.parametrize("m,b", [(60, 20), (180, 32), (1100, 32)])
+def test_panel_waits(cm, knob, m, b):
+    A = fx.gaussian(m, b, m + b)
+    try:
+        cm.set_tuning(knob, 1)
+        assert status_of(cm, lambda: cm.hh_recon_qr(np.asfortranarray(A.copy()))) == TIMEOUT
+    finally:
+        cm.set_tuning(knob, POLLS)
+    YR = np.asfortranarray(A.copy())
+    W, T = cm.hh_recon_qr(YR)
+    YRo, Wo = co.hh_recon_qr(A, b)
+    tol = 2e-12 * max(1.0, b / 16)
+    assert np.abs(YR - YRo).max() <= tol * max(1.0, np.abs(YRo).max())
+    assert np.abs(W - Wo).max() <= tol
+
+
+def test_wait_limits_are_checked(cm):
+    for knob in ("panel_smem_polls", "panel_polls"):
+        with pytest.raises(cm.CandmcError):
+            cm.set_tuning(knob, 0)
