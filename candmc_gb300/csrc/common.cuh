@@ -51,6 +51,10 @@ __device__ __forceinline__ double mat_at(const MatRef& X, int64_t i, int64_t j) 
   }
 }
 
+// Records a failure in a call's status word; the first one stays (what follows from
+// it, such as non-finite values behind a wait that ran out, does not replace it).
+__device__ __forceinline__ void record_status(int* status, int code) { atomicCAS(status, CANDMC_OK, code); }
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -913,7 +913,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
     }
   }
   __syncthreads();
-  if (s_fail && tid == 0) atomicExch(a.status, CANDMC_ERR_TIMEOUT);
+  if (s_fail && tid == 0) record_status(a.status, CANDMC_ERR_TIMEOUT);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (warp == 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
@@ -1277,7 +1277,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_tn(OzArgs a) {
     asm volatile("cp.async.wait_all;" ::: "memory");
   }
   __syncthreads();
-  if (s_fail && tid == 0) atomicExch(a.status, CANDMC_ERR_TIMEOUT);
+  if (s_fail && tid == 0) record_status(a.status, CANDMC_ERR_TIMEOUT);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (warp == 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));

@@ -231,7 +231,7 @@ __device__ void hr_root_finalize(const HrArgs& a, double* smem) {
     if (!isfinite(v)) bad = 1;
     a.Uinv[idx] = v;
   }
-  if (bad) atomicExch(a.status, CANDMC_ERR_NUMERIC);
+  if (bad) record_status(a.status, CANDMC_ERR_NUMERIC);
 }
 
 __global__ void __launch_bounds__(kThreads) hr_leaf_tree(HrArgs a) {

@@ -45,7 +45,7 @@ k_signed_nlu(double* A, double* R, int b, int64_t lda, int64_t ldr, int64_t* sig
   if (use_smem) {
     for (int idx = tid; idx < b * b; idx += blockDim.x) A[(idx / b) * lda + idx % b] = sh[idx];
   }
-  if (bad) atomicExch(status, CANDMC_ERR_NUMERIC);
+  if (bad) record_status(status, CANDMC_ERR_NUMERIC);
 }
 
 int signed_nlu(double* A, double* R, int64_t b, int64_t lda, int64_t ldr, int64_t* signs,

@@ -680,7 +680,7 @@ __device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
 // other CTAs' waits.
 __device__ __forceinline__ void h6_give_up(int* fail, int* status) {
   if (fail) atomicExch(fail, 1);
-  atomicExch(status, CANDMC_ERR_TIMEOUT);
+  record_status(status, CANDMC_ERR_TIMEOUT);
 }
 
 constexpr int kBlk = kDirectB * kLd;        // doubles of a 32 x 32 shared block
@@ -846,7 +846,7 @@ __device__ void h4_root(const Hr4Args& a, double* sm) {
       named_bar(2, 128);
     }
     if (!h) {
-      if (bad) atomicExch(a.status, CANDMC_ERR_NUMERIC);
+      if (bad) record_status(a.status, CANDMC_ERR_NUMERIC);
       __threadfence();
       __syncwarp();
       if (lane == 0 && a.Pc && !s_late) st_release(a.done + a.base[a.depth] + 1, 1u);

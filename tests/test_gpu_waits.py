@@ -12,7 +12,7 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 POLLS = 1 << 22
-TIMEOUT = 4
+TIMEOUT, NUMERIC = 4, 5
 
 
 @pytest.fixture(scope="module")
@@ -49,6 +49,31 @@ def test_panel_waits(cm, knob, m, b):
     tol = 2e-12 * max(1.0, b / 16)
     assert np.abs(YR - YRo).max() <= tol * max(1.0, np.abs(YRo).max())
     assert np.abs(W - Wo).max() <= tol
+
+
+@pytest.mark.parametrize("first", ["nan", "wait"])
+def test_first_failure_is_reported(cm, first):
+    """Of two batched calls that fail, one for a NaN and one for a wait, the status
+    word has the first one's failure."""
+    def call(what):
+        A = fx.gaussian(200, 16, 3)
+        if what == "nan":
+            A[100, 3] = np.nan
+        else:
+            cm.set_tuning("panel_smem_polls", 1)
+        dA = torch.from_numpy(A).cuda().t().contiguous().t()
+        db = torch.ones((200, 1), dtype=torch.float64, device="cuda")
+        try:
+            cm.batched_ls([dA], [db])
+            torch.cuda.synchronize()
+        finally:
+            cm.set_tuning("panel_smem_polls", POLLS)
+
+    assert status_of(cm, cm.batched_status) == 0
+    call(first)
+    call("wait" if first == "nan" else "nan")
+    assert status_of(cm, cm.batched_status) == (NUMERIC if first == "nan" else TIMEOUT)
+    assert status_of(cm, cm.batched_status) == 0
 
 
 def test_wait_limits_are_checked(cm):
