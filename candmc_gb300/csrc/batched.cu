@@ -205,6 +205,11 @@ extern "C" int candmc_set_tuning(const char* key, int64_t value) {
     (std::string(key) == "panel_polls" ? g_panel_polls : g_panel_smem_polls) = (int)value;
     return CANDMC_OK;
   }
+  if (std::string(key) == "oz_polls") {
+    if (value < 0 || value > (1 << 30)) return set_error(CANDMC_ERR_ARG, "oz_polls in [0, 2^30]");
+    g_oz_polls = (int)value;
+    return CANDMC_OK;
+  }
   return set_error(CANDMC_ERR_ARG, "unknown tuning key");
 }
 
@@ -226,13 +231,14 @@ extern "C" int candmc_batched_ls(int64_t nprob, const int64_t* m, const int64_t*
   }
   if (!use_graph) return batched_issue(nprob, m, n, A, lda, B, nstreams, s);
   std::vector<int64_t> key;
-  key.reserve(5 * nprob + 8);
+  key.reserve(5 * nprob + 9);
   key.push_back(nprob);
   key.push_back(nstreams);
   key.push_back(g_leaf_rows);
   key.push_back(g_pipe_tree);
   key.push_back(g_panel_polls);
   key.push_back(g_panel_smem_polls);
+  key.push_back(g_oz_polls);
   key.push_back(g_batched_form);
   key.push_back(g_panel_oz_min_rows);
   for (int64_t i = 0; i < nprob; ++i) {

@@ -41,6 +41,8 @@ extern thread_local int64_t t_leaf_rows;
 // SMs left free of persistent Ozaki CTAs while a lookahead factorization runs,
 // so the panel stream is not starved (tuning knob "oz_reserve_sms")
 extern int g_oz_reserve_sms;
+// polls of the Ozaki kernels' waits between their warps (tuning knob "oz_polls")
+extern int g_oz_polls;
 // per host thread: > 0 caps the persistent Ozaki grid (set for the duration
 // of a lookahead factorization)
 extern thread_local int t_oz_cap;

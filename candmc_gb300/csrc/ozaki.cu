@@ -61,6 +61,7 @@ struct OzCfg {
   static constexpr int SMEM = OZ_STAGES * STAGE_BYTES + 1024;
 };
 constexpr int OZ_WAIT_LIMIT = 1 << 22;                // bounded mbarrier polls
+int g_oz_polls = OZ_WAIT_LIMIT;                       // those of the roles on one another (knob "oz_polls")
 
 // element (r, k) of an R x K operand slice plane in core-matrix K-major order
 __host__ __device__ __forceinline__ int64_t cm_off(int64_t r, int64_t k, int64_t R) {
@@ -368,6 +369,7 @@ struct OzArgs {
   int64_t fp64_rows;         // kOzPairs: rows < fp64_rows are written as FP64 (final)
   int c_assign;              // kOzDoubles: C = product (C is not read)
   int* status;
+  int polls;                 // limit of the roles' waits on one another
   int n_mt, n_nt, n_ks;      // work items: M tiles x N tiles x K splits
 };
 
@@ -504,11 +506,13 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, unsigned
       : "memory");
 }
 
-// bounded wait; gives up early when another role of the CTA failed
-__device__ __forceinline__ bool oz_wait(uint64_t* b, uint32_t parity, volatile int* fail) {
+// Bounded wait of a whole warp; gives up early when another role of the CTA failed.
+// Warp collectives (votes, elections, TMEM loads) follow on either outcome, so the
+// lanes vote on it: all of them leave by the same poll with the same result.
+__device__ __forceinline__ bool oz_wait(uint64_t* b, uint32_t parity, volatile int* fail, int polls) {
   const uint32_t addr = smem_u32(b);
 #pragma unroll 1
-  for (int it = 0; it < OZ_WAIT_LIMIT; ++it) {
+  for (int it = 0; it < polls; ++it) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\t"
@@ -516,11 +520,20 @@ __device__ __forceinline__ bool oz_wait(uint64_t* b, uint32_t parity, volatile i
         : "=r"(done)
         : "r"(addr), "r"(parity)
         : "memory");
-    if (done) return true;
-    if ((it & 63) == 63 && *fail) return false;
+    if (__all_sync(0xffffffffu, done)) return true;
+    if ((it & 63) == 63 && __any_sync(0xffffffffu, *fail)) return false;
   }
   *fail = 1;
+  __syncwarp();
   return false;
+}
+
+// The last of the `fills` fills of each of n stages has arrived (a bounded wait of the
+// producer's warp): a CTA that gave up must not end with copies into it in flight.
+__device__ __forceinline__ void oz_copies_done(uint64_t* full, int n, int fills) {
+  volatile int unused = 0;
+  for (int st = 0; st < n && st < fills; ++st)
+    oz_wait(&full[st], (uint32_t)((fills - 1 - st) / n & 1), &unused, OZ_WAIT_LIMIT);
 }
 
 // Where a product of slice A_i stands among the products of A_i in one step:
@@ -750,7 +763,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
     // ---------------- producer: the whole warp walks the stages, one elected lane copies
     const int abytes = (E == kOzSums && a.AR < OZ_M) ? (int)a.AR * 32 : OZ_ABYTES;
     const int64_t aplane = a.AR * a.Kpad, bplane = a.BR * a.Kpad;
-    int st = 0;
+    int st = 0, fills = 0;
     uint32_t parity = 1;
     bool ok = true;
     for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
@@ -758,8 +771,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
       const __nv_bfloat16* as = a.As + (int64_t)it.kbeg * a.AR + it.m0 * 16;
       const __nv_bfloat16* bs = a.Bs + (int64_t)it.kbeg * a.BR + it.n0 * 16;
       for (int k = it.kbeg; k < it.kend; k += 16) {
-        ok = oz_wait(&empty_b[st], parity, &s_fail);
+        ok = oz_wait(&empty_b[st], parity, &s_fail, a.polls);
         if (!ok) break;
+        ++fills;
         if (elect_one()) {
           mbar_expect_tx(&full_b[st], (unsigned)(S * (abytes + OZ_BBYTES)));
           const uint32_t sa = smem_u32(ring + (size_t)st * STAGE_BYTES), sb = sa + S * OZ_ABYTES;
@@ -778,6 +792,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
         }
       }
     }
+    oz_copies_done(full_b, OZ_STAGES, fills);
   } else if (warp == 1) {
     // ---------------- MMA issuer: the whole warp walks the stages, one elected lane issues
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_N >> 3) << 17) |
@@ -795,10 +810,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
       for (int left = (it.kend - it.kbeg) >> 4; left > 0 && ok; left -= steps_per_group) {
         const int steps = min(left, steps_per_group);
         // the epilogue has read the previous group's accumulators
-        ok = oz_wait(&acc_empty, acc_parity, &s_fail);
+        ok = oz_wait(&acc_empty, acc_parity, &s_fail, a.polls);
         acc_parity ^= 1;
         for (int t = 0; t < steps && ok; ++t) {
-          ok = oz_wait(&full_b[st], parity, &s_fail);
+          ok = oz_wait(&full_b[st], parity, &s_fail, a.polls);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint64_t da = ring_desc + (uint64_t)(st * (STAGE_BYTES >> 4));
@@ -815,15 +830,16 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
     // every MMA this warp issued has completed before TMEM is released
     umma_commit(&fin);
     volatile int dummy = 0;
-    oz_wait(&fin, 0u, &dummy);
+    oz_wait(&fin, 0u, &dummy, OZ_WAIT_LIMIT);
   } else {
     // ---------------- epilogue: warps 2 .. 2 + OZ_EPI_WARPS - 1
     const int q = warp & 3;                // TMEM lane quarter this warp may access
     const int part = (warp - 2) >> 2;      // column part
     const int row = q * 32 + lane;
     int64_t ngroups = 0;
+    bool ok = true;
     df2 acc[OZ_EPI_COLS / 2];   // this group's product, or the sums over the item's groups
-    for (int w = blockIdx.x; w < nitems && !s_fail; w += gridDim.x) {
+    for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
       const OzItem it = oz_item(a, w);
       const int nsteps = (it.kend - it.kbeg) >> 4;
       const int64_t gm = it.m0 + row, gn0 = it.n0 + part * OZ_EPI_COLS;
@@ -851,7 +867,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
         int* ebs = s_eb[warp - 2];
         ebs[lane] = eb << 23;
         __syncwarp();
-        if (!oz_wait(&acc_full, (uint32_t)(ngroups & 1), &s_fail)) break;
+        ok = oz_wait(&acc_full, (uint32_t)(ngroups & 1), &s_fail, a.polls);
+        if (!ok) break;
         ++ngroups;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         oz_drain<G, E == kOzSums>(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(part * OZ_EPI_COLS), ebs, eb, eA, acc);
@@ -909,7 +926,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_mma(OzArgs a) {
           }
         }
       }
-      if (E == kOzSums && !s_fail) oz_store_sums(a, it, row, part, acc);
+      if (E == kOzSums && ok) oz_store_sums(a, it, row, part, acc);
     }
   }
   __syncthreads();
@@ -1024,15 +1041,16 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_tn(OzArgs a) {
     // ---------------- producer of A: the whole warp walks the stages, one elected lane copies
     const int abytes = (a.AR < OZ_M) ? (int)a.AR * 32 : OZ_ABYTES;
     const int64_t aplane = a.AR * a.Kpad;
-    int st = 0;
+    int st = 0, fills = 0;
     uint32_t parity = 1;
     bool ok = true;
     for (int w = blockIdx.x; w < nitems && ok; w += gridDim.x) {
       const OzItem it = oz_item(a, w);
       const __nv_bfloat16* as = a.As + (int64_t)it.kbeg * a.AR;
       for (int k = it.kbeg; k < it.kend; k += 16, as += a.AR * 16) {
-        ok = oz_wait(&a_empty[st], parity, &s_fail);
+        ok = oz_wait(&a_empty[st], parity, &s_fail, a.polls);
         if (!ok) break;
+        ++fills;
         if (elect_one()) {
           mbar_expect_tx(&a_full[st], (unsigned)(S * abytes));
           const uint32_t sa = smem_u32(ring + st * Cfg::A);
@@ -1046,6 +1064,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_tn(OzArgs a) {
         }
       }
     }
+    oz_copies_done(a_full, TN_ASTAGES, fills);
   } else if (warp == 1) {
     // ---------------- MMA issuer: the whole warp walks the stages, one elected lane issues
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_N >> 3) << 17) |
@@ -1061,10 +1080,10 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_tn(OzArgs a) {
       const OzItem it = oz_item(a, w);
       for (int k = it.kbeg; k < it.kend && ok; k += 128) {
         // the previous group's accumulators have been read
-        ok = oz_wait(&acc_empty, acc_parity, &s_fail);
+        ok = oz_wait(&acc_empty, acc_parity, &s_fail, a.polls);
         acc_parity ^= 1;
         for (int t = 0; t < 8 && ok; ++t) {
-          ok = oz_wait(&a_full[sa], a_parity, &s_fail) && oz_wait(&b_full[sb], b_parity, &s_fail);
+          ok = oz_wait(&a_full[sa], a_parity, &s_fail, a.polls) && oz_wait(&b_full[sb], b_parity, &s_fail, a.polls);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           oz_issue_step<S, G>(tmem, a_desc + (uint64_t)(sa * (Cfg::A >> 4)), b_desc + (uint64_t)(sb * (Cfg::B >> 4)),
@@ -1086,7 +1105,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_tn(OzArgs a) {
     // every MMA this warp issued has completed before TMEM is released
     umma_commit(&fin);
     volatile int dummy = 0;
-    oz_wait(&fin, 0u, &dummy);
+    oz_wait(&fin, 0u, &dummy, OZ_WAIT_LIMIT);
   } else {
     // ---------------- slicing of C and sums: warps 2 .. 2 + OZ_EPI_WARPS - 1
     const int cw = warp - 2;
@@ -1154,7 +1173,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_tn(OzArgs a) {
       const int c = part * OZ_EPI_COLS + lane;
       const int eb = tn_exp(s_mx[par][0][c], s_mx[par][1][c]);
       s_eb[cw][lane] = eb << 23;
-      if (!oz_wait(&acc_full, par, &s_fail)) return false;
+      if (!oz_wait(&acc_full, par, &s_fail, a.polls)) return false;
       ++drained;
       __syncwarp();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -1208,7 +1227,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_tn(OzArgs a) {
         }
       }
       load_from(nit.n0, nk);
-      ok = oz_wait(&exp_full, group & 1, &s_fail);
+      ok = oz_wait(&exp_full, group & 1, &s_fail, a.polls);
       if (!ok) break;
 #pragma unroll
       for (int h = 0; h < 2; ++h)
@@ -1250,7 +1269,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_tn(OzArgs a) {
               __syncwarp();
               scan_block(u - 1);
             }
-            ok = oz_wait(&b_empty[team], b_parity, &s_fail);
+            ok = oz_wait(&b_empty[team], b_parity, &s_fail, a.polls);
             if (!ok) break;
           }
 #pragma unroll
@@ -1439,6 +1458,7 @@ template <int S, OzEpilogue E>
 static int launch_oz_mma(OzArgs a, int64_t gm, int64_t gn, int64_t gk, int cls, double flops, cudaStream_t s) {
   static std::atomic<bool> attr{false};
   CANDMC_RET(allow_smem(k_oz_mma<S, E>, OzCfg<S>::SMEM, attr));
+  a.polls = g_oz_polls;
   a.n_mt = (int)gm;
   a.n_nt = (int)gn;
   a.n_ks = (int)gk;
@@ -1452,6 +1472,7 @@ template <int S>
 static int launch_oz_tn(OzArgs a, int64_t gn, int64_t gk, int cls, double flops, cudaStream_t s) {
   static std::atomic<bool> attr{false};
   CANDMC_RET(allow_smem(k_oz_tn<S>, TnCfg<S>::SMEM, attr));
+  a.polls = g_oz_polls;
   a.n_mt = 1;
   a.n_nt = (int)gn;
   a.n_ks = (int)gk;

@@ -325,7 +325,8 @@ int candmc_batched_status(void* stream, int* status);
  * emulated FP64 on FP64 storage; CANDMC_PREC_FP64: on the FP64 pipe); "panel_polls", "panel_smem_polls" (polls
  * after which a wait of the panel kernels on another thread block, or on another
  * warp of its own, gives up with CANDMC_ERR_TIMEOUT; 1..2^30, default 2^22, about
- * half a second) */
+ * half a second); "oz_polls" (the same for the waits between the warps of the
+ * tensor-core contractions; 0..2^30, default 2^22) */
 int candmc_set_tuning(const char* key, int64_t value);
 
 /* ---- least-squares request server (no counterpart in the reference) ---------

@@ -76,7 +76,36 @@ def test_first_failure_is_reported(cm, first):
     assert status_of(cm, cm.batched_status) == 0
 
 
+# the contractions: float pairs (Y^T C sliced on the way, C -= Y Z) and a panel's own
+# FP64 columns, in the seven- and three-slice forms.  With few polls a wait may or may
+# not run out, at any place: the call reports it, or its result is the usual one.
+@pytest.mark.parametrize("precision", ["ozaki", "fp32"])
+@pytest.mark.parametrize("m,n,b,min_rows", [(300, 200, 32, 8192), (1500, 1300, 64, 1024)])
+def test_contraction_waits(cm, precision, m, n, b, min_rows):
+    A = np.asfortranarray(fx.gaussian(m, n, m))
+
+    def run():
+        d = A.copy(order="F")
+        return status_of(cm, lambda: cm.QR_2D(d, b, precision=precision)), d
+
+    try:
+        cm.set_tuning("panel_oz_min_rows", min_rows)
+        st, want = run()
+        assert st == 0
+        for polls in (0, 1, 2, 4, 16):
+            cm.set_tuning("oz_polls", polls)
+            st, got = run()
+            assert st == TIMEOUT if polls == 0 else st in (0, TIMEOUT), polls
+            assert st == TIMEOUT or np.array_equal(got, want), polls
+        cm.set_tuning("oz_polls", POLLS)
+        st, got = run()
+        assert st == 0 and np.array_equal(got, want)
+    finally:
+        cm.set_tuning("oz_polls", POLLS)
+        cm.set_tuning("panel_oz_min_rows", 8192)
+
+
 def test_wait_limits_are_checked(cm):
-    for knob in ("panel_smem_polls", "panel_polls"):
+    for knob, bad in (("panel_smem_polls", 0), ("panel_polls", 0), ("oz_polls", -1)):
         with pytest.raises(cm.CandmcError):
-            cm.set_tuning(knob, 0)
+            cm.set_tuning(knob, bad)
