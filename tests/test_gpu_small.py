@@ -119,3 +119,55 @@ def test_fp64_products(cm, m, nb, n, masked):
 @pytest.mark.parametrize("m,nb,n", [(1111, 65, 4900), (900, 128, 2500), (256, 70, 9800), (2050, 33, 3300)])
 def test_fp64_products_wide(cm, m, nb, n):
     test_fp64_products(cm, m, nb, n, False)
+
+
+def invert_upper(W):
+    """Column by column back substitution: element (i, c) from rows and columns i..c."""
+    n = len(W)
+    X = np.zeros((n, n))
+    for c in range(n):
+        x = np.zeros(c + 1)
+        x[c] = 1.0
+        for k in range(c, -1, -1):
+            x[k] /= W[k, k]
+            x[:k] -= W[:k, k] * x[k]
+        X[:c + 1, c] = x
+    return X
+
+
+# What stays finite: the rows of -W^-T Y1 whose columns of the inverse do not reach the
+# odd entry.  Where all stay finite, the substitution's bound |W^-1| |W| |W^-1| n 2^-53.
+@pytest.mark.parametrize("kind", ["zero pivot", "nan", "inf", "small pivot", "large pivot", "tiny pivot",
+                                  "small entry", "quotient"])
+@pytest.mark.parametrize("n", [2, 5, 32, 33, 64, 100, 300])
+def test_triangular_inverse_extremes(cm, n, kind):
+    W, Y1 = triangle(n, False, n), triangle(n, True, n + 1)
+    q = n // 2
+    if kind == "zero pivot":
+        W[q, q] = 0.0
+    elif kind == "nan":
+        W[0, q] = np.nan
+    elif kind == "inf":
+        W[0, q] = np.inf
+    elif kind == "small pivot":
+        W[q, q] = 2.0 ** -600
+    elif kind == "large pivot":
+        W[q, q] = 2.0 ** 1000
+    elif kind == "tiny pivot":   # its reciprocal overflows
+        W[q, q] = 2.0 ** -1060
+    elif kind == "small entry":   # W[0, q] / W[q, q] underflows
+        W[0, q], W[q, q] = 2.0 ** -700, 2.0 ** 400
+    else:   # W[0, q] / W[q, q] overflows
+        W[0, q], W[q, q] = 2.0 ** 700, 2.0 ** -400
+    got = cm.compute_invT_from_W(dev(W), dev(Y1)).cpu().numpy()
+    with np.errstate(all="ignore"):
+        Wi = invert_upper(W)
+        up = np.triu(np.ones((n, n), dtype=bool))
+        cols = np.isfinite(np.where(up, Wi, 0.0)).all(axis=0)
+        assert np.isfinite(got[cols]).all() and not np.isfinite(got[~cols]).all(axis=1).any()
+        if kind not in ("small pivot", "large pivot", "small entry"):
+            assert not cols.all() and cols[:q].all()
+        V = Wi[:, cols]
+        fin = lambda a: np.abs(np.where(np.isfinite(a), a, 0.0))
+        bound = 4 * n * 2.0 ** -53 * (fin(Wi) @ (fin(W) @ np.abs(V))).T @ np.abs(Y1)
+        assert (np.abs(got[cols] + V.T @ Y1) <= bound).all()
