@@ -453,11 +453,15 @@ k_merge_t(const double* G, double* T, int64_t ldT, int b1, int b2, int nbp) {
   const int NG = kThreads / nbp;
   const int i = threadIdx.x % nbp, g = threadIdx.x / nbp, j = blockIdx.x;
   const double* t22 = T + (int64_t)(b1 + j) * ldT + b1;
-  for (int k = threadIdx.x; k <= j; k += kThreads) col[k] = t22[k];
-  __syncthreads();
   double v = 0.0;
-  if (i < b1)
-    for (int k = g; k <= j; k += NG) v = fma(G[(int64_t)k * b1 + i], col[k], v);
+  for (int k0 = 0; k0 <= j; k0 += kThreads) {   // b2 may exceed kThreads (an odd width's wider half)
+    const int kn = j + 1 - k0 < kThreads ? j + 1 - k0 : kThreads;
+    if (k0) __syncthreads();
+    if ((int)threadIdx.x < kn) col[threadIdx.x] = t22[k0 + threadIdx.x];
+    __syncthreads();
+    if (i < b1)
+      for (int k = g; k < kn; k += NG) v = fma(G[(int64_t)(k0 + k) * b1 + i], col[k], v);
+  }
   part[g * nbp + i] = v;
   __syncthreads();
   if (g == 0) {
@@ -689,7 +693,7 @@ int small_gemm(int64_t M, int64_t N, int64_t K, double alpha, MatRef A, MatRef B
 }
 
 int merge_t(const double* G, double* T, int64_t ldT, int b1, int b2, cudaStream_t s) {
-  if (b1 > kThreads || b2 > kThreads) return set_error(CANDMC_ERR_ARG, "merge_t needs widths of at most 256");
+  if (b1 > kThreads) return set_error(CANDMC_ERR_ARG, "merge_t needs a first factor of at most 256 columns");
   int nbp = 1;
   while (nbp < b1) nbp <<= 1;
   ProfScope ps(CANDMC_KCLASS_SMALL, 2.0 * b1 * b2 * (b1 + b2), s);

@@ -98,3 +98,21 @@ def test_merged_factors(cm, m, b, oz):
         assert np.abs(T.cpu().numpy() - To).max() <= tol
         assert np.array_equal(np.tril(T.cpu().numpy(), -1), np.zeros((b, b)))
     assert np.abs(d.cpu().numpy() - YRo).max() <= tol * max(1.0, np.abs(YRo).max())
+
+
+def test_widest_panel(cm):
+    """513 columns, the widest panel: halves of 256 and 257; 514 is refused."""
+    m, b = 700, 513
+    A = fx.gaussian(m, b, 11)
+    YRo, Wo = co.hh_recon_qr(A, b)
+    To = co.T_from_W(Wo, lp.unit_lower(YRo, b)[:b])
+    tol = 2e-12 * max(1.0, b / 16)
+    d = torch.from_numpy(A).cuda().t().contiguous().t()
+    W, T = cm.hh_recon_qr(d)
+    torch.cuda.synchronize()
+    assert np.abs(d.cpu().numpy() - YRo).max() <= tol * max(1.0, np.abs(YRo).max())
+    assert np.abs(W.cpu().numpy() - Wo).max() <= tol
+    assert np.abs(T.cpu().numpy() - To).max() <= tol
+    d = torch.zeros((514, m), dtype=torch.float64, device="cuda").t()
+    with pytest.raises(cm.CandmcError):
+        cm.hh_recon_qr(d)
