@@ -759,7 +759,8 @@ int gemm_tn_reduce(MatRef Y, MatRef C, int64_t m, int nb, int64_t n, MatRef Top,
     CANDMC_CK(cudaGetLastError());
     return reduce_apply(part.d(), nsplit, nb, nb, 1, Top, alpha, Z, ldz, s);
   }
-  if (m * nb * n <= kSmallProduct) return small_tn(Y, C, m, nb, n, Top, alpha, Z, ldz, s);
+  // (small_tn's grid takes 65535 tiles of 16 columns; the product below goes in pieces)
+  if (m * nb * n <= kSmallProduct && n <= 16 * (int64_t)65535) return small_tn(Y, C, m, nb, n, Top, alpha, Z, ldz, s);
   // column groups: 4, or 1 (and eight groups of rows) when there are at most
   // two column blocks; row tiles of at most 64 rows, all alike
   const int cg = n > 8 ? 4 : 1;

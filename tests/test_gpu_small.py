@@ -171,3 +171,15 @@ def test_triangular_inverse_extremes(cm, n, kind):
         fin = lambda a: np.abs(np.where(np.isfinite(a), a, 0.0))
         bound = 4 * n * 2.0 ** -53 * (fin(Wi) @ (fin(W) @ np.abs(V))).T @ np.abs(Y1)
         assert (np.abs(got[cols] + V.T @ Y1) <= bound).all()
+
+
+# short products wider than a launch grid of 16-column tiles (65535 of them); each
+# output is a sum of m products on both sides, m 2^-53 sum |x||y| apiece
+@pytest.mark.parametrize("m,b1,n", [(1, 18, 1100000), (4, 4, 1048561), (4, 4, 1048560)])
+def test_short_wide_products(cm, m, b1, n):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    Y1 = torch.randn(b1, m, dtype=torch.float64, device="cuda", generator=g).t()
+    Y2 = torch.randn(n, m, dtype=torch.float64, device="cuda", generator=g).t()
+    got = cm.compute_invT_from_Y2(Y1, Y2)
+    want, size = Y1.t() @ Y2, Y1.t().abs() @ Y2.abs()
+    assert bool(((got - want).abs() <= 2 * m * 2.0 ** -53 * size).all())
