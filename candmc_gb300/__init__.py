@@ -303,7 +303,8 @@ def ls_solve(A, B, b=128, precision="fp64", max_refine=20, tol=1e-15, stream=Non
 
 
 def set_tuning(key, value):
-    """Set a tuning knob of the library ("leaf_rows": target rows per TSQR leaf)."""
+    """Set a tuning knob of the library ("leaf_rows": target rows per TSQR leaf, 0 for
+    the choice by the panel's height)."""
     check(lib().candmc_set_tuning(key.encode(), int(value)), "set_tuning")
 
 

@@ -1,7 +1,8 @@
 """Project-written autotuner for the batched least-squares schedule.
 
 The knobs are the number of streams the batch is dealt onto and the target
-rows per TSQR leaf (candmc_set_tuning("leaf_rows")).  `tune_batched` times
+rows per TSQR leaf (candmc_set_tuning("leaf_rows"); 0, the library's default,
+chooses them by each panel's height).  `tune_batched` times
 every combination on a sample of the problem set with CUDA events and keeps
 the fastest; results are cached in a JSON database keyed by the width mix and
 the (log2-bucketed) row range, at $CANDMC_TUNING_DB or
@@ -11,8 +12,8 @@ import json
 import math
 import os
 
-DEFAULT = {"nstreams": 16, "leaf_rows": 64}
-GRID = {"nstreams": (4, 8, 16, 32), "leaf_rows": (64, 128, 256)}
+DEFAULT = {"nstreams": 16, "leaf_rows": 0}
+GRID = {"nstreams": (4, 8, 16, 32), "leaf_rows": (0, 64, 128, 256)}
 
 
 def db_path():

@@ -165,7 +165,7 @@ extern "C" int candmc_batched_status(void* stream, int* status) {
 extern "C" int candmc_set_tuning(const char* key, int64_t value) {
   if (!key) return set_error(CANDMC_ERR_ARG, "tuning key");
   if (std::string(key) == "leaf_rows") {
-    if (value < 32 || value > 256) return set_error(CANDMC_ERR_ARG, "leaf_rows in [32, 256]");
+    if (value != 0 && (value < 32 || value > 256)) return set_error(CANDMC_ERR_ARG, "leaf_rows 0 or in [32, 256]");
     g_leaf_rows = value;
     return CANDMC_OK;
   }
@@ -175,7 +175,8 @@ extern "C" int candmc_set_tuning(const char* key, int64_t value) {
     return CANDMC_OK;
   }
   if (std::string(key) == "pipe_leaf_rows") {
-    if (value < 32 || value > 256) return set_error(CANDMC_ERR_ARG, "pipe_leaf_rows in [32, 256]");
+    if (value != 0 && (value < 32 || value > 256))
+      return set_error(CANDMC_ERR_ARG, "pipe_leaf_rows 0 or in [32, 256]");
     g_pipe_leaf_rows = value;
     return CANDMC_OK;
   }

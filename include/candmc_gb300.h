@@ -307,14 +307,15 @@ int candmc_batched_ls_f32(int64_t nprob, const int64_t* m, const int64_t* n, flo
  * device-side failures surface here. */
 int candmc_batched_status(void* stream, int* status);
 
-/* tuning knobs: "leaf_rows" (target rows per TSQR leaf, 32..256; unset: 128, 256 for
- * panels of 32768 rows or more, 64 for panels of up to about 4000);
+/* tuning knobs: "leaf_rows" (target rows per TSQR leaf, 32..256; 0, the default: by
+ * the panel's height, 128, 256 for panels of 32768 rows or more, 64 for panels of up
+ * to about 4000);
  * "pipe_tree" (1, the default: the levels of the TSQR tree overlap column by
  * column; 0: level by level); "oz_reserve_sms" (SMs kept free of the
  * persistent emulated-FP64 update kernel during QR_2D_pipe, for the panel
  * stream; default 32); "pipe_leaf_rows" (leaf height of the panels QR_2D_pipe
- * factors, 32..256; unset: as "leaf_rows" unset; panels of 32768 rows or more
- * take at least 256); "panel_oz_min_rows" (in the emulated-FP64
+ * factors, 32..256; 0, the default: by the height, as with "leaf_rows" 0; panels of
+ * 32768 rows or more take at least 256); "panel_oz_min_rows" (in the emulated-FP64
  * and FP32 forms, panels with at least this many rows apply each half's Q^T to
  * the other half of the panel in emulated FP64 on the tensor cores instead of
  * the FP64 pipe; default 8192, 0 disables); "ls_refine" (candmc_ls_solve's refinement: 0, the

@@ -17,3 +17,16 @@ def pytest_configure(config):
 def golden():
     import numpy as np
     return np.load(os.path.join(ROOT, "tests", "golden", "golden.npz"))
+
+
+@pytest.fixture(autouse=True)
+def default_leaf_heights(request):
+    """Every GPU test starts with the leaf heights that users get, whatever an earlier
+    test in the process has set."""
+    if request.node.get_closest_marker("gpu"):
+        import torch
+        if torch.cuda.is_available():
+            import candmc_gb300 as cm
+            cm.set_tuning("leaf_rows", 0)
+            cm.set_tuning("pipe_leaf_rows", 0)
+    yield
