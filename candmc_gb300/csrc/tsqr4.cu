@@ -229,9 +229,10 @@ struct Crit {
 // is refined here, beside the dot product, written to s_gam[j - 1] and
 // announced on barrier kGamBar, where the column warps wait for it after their
 // own dot products: the step barrier need not wait for it.
+// Leaf: the block has `rows` rows, zero beyond them.
 template <int R, bool NODE>
 __device__ __forceinline__ void h7_crit(double* S, int ld, int j, Crit<R>& cr, double* s_h, double* s_gam,
-                                        int nthreads) {
+                                        int nthreads, int rows) {
   const int lane = threadIdx.x & 31;
   double (&v)[R] = cr.v;
   double* col = S + (size_t)j * ld;
@@ -266,15 +267,28 @@ __device__ __forceinline__ void h7_crit(double* S, int ld, int j, Crit<R>& cr, d
   q = warp_sum(q);
   const double alpha = __shfl_sync(0xffffffffu, x[0], j);
   double h, beta;
-  if (!__any_sync(0xffffffffu, nz != 0)) {   // an empty tail: a sign flip
+  const int qh = __double2hiint(q);
+  const bool usual = qh >= ((1023 - 60) << 20) && qh < ((1023 + 60) << 20);
+  bool empty = !__any_sync(0xffffffffu, nz != 0);
+  if (!NODE && !usual && !empty) {
+    // a product 0 * NaN leaves NaN beyond the rows too; they are not part of the tail
+    nz = 0;
+#pragma unroll
+    for (int t = 0; t < R; ++t) {
+      const int r = lane + 32 * t;
+      if (r >= rows) x[t] = 0.0;
+      else if (r > j) nz |= hi_abs(x[t]) | __double2loint(x[t]);
+    }
+    empty = !__any_sync(0xffffffffu, nz != 0);
+  }
+  if (empty) {   // an empty tail: a sign flip
     h = 1.0;
     cr.seed = 2.0;
     cr.den = 0.5;
     beta = flip_if(alpha, true);
   } else {
-    const int qh = __double2hiint(q);
     const bool neg = __double2hiint(alpha) < 0;
-    if (qh >= ((1023 - 60) << 20) && qh < ((1023 + 60) << 20)) {
+    if (usual) {
       double sigma;
       h7_scalars(alpha, q, &sigma, &cr.seed, &cr.den);
       h = alpha + flip_if(sigma, neg);
@@ -367,7 +381,7 @@ struct NoPublish {
 // seven warps per step.  The publishing warp follows the count of finished
 // columns on its own, so that its fences (about 1 us) hold nobody up.
 template <int R, bool NODE, class Pub = NoPublish>
-__device__ void h7_factor(double* S, int ld, int b, double* s_h, double* s_gam, volatile int* s_done,
+__device__ void h7_factor(double* S, int ld, int rows, int b, double* s_h, double* s_gam, volatile int* s_done,
                           Pub pub = Pub()) {
   const int lane = threadIdx.x & 31, warp = warp_id();
   const int q = bulk_index(warp);
@@ -383,7 +397,7 @@ __device__ void h7_factor(double* S, int ld, int b, double* s_h, double* s_gam, 
     for (int j = 0; j < b; ++j) {
       named_bar(kStepBar, kLeafStepThreads);
       if (warp == 0) {
-        h7_crit<R, NODE>(S, ld, j, cr, s_h, s_gam, kLeafStepThreads);
+        h7_crit<R, NODE>(S, ld, j, cr, s_h, s_gam, kLeafStepThreads, rows);
         __threadfence_block();
         __syncwarp();
         if (lane == 0) *s_done = j + 1;
@@ -902,14 +916,14 @@ __device__ __forceinline__ int h7_slots(int L) {
 }
 
 template <class Pub>
-__device__ void h7_leaf_factor(double* S, int ldS, int slots, int b, double* s_h, double* s_gam, Pub pub) {
+__device__ void h7_leaf_factor(double* S, int ldS, int slots, int L, int b, double* s_h, double* s_gam, Pub pub) {
   __shared__ volatile int s_done;
   switch (slots) {
-    case 1: h7_factor<1, false>(S, ldS, b, s_h, s_gam, &s_done, pub); break;
-    case 2: h7_factor<2, false>(S, ldS, b, s_h, s_gam, &s_done, pub); break;
-    case 3: h7_factor<3, false>(S, ldS, b, s_h, s_gam, &s_done, pub); break;
-    case 4: h7_factor<4, false>(S, ldS, b, s_h, s_gam, &s_done, pub); break;
-    default: h7_factor<kMaxR, false>(S, ldS, b, s_h, s_gam, &s_done, pub); break;
+    case 1: h7_factor<1, false>(S, ldS, L, b, s_h, s_gam, &s_done, pub); break;
+    case 2: h7_factor<2, false>(S, ldS, L, b, s_h, s_gam, &s_done, pub); break;
+    case 3: h7_factor<3, false>(S, ldS, L, b, s_h, s_gam, &s_done, pub); break;
+    case 4: h7_factor<4, false>(S, ldS, L, b, s_h, s_gam, &s_done, pub); break;
+    default: h7_factor<kMaxR, false>(S, ldS, L, b, s_h, s_gam, &s_done, pub); break;
   }
 }
 
@@ -936,7 +950,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2) k_hr4_leaf_tree(Hr4Args a) {
   // ---- leaf: Householder QR of rows [r0, r0 + L); the rows beyond L are zero
   const int slots = h7_slots(L);
   h4_load_block(S, ldS, a.A + r0, a.lda, L, b, 32 * slots);
-  h7_leaf_factor(S, ldS, slots, b, s_h, s_gam, NoPublish());
+  h7_leaf_factor(S, ldS, slots, L, b, s_h, s_gam, NoPublish());
   double* Rl = a.Rn + (size_t)(a.base[0] + leaf) * b * b;
   for (int idx = tid; idx < b * b; idx += blockDim.x) {
     const int r = idx % b, c = idx / b;
@@ -977,7 +991,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2) k_hr4_leaf_tree(Hr4Args a) {
     }
     // reflector j: head row j (child 0), tail = rows 0..j of every other child
     // (the children are upper triangular, so nothing below their diagonals is touched)
-    h7_factor<kFan, true>(S, ldS, b, s_h, s_gam, &s_done);
+    h7_factor<kFan, true>(S, ldS, kFan * 32, b, s_h, s_gam, &s_done);
     for (int idx = tid; idx < b * b; idx += blockDim.x) {
       const int r = idx % b, c = idx / b;
       Rpar[idx] = (r <= c) ? S[c * ldS + r] : 0.0;
@@ -1089,7 +1103,7 @@ __device__ void h6_leaf(const Hr4Args& a, int leaf, double* sm, double* s_h, dou
   const int slots = h7_slots(L);
   if (tid == 0) s_short = 0;   // read after the barriers of the factorization
   h4_load_block(S, ldS, a.A + r0, a.lda, L, b, 32 * slots);
-  h7_leaf_factor(S, ldS, slots, b, s_h, s_gam,
+  h7_leaf_factor(S, ldS, slots, L, b, s_h, s_gam,
                  Publish{a.Rn + (size_t)leaf * b * b, b, a.prog + leaf, &s_short, a.smem_polls, a.fail, a.status});
   if (s_short) return;
   h7_leaf_v(S, ldS, L, 32 * slots, b, s_h, VT, a.Vw + r0, a.m);
@@ -1340,7 +1354,7 @@ __device__ void h6_node(const Hr4Args& a, int f, double* sm, double* s_h, double
           break;
         }
         if (warp == 0) {
-          h7_crit<kFan, true>(S, ld, j, cr, s_h, s_gam, kStepThreads);
+          h7_crit<kFan, true>(S, ld, j, cr, s_h, s_gam, kStepThreads, 0);
           __threadfence_block();
           __syncwarp();
           if (lane == 0) s_done = j + 1;

@@ -116,3 +116,21 @@ def test_widest_panel(cm):
     d = torch.zeros((514, m), dtype=torch.float64, device="cuda").t()
     with pytest.raises(cm.CandmcError):
         cm.hh_recon_qr(d)
+
+
+@pytest.mark.parametrize("b", [1, 2, 20, 31, 32, 40, 70])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_non_finite_last_column(cm, b, bad):
+    """The last reflector of a square panel has an empty tail, whatever its column
+    holds: a non-finite entry there stays in that column of R."""
+    A = fx.gaussian(b, b, b)
+    out = []
+    for v in (A[b // 2, -1], bad):
+        A[b // 2, -1] = v
+        d = torch.from_numpy(A).cuda().t().contiguous().t()
+        W, T = cm.hh_recon_qr(d)
+        torch.cuda.synchronize()
+        out.append((d.cpu().numpy(), W.cpu().numpy(), T.cpu().numpy()))
+    (YR, W, T), (YR2, W2, T2) = out
+    assert np.array_equal(YR[:, :-1], YR2[:, :-1]) and np.array_equal(W, W2) and np.array_equal(T, T2)
+    assert np.isfinite(YR).all() and not np.isfinite(YR2[:, -1]).all()
