@@ -501,10 +501,13 @@ __device__ __forceinline__ int up8(int b) { return (b + 7) & ~7; }
 // inv([[A, B], [0, C]]) = [[A^-1, -A^-1 B C^-1], [0, C^-1]].  Every level is
 // two small products computed in parallel, so the dependent FP64 chain is
 // about 2 (1 + 2 + 4 + 8 + 16) operations instead of the b^2 / 2 of a
-// substitution.  scratch: 512 doubles.
+// substitution.  Only the leading w x w part (w = h4_width(b)) is read and written.
+// scratch: 512 doubles.
+__device__ __forceinline__ int h4_width(int b) { return b <= 8 ? 8 : b <= 16 ? 16 : kDirectB; }
+
 template <int H>
-__device__ __forceinline__ void h4_tri_level(const double* X, double* Xi, double* scratch) {
-  constexpr int n = kDirectB / 2 * H;   // elements of the level's off-diagonal blocks
+__device__ __forceinline__ void h4_tri_level(const double* X, double* Xi, double* scratch, int width) {
+  const int n = width / 2 * H;   // elements of the level's off-diagonal blocks
   constexpr int step = H < 8 ? H : 8;
   const int idx = threadIdx.x;
   const int p = idx / (H * H), e = idx % (H * H), i = e % H, j = e / H, i0 = p * 2 * H, c0 = i0 + H;
@@ -536,17 +539,18 @@ __device__ __forceinline__ void h4_tri_level(const double* X, double* Xi, double
   __syncthreads();
 }
 
-__device__ void h4_tri_inv(const double* X, double* Xi, double* scratch) {
-  for (int idx = threadIdx.x; idx < kDirectB * kDirectB; idx += blockDim.x) {
+__device__ void h4_tri_inv(const double* X, int b, double* Xi, double* scratch) {
+  const int width = h4_width(b);
+  for (int idx = threadIdx.x; idx < width * kDirectB; idx += blockDim.x) {
     const int i = idx & 31, k = idx >> 5;
-    Xi[k * kLd + i] = i == k ? quick_rcp(X[i * kLd + i]) : 0.0;
+    if (i < width) Xi[k * kLd + i] = i == k ? quick_rcp(X[i * kLd + i]) : 0.0;
   }
   __syncthreads();
-  h4_tri_level<1>(X, Xi, scratch);
-  h4_tri_level<2>(X, Xi, scratch);
-  h4_tri_level<4>(X, Xi, scratch);
-  h4_tri_level<8>(X, Xi, scratch);
-  h4_tri_level<16>(X, Xi, scratch);
+  h4_tri_level<1>(X, Xi, scratch, width);
+  h4_tri_level<2>(X, Xi, scratch, width);
+  h4_tri_level<4>(X, Xi, scratch, width);
+  if (width > 8) h4_tri_level<8>(X, Xi, scratch, width);
+  if (width > 16) h4_tri_level<16>(X, Xi, scratch, width);
 }
 
 // b x b block from global memory (ld b) into a shared block (ld kLd), zero beyond b
@@ -559,10 +563,10 @@ __device__ void h4_load(double* dst, const double* src, int b) {
 }
 
 // Rows [0, L) of b columns of a column-major block (ld lda) into S (ld ldS),
-// zero up to row `rows` (a multiple of 32) and column 32: eight loads in
+// zero up to row `rows` (a multiple of 32) and column h4_width(b): eight loads in
 // flight per thread before any store.
 __device__ void h4_load_block(double* S, int ldS, const double* A, int64_t lda, int L, int b, int rows) {
-  const int n = rows * kDirectB;
+  const int n = rows * h4_width(b);
   for (int e0 = threadIdx.x; e0 < n; e0 += 8 * kLeafThreads) {
     double t[8];
 #pragma unroll
@@ -580,31 +584,36 @@ __device__ void h4_load_block(double* S, int ldS, const double* A, int64_t lda, 
 
 constexpr int kGramScratch = 4 * 640;   // h7_gram's partial sums (doubles)
 
-// T^-1 = striu(V^T V) + diag(V^T V) / 2 of normalised reflectors into G (32 x
-// 32, ld kLd; columns beyond b get a unit diagonal).  V: rows 0..31 in VT (ld
-// kLd, masked to the reflectors' structure), rows 32..rows-1 in S (ld ldS).
-// Eight warps split the rows; each holds the ten upper 8 x 8 tiles (lane l:
-// row l % 8 of a tile, columns l / 8 and l / 8 + 4), so a row costs 20 FP64
+// T^-1 = striu(V^T V) + diag(V^T V) / 2 of normalised reflectors into G (w x w,
+// w = h4_width(b), ld kLd; columns beyond b get a unit diagonal).  V: rows 0..31 in
+// VT (ld kLd, masked to the reflectors' structure), rows 32..rows-1 in S (ld ldS).
+// Eight warps split the rows; each holds the upper 8 x 8 tiles (lane l: row l % 8
+// of a tile, columns l / 8 and l / 8 + 4), so a row of 32 columns costs 20 FP64
 // instructions and no shuffles; the eight partial sums meet in shared memory.
-__device__ void h7_gram(const double* VT, const double* S, int ldS, int rows, int b, double* G, double* part) {
+// NT = w / 8: with all ten tiles at every width, a 2000000 x 1 panel spent 3.3 ms in
+// its leaves, most of it on columns that are not there.
+template <int NT>
+__device__ __forceinline__ void h7_gram_tiles(const double* VT, const double* S, int ldS, int rows, int b, double* G,
+                                              double* part) {
+  constexpr int TILES = NT * (NT + 1) / 2, PART = 64 * TILES;
   const int lane = threadIdx.x & 31, warp = warp_id();
   const int i = lane & 7, jj = lane >> 3;
-  double acc[10][2];
+  double acc[TILES][2];
 #pragma unroll
-  for (int t = 0; t < 10; ++t) acc[t][0] = acc[t][1] = 0.0;
+  for (int t = 0; t < TILES; ++t) acc[t][0] = acc[t][1] = 0.0;
   if (warp < 8) {
     for (int r = warp; r < rows; r += 8) {
       const double* X = r < kDirectB ? VT : S;
       const int ld = r < kDirectB ? kLd : ldS;
-      double x[4], y0[4], y1[4];
+      double x[NT], y0[NT], y1[NT];
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
+      for (int t = 0; t < NT; ++t) {
         x[t] = X[(8 * t + i) * ld + r];
         y0[t] = X[(8 * t + jj) * ld + r];
         y1[t] = X[(8 * t + jj + 4) * ld + r];
       }
 #pragma unroll
-      for (int tj = 0; tj < 4; ++tj)
+      for (int tj = 0; tj < NT; ++tj)
 #pragma unroll
         for (int ti = 0; ti <= tj; ++ti) {
           const int t = tj * (tj + 1) / 2 + ti;
@@ -614,30 +623,36 @@ __device__ void h7_gram(const double* VT, const double* S, int ldS, int rows, in
     }
     if (warp >= 4) {
 #pragma unroll
-      for (int t = 0; t < 10; ++t) {
-        part[(warp - 4) * 640 + t * 64 + lane] = acc[t][0];
-        part[(warp - 4) * 640 + t * 64 + 32 + lane] = acc[t][1];
+      for (int t = 0; t < TILES; ++t) {
+        part[(warp - 4) * PART + t * 64 + lane] = acc[t][0];
+        part[(warp - 4) * PART + t * 64 + 32 + lane] = acc[t][1];
       }
     }
   }
   __syncthreads();
   if (warp < 4) {
 #pragma unroll
-    for (int t = 0; t < 10; ++t) {
-      part[warp * 640 + t * 64 + lane] += acc[t][0];
-      part[warp * 640 + t * 64 + 32 + lane] += acc[t][1];
+    for (int t = 0; t < TILES; ++t) {
+      part[warp * PART + t * 64 + lane] += acc[t][0];
+      part[warp * PART + t * 64 + 32 + lane] += acc[t][1];
     }
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < 640; e += blockDim.x) {
+  for (int e = threadIdx.x; e < PART; e += blockDim.x) {
     const int t = e >> 6, u = (e >> 5) & 1, l = e & 31;
     int tj = 0;
     while ((tj + 1) * (tj + 2) / 2 <= t) ++tj;
     const int r = 8 * (t - tj * (tj + 1) / 2) + (l & 7), c = 8 * tj + (l >> 3) + 4 * u;
-    const double g = (part[e] + part[640 + e]) + (part[1280 + e] + part[1920 + e]);
+    const double g = (part[e] + part[PART + e]) + (part[2 * PART + e] + part[3 * PART + e]);
     if (r <= c) G[c * kLd + r] = r == c ? (c < b ? 0.5 * g : 1.0) : g;
   }
   __syncthreads();
+}
+
+__device__ void h7_gram(const double* VT, const double* S, int ldS, int rows, int b, double* G, double* part) {
+  if (b <= 8) h7_gram_tiles<1>(VT, S, ldS, rows, b, G, part);
+  else if (b <= 16) h7_gram_tiles<2>(VT, S, ldS, rows, b, G, part);
+  else h7_gram_tiles<4>(VT, S, ldS, rows, b, G, part);
 }
 
 struct Hr4Args {
@@ -896,7 +911,7 @@ __device__ void h7_leaf_v(double* S, int ldS, int L, int rows, int b, double* s_
   const int tid = threadIdx.x;
   if (tid < kDirectB) s_h[tid] = tid < b ? quick_rcp(s_h[tid]) : 0.0;
   __syncthreads();
-  const int n = rows * kDirectB;
+  const int n = rows * h4_width(b);
   for (int e = tid; e < n; e += kLeafThreads) {
     const int c = e / rows, r = e - c * rows;
     double v = 0.0;
@@ -958,7 +973,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2) k_hr4_leaf_tree(Hr4Args a) {
   }
   h7_leaf_v(S, ldS, L, 32 * slots, b, s_h, VT, a.Vw + r0, a.m);
   h7_gram(VT, S, ldS, 32 * slots, b, G, scratch);
-  h4_tri_inv(G, Tt, scratch);
+  h4_tri_inv(G, b, Tt, scratch);
   double* Tleaf = a.Tl + (size_t)leaf * b * b;
   for (int idx = tid; idx < b * b; idx += blockDim.x) Tleaf[idx] = (idx % b <= idx / b) ? Tt[(idx / b) * kLd + idx % b] : 0.0;
 
@@ -984,7 +999,7 @@ __global__ void __launch_bounds__(kLeafThreads, 2) k_hr4_leaf_tree(Hr4Args a) {
     __threadfence();
     // stack the children's R factors: child k occupies rows [32 k, 32 k + b)
     // (rows b..31 of every child, and the children beyond nch, stay zero)
-    for (int idx = tid; idx < kDirectB * kFan * 32; idx += blockDim.x) {
+    for (int idx = tid; idx < h4_width(b) * kFan * 32; idx += blockDim.x) {
       const int c = idx / (kFan * 32), r = idx % (kFan * 32), k = r >> 5, i = r & 31;
       const double* Rk = a.Rn + (size_t)(a.base[lvl] + parent * kFan + k) * b * b;
       S[c * ldS + r] = (k < nch && c < b && i <= c) ? __ldcg(Rk + c * b + i) : 0.0;
@@ -999,14 +1014,14 @@ __global__ void __launch_bounds__(kLeafThreads, 2) k_hr4_leaf_tree(Hr4Args a) {
     // V = [I; V_1; ..; V_{nch-1}] (V_k upper triangular), normalised
     if (tid < kDirectB) s_h[tid] = tid < b ? quick_rcp(s_h[tid]) : 0.0;
     __syncthreads();
-    for (int idx = tid; idx < kDirectB * kFan * 32; idx += blockDim.x) {
+    for (int idx = tid; idx < h4_width(b) * kFan * 32; idx += blockDim.x) {
       const int c = idx / (kFan * 32), r = idx % (kFan * 32);
       if (r >= 32) S[c * ldS + r] *= s_h[c];
       else VT[c * kLd + r] = (r == c && c < b) ? 1.0 : 0.0;
     }
     __syncthreads();
     h7_gram(VT, S, ldS, kFan * 32, b, G, scratch);
-    h4_tri_inv(G, Tt, scratch);
+    h4_tri_inv(G, b, Tt, scratch);
     double* Qp = a.Qn + (size_t)(a.base[lvl + 1] + parent) * kFan * b * b;
     // Q_1 = I - T;  Q_k = -V_k T
     for (int idx = tid; idx < b * b; idx += blockDim.x) {
@@ -1108,7 +1123,7 @@ __device__ void h6_leaf(const Hr4Args& a, int leaf, double* sm, double* s_h, dou
   if (s_short) return;
   h7_leaf_v(S, ldS, L, 32 * slots, b, s_h, VT, a.Vw + r0, a.m);
   h7_gram(VT, S, ldS, 32 * slots, b, G, scratch);
-  h4_tri_inv(G, Tt, scratch);
+  h4_tri_inv(G, b, Tt, scratch);
   double* Tleaf = a.Tl + (size_t)leaf * b * b;
   for (int idx = tid; idx < b * b; idx += blockDim.x) Tleaf[idx] = (idx % b <= idx / b) ? Tt[(idx / b) * kLd + idx % b] : 0.0;
   if (leaf == 0 && a.Pc) {
