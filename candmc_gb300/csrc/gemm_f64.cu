@@ -540,11 +540,27 @@ k_reduce_apply(const double* Zp, int nsplit, int64_t split_stride, int nb, int n
 // diagonal first, a chain of 32 shuffles and fmas.  Bound by those chains: 25 us
 // at n = 128, where a thread per column took 480 us (600 us for the diagonal
 // blocks of a least-squares R).
-// Element (i, c) of the inverse depends on rows and columns i..c only.  A block with a
-// zero on the diagonal, a non-finite entry or one so large or small that a quotient by
-// the diagonal could leave the normal range (`rough`) is worked entry by entry: the
-// terms of column c alone, each divided where it is used.
+// Element (i, c) of the inverse depends on rows and columns i..c only, but the blocks
+// multiply by whole columns and by reciprocals: a column that comes out non-finite, or
+// that used a pivot outside 2^+-200 (where a quotient could leave the normal range), is
+// worked again by itself (tri_column).
 constexpr int kTriWarps = 4;
+
+// Column c of the inverse of the upper triangle X(i, k) = X[i xi + k xk] into x[i xs],
+// i <= c: plain back substitution by one warp, every entry divided where it is used.
+__device__ __noinline__ void tri_column(const double* X, int64_t xi, int64_t xk, int unit, int c, double* x, int64_t xs) {
+  const int lane = threadIdx.x & 31;
+  for (int i = lane; i <= c; i += 32) x[i * xs] = i == c ? 1.0 : 0.0;
+  for (int k = c; k >= 0; --k) {
+    __syncwarp();
+    double v = x[k * xs];
+    if (!unit) v /= X[k * (xi + xk)];
+    __syncwarp();
+    if (lane == 0) x[k * xs] = v;
+    for (int i = lane; i < k; i += 32) x[i * xs] = fma(-X[i * xi + k * xk], v, x[i * xs]);
+  }
+}
+
 __global__ void __launch_bounds__(32 * kTriWarps)
 k_tri_inv(const double* X, int64_t ldx, int n, int64_t ntot, int64_t xstep, int lower, int unit, double* Xi,
           int64_t ldi, int64_t istep) {
@@ -570,37 +586,27 @@ k_tri_inv(const double* X, int64_t ldx, int n, int64_t ntot, int64_t xstep, int 
 #pragma unroll
     for (int u = 0; u < per; ++u) nxt[u] = at(ib, kb, tid + 32 * kTriWarps * u);
   };
-  // the fetched block into shared memory (diag: a diagonal one); true when it is rough
-  auto stage = [&](bool diag) -> bool {
-    bool rough = false;
+  auto stage = [&]() {
 #pragma unroll
     for (int u = 0; u < per; ++u) {
       const int e = tid + 32 * kTriWarps * u;
       sU[lower ? (e & 31) * ld + (e >> 5) : (e >> 5) * ld + (e & 31)] = nxt[u];
-      const unsigned h = (unsigned)__double2hiint(nxt[u]) & 0x7fffffffu;
-      const bool zero = (h | (unsigned)__double2loint(nxt[u])) == 0;
-      rough |= zero ? diag && (e >> 5) == (e & 31) : h - ((1023u - 500u) << 20) >= (1000u << 20);   // outside 2^+-500
     }
-    return __syncthreads_or(rough) != 0;
   };
   if (c < n)
     for (int i = 32 * (J + 1) + lane; i < n; i += 32) Xi[i * ri + c * ci] = 0.0;
+  bool again = false;   // this lane's entries, or pivots of the blocks passed
   fetch(J, J);
   for (int ib = J; ib >= 0; --ib) {
     const int i = 32 * ib + lane;
     double r0 = (i == c && c < nq) ? 1.0 : 0.0, r1 = 0.0;
     for (int kb = J; kb > ib; --kb) {
       __syncthreads();
-      const bool rough = stage(false);
+      stage();
       if (kb - 1 >= ib) fetch(ib, kb - 1);
+      __syncthreads();
       const int kk = 32 * kb + lane;
       const double x = (c < n && kk < n) ? Xi[kk * ri + c * ci] : 0.0;
-      if (rough) {
-#pragma unroll 1
-        for (int k = 0; k < 32 && 32 * kb + k <= c; ++k)
-          r0 = fma(-sU[k * ld + lane], __shfl_sync(0xffffffffu, x, k), r0);
-        continue;
-      }
 #pragma unroll 8
       for (int k = 0; k < 32; k += 2) {
         r0 = fma(-sU[k * ld + lane], __shfl_sync(0xffffffffu, x, k), r0);
@@ -608,20 +614,9 @@ k_tri_inv(const double* X, int64_t ldx, int n, int64_t ntot, int64_t xstep, int 
       }
     }
     __syncthreads();
-    const bool rough = stage(true);
+    stage();
     if (ib > 0) fetch(ib - 1, J);
-    if (rough) {
-      double r = r0 + r1;
-#pragma unroll 1
-      for (int k = min(31, c - 32 * ib); k >= 0; --k) {
-        if (lane == k) r /= sU[k * ld + k];
-        const double xk = __shfl_sync(0xffffffffu, r, k);
-        if (lane < k) r = fma(-sU[k * ld + lane], xk, r);
-      }
-      if (c < n && i < n) Xi[i * ri + c * ci] = r;
-      __syncwarp();
-      continue;
-    }
+    __syncthreads();
     if (tid < 32) s_rd[tid] = 1.0 / sU[tid * ld + tid];
     __syncthreads();
     // columns k divided by U[k][k]: r_i -= (U[i][k] / U[k][k]) r_k, then x = r / diag
@@ -637,9 +632,15 @@ k_tri_inv(const double* X, int64_t ldx, int n, int64_t ntot, int64_t xstep, int 
       const double rk = __shfl_sync(0xffffffffu, r, k);
       if (lane < k) r = fma(-sU[k * ld + lane], rk, r);
     }
-    if (c < n && i < n) Xi[i * ri + c * ci] = r * s_rd[lane];
+    const double rd = s_rd[lane], x = r * rd;
+    again |= ((unsigned)__double2hiint(x) & 0x7fffffffu) >= 0x7ff00000u ||
+             ((unsigned)__double2hiint(rd) & 0x7fffffffu) - ((1023u - 200u) << 20) > (400u << 20);
+    if (c < n && i < n) Xi[i * ri + c * ci] = x;
     __syncwarp();
   }
+  if (!__any_sync(0xffffffffu, again) || c >= nq) return;
+  for (int i = c + 1 + lane; i < 32 * (J + 1) && i < n; i += 32) Xi[i * ri + c * ci] = 0.0;
+  tri_column(X, lower ? ldx : 1, lower ? 1 : ldx, unit, c, Xi + c * ci, ri);
 }
 
 // Copy op(X) (masked) into a dense n x k buffer (ld ldo).
