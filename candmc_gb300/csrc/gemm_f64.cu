@@ -26,12 +26,13 @@ namespace candmc {
 // mode 0: store into out + split * split_stride (partials), ld ldo.
 // mode 1: out(i, j) -= result (out is the trailing matrix itself).
 constexpr int TK = 16;
+static_assert(kThreads == 16 * TK, "one tile element a thread");
 constexpr int64_t kSmallProduct = 20000000;
 
 __global__ void __launch_bounds__(kThreads)
 k_gemm_f64(MatRef A, MatRef B, int64_t M, int64_t N, int64_t K, int64_t kchunk, double* out,
            int64_t ldo, int64_t split_stride, int mode) {
-  constexpr int U = 1, TM = 16, TN = 16;
+  constexpr int TM = 16, TN = 16;
   __shared__ double sA[TK][TM + 1];
   __shared__ double sB[TK][TN + 1];
   const int tid = threadIdx.x;
@@ -39,54 +40,31 @@ k_gemm_f64(MatRef A, MatRef B, int64_t M, int64_t N, int64_t K, int64_t kchunk, 
   const int64_t i0 = (int64_t)blockIdx.x * TM, j0 = (int64_t)blockIdx.y * TN;
   const int64_t k0 = (int64_t)blockIdx.z * kchunk;
   const int64_t k1 = (k0 + kchunk < K) ? k0 + kchunk : K;
-  double acc[U][U];
-#pragma unroll
-  for (int u = 0; u < U; ++u)
-#pragma unroll
-    for (int v = 0; v < U; ++v) acc[u][v] = 0.0;
-
+  double acc = 0.0;
   for (int64_t kb = k0; kb < k1; kb += TK) {
-    // A tile: TM x TK.  Coalesce along the stored row index.
-    for (int idx = tid; idx < TM * TK; idx += kThreads) {
+    // one element of each tile a thread, coalesced along the stored row index
+    {
       int ii, kk;
-      if (A.trans) { kk = idx % TK; ii = idx / TK; } else { ii = idx % TM; kk = idx / TM; }
-      int64_t gi = i0 + ii, gk = kb + kk;
+      if (A.trans) { kk = tid % TK; ii = tid / TK; } else { ii = tid % TM; kk = tid / TM; }
+      const int64_t gi = i0 + ii, gk = kb + kk;
       sA[kk][ii] = (gi < M && gk < k1) ? mat_at(A, gi, gk) : 0.0;
     }
-    for (int idx = tid; idx < TK * TN; idx += kThreads) {
+    {
       int jj, kk;
-      if (B.trans) { jj = idx % TN; kk = idx / TN; } else { kk = idx % TK; jj = idx / TK; }
-      int64_t gj = j0 + jj, gk = kb + kk;
+      if (B.trans) { jj = tid % TN; kk = tid / TN; } else { kk = tid % TK; jj = tid / TK; }
+      const int64_t gj = j0 + jj, gk = kb + kk;
       sB[kk][jj] = (gj < N && gk < k1) ? mat_at(B, gk, gj) : 0.0;
     }
     __syncthreads();
 #pragma unroll
-    for (int kk = 0; kk < TK; ++kk) {
-      double a[U], bb[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) a[u] = sA[kk][ti + 16 * u];
-#pragma unroll
-      for (int v = 0; v < U; ++v) bb[v] = sB[kk][tj + 16 * v];
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-#pragma unroll
-        for (int v = 0; v < U; ++v) acc[u][v] = fma(a[u], bb[v], acc[u][v]);
-    }
+    for (int kk = 0; kk < TK; ++kk) acc = fma(sA[kk][ti], sB[kk][tj], acc);
     __syncthreads();
   }
-  double* o = out + (mode == 0 ? (int64_t)blockIdx.z * split_stride : 0);
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    int64_t gi = i0 + ti + 16 * u;
-    if (gi >= M) continue;
-#pragma unroll
-    for (int v = 0; v < U; ++v) {
-      int64_t gj = j0 + tj + 16 * v;
-      if (gj >= N) continue;
-      if (mode == 0) o[gj * ldo + gi] = acc[u][v];
-      else o[gj * ldo + gi] -= acc[u][v];
-    }
-  }
+  const int64_t gi = i0 + ti, gj = j0 + tj;
+  if (gi >= M || gj >= N) return;
+  double* o = out + (mode == 0 ? (int64_t)blockIdx.z * split_stride : 0) + gj * ldo + gi;
+  if (mode == 0) *o = acc;
+  else *o -= acc;
 }
 
 // An operand as element (i, j) = p[i si + j sj] with its mask as what to keep by

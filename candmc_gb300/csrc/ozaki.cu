@@ -63,11 +63,6 @@ struct OzCfg {
 constexpr int OZ_WAIT_LIMIT = 1 << 22;                // bounded mbarrier polls
 int g_oz_polls = OZ_WAIT_LIMIT;                       // those of the roles on one another (knob "oz_polls")
 
-// element (r, k) of an R x K operand slice plane in core-matrix K-major order
-__host__ __device__ __forceinline__ int64_t cm_off(int64_t r, int64_t k, int64_t R) {
-  return (k >> 4) * (R * 16) + (r >> 3) * 128 + ((k & 15) >> 3) * 64 + (r & 7) * 8 + (k & 7);
-}
-
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -87,12 +82,6 @@ __device__ __forceinline__ f2 two_sum(float a, float b) {
 __device__ __forceinline__ f2 fast_two_sum(float a, float b) {
   float s = a + b;
   return {s, b - (s - a)};
-}
-
-// (h, l) + g
-__device__ __forceinline__ f2 df_add_f(f2 x, float g) {
-  f2 s = two_sum(x.h, g);
-  return fast_two_sum(s.h, s.l + x.l);
 }
 
 // x + y

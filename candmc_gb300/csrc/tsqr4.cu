@@ -161,7 +161,6 @@ __device__ __forceinline__ void bar_arrive(int id, int n) {
 }
 
 __device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
-__device__ __forceinline__ bool bits_nonzero(double x) { return (hi_abs(x) | __double2loint(x)) != 0; }
 // x with its sign flipped when `neg` is set
 __device__ __forceinline__ double flip_if(double x, bool neg) {
   return __hiloint2double(__double2hiint(x) ^ (neg ? 0x80000000 : 0), __double2loint(x));
@@ -788,8 +787,8 @@ __device__ void h4_root(const Hr4Args& a, double* sm) {
     }
     __threadfence_block();
   };
-  // acc minus the sum over k < c, k = h (mod 4), of X[:, k] v[k]: X's columns
-  // from c on are still zero, so the last step may reach beyond c
+  // acc minus the sum over k < c, k = h (mod 4), of X[:, k] v[k], four terms at a
+  // time (those from c on read as zero)
   const int h = warp - 1;   // of the four warps 1..4
   auto minus_sum = [&](double acc, const double* X, const double* v, int ldv, int c) -> double {
 #pragma unroll 1
