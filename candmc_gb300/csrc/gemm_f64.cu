@@ -515,7 +515,7 @@ k_reduce_apply(const double* Zp, int nsplit, int64_t split_stride, int nb, int n
 // with one row per lane: the CTA stages 32 x 32 blocks of the triangle (the
 // next one loads while this one is used), a block above the diagonal costs 32
 // FP64 instructions a column and a diagonal block, its columns divided by the
-// diagonal first, a chain of 32 shuffles and fmas.  Bound by those chains: 25 us
+// diagonal first, a chain of 32 shuffles and fmas.  Bound by those chains: 28 us
 // at n = 128, where a thread per column took 480 us (600 us for the diagonal
 // blocks of a least-squares R).
 // Element (i, c) of the inverse depends on rows and columns i..c only, but the blocks
