@@ -495,9 +495,10 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, unsigned
       : "memory");
 }
 
-// Bounded wait of a whole warp; gives up early when another role of the CTA failed.
-// Warp collectives (votes, elections, TMEM loads) follow on either outcome, so the
-// lanes vote on it: all of them leave by the same poll with the same result.
+// Bounded wait of a whole warp.  Warp collectives (votes, elections, TMEM loads) follow
+// on either outcome, so the lanes vote on it: all of them leave by the same poll with
+// the same result.  A role whose partner has given up runs out by itself: a look at
+// the flag in the loop is code at every wait, and these kernels are bound by it.
 __device__ __forceinline__ bool oz_wait(uint64_t* b, uint32_t parity, volatile int* fail, int polls) {
   const uint32_t addr = smem_u32(b);
 #pragma unroll 1
@@ -510,7 +511,6 @@ __device__ __forceinline__ bool oz_wait(uint64_t* b, uint32_t parity, volatile i
         : "r"(addr), "r"(parity)
         : "memory");
     if (__all_sync(0xffffffffu, done)) return true;
-    if ((it & 63) == 63 && __any_sync(0xffffffffu, *fail)) return false;
   }
   *fail = 1;
   __syncwarp();
